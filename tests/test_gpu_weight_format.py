@@ -51,3 +51,17 @@ def test_disk_format_round_trip(pkg, gpu, oracle, tmp_path):
         pkg.disk_format.load_linear(prefix, N + 1, K)       # short files
     with pytest.raises(FileNotFoundError):
         pkg.disk_format.load_linear(prefix + "missing/", N, K)
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+@pytest.mark.parametrize("N,K", [(1, 64), (3, 320), (131, 192)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_gpu_weight_quantizer_list_ends_and_alignment(pkg, gpu, oracle, fmt, N, K, shift):
+    """Pair counts around the kernel's unit of work, and a source that is only 4-byte aligned."""
+    import torch
+    w = np.random.default_rng(N + K).standard_normal(N * K + 1).astype(np.float32)
+    wd = torch.from_numpy(w).cuda()[shift:shift + N * K].view(N, K)
+    nib, d, m, zp = (t.cpu().numpy() for t in gpu.quantize_weights(fmt, wd))
+    for got, want in zip((nib, d, m), oracle.quantize_weight(fmt, w[shift:shift + N * K].reshape(N, K))):
+        assert np.array_equal(got, want)
+    assert (zp == (8 if fmt == 0 else 0)).all()
