@@ -30,12 +30,6 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void *smem_row)
-{
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(smem_u32(smem_row)));
-}
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void *smem_row)
 {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -120,7 +114,7 @@ __global__ void __launch_bounds__(128) k_attention_prefill_mma(const float *__re
             for (int np = 0; np < 4; np++) {
                 // four 8x8 matrices: keys 16 np .. + 7 and + 8 .. + 15, dims 16 kk .. + 7 and + 8 .. + 15
                 uint32_t b[4];
-                ldmatrix_x4(b, &ks[np * 16 + (lane & 7) + ((lane >> 4) << 3)][kk * 16 + (((lane >> 3) & 1) << 3)]);
+                ldmatrix_x4(b, smem_u32(&ks[np * 16 + (lane & 7) + ((lane >> 4) << 3)][kk * 16 + (((lane >> 3) & 1) << 3)]));
                 mma_f16(s[2 * np], qh[kk], b[0], b[1]);
                 mma_f16(s[2 * np], ql[kk], b[0], b[1]);
                 mma_f16(s[2 * np + 1], qh[kk], b[2], b[3]);

@@ -36,6 +36,24 @@ int after_launch(inkq_ctx *ctx, const char *what)
     return INKQ_OK;
 }
 
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+int encode_map_2d(inkq_ctx *ctx, CUtensorMap *map, CUtensorMapDataType dt, int elem_bytes, const void *base, uint64_t dim0, uint64_t dim1, uint32_t box0,
+                  uint32_t box1, CUtensorMapSwizzle swz, uint64_t pitch_elems)
+{
+    const cuuint64_t gdim[2] = {dim0, dim1};
+    const cuuint64_t gstride[1] = {pitch_elems * static_cast<uint64_t>(elem_bytes)};
+    const cuuint32_t box[2] = {box0, box1};
+    const cuuint32_t estr[2] = {1u, 1u};
+    const CUresult cr = reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled)(map, dt, 2, const_cast<void *>(base), gdim, gstride, box, estr,
+                                                                           CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                                                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) return fail(ctx, INKQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(cr)));
+    return INKQ_OK;
+}
+
 static int use(inkq_ctx *ctx)
 {
     if (ctx == nullptr) return fail(nullptr, INKQ_ERR_INVALID, "null context");

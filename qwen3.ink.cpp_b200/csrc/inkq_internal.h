@@ -1,6 +1,7 @@
 // Internal definitions shared by the .cu files: handle structs, device layouts,
 // error plumbing.  Nothing here is part of the public ABI (see include/inkq.h).
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -163,6 +164,10 @@ static inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 b
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Tiled 2-D tensor map (rows of dim0 elements, pitch_elems apart), 128-byte L2 promotion, zero fill outside
+int encode_map_2d(inkq_ctx *ctx, CUtensorMap *map, CUtensorMapDataType dt, int elem_bytes, const void *base, uint64_t dim0, uint64_t dim1, uint32_t box0,
+                  uint32_t box1, CUtensorMapSwizzle swz, uint64_t pitch_elems);
+
 // Checks the launch, counts it.
 int after_launch(inkq_ctx *ctx, const char *what);
 
@@ -188,6 +193,9 @@ int launch_block_dots(inkq_ctx *ctx, const Act *a, const Weight *w, int32_t *dot
 // multiple of 4; C and the extra destinations still point at row 0)
 int launch_gemm_tc(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc, int32_t *dots, const ExtraDst *extra = nullptr,
                    int tn_begin = 0, int tn_count = -1, int m_begin = 0, int m_count = -1);
+// launch_gemm_tc's share with few activation rows (qgemm_rows.cu): m_count <= GEMM_ROWS_MAX
+constexpr int GEMM_ROWS_MAX = 32;
+int launch_gemm_rows(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc, const ExtraDst *extra, int m_begin, int m_count);
 int launch_gemm_w41_f16(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc);   // CUDA cores
 int launch_gemm_w41_tc(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc);    // tcgen05 kind::f16
 int launch_gemv_w41(inkq_ctx *ctx, const uint16_t *a16, const Weight *w, float *C);                        // M == 1, bandwidth-bound

@@ -18,6 +18,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p)
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One lane of a converged warp.  Unlike a comparison of the lane number, the compiler knows that exactly one lane is
+// active behind it, so uniform operands (descriptors, addresses) need no loop over lanes.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
 {
@@ -215,6 +224,68 @@ template <int N>
 __device__ __forceinline__ void setmaxnreg_dec()
 {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+
+// ---- warp-level matrix operands, shared loads by address -------------------------------------
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t saddr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr) : "memory");
+}
+__device__ __forceinline__ uint32_t lds_u16(uint32_t saddr)
+{
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(saddr) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint2 lds_u32x2(uint32_t saddr)
+{
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(saddr) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 lds_f4(uint32_t saddr)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(saddr) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned long long lds_u64(uint32_t saddr)
+{
+    unsigned long long v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(saddr) : "memory");
+    return v;
+}
+
+// ---- packed fp32 pairs -------------------------------------------------------------------------
+// Two fp32 values in one 64-bit register and the IEEE (round-to-nearest) packed multiply / fused multiply-add of
+// sm_100a: each half rounds exactly like the scalar instruction, so results stay bit-identical while the issue slots
+// are halved.
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// Two int32 -> packed fp32 pair, exact below 2^24 in magnitude
+__device__ __forceinline__ unsigned long long cvt2_exact(uint32_t v0, uint32_t v1)
+{
+    return pack2(static_cast<float>(static_cast<int32_t>(v0)), static_cast<float>(static_cast<int32_t>(v1)));
 }
 
 // ---- misc -----------------------------------------------------------------------------

@@ -157,37 +157,6 @@ __device__ __forceinline__ void mbar_arrive_elect(uint64_t *bar)
         : "memory");
 }
 
-// Two fp32 values in one 64-bit register and the IEEE (round-to-nearest) packed
-// multiply / fused multiply-add of sm_100: each half rounds exactly like the scalar
-// instruction, so results stay bit-identical while the issue slots are halved.
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b)
-{
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c)
-{
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-// Two block dots -> packed fp32 pair, exactly (a block dot is at most 32 * 128 * 15 = 61440 in magnitude).
-__device__ __forceinline__ unsigned long long cvt2_exact(uint32_t v0, uint32_t v1)
-{
-    return pack2(static_cast<float>(static_cast<int32_t>(v0)), static_cast<float>(static_cast<int32_t>(v1)));
-}
-
 // Loads N consecutive TMEM columns of this thread's lane; N a multiple of 4 up to 16.
 template <int N>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t *r)
@@ -562,10 +531,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 // The opt-in for large dynamic shared memory is a per-device function attribute: remember per device
 // (and per instantiation, through the template's own statics) whether it has been set.
 constexpr int MAX_DEVICES = 64;
@@ -611,20 +576,6 @@ static int launch_cw(inkq_ctx *ctx, int cw, const CUtensorMap *maps, const TcPar
     return fail(ctx, INKQ_ERR_INVALID, "internal: bad column width");
 }
 
-static int encode2d(inkq_ctx *ctx, CUtensorMap *map, CUtensorMapDataType dt, int elem_bytes, const void *base, uint64_t dim0, uint64_t dim1,
-                    uint32_t box0, uint32_t box1, CUtensorMapSwizzle swz, uint64_t pitch_elems = 0)
-{
-    const cuuint64_t gdim[2] = {dim0, dim1};
-    const cuuint64_t gstride[1] = {(pitch_elems ? pitch_elems : dim0) * static_cast<uint64_t>(elem_bytes)};
-    const cuuint32_t box[2] = {box0, box1};
-    const cuuint32_t estr[2] = {1u, 1u};
-    CUresult cr = reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled)(map, dt, 2, const_cast<void *>(base), gdim, gstride, box, estr,
-                                                                     CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                                                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) return fail(ctx, INKQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(cr)));
-    return INKQ_OK;
-}
-
 // Relative cost of one tile by its width block_m = 16 * index (any common factor cancels; measured on a B200 with
 // one tile per SM at K = 4096: 32.2, 35.4, 39.3, 45.7, 51.7, 58.4, 66.0, 76.6 us): narrow tiles are bounded by the chain of
 // K=32 MMAs and their commits, wide ones by the epilogue arithmetic.  The ratios hardly depend on K (both terms are per block).
@@ -639,6 +590,9 @@ int launch_gemm_tc(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int l
         return fail(ctx, INKQ_ERR_INVALID, "bad activation row window");
     if (ctx->encode_tiled == nullptr) return fail(ctx, INKQ_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled entry point not available");
     if (w->sc32 == nullptr) return fail(ctx, INKQ_ERR_INVALID, "this weight holds no fp32 scale records (weight-only layers use inkq_gemm_w41_f16act)");
+    // few rows: the kernel without tensor memory (qgemm_rows.cu)
+    if (m_count <= GEMM_ROWS_MAX && dots == nullptr && tn_begin == 0 && tn_count == w->tiles)
+        return launch_gemm_rows(ctx, a, w, C, ldc, extra, m_begin, m_count);
     const int M = m_count;
     // Split of the M activation rows into tiles of block_m columns (a multiple of 16, at most 128).  With few
     // weight tiles (a shard of a column-sharded layer) narrower tiles fill more SMs; the choice minimises
@@ -663,11 +617,11 @@ int launch_gemm_tc(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int l
 
     CUtensorMap maps[3];
     // a row window starts m_begin rows into q and m_begin entries into every block's line of the planes
-    int rc = encode2d(ctx, &maps[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->q + static_cast<size_t>(m_begin) * a->K, a->K, M, 128u, block_m,
-                      CU_TENSOR_MAP_SWIZZLE_128B);
-    if (!rc) rc = encode2d(ctx, &maps[1], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->d + m_begin, a->M_ld - m_begin, nb, block_m, STAGE_BLOCKS,
+    int rc = encode_map_2d(ctx, &maps[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->q + static_cast<size_t>(m_begin) * a->K, a->K, M, 128u, block_m,
+                           CU_TENSOR_MAP_SWIZZLE_128B, a->K);
+    if (!rc) rc = encode_map_2d(ctx, &maps[1], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->d + m_begin, a->M_ld - m_begin, nb, block_m, STAGE_BLOCKS,
                            CU_TENSOR_MAP_SWIZZLE_NONE, a->M_ld);
-    if (!rc) rc = encode2d(ctx, &maps[2], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->s + m_begin, a->M_ld - m_begin, nb, block_m, STAGE_BLOCKS,
+    if (!rc) rc = encode_map_2d(ctx, &maps[2], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->s + m_begin, a->M_ld - m_begin, nb, block_m, STAGE_BLOCKS,
                            CU_TENSOR_MAP_SWIZZLE_NONE, a->M_ld);
     if (rc) return rc;
 

@@ -104,6 +104,27 @@ def test_gemm_bit_identical_to_oracle(pkg, gpu, oracle, impl, scheme, scale_mode
     assert np.array_equal(got[:M, :N].view(np.uint32), ref.view(np.uint32)), f"max abs diff {np.abs(got[:M, :N] - ref).max()}"
 
 
+@pytest.mark.parametrize("scheme", [0, 1, 2])
+@pytest.mark.parametrize("scale_mode", [0, 1])
+@pytest.mark.parametrize("N,K", [(200, 64), (264, 448), (9736, 320)])     # few and many weight tiles, ragged last tile, partial last stages
+def test_gemm_tile_edges(pkg, gpu, scheme, scale_mode, N, K):
+    """Both sides of every tile width (8-row steps up to 32 rows, 16-row steps above) against the CUDA-core kernel."""
+    import torch
+    w = pkg.synth.weights(N, K, 7)
+    if scale_mode == 0:
+        w["d"] = (w["d"] * np.float32(1.0003)).astype(np.float32)
+    wh = gpu.weight(scheme, scale_mode, w["nib"], w["d"], w["m"] if scheme == 0 else None, w["zp"] if scheme == 2 else None)
+    x = torch.from_numpy(pkg.synth.activations(260, K, 7)).cuda()
+    act = gpu.act(260, K)
+    for M in (2, 8, 9, 16, 17, 24, 25, 32, 33, 48, 49, 64, 65, 127, 129, 260):
+        C, ref = torch.full((M + 1, N), -5.0, device="cuda"), torch.empty((M, N), device="cuda")
+        gpu.quantize(act, x, M, 2 if scheme == 0 else 0)
+        gpu.gemm(act, wh, C, N)
+        gpu.gemm_simt(act, wh, ref, N)
+        gpu.synchronize()
+        assert torch.equal(C[:M], ref) and bool((C[M] == -5.0).all()), M
+
+
 @pytest.mark.parametrize("M", [2, 5, 6, 7, 13])
 def test_gemm_matches_reference_golden(pkg, gpu, golden, M):
     import torch
