@@ -256,6 +256,14 @@ __device__ __forceinline__ unsigned long long lds_u64(uint32_t saddr)
     return v;
 }
 
+// fp16 product 16 x 8 x 16 with fp32 accumulation, d += a b
+__device__ __forceinline__ void mma_f16_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // ---- packed fp32 pairs -------------------------------------------------------------------------
 // Two fp32 values in one 64-bit register and the IEEE (round-to-nearest) packed multiply / fused multiply-add of
 // sm_100a: each half rounds exactly like the scalar instruction, so results stay bit-identical while the issue slots
@@ -293,6 +301,13 @@ __device__ __forceinline__ uint4 ldg_stream_v4(const void *p)
 {
     uint4 v;
     asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+// The same for rows that are read in 64-byte pieces: the request brings the 256 bytes around it into L2
+__device__ __forceinline__ uint4 ldg_stream_v4_l2(const void *p)
+{
+    uint4 v;
+    asm("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 // 32 contiguous bytes in one request (256-bit load; p must be 32-byte aligned): a whole sector per lane
