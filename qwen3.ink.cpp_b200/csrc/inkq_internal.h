@@ -198,6 +198,8 @@ constexpr int GEMM_ROWS_MAX = 32;
 int launch_gemm_rows(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc, const ExtraDst *extra, int m_begin, int m_count);
 int launch_gemm_w41_f16(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc);   // CUDA cores
 int launch_gemm_w41_tc(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc);    // tcgen05 kind::f16
+bool gemm_w41_rows_fits(const uint16_t *a16, int M, int K);                                                   // whether the next one serves this call
+int launch_gemm_w41_rows(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc);  // M = 2 .. 16, bandwidth-bound
 int launch_gemv_w41(inkq_ctx *ctx, const uint16_t *a16, const Weight *w, float *C);                        // M == 1, bandwidth-bound
 // inkq_linear with further destinations for every output element (defined in inkq_api.cu)
 int linear_impl(inkq_ctx *ctx, const inkq_weight *w, const float *x_dev, int M, float *C_dev, int ldc, const ExtraDst *extra);

@@ -237,6 +237,8 @@ def test_mismatched_quantizer_mode_is_rejected(pkg, gpu, oracle):
 
 # ------------------------------------------------------------------ weight-only W41 and fp16 lm_head
 @pytest.mark.parametrize("M,N,K", [(9, 72, 256), (1, 256, 128), (1, 1064, 512), (1, 4096, 4096), (1, 512, 12288),   # M == 1: the streaming kernel
+                                   # M = 2 .. 16: products in registers, ragged row tiles, fewer and more pairs than warps x depth
+                                   (2, 72, 64), (8, 2440, 1088), (10, 136, 8256), (15, 24, 320), (16, 4808, 576), (16, 136, 12288),
                                    (16, 128, 64), (322, 384, 512), (200, 136, 1024), (400, 264, 192),
                                    # enough work items for the two-weight-tiles-per-CTA variant: an odd tile count (the last
                                    # group holds one tile), and two activation tiles of 160 rows
@@ -285,7 +287,9 @@ def test_weight_only_w41_dequantisation_bits(pkg, gpu, oracle):
     assert np.array_equal(C.cpu().numpy(), ref) and np.array_equal(Cs.cpu().numpy(), ref)
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 1000, 4096), (1, 16, 64), (5, 264, 512)])
+@pytest.mark.parametrize("M,N,K", [(1, 1000, 4096), (1, 16, 64), (5, 264, 512),
+                                   # warp-level products: one and two passes of rows, ragged row tiles, more and fewer K steps than warps x depth
+                                   (2, 1000, 4096), (8, 2408, 2560), (9, 40, 5120), (15, 24, 32), (3, 2400, 544), (4, 72, 40)])
 def test_lm_head_f16(pkg, gpu, oracle, M, N, K):
     import torch
     w16 = pkg.synth.lm_head(N, K, 6)
