@@ -835,7 +835,7 @@ def run_ours(args, rank, world, local_rank):
                             "traffic": 41.12e6 if full_shape else None,
                             "traffic_source": "profiles/qgemm_tc_pp322.md: dram__bytes_read.sum + dram__bytes_write.sum of one launch at this shape "
                                               "(not measured by this run)" if full_shape else None,
-                            "kernel": "k_qgemm_tc", "us_per_launch": ms_g * 1e3,
+                            "kernel": "k_qgemm_rows", "us_per_launch": ms_g * 1e3,
                             "peak_note": f"2 x the {pk['source']} dense bf16 figure ({pk['bf16_tflops']} TFLOP/s); int8 itself is not in MEASURED_PEAKS.json",
                             "cuda_core_note": "every K=32 MMA is followed by an fp32 scale+accumulate of its whole tile on the CUDA cores "
                                               "(M*N*K/32 block dots per launch); that, not the tensor pipe, bounds this kernel"}
@@ -873,7 +873,7 @@ def run_ours(args, rank, world, local_rank):
     line = {"metric": "qgemm_int8_tops_pp322" if wl in ("qgemm_pp322", "qgemv_sweep") else f"qgemm_int8_tops_{wl.split('_')[1]}",
             "value": tops, "unit": "TOPS", "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "repeats": repeats,
             "timed_region_s": ms * 1e-3, "ms_per_step": ms / n_steps, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-            "dtype": "s8 x u4 -> s32 block dots (tcgen05 kind::i8), fp32 scale/accumulate", "data": "synthetic",
+            "dtype": "s8 x u4 -> s32 block dots (mma.sync m16n8k32), fp32 scale/accumulate", "data": "synthetic",
             "config": base_config(wl if wl != "qgemv_sweep" else "qgemm_pp322", M, N, K),
             "run": {"parallelism": exchange, "timing": "CUDA graph of the K steps, replayed" if graph is not None else "eager launches",
                     "l2": f"{sets} distinct weight sets ({sets * w_bytes_one / 1e6:.0f} MB per rank) rotated between steps, > 126 MB L2"},

@@ -525,7 +525,7 @@ int inkq_gemm(inkq_ctx *ctx, const inkq_act *act, const inkq_weight *w, float *C
     if (rc) return rc;
     if ((rc = check_mm(ctx, act, w, C_dev))) return rc;
     INKQ_REQUIRE(ctx, ldc >= w->rows, "ldc is smaller than the number of weight rows");
-    return launch_gemm_tc(ctx, act, w, C_dev, ldc, nullptr);
+    return launch_gemm(ctx, act, w, C_dev, ldc, nullptr);
 }
 
 int inkq_gemm_simt(inkq_ctx *ctx, const inkq_act *act, const inkq_weight *w, float *C_dev, int ldc)
@@ -582,7 +582,7 @@ int inkq_debug_block_dots_tc(inkq_ctx *ctx, const inkq_act *act, const inkq_weig
     if (rc) return rc;
     INKQ_REQUIRE(ctx, act != nullptr && w != nullptr && dots_dev != nullptr, "null handle or output");
     INKQ_REQUIRE(ctx, act->M > 0 && act->K == w->K, "activation handle empty or K mismatch");
-    return launch_gemm_tc(ctx, act, w, nullptr, 0, dots_dev);
+    return launch_gemm(ctx, act, w, nullptr, 0, dots_dev);
 }
 
 // ---- linear forward ---------------------------------------------------------------------
@@ -659,7 +659,7 @@ int inkq::linear_impl(inkq_ctx *ctx, const inkq_weight *w, const float *x_dev, i
     if (w->scheme == INKQ_A81W41) qmode = (M > 1) ? INKQ_Q8_1_F32 : INKQ_Q8_1_F16;  // QwenOperator.cc:96-120
     else qmode = INKQ_Q8_0_F16;
     if ((rc = inkq_quantize(ctx, qmode, x_dev, M, w->K, act))) return rc;
-    if (M > 1) return launch_gemm_tc(ctx, act, w, C_dev, ldc, nullptr, extra);
+    if (M > 1) return launch_gemm(ctx, act, w, C_dev, ldc, nullptr, extra);
     return launch_gemv(ctx, act, w, C_dev, extra);
 }
 
@@ -721,7 +721,7 @@ int inkq_linear_host(inkq_ctx *ctx, const inkq_weight *w, const float *x_host, i
             const int rows = m0[c + 1] - m0[c];
             INKQ_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->h2d_ev[c], 0));
             if ((rc = launch_quantize_rows(ctx, qmode, ctx->lin_x + static_cast<size_t>(m0[c]) * w->K, m0[c], rows, M, w->K, act))) return rc;
-            if ((rc = launch_gemm_tc(ctx, act, w, ctx->lin_c, w->rows, nullptr, nullptr, 0, -1, m0[c], rows))) return rc;
+            if ((rc = launch_gemm(ctx, act, w, ctx->lin_c, w->rows, nullptr, nullptr, m0[c], rows))) return rc;
             INKQ_CUDA(ctx, cudaEventRecord(ctx->chunk_ev[c], ctx->stream));
             INKQ_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_stream, ctx->chunk_ev[c], 0));
             INKQ_CUDA(ctx, cudaMemcpy2DAsync(C_host + static_cast<size_t>(m0[c]) * ldc, static_cast<size_t>(ldc) * sizeof(float),

@@ -188,14 +188,9 @@ int launch_gemv(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const Ex
 int launch_gemv_fused(inkq_ctx *ctx, const Weight *w, const float *x, int pro, const float *g, float eps, float *C, int accumulate);
 int launch_gemm_simt(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc);
 int launch_block_dots(inkq_ctx *ctx, const Act *a, const Weight *w, int32_t *dots);
-// tn_begin / tn_count: the launch covers the weight tiles (of 128 rows) tn_begin .. tn_begin + tn_count - 1 (default: all)
-// tn_begin / tn_count: a range of the weight's 128-row tiles; m_begin / m_count: a window of the activation rows (m_begin a
-// multiple of 4; C and the extra destinations still point at row 0)
-int launch_gemm_tc(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc, int32_t *dots, const ExtraDst *extra = nullptr,
-                   int tn_begin = 0, int tn_count = -1, int m_begin = 0, int m_count = -1);
-// launch_gemm_tc's share with few activation rows (qgemm_rows.cu): m_count <= GEMM_ROWS_MAX
-constexpr int GEMM_ROWS_MAX = 32;
-int launch_gemm_rows(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc, const ExtraDst *extra, int m_begin, int m_count);
+// QGEMM (qgemm_rows.cu); m_begin / m_count: a window of the activation rows (m_begin a multiple of 4; C and the extra
+// destinations still point at row 0).  dots: raw int32 block dots instead of C
+int launch_gemm(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc, int32_t *dots, const ExtraDst *extra = nullptr, int m_begin = 0, int m_count = -1);
 int launch_gemm_w41_f16(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc);   // CUDA cores
 int launch_gemm_w41_tc(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc);    // tcgen05 kind::f16
 bool gemm_w41_rows_fits(const uint16_t *a16, int M, int K);                                                   // whether the next one serves this call

@@ -151,27 +151,13 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr, uint32_t lbo_
     d |= static_cast<uint64_t>(swizzle_mode & 7u) << 61;
     return d;
 }
-// Instruction descriptor for kind::i8: D = s32, A and B signed 8-bit, both K-major.
-//   bits [4,6) D format (2 = s32); [7,10) A format (1 = s8); [10,13) B format (1 = s8);
-//   bit 15 / 16 A / B major (0 = K); [17,23) N >> 3; [24,29) M >> 4.
-__device__ __host__ __forceinline__ uint32_t umma_idesc_i8(int umma_m, int umma_n)
-{
-    return (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(umma_n >> 3) << 17) | (static_cast<uint32_t>(umma_m >> 4) << 24);
-}
-// Instruction descriptor for kind::f16: D = f32 (1), A and B fp16 (0), K-major.
+// Instruction descriptor for kind::f16: D = f32 (1), A and B fp16 (0), both K-major.
+//   bits [4,6) D format; [7,10) A format; [10,13) B format; bit 15 / 16 A / B major (0 = K); [17,23) N >> 3; [24,29) M >> 4.
 __device__ __host__ __forceinline__ uint32_t umma_idesc_f16(int umma_m, int umma_n)
 {
     return (1u << 4) | (0u << 7) | (0u << 10) | (static_cast<uint32_t>(umma_n >> 3) << 17) | (static_cast<uint32_t>(umma_m >> 4) << 24);
 }
 // One thread issues.  D[tmem] (+)= A[smem] * B[smem]; accumulate = 0 overwrites D.
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
@@ -187,20 +173,6 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar)
 }
 
 // ---- TMEM -> registers (whole warp; lane i reads TMEM lane base+i, N consecutive columns) ----
-__device__ __forceinline__ void tmem_ld_x4(uint32_t taddr, uint32_t *r)
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(taddr)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld_x8(uint32_t taddr, uint32_t *r)
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-}
 __device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, uint32_t *r)
 {
     asm volatile(
@@ -211,20 +183,6 @@ __device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, uint32_t *r)
         : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Per-warpgroup register re-balancing; all four warps of a warpgroup execute the same one.
-// inc blocks until the CTA's other warpgroups have released enough registers with dec: the
-// caller must make sure the requests never exceed the releases.
-template <int N>
-__device__ __forceinline__ void setmaxnreg_inc()
-{
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
-}
-template <int N>
-__device__ __forceinline__ void setmaxnreg_dec()
-{
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
-}
 
 // ---- warp-level matrix operands, shared loads by address -------------------------------------
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t saddr)

@@ -1,20 +1,30 @@
-// QGEMM for a few activation rows (2 to 32: sequences decoded together, short prompts): warp-level int8 matrix products
-// whose block dots are scaled where they appear, in registers.
+// QGEMM (2 and more activation rows: sequences decoded together, prompts): warp-level int8 matrix products whose block dots
+// are scaled where they appear, in registers.
 //
 // Stands in for gemm_repack_A81W41_fp32 (qwen3/src/qwen/quantized_gemx_kernels.cc:349-582)
 // and gemm_repack_A80W40 (:195-347); A80W4Z has no reference kernel and follows the A80W40
-// code with q_w = nibble - zp.  Same result bits as qgemm_tc.cu, which serves more rows.
+// code with q_w = nibble - zp.  Same result bits as qgemm_simt.cu.
 //
 //   C[m][n] = sum over 32-element blocks b of  d_a[m,b]*d_w[n,b]*I[m,n,b] + m_w[n,b]*s_a[m,b]
 //   I[m,n,b] = sum_e q_a[m,32b+e] * q_w[n,32b+e]                       (exact int32)
 //
-// What bounds it: the weight stream, and for layers with few rows the chain of a warp's dependent instructions over K (the
-// reference's order forbids splitting an output's sum).  mma.sync.m16n8k32 leaves the 16 x 8 dots of one block (K = 32)
-// in the registers of the threads that scale them, so there is no tensor-memory round trip and no hand-shake between warps,
-// which cost the tcgen05 kernel ~350 cycles per pair of blocks however narrow the tile.  Every warp owns 16 weight rows
-// and all columns: each weight byte is fetched once.  Stages of four pairs (256 K-elements) are unrolled, so that
-// the fragment loads and products of one pair overlap the scaling of the one before.  Measured (prefetched weights of
-// distinct layers, A81W41): 24576 x 4096 with 5 rows 59 -> 15 us (4.2 TB/s), 4096 x 4096 with 5 rows 37 -> 8.5 us.
+// Why mma.sync: it leaves the 16 x 8 dots of one block (K = 32) in the registers of the threads that scale them.  Every block
+// of every output needs its own fp32 conversion, scale product and one or two fused multiply-adds in the reference's order, so
+// the CUDA cores bound this path and not the tensor cores: a tcgen05 form (block dots in tensor memory, or as e4m3 parts with
+// the weights in tensor memory) keeps the tensor pipe 94 % idle and pays for the way back to registers, ~350 cycles of
+// hand-shakes per pair of blocks in narrow tiles and shared-memory bandwidth in wide ones.
+//
+// What bounds it.  Up to 32 rows: the weight stream, and for layers with few rows the chain of a warp's dependent instructions
+// over K (an output's sum may not be split).  Every warp owns 16 weight rows and all columns: each weight byte is fetched once.
+// Stages of four pairs (256 K-elements) are unrolled, so that the fragment loads and products of one pair overlap the scaling of
+// the one before.  More rows: the register file and the FMA pipe.  Alone in registers, a block's 16 x 8 dots take a scheduler 22
+// cycles with four warps (27 with mins, of which 20 are the packed multiplications, three operands of 64 bits each); the kernel
+// runs at 85 to 92 % of that rate.  The weights are read from L2 once per tile of columns (CTAs of one weight tile are neighbours).
+// Measured (prefetched weights of distinct layers; before: the tcgen05 kernel this one replaced), A81W41: 24576 x 4096 with 5 rows
+// 59 -> 15 us (4.2 TB/s), 4096 x 4096 with 5 rows 37 -> 8.5, 12288 x 4096 with 48 rows 39 -> 25, with 128 rows 72 -> 52, with 322
+// rows 128 -> 117, with 2048 rows 728 -> 644; A80W40 with 322 rows 111 -> 98, with 2048 rows 634 -> 562; A80W4Z 4096 x 12288 with
+// 77 rows 83 -> 57.  Slower: scalar multiplications (+12 %), the conversion by a bias in the product's accumulator operand
+// (+20 %: it has to be moved there), fp16 operands with fp32 accumulators (+25 %) and e4m3 parts (x2).
 //
 // Operands: the weights are the MMA's A side, the activation rows its B side.  A packed byte holds element e of both blocks of
 // a pair, so one ldmatrix.x4 fetches the A fragments of two blocks.  Stages pass through a ring in shared memory: tiled TMA
@@ -29,6 +39,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <initializer_list>
 #include <mutex>
 
 #include "inkq_internal.h"
@@ -37,31 +48,38 @@
 namespace inkq {
 namespace qrows {
 
-constexpr int SP = 4;             // pairs per stage
 constexpr int MAX_STAGES = 8;
 constexpr int SMEM_ONE_CTA = 116 * 1024;   // more than half of an SM's shared memory
-constexpr int SMEM_CTA = 111 * 1024;       // two CTAs per SM
+constexpr int SMEM_SM = 222 * 1024;        // for all CTAs of an SM
 
 struct Params {
     const uint8_t *nibT;
     const unsigned char *sc;   // fp16 or fp32 scale records
     const uchar2 *zpT;
     float *C;
+    int32_t *dots;    // DUMP: raw int32 block dots [M][rows][K/32] instead of C
     ExtraDst extra;   // further destinations of every C element (peers of a column-sharded layer)
     int *flag;
-    int M, rows, pairs, ldc;
+    int M, rows, pairs, ldc, tiles_m;
 };
 
-// SCH: weight scheme; S16: fp16 scale records; WR: warps (16 weight rows each); NT: 8-column groups.
-template <int SCH, bool S16, int WR, int NT>
+// Shape of a tile: WR x WC warps, each with MT groups of 16 weight rows and NT groups of 8 activation rows; SP pairs per stage;
+// CTAS resident CTAs per SM.
+template <int WR_, int WC_, int MT_, int NT_, int SP_, int CTAS_ = 2>
+struct Tile {
+    static constexpr int WR = WR_, WC = WC_, MT = MT_, NT = NT_, SP = SP_, CTAS = CTAS_;
+};
+
+// SCH: weight scheme; S16: fp16 scale records
+template <int SCH, bool S16, class T>
 struct Cfg {
-    static constexpr int ROWS = 16 * WR, BM = 8 * NT, THREADS = 32 * WR;
+    static constexpr int SP = T::SP, ROWS = 16 * T::WR * T::MT, BM = 8 * T::NT * T::WC, WARPS = T::WR * T::WC, THREADS = 32 * WARPS;
     static constexpr int PLANES = (SCH == INKQ_A81W41) ? 2 : 1;
     static constexpr int Q_BYTES = BM * 64 * SP, PLANE_BYTES = 2 * SP * BM * 4;
     static constexpr int W_PAIR = ROWS * 32, SC_REC = S16 ? 8 : 16, SC_PAIR = ROWS * SC_REC, Z_PAIR = (SCH == INKQ_A80W4Z) ? ROWS * 2 : 0;
     static constexpr int W_OFF = Q_BYTES, SC_OFF = W_OFF + SP * W_PAIR, Z_OFF = SC_OFF + SP * SC_PAIR, D_OFF = Z_OFF + SP * Z_PAIR, S_OFF = D_OFF + PLANE_BYTES;
     static constexpr int STAGE_BYTES = (D_OFF + PLANES * PLANE_BYTES + 1023) / 1024 * 1024;
-    static constexpr int FIT = (SMEM_CTA - 1024 - 256) / STAGE_BYTES, STAGES = FIT > MAX_STAGES ? MAX_STAGES : FIT;
+    static constexpr int FIT = (SMEM_SM / T::CTAS - 1024 - 256) / STAGE_BYTES, STAGES = FIT > MAX_STAGES ? MAX_STAGES : FIT;
     static constexpr int LEAD = STAGES >= 4 ? STAGES - 2 : STAGES - 1;   // stages requested ahead of the one being multiplied
     static constexpr int SMEM = 1024 + STAGES * STAGE_BYTES + 256;
     static_assert(STAGES >= 3, "shared memory budget");
@@ -95,12 +113,13 @@ __device__ __forceinline__ void wait_bounded(uint64_t *bar, uint32_t parity, vol
     }
 }
 
-template <int SCH, bool S16, int WR, int NT>
-__global__ void __launch_bounds__(32 * WR, 2)
+template <int SCH, bool S16, class T, bool DUMP>
+__global__ void __launch_bounds__(32 * T::WR * T::WC, T::CTAS)
     k_qgemm_rows(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_s,
                  const Params prm)
 {
-    using G = Cfg<SCH, S16, WR, NT>;
+    using G = Cfg<SCH, S16, T>;
+    constexpr int SP = T::SP, MT = T::MT, NT = T::NT;
     constexpr bool HAS_MIN = SCH == INKQ_A81W41;
     constexpr int STAGES = G::STAGES, LEAD = G::LEAD;
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
@@ -109,7 +128,8 @@ __global__ void __launch_bounds__(32 * WR, 2)
     volatile int *abort_flag = reinterpret_cast<volatile int *>(empty + STAGES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row_base = blockIdx.x * G::ROWS, row_in_tile = row_base % TILE_N;   // first weight row of the CTA
+    const int tn = blockIdx.x / prm.tiles_m, m_base = (blockIdx.x - tn * prm.tiles_m) * G::BM;   // first activation row of the CTA
+    const int row_base = tn * G::ROWS, row_in_tile = row_base % TILE_N;                          // and its first weight row
     const size_t slab = static_cast<size_t>(row_base / TILE_N) * prm.pairs;
     const int k_stages = (prm.pairs + SP - 1) / SP;
 
@@ -133,15 +153,15 @@ __global__ void __launch_bounds__(32 * WR, 2)
     auto issue_activations = [&](int ks, int slot) {   // boxes are always full size; parts out of range arrive as zeros
         unsigned char *st = smem + slot * G::STAGE_BYTES;
 #pragma unroll
-        for (int b = 0; b < SP / 2; b++) tma_tensor2d_g2s(st + b * (G::BM * 128), &map_q, ks * (64 * SP) + b * 128, 0, &full[slot]);
-        tma_tensor2d_g2s(st + G::D_OFF, &map_d, 0, ks * (2 * SP), &full[slot]);
-        if (G::PLANES == 2) tma_tensor2d_g2s(st + G::S_OFF, &map_s, 0, ks * (2 * SP), &full[slot]);
+        for (int b = 0; b < SP / 2; b++) tma_tensor2d_g2s(st + b * (G::BM * 128), &map_q, ks * (64 * SP) + b * 128, m_base, &full[slot]);
+        tma_tensor2d_g2s(st + G::D_OFF, &map_d, m_base, ks * (2 * SP), &full[slot]);
+        if (G::PLANES == 2) tma_tensor2d_g2s(st + G::S_OFF, &map_s, m_base, ks * (2 * SP), &full[slot]);
     };
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < STAGES; i++) {
             mbar_init(&full[i], 1);
-            mbar_init(&empty[i], WR);
+            mbar_init(&empty[i], G::WARPS);
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -159,59 +179,61 @@ __global__ void __launch_bounds__(32 * WR, 2)
     }
     __syncthreads();
 
-    const int row0 = warp * 16;                              // the warp's first row inside the CTA's tile
+    const int row0 = (warp % T::WR) * (16 * MT), col0 = (warp / T::WR) * (8 * NT);   // the warp's first row and column inside the tile
     const int g = lane >> 2, t2 = (lane & 3) * 2;            // fragment coordinates: rows g, g + 8; columns t2, t2 + 1
     // ldmatrix row addresses.  A: matrices (rows 0-7, chunk 0), (rows 8-15, chunk 0), (rows 0-7, chunk 1), (rows 8-15, chunk 1)
     const int a_row = row0 + ((lane >> 3) & 1) * 8 + (lane & 7);
     const uint32_t a_off = G::W_OFF + a_row * 32 + ((((lane >> 4) & 1) ^ ((a_row >> 2) & 1)) << 4);
     // B: matrix j = 16-byte chunk j of a pair's 64 bytes (low block: chunks 0, 1; high block: 2, 3); rows of 128 B, swizzled;
     // the second pair of a row lies at this offset with bit 6 flipped
-    const uint32_t b_off = (lane & 7) * 128 + (((lane >> 3) ^ (lane & 7)) << 4);
+    const uint32_t b_off = (col0 + (lane & 7)) * 128 + (((lane >> 3) ^ (lane & 7)) << 4);
     const uint32_t base = smem_u32(smem);
 
-    unsigned long long acc[NT][2];   // columns (t2, t2 + 1) of rows g and g + 8
+    unsigned long long acc[MT][NT][2];   // columns (t2, t2 + 1) of rows g and g + 8
 #pragma unroll
-    for (int j = 0; j < NT; j++) acc[j][0] = acc[j][1] = 0ull;
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int j = 0; j < NT; j++) acc[i][j][0] = acc[i][j][1] = 0ull;
 
-    auto multiply_pair = [&](int pj, uint32_t st) {
-        uint32_t pk[4], alo[4], ahi[4];
-        ldmatrix_x4(pk, st + a_off + pj * G::W_PAIR);
-        float4 w[2];   // {d_lo, d_hi, m_lo, m_hi} of rows g and g + 8
-        uint32_t z_lo[2] = {0u, 0u}, z_hi[2] = {0u, 0u};
+    auto multiply_pair = [&](int p, int pj, uint32_t st) {   // pair p of the row, pj of the stage
+        uint32_t alo[MT][4], ahi[MT][4];
+        float4 w[MT][2];   // {d_lo, d_hi, m_lo, m_hi} of rows g and g + 8
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int r = row0 + g + 8 * h;
-            if (S16) {
-                const uint2 p = lds_u32x2(st + G::SC_OFF + pj * G::SC_PAIR + r * 8);
-                const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&p.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&p.y));
-                w[h] = make_float4(a.x, a.y, b.x, b.y);
-            } else {
-                w[h] = lds_f4(st + G::SC_OFF + pj * G::SC_PAIR + r * 16);
-            }
-            if (SCH == INKQ_A80W40) z_lo[h] = z_hi[h] = 0x08080808u;
-            if (SCH == INKQ_A80W4Z) {
-                const uint32_t z = lds_u16(st + G::Z_OFF + pj * G::Z_PAIR + r * 2);
-                z_lo[h] = (z & 0xFFu) * 0x01010101u;
-                z_hi[h] = (z >> 8) * 0x01010101u;
-            }
-        }
+        for (int i = 0; i < MT; i++) {
+            uint32_t pk[4], z_lo[2] = {0u, 0u}, z_hi[2] = {0u, 0u};
+            ldmatrix_x4(pk, st + a_off + pj * G::W_PAIR + i * (16 * 32));
 #pragma unroll
-        for (int e = 0; e < 4; e++) {   // registers 0, 2: row g; 1, 3: row g + 8
-            alo[e] = pk[e] & 0x0F0F0F0Fu;
-            ahi[e] = (pk[e] >> 4) & 0x0F0F0F0Fu;
-            if (!HAS_MIN) {   // byte-wise (nibble - z) without borrows between bytes: set bit 7, subtract, clear
-                alo[e] = ((alo[e] | 0x80808080u) - z_lo[e & 1]) ^ 0x80808080u;
-                ahi[e] = ((ahi[e] | 0x80808080u) - z_hi[e & 1]) ^ 0x80808080u;
+            for (int h = 0; h < 2; h++) {
+                const int r = row0 + i * 16 + g + 8 * h;
+                if (S16) {
+                    const uint2 v = lds_u32x2(st + G::SC_OFF + pj * G::SC_PAIR + r * 8);
+                    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
+                    w[i][h] = make_float4(a.x, a.y, b.x, b.y);
+                } else {
+                    w[i][h] = lds_f4(st + G::SC_OFF + pj * G::SC_PAIR + r * 16);
+                }
+                if (SCH == INKQ_A80W40) z_lo[h] = z_hi[h] = 0x08080808u;
+                if (SCH == INKQ_A80W4Z) {
+                    const uint32_t z = lds_u16(st + G::Z_OFF + pj * G::Z_PAIR + r * 2);
+                    z_lo[h] = (z & 0xFFu) * 0x01010101u;
+                    z_hi[h] = (z >> 8) * 0x01010101u;
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e++) {   // registers 0, 2: row g; 1, 3: row g + 8
+                alo[i][e] = pk[e] & 0x0F0F0F0Fu;
+                ahi[i][e] = (pk[e] >> 4) & 0x0F0F0F0Fu;
+                if (!HAS_MIN) {   // byte-wise (nibble - z) without borrows between bytes: set bit 7, subtract, clear
+                    alo[i][e] = ((alo[i][e] | 0x80808080u) - z_lo[e & 1]) ^ 0x80808080u;
+                    ahi[i][e] = ((ahi[i][e] | 0x80808080u) - z_hi[e & 1]) ^ 0x80808080u;
+                }
             }
         }
 #pragma unroll
         for (int j = 0; j < NT; j++) {
             uint32_t b[4];
             ldmatrix_x4(b, st + (pj >> 1) * (G::BM * 128) + (b_off ^ ((pj & 1) << 6)) + j * (8 * 128));
-            int lo[4], hi[4];
-            mma_block(lo, alo, b[0], b[1]);
-            mma_block(hi, ahi, b[2], b[3]);
-            const uint32_t pl = st + (2 * pj) * (G::BM * 4) + (j * 8 + t2) * 4;
+            const uint32_t pl = st + (2 * pj) * (G::BM * 4) + (col0 + j * 8 + t2) * 4;
             const unsigned long long d_lo = lds_u64(pl + G::D_OFF), d_hi = lds_u64(pl + G::D_OFF + G::BM * 4);
             unsigned long long s_lo = 0ull, s_hi = 0ull;
             if (HAS_MIN) {
@@ -219,15 +241,33 @@ __global__ void __launch_bounds__(32 * WR, 2)
                 s_hi = lds_u64(pl + G::S_OFF + G::BM * 4);
             }
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                unsigned long long a = acc[j][h];
-                a = fma2(cvt2_exact(lo[2 * h], lo[2 * h + 1]), mul2(d_lo, pack2(w[h].x, w[h].x)), a);
-                a = fma2(cvt2_exact(hi[2 * h], hi[2 * h + 1]), mul2(d_hi, pack2(w[h].y, w[h].y)), a);
-                if (HAS_MIN) {
-                    a = fma2(pack2(w[h].z, w[h].z), s_lo, a);
-                    a = fma2(pack2(w[h].w, w[h].w), s_hi, a);
+            for (int i = 0; i < MT; i++) {
+                int lo[4], hi[4];
+                mma_block(lo, alo[i], b[0], b[1]);
+                mma_block(hi, ahi[i], b[2], b[3]);
+                if (DUMP) {
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int n = row_base + row0 + i * 16 + g + (e >> 1) * 8, m = m_base + col0 + j * 8 + t2 + (e & 1);
+                        if (n < prm.rows && m < prm.M) {
+                            int32_t *o = prm.dots + (static_cast<size_t>(m) * prm.rows + n) * (2 * prm.pairs) + 2 * p;
+                            o[0] = lo[e];
+                            o[1] = hi[e];
+                        }
+                    }
+                    continue;
                 }
-                acc[j][h] = a;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    unsigned long long a = acc[i][j][h];
+                    a = fma2(cvt2_exact(lo[2 * h], lo[2 * h + 1]), mul2(d_lo, pack2(w[i][h].x, w[i][h].x)), a);
+                    a = fma2(cvt2_exact(hi[2 * h], hi[2 * h + 1]), mul2(d_hi, pack2(w[i][h].y, w[i][h].y)), a);
+                    if (HAS_MIN) {
+                        a = fma2(pack2(w[i][h].z, w[i][h].z), s_lo, a);
+                        a = fma2(pack2(w[i][h].w, w[i][h].w), s_hi, a);
+                    }
+                    acc[i][j][h] = a;
+                }
             }
         }
     };
@@ -246,16 +286,16 @@ __global__ void __launch_bounds__(32 * WR, 2)
             fill = 0;
             fill_phase ^= 1;
         }
-        if (++turn == WR) turn = 0;
+        if (++turn == G::WARPS) turn = 0;
         wait_bounded(&full[slot], phase, abort_flag, prm.flag);
         const uint32_t st = base + slot * G::STAGE_BYTES;
         const int np = min(SP, prm.pairs - ks * SP);
         if (np == SP) {
 #pragma unroll
-            for (int pj = 0; pj < SP; pj++) multiply_pair(pj, st);
+            for (int pj = 0; pj < SP; pj++) multiply_pair(ks * SP + pj, pj, st);
         } else {
 #pragma unroll 1
-            for (int pj = 0; pj < np; pj++) multiply_pair(pj, st);
+            for (int pj = 0; pj < np; pj++) multiply_pair(ks * SP + pj, pj, st);
         }
         __syncwarp();
         if (elect_one()) mbar_arrive(&empty[slot]);
@@ -268,37 +308,40 @@ __global__ void __launch_bounds__(32 * WR, 2)
         // copies of stages nobody waited for may still be in flight: wait (bounded) for the last fill of each slot
         for (int s = 0; s < STAGES && s < k_stages; s++) mbar_wait_drain(&full[s], ((k_stages - 1 - s) / STAGES) & 1);
     }
+    if (DUMP) return;
 #pragma unroll
     for (int j = 0; j < NT; j++)
 #pragma unroll
         for (int c = 0; c < 2; c++) {
-            const int m = j * 8 + t2 + c;
+            const int m = m_base + col0 + j * 8 + t2 + c;
             if (m < prm.M) {
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int n = row_base + row0 + h * 8 + g;
-                    if (n < prm.rows) {
-                        float v0, v1;
-                        unpack2(acc[j][h], v0, v1);
-                        const float v = c ? v1 : v0;
-                        const size_t off = static_cast<size_t>(m) * prm.ldc + n;
-                        prm.C[off] = v;
+                for (int i = 0; i < MT; i++)
 #pragma unroll
-                        for (int e = 0; e < MAX_PEERS - 1; e++)   // static indices: the parameter array stays out of local memory
-                            if (e < prm.extra.n) prm.extra.p[e][off] = v;
+                    for (int h = 0; h < 2; h++) {
+                        const int n = row_base + row0 + i * 16 + h * 8 + g;
+                        if (n < prm.rows) {
+                            float v0, v1;
+                            unpack2(acc[i][j][h], v0, v1);
+                            const float v = c ? v1 : v0;
+                            const size_t off = static_cast<size_t>(m) * prm.ldc + n;
+                            prm.C[off] = v;
+#pragma unroll
+                            for (int e = 0; e < MAX_PEERS - 1; e++)   // static indices: the parameter array stays out of local memory
+                                if (e < prm.extra.n) prm.extra.p[e][off] = v;
+                        }
                     }
-                }
             }
         }
 }
 
 constexpr int MAX_DEVICES = 64;
 
-template <int SCH, bool S16, int WR, int NT>
-static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin, const Params &prm)
+template <int SCH, bool S16, class T, bool DUMP = false>
+static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin, Params prm)
 {
-    using G = Cfg<SCH, S16, WR, NT>;
-    auto kernel = k_qgemm_rows<SCH, S16, WR, NT>;
+    using G = Cfg<SCH, S16, T>;
+    auto kernel = k_qgemm_rows<SCH, S16, T, DUMP>;
     // The opt-in for large dynamic shared memory is a per-device function attribute: remembered per device and instantiation
     static std::mutex mu;
     static bool configured[MAX_DEVICES] = {};
@@ -316,48 +359,122 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
     // a row window starts m_begin rows into q and m_begin entries into every block's line of the planes
     int rc = encode_map_2d(ctx, &mq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->q + static_cast<size_t>(m_begin) * a->K, a->K, prm.M, 128u, G::BM,
                            CU_TENSOR_MAP_SWIZZLE_128B, a->K);
-    if (!rc) rc = encode_map_2d(ctx, &md, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->d + m_begin, a->M_ld - m_begin, nb, G::BM, 2 * SP, CU_TENSOR_MAP_SWIZZLE_NONE,
+    if (!rc) rc = encode_map_2d(ctx, &md, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->d + m_begin, a->M_ld - m_begin, nb, G::BM, 2 * G::SP, CU_TENSOR_MAP_SWIZZLE_NONE,
                                 a->M_ld);
     ms = md;
     if (!rc && G::PLANES == 2)
-        rc = encode_map_2d(ctx, &ms, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->s + m_begin, a->M_ld - m_begin, nb, G::BM, 2 * SP, CU_TENSOR_MAP_SWIZZLE_NONE, a->M_ld);
+        rc = encode_map_2d(ctx, &ms, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->s + m_begin, a->M_ld - m_begin, nb, G::BM, 2 * G::SP, CU_TENSOR_MAP_SWIZZLE_NONE, a->M_ld);
     if (rc) return rc;
-    const int grid = (w->rows + G::ROWS - 1) / G::ROWS;
-    // No more CTAs than SMs: one per SM.  The grid may be placed while the kernel before it still occupies SMs, and would
-    // otherwise double up on the free ones (4096 x 12288 behind its quantizer: 95 -> 60 us with 77 rows in an earlier form).
-    const int smem = grid <= ctx->num_sms && G::SMEM < SMEM_ONE_CTA ? SMEM_ONE_CTA : G::SMEM;
+    prm.tiles_m = (prm.M + G::BM - 1) / G::BM;
+    const int grid = (w->rows + G::ROWS - 1) / G::ROWS * prm.tiles_m;
+    // Shared memory for no more CTAs per SM than an even spread needs.  The grid may be placed while the kernel before it
+    // still occupies SMs, and would otherwise pile up on the free ones (4096 x 12288 behind its quantizer: 95 -> 60 us with 77
+    // rows in an earlier form).
+    const int per_sm = (grid + ctx->num_sms - 1) / ctx->num_sms, spread = per_sm == 1 ? SMEM_ONE_CTA : SMEM_SM / (per_sm < T::CTAS ? per_sm : T::CTAS);
+    const int smem = spread > G::SMEM ? spread : G::SMEM;
     const cudaError_t le = launch_pdl(kernel, dim3(grid), dim3(G::THREADS), smem, ctx->stream, mq, md, ms, prm);
     if (le != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("k_qgemm_rows launch: ") + cudaGetErrorString(le));
     return after_launch(ctx, "k_qgemm_rows");
 }
 
+// Tiles for more than 32 activation rows: shape, then the time (us) of 1 .. CTAS tiles on every SM at K = 4096, without the
+// ~3 us that a launch takes, with the mins of A81W41 and without them.  Measured with prefetched weights of distinct layers;
+// only the ratios matter, and they hardly depend on K.  Per column the wide tiles cost least (fragments and scales of the weight
+// rows are fetched once for more columns) until the accumulators crowd the 128 registers that two CTAs of 256 threads leave
+// (112 columns of 32-row warps spill a little).  Half-height tiles split a layer with few weight rows over more SMs.
+#define QROWS_TILES(X)                                                                    \
+    X(0, (4, 1, 2, 2, 2, 4), (15.7f, 21.4f, 29.9f, 38.6f), (15.4f, 21.2f, 28.3f, 36.7f)) \
+    X(1, (4, 2, 2, 2, 2, 2), (21.7f, 37.1f), (21.0f, 36.3f))                              \
+    X(2, (4, 2, 2, 3, 2, 2), (27.7f, 48.9f), (26.1f, 45.3f))                              \
+    X(3, (4, 2, 2, 4, 2, 2), (34.6f, 62.5f), (31.7f, 55.8f))                              \
+    X(4, (4, 2, 2, 5, 2, 2), (43.3f, 78.1f), (37.6f, 66.7f))                              \
+    X(5, (4, 2, 2, 7, 2, 2), (72.0f, 122.5f), (55.2f, 94.1f))                             \
+    X(6, (4, 2, 1, 3, 2, 2), (17.9f, 29.8f), (16.3f, 26.5f))                              \
+    X(7, (4, 2, 1, 4, 2, 2), (21.9f, 36.4f), (19.3f, 31.5f))                              \
+    X(8, (4, 2, 1, 6, 2, 2), (28.3f, 50.2f), (25.1f, 42.3f))                              \
+    X(9, (4, 2, 1, 7, 2, 2), (31.7f, 56.8f), (28.2f, 48.7f))
+
+#define QROWS_UNWRAP(...) __VA_ARGS__
+struct TileCost {
+    int rows, cols, ctas;
+    float with_min[4], without[4];
+};
+template <class T>
+constexpr TileCost tile_cost(std::initializer_list<float> with_min, std::initializer_list<float> without)
+{
+    TileCost c{16 * T::WR * T::MT, 8 * T::NT * T::WC, T::CTAS, {}, {}};
+    int i = 0;
+    for (float v : with_min) c.with_min[i++] = v;
+    i = 0;
+    for (float v : without) c.without[i++] = v;
+    return c;
+}
+static constexpr TileCost tile_costs[] = {
+#define QROWS_COST(i, shape, with_min, without) tile_cost<Tile<QROWS_UNWRAP shape>>({QROWS_UNWRAP with_min}, {QROWS_UNWRAP without}),
+    QROWS_TILES(QROWS_COST)
+};
+
+// The tile with the least time for M activation rows: a CTA takes one tile, so the busiest SM works through
+// n = ceil(tiles / SMs) of them, CTAS at a time (3 tiles of 128 x 64 on every SM: 94.2 us against 62.5 + 34.6 by the table).
+static int pick_tile(const inkq_ctx *ctx, bool has_min, int rows, int M)
+{
+    int best = 0;
+    float best_time = 0.f;
+    for (int i = 0; i < static_cast<int>(sizeof(tile_costs) / sizeof(tile_costs[0])); i++) {
+        const TileCost &c = tile_costs[i];
+        const float *t = has_min ? c.with_min : c.without;
+        const long long total = static_cast<long long>((rows + c.rows - 1) / c.rows) * ((M + c.cols - 1) / c.cols);
+        const long long n = (total + ctx->num_sms - 1) / ctx->num_sms;
+        const float time = static_cast<float>(n / c.ctas) * t[c.ctas - 1] + (n % c.ctas != 0 ? t[n % c.ctas - 1] : 0.f);
+        if (i == 0 || time < best_time) {
+            best = i;
+            best_time = time;
+        }
+    }
+    return best;
+}
+
 template <int SCH, bool S16>
 static int launch_sized(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin, const Params &prm)
 {
-    // 64 instead of 128 rows per CTA when the layer has too few 128-row tiles to occupy the SMs (measured: 6144 x 4096 with 24
-    // rows 18.0 -> 13.4 us; 24576 x 4096 with 5 rows 16.3 against 23.1 us the other way round)
+    if (prm.M > 32) {
+        const int tile = pick_tile(ctx, SCH == INKQ_A81W41, prm.rows, prm.M);
+        switch (tile) {
+#define QROWS_CASE(i, shape, with_min, without) case i: return launch_one<SCH, S16, Tile<QROWS_UNWRAP shape>>(ctx, a, w, m_begin, prm);
+            QROWS_TILES(QROWS_CASE)
+        }
+    }
+    // Up to 32 rows one tile holds all of them, so every weight byte is fetched once.  64 instead of 128 weight rows per CTA when
+    // the layer has too few 128-row tiles to occupy the SMs (measured: 6144 x 4096 with 24 rows 18.0 -> 13.4 us; 24576 x 4096
+    // with 5 rows 16.3 against 23.1 us the other way round)
     const bool narrow = w->tiles * 2 <= ctx->num_sms;
     switch ((prm.M + 7) / 8) {
-        case 1: return narrow ? launch_one<SCH, S16, 4, 1>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, 8, 1>(ctx, a, w, m_begin, prm);
-        case 2: return narrow ? launch_one<SCH, S16, 4, 2>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, 8, 2>(ctx, a, w, m_begin, prm);
-        case 3: return narrow ? launch_one<SCH, S16, 4, 3>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, 8, 3>(ctx, a, w, m_begin, prm);
-        case 4: return narrow ? launch_one<SCH, S16, 4, 4>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, 8, 4>(ctx, a, w, m_begin, prm);
+        case 1: return narrow ? launch_one<SCH, S16, Tile<4, 1, 1, 1, 4>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, 1, 4>>(ctx, a, w, m_begin, prm);
+        case 2: return narrow ? launch_one<SCH, S16, Tile<4, 1, 1, 2, 4>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, 2, 4>>(ctx, a, w, m_begin, prm);
+        case 3: return narrow ? launch_one<SCH, S16, Tile<4, 1, 1, 3, 4>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, 3, 4>>(ctx, a, w, m_begin, prm);
+        case 4: return narrow ? launch_one<SCH, S16, Tile<4, 1, 1, 4, 4>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, 4, 4>>(ctx, a, w, m_begin, prm);
     }
     return fail(ctx, INKQ_ERR_INVALID, "internal: too many rows for k_qgemm_rows");
 }
 
 }  // namespace qrows
 
-int launch_gemm_rows(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc, const ExtraDst *extra, int m_begin, int m_count)
+int launch_gemm(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc, int32_t *dots, const ExtraDst *extra, int m_begin, int m_count)
 {
     using namespace qrows;
-    const bool s16 = w->scale_mode == INKQ_SCALES_F16;
+    if (m_count < 0) m_count = a->M - m_begin;   // default: every row from m_begin on
+    if (m_begin < 0 || (m_begin & 3) != 0 || m_count < 1 || m_begin + m_count > a->M || (m_begin != 0 && dots != nullptr))
+        return fail(ctx, INKQ_ERR_INVALID, "bad activation row window");
+    if (ctx->encode_tiled == nullptr) return fail(ctx, INKQ_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled entry point not available");
+    if (w->sc32 == nullptr) return fail(ctx, INKQ_ERR_INVALID, "this weight holds no fp32 scale records (weight-only layers use inkq_gemm_w41_f16act)");
+    const bool s16 = w->scale_mode == INKQ_SCALES_F16 && dots == nullptr;
     Params prm;
     prm.nibT = w->nibT;
     prm.sc = s16 ? reinterpret_cast<const unsigned char *>(w->sc16) : reinterpret_cast<const unsigned char *>(w->sc32);
     prm.zpT = w->zpT;
     const size_t c_off = static_cast<size_t>(m_begin) * ldc;
-    prm.C = C + c_off;
+    prm.C = (C != nullptr) ? C + c_off : nullptr;
+    prm.dots = dots;
     prm.extra = ExtraDst{};
     if (extra != nullptr) {
         prm.extra = *extra;
@@ -368,6 +485,12 @@ int launch_gemm_rows(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int
     prm.rows = w->rows;
     prm.pairs = w->pairs;
     prm.ldc = ldc;
+    if (dots != nullptr) {
+        using T = Tile<4, 2, 1, 3, 2>;
+        if (w->scheme == INKQ_A81W41) return launch_one<INKQ_A81W41, false, T, true>(ctx, a, w, m_begin, prm);
+        if (w->scheme == INKQ_A80W40) return launch_one<INKQ_A80W40, false, T, true>(ctx, a, w, m_begin, prm);
+        return launch_one<INKQ_A80W4Z, false, T, true>(ctx, a, w, m_begin, prm);
+    }
     if (w->scheme == INKQ_A81W41) return s16 ? launch_sized<INKQ_A81W41, true>(ctx, a, w, m_begin, prm) : launch_sized<INKQ_A81W41, false>(ctx, a, w, m_begin, prm);
     if (w->scheme == INKQ_A80W40) return s16 ? launch_sized<INKQ_A80W40, true>(ctx, a, w, m_begin, prm) : launch_sized<INKQ_A80W40, false>(ctx, a, w, m_begin, prm);
     return s16 ? launch_sized<INKQ_A80W4Z, true>(ctx, a, w, m_begin, prm) : launch_sized<INKQ_A80W4Z, false>(ctx, a, w, m_begin, prm);

@@ -125,6 +125,25 @@ def test_gemm_tile_edges(pkg, gpu, scheme, scale_mode, N, K):
         assert torch.equal(C[:M], ref) and bool((C[M] == -5.0).all()), M
 
 
+@pytest.mark.parametrize("scheme", [0, 1, 2])
+@pytest.mark.parametrize("scale_mode", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(33, 24576, 192), (281, 8192, 64), (65, 6144, 320), (113, 12232, 192), (481, 12288, 64), (700, 24576, 64),
+                                   (322, 12288, 192), (409, 1000, 320), (57, 24568, 64), (100, 4096, 192), (322, 4096, 64), (322, 6144, 192)])
+def test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K):
+    """Sizes that between them select every tile of more than 32 columns, ragged in rows, columns and stages."""
+    import torch
+    w = pkg.synth.weights(N, K, 11)
+    wh = gpu.weight(scheme, scale_mode, w["nib"], w["d"], w["m"] if scheme == 0 else None, w["zp"] if scheme == 2 else None)
+    x = torch.from_numpy(pkg.synth.activations(M, K, 11)).cuda()
+    act = gpu.act(M, K)
+    C, ref = torch.full((M + 1, N), -5.0, device="cuda"), torch.empty((M, N), device="cuda")
+    gpu.quantize(act, x, M, 2 if scheme == 0 else 0)
+    gpu.gemm(act, wh, C, N)
+    gpu.gemm_simt(act, wh, ref, N)
+    gpu.synchronize()
+    assert torch.equal(C[:M], ref) and bool((C[M] == -5.0).all())
+
+
 @pytest.mark.parametrize("M", [2, 5, 6, 7, 13])
 def test_gemm_matches_reference_golden(pkg, gpu, golden, M):
     import torch
