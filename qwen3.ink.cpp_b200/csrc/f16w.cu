@@ -7,6 +7,8 @@
 // notebooks/evaluate-qwen3_8b_W4.ipynb cell 13: the weight is replaced by
 // w16 = fp16(q*d + m) and a stock fp16 linear with fp32 accumulation runs.
 //
+// k_f16w_rows (further down) serves rows of a multiple of 64 elements, k_f16w_gemv the others.
+//
 // k_f16w_gemv is bandwidth-bound: one warp per weight row, 128-bit streaming loads,
 // eight loads in flight per lane, activations staged once per CTA in shared memory.
 // Reduction order (fixed): lane l accumulates the 8-element chunks c with
@@ -97,21 +99,24 @@ __global__ void __launch_bounds__(256) k_f16w_gemv(const uint16_t *__restrict__ 
     }
 }
 
-// ---- 2 to 8 activation rows per pass --------------------------------------------------------------------------------
+// ---- up to 8 activation rows per pass, K a multiple of 64 ------------------------------------------------------------
 // The CUDA-core kernel above needs, per weight and row, a conversion, an fp32 fma and its share of a 16-byte shared load: with
-// four rows it is bound by instruction issue (4 rows 631 us for the 1.2 GB lm_head, 195 us with one).  Here 16 weight rows x 8
+// four rows it is bound by instruction issue (4 rows 631 us for the 1.2 GB lm_head, 194 us with one).  Here 16 weight rows x 8
 // activation rows x 16 k are one warp-level fp16 product with fp32 accumulation; the fp32 activations enter as an fp16 value and
 // an fp16 remainder of the row scaled by a power of two (22 significant bits, as in the tensor-core GEMM), so both products
-// are exact.  A tile's K is split over the CTA's 16 warps, whose partial sums are added in ascending order.
+// are exact.  A tile's K is split over the CTA's 16 warps, whose partial sums are added in ascending order.  A row's result does
+// not depend on the rows beside it, and one row takes this kernel too: a batch gives the same bits as its rows one by one.
 //
-// The weights come straight from global memory into A fragments: the order of k inside a product is free, so a lane takes 16
-// contiguous bytes of its two rows per 32 k - the fragments of two products - and the activations are read alike.  Each
-// lane keeps F16R_DEPTH such steps in flight across tile borders (128 KB per SM).  Measured: 151936 x 4096, 8 rows 1258 ->
-// 230 us.
-constexpr int F16R_WARPS = 16, F16R_DEPTH = 8, F16R_COLS = 8;
+// Bound by the weight stream.  The weights come straight from global memory into A fragments: the order of k inside a product
+// is free, so a lane takes 32 contiguous bytes of its two rows per 64 k - the fragments of four products, 128 bytes per row and
+// request - and the activations are read alike.  Each lane keeps F16R_DEPTH such steps in flight across tile borders (128 KB
+// per SM).  Measured: 151936 x 4096, 8 rows 1258 us on the CUDA cores, 230 with 64-byte pieces, 200 now (6.2 TB/s); one row 194
+// on the CUDA cores, 197 now (32000 x 4096: 54 -> 50, 151936 x 2048: 111 -> 100, set-up hidden behind the kernel before).
+constexpr int F16R_WARPS = 16, F16R_DEPTH = 4, F16R_COLS = 8;
 
-// bytes between two rows of the staged activations: 64 modulo 128, so that the rows of an 8-lane phase fall into different banks
-__host__ __device__ constexpr int f16r_pitch(int K) { return (K * 2 + 127) / 128 * 128 + 64; }
+// bytes between two rows of the staged activations: 16 modulo 128, so that the 16-byte pieces of an 8-lane phase (two rows, every
+// other piece of 128 bytes) fall into different banks
+__host__ __device__ constexpr int f16r_pitch(int K) { return (K * 2 + 127) / 128 * 128 + 16; }
 
 __global__ void __launch_bounds__(F16R_WARPS * 32, 1)
     k_f16w_rows(const uint16_t *__restrict__ w, const float *__restrict__ x, int m0, int mt, int rows, int K, float *__restrict__ C, int ldc, const ExtraDst extra)
@@ -122,18 +127,18 @@ __global__ void __launch_bounds__(F16R_WARPS * 32, 1)
     float *part = reinterpret_cast<float *>(xl + F16R_COLS * pitch);                              // [2][warps][8 columns][16 rows]
     float *inv = part + 2 * F16R_WARPS * F16R_COLS * 16;                                           // [8]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int k32 = K / 32, steps = (k32 + F16R_WARPS - 1) / F16R_WARPS;                          // steps of 32 k per warp and tile
+    const int k64 = K / 64, steps = (k64 + F16R_WARPS - 1) / F16R_WARPS;                          // steps of 64 k per warp and tile
     const int tiles = (rows + 15) / 16;
 
-    uint4 a[F16R_DEPTH][2];                                                                       // rows g and g + 8
+    uint4 a[F16R_DEPTH][2][2];                                                                    // rows g and g + 8, 16 k each
     int ptile = blockIdx.x, ps = 0;                                                               // next step to request
-    auto request = [&](uint4 (&v)[2]) {
+    auto request = [&](uint4 (&v)[2][2]) {
         const int k = warp * steps + ps, r0 = ptile * 16 + g;
-        v[0] = v[1] = make_uint4(0, 0, 0, 0);
-        if (ptile < tiles && k < k32) {
-            const uint16_t *src = w + static_cast<size_t>(r0) * K + k * 32 + t * 8;
-            if (r0 < rows) v[0] = ldg_stream_v4_l2(src);
-            if (r0 + 8 < rows) v[1] = ldg_stream_v4_l2(src + static_cast<size_t>(8) * K);
+        v[0][0] = v[0][1] = v[1][0] = v[1][1] = make_uint4(0, 0, 0, 0);
+        if (ptile < tiles && k < k64) {
+            const uint16_t *src = w + static_cast<size_t>(r0) * K + k * 64 + t * 16;
+            if (r0 < rows) ldg_stream_v8(src, v[0][0], v[0][1]);
+            if (r0 + 8 < rows) ldg_stream_v8(src + static_cast<size_t>(8) * K, v[1][0], v[1][1]);
         }
         if (++ps == steps) {
             ps = 0;
@@ -182,7 +187,7 @@ __global__ void __launch_bounds__(F16R_WARPS * 32, 1)
     }
     __syncthreads();
 
-    const unsigned char *bh = xh + g * pitch + t * 16, *bl = xl + g * pitch + t * 16;            // column g of the activations
+    const unsigned char *bh = xh + g * pitch + t * 32, *bl = xl + g * pitch + t * 32;            // column g of the activations
     int tile = blockIdx.x, s = 0, buf = 0;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     while (tile < tiles) {
@@ -190,15 +195,19 @@ __global__ void __launch_bounds__(F16R_WARPS * 32, 1)
         for (int u = 0; u < F16R_DEPTH; u++) {
             if (tile < tiles) {   // uniform over the CTA
                 const int k = warp * steps + s;
-                if (k < k32) {
-                    const uint4 h = *reinterpret_cast<const uint4 *>(bh + k * 64), l = *reinterpret_cast<const uint4 *>(bl + k * 64);
-                    float sum[4] = {0.f, 0.f, 0.f, 0.f};   // the products' own accumulation truncates: 32 terms at a time, rounded sums beyond
-                    mma_f16_16x8x16(sum, a[u][0].x, a[u][1].x, a[u][0].y, a[u][1].y, l.x, l.y);
-                    mma_f16_16x8x16(sum, a[u][0].z, a[u][1].z, a[u][0].w, a[u][1].w, l.z, l.w);
-                    mma_f16_16x8x16(sum, a[u][0].x, a[u][1].x, a[u][0].y, a[u][1].y, h.x, h.y);
-                    mma_f16_16x8x16(sum, a[u][0].z, a[u][1].z, a[u][0].w, a[u][1].w, h.z, h.w);
+                if (k < k64) {
 #pragma unroll
-                    for (int i = 0; i < 4; i++) acc[i] = __fadd_rn(acc[i], sum[i]);
+                    for (int i = 0; i < 2; i++) {
+                        const uint4 h = *reinterpret_cast<const uint4 *>(bh + k * 128 + i * 16), l = *reinterpret_cast<const uint4 *>(bl + k * 128 + i * 16);
+                        const uint4 &p = a[u][0][i], &q = a[u][1][i];
+                        float sum[4] = {0.f, 0.f, 0.f, 0.f};   // the products' own accumulation truncates: 32 terms at a time, rounded sums beyond
+                        mma_f16_16x8x16(sum, p.x, q.x, p.y, q.y, l.x, l.y);
+                        mma_f16_16x8x16(sum, p.z, q.z, p.w, q.w, l.z, l.w);
+                        mma_f16_16x8x16(sum, p.x, q.x, p.y, q.y, h.x, h.y);
+                        mma_f16_16x8x16(sum, p.z, q.z, p.w, q.w, h.z, h.w);
+#pragma unroll
+                        for (int e = 0; e < 4; e++) acc[e] = __fadd_rn(acc[e], sum[e]);
+                    }
                 }
                 request(a[u]);
                 if (++s == steps) {   // the tile is complete: add the warps' partials
@@ -238,14 +247,8 @@ int launch_f16w_matmul(inkq_ctx *ctx, const F16W *w, const float *x, int M, floa
     ExtraDst extra = {};
     if (extra_in != nullptr) extra = *extra_in;
     const int grid = min((w->rows + 7) / 8, ctx->num_sms * 8);
-    if (M == 1) {
-        const size_t smem = static_cast<size_t>(w->K) * sizeof(float);
-        if (smem > 48 * 1024) cudaFuncSetAttribute(k_f16w_gemv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        k_f16w_gemv<1><<<grid, 256, smem, ctx->stream>>>(w->w, x, 0, M, w->rows, w->K, C, ldc, extra);
-        return after_launch(ctx, "k_f16w_gemv");
-    }
     const size_t rows_smem = static_cast<size_t>(2 * F16R_COLS) * f16r_pitch(w->K) + sizeof(float) * (2 * F16R_WARPS * F16R_COLS * 16 + F16R_COLS);
-    if (w->K % 32 == 0 && rows_smem <= 226 * 1024) {
+    if (w->K % 64 == 0 && rows_smem <= 226 * 1024) {
         INKQ_CUDA(ctx, cudaFuncSetAttribute(k_f16w_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(rows_smem)));
         const int tiles = (w->rows + 15) / 16;
         for (int m0 = 0; m0 < M; m0 += F16R_COLS) {
@@ -257,7 +260,13 @@ int launch_f16w_matmul(inkq_ctx *ctx, const F16W *w, const float *x, int M, floa
         }
         return INKQ_OK;
     }
-    // other row lengths: four rows per pass on the CUDA cores
+    // other row lengths: one or four rows per pass on the CUDA cores
+    if (M == 1) {
+        const size_t smem = static_cast<size_t>(w->K) * sizeof(float);
+        if (smem > 48 * 1024) cudaFuncSetAttribute(k_f16w_gemv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        k_f16w_gemv<1><<<grid, 256, smem, ctx->stream>>>(w->w, x, 0, M, w->rows, w->K, C, ldc, extra);
+        return after_launch(ctx, "k_f16w_gemv");
+    }
     const size_t smem = 4 * static_cast<size_t>(w->K) * sizeof(float);
     if (smem > 200 * 1024) return fail(ctx, INKQ_ERR_UNSUPPORTED, "K too large for the fp16-weight matmul");
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_f16w_gemv<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));

@@ -261,13 +261,6 @@ __device__ __forceinline__ uint4 ldg_stream_v4(const void *p)
     asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
-// The same for rows that are read in 64-byte pieces: the request brings the 256 bytes around it into L2
-__device__ __forceinline__ uint4 ldg_stream_v4_l2(const void *p)
-{
-    uint4 v;
-    asm("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
 // 32 contiguous bytes in one request (256-bit load; p must be 32-byte aligned): a whole sector per lane
 __device__ __forceinline__ void ldg_stream_v8(const void *p, uint4 &lo, uint4 &hi)
 {

@@ -308,7 +308,8 @@ def test_weight_only_w41_dequantisation_bits(pkg, gpu, oracle):
 
 @pytest.mark.parametrize("M,N,K", [(1, 1000, 4096), (1, 16, 64), (5, 264, 512),
                                    # warp-level products: one and two passes of rows, ragged row tiles, more and fewer K steps than warps x depth
-                                   (2, 1000, 4096), (8, 2408, 2560), (9, 40, 5120), (15, 24, 32), (3, 2400, 544), (4, 72, 40)])
+                                   (2, 1000, 4096), (8, 2408, 2560), (9, 40, 5120), (15, 24, 32), (3, 2400, 544), (4, 72, 40),
+                                   (3, 1000, 4160), (1, 24, 544)])
 def test_lm_head_f16(pkg, gpu, oracle, M, N, K):
     import torch
     w16 = pkg.synth.lm_head(N, K, 6)
