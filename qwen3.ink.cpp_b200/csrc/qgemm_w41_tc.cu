@@ -7,35 +7,44 @@
 //   w16[n][k] = fp16(q[n][k] * d[n][k/32] + m[n][k/32])      (one rounding: a half-precision fma)
 //   C[m][n]   = sum_k a16[m][k] * w16[n][k]                   (fp32 accumulate)
 // Unlike the A8W4 schemes there is no per-block epilogue: the whole K extent accumulates inside
-// tensor memory and the CUDA cores only dequantise (2.1 instructions per weight, once per tile)
-// and store the finished tile, so this kernel is bound by the tensor pipe / shared-memory
-// operand bandwidth, not by the epilogue.
+// tensor memory and the CUDA cores only dequantise (1.75 instructions per weight, once per tile of columns)
+// and store the finished tile.
 //
-// "Swap-AB" like the int8 kernel: the 128 weight rows of a tile are the UMMA M side (TMEM lanes),
-// block_m = 16..192 activation rows (a multiple of 16, chosen on the host) the UMMA N side (TMEM
-// columns).  One stage = one pair of quantization blocks = 64 K-elements = four K=16 MMAs.
+// "Swap-AB": the 128 weight rows of a tile are the UMMA M side (TMEM lanes), block_m = 16..256 activation rows
+// the UMMA N side.  One stage = one pair of quantization blocks = 64 K-elements = four K=16 MMAs per weight tile.
+// The dequantised weights go from registers straight into tensor memory and are the MMA's A operand there: with A in
+// shared memory (16 KB written and read again per stage and tile) the shared-memory port was as busy as the tensor pipe.
+// What bounds it: up to ~100 columns the dequantising warps (~740 cycles per stage of two weight tiles: fp16 and ALU pipes at half
+// rate, plus waiting, storing and handing over), above the tensor pipe.  Measured at K = 4096 (before: A in shared memory, 8
+// dequantising warps): 12288 rows x 17 columns 29 -> 22 us, x 64 31 -> 22, x 322 53 -> 33, x 2048 178 -> 157 (1.31 PFLOP/s); 4096 x
+// 322 33 -> 22; 24576 x 512 123 -> 78.  Slower: one chunk per thread and turn (+15 %), the stores of a stage completing under the
+// next one's arithmetic (+5 %: one slot less), two stages per copy (+10 %).
 //
-// Persistent, warp-specialised, one CTA per SM, 512 threads:
-//   warp 0       TMA producer: per stage one tiled 2-D copy of the fp16 activations
+// Persistent, warp-specialised, one CTA per SM, 768 threads:
+//   warps 0, 3   TMA producers (activations; weights): per stage one tiled 2-D copy of the fp16 activations
 //                [block_m rows][64 halves = 128 B] (128-byte swizzle, rows beyond M zero-filled)
-//                and two untiled bulk copies: the pair's packed nibbles (4096 B) and its fp16
+//                and per weight tile two untiled bulk copies: the pair's packed nibbles (4096 B) and its fp16
 //                scales {d_lo, d_hi, m_lo, m_hi} per row (1024 B)
-//   warp 1       MMA issuer (one elected thread), commits free the stages
+//   warp 1       MMA issuer (one elected thread); one commit per stage frees its shared memory and its weights' columns
 //   warp 2       tensor-memory allocation / release
-//   warps 4-11   dequantise: thread = (row, low or high nibble block): 32 nibbles -> 32 halves with
-//                prmt (nibble -> 1024+q as fp16 bits), sub.f16x2, fma.rn.f16x2, written in the
-//                canonical no-swizzle K-major core-matrix layout (conflict-free on both sides)
-//   warps 12-15  epilogue: tcgen05.ld of the finished fp32 tile, coalesced stores of C
-// One ring of stages for all roles (raw operands + dequantised weights per stage), released by one tcgen05.commit
-// per stage (back-to-back MMAs with a commit after every one or two run 2-3x slower than with one commit per 4-16;
-// measured: 363 / 208 / 128 / 70 cycles per 128x112x32 MMA with 1 / 2 / 4 / 16 MMAs per commit).
-// Every mbarrier wait is bounded; on expiry the kernel sets a device flag and all roles drain.
+//   warps 4-19   dequantise: a thread takes one 16-byte chunk of a row = 16 weights of both blocks: byte pairs spread by
+//                prmt, nibble -> 1024 + q as fp16 bits, minus 1024, fma.rn.f16x2 (one rounding of q*d + m), tcgen05.st.
+//                Two chunks per turn: of two weight tiles every other stage, of one every fourth
+//   warps 20-23  epilogue: tcgen05.ld of the finished fp32 tile, coalesced stores of C; the dequantising warps
+//                help with a CTA's last tile
+// Rings: as many raw stages as fit into shared memory, up to four slots of dequantised weights and one or two accumulators
+// in tensor memory, whichever the tile's width leaves room for.
+// Every mbarrier wait is bounded: when one runs out the kernel sets a device flag, every later wait returns at once, all
+// loops run to their end inside their buffers and the host reports INKQ_ERR_TIMEOUT with the context usable.
 //
 // Algorithmic work per launch: 2*M*N*K flop; bytes: N*K*0.625 weights + M*K*2 activations (re-read
 // from L2 once per weight tile) + M*N*4 output.
 #include <cuda.h>
 #include <cuda_fp16.h>
-#include <stdlib.h>
+
+#include <math.h>
+
+#include <mutex>
 
 #include "inkq_internal.h"
 #include "ptx.cuh"
@@ -43,27 +52,33 @@
 namespace inkq {
 
 namespace w41 {
-constexpr int THREADS = 512;
-constexpr int DEQ_WARPS = 8, EPI_WARPS = 4;
+constexpr int DEQ_WARPS = 16, EPI_WARPS = 4, THREADS = 32 * (4 + DEQ_WARPS + EPI_WARPS);
 constexpr int RAW_W_BYTES = TILE_N * 32;                // packed nibbles of one (tile, pair): 4096
 constexpr int RAW_S_BYTES = TILE_N * 8;                 // its fp16 scales: 1024
-constexpr int U16_TILE_BYTES = TILE_N * 64 * 2;         // one dequantised (tile, pair): 16384
-constexpr int ACC_COLS = 256;                          // TMEM columns of one accumulator (block_m <= 256)
-// NT = weight tiles (of 128 rows) a CTA multiplies with one activation stage.  NT = 2 halves the activation bytes
-// fetched from L2 per output (the limiter of the NT = 1 kernel) at the price of a single accumulator slot:
-//   NT = 1: block_m <= 192, 4 stages, two accumulator slots of 256 columns (epilogue overlaps the next tile)
-//   NT = 2: block_m <= 256, 3 stages, one slot: tile 0 in columns [0, 256), tile 1 in [256, 512)
-template <int NT>
-struct Cfg {
-    static constexpr int MAX_BLOCK_M = (NT == 1) ? 192 : 256;
-    static constexpr int RAW_A_BYTES = MAX_BLOCK_M * 128;
-    static constexpr int RAW_STAGE_BYTES = ((RAW_A_BYTES + NT * (RAW_W_BYTES + RAW_S_BYTES)) + 1023) / 1024 * 1024;
-    static constexpr int STAGES = (NT == 1) ? 4 : 3;
-    static constexpr int U16_STAGE_BYTES = NT * U16_TILE_BYTES;
-    static constexpr int ACC_STAGES = (NT == 1) ? 2 : 1;
-    static constexpr int SMEM_BYTES = 1024 /*align slack*/ + STAGES * (RAW_STAGE_BYTES + U16_STAGE_BYTES) + 256 /*barriers*/;
-    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+constexpr int A_COLS = 32;                              // tensor-memory columns of one dequantised (tile, pair): 64 halves per lane
+constexpr int MAX_STAGES = 12, MAX_A_SLOTS = 4, MAX_ACC_SLOTS = 2;
+constexpr int DONE_RING = 16;                           // "the MMAs of pair g have completed", indexed by g % DONE_RING
+static_assert(MAX_STAGES < DONE_RING && MAX_A_SLOTS < DONE_RING, "rings");
+constexpr int BAR_BYTES = 512, SMEM_BYTES = 226 * 1024;
+
+// Weight tiles (of 128 rows) a CTA multiplies with one activation stage, and the activation rows of a stage.  Two weight
+// tiles halve the activation bytes fetched from L2 per output.
+struct Shape {
+    int nt, block_m;
+    constexpr int raw_bytes() const { return block_m * 128 + nt * (RAW_W_BYTES + RAW_S_BYTES); }
+    constexpr int stages() const
+    {
+        const int fit = (SMEM_BYTES - 1024 - BAR_BYTES) / raw_bytes();
+        return fit < MAX_STAGES ? fit : MAX_STAGES;
+    }
+    constexpr int acc_slots() const { return 2 * nt * block_m + 3 * nt * A_COLS <= 512 ? 2 : 1; }
+    constexpr int a_slots() const
+    {
+        const int fit = (512 - acc_slots() * nt * block_m) / (nt * A_COLS);
+        return fit < MAX_A_SLOTS ? fit / 2 * 2 : MAX_A_SLOTS;
+    }
 };
+static_assert(Shape{2, 192}.a_slots() >= 2 && Shape{1, 256}.a_slots() >= 2 && Shape{1, 256}.stages() >= 2 && Shape{2, 192}.stages() >= 3, "shapes");
 
 struct Params {
     const uint8_t *nibT;
@@ -71,68 +86,100 @@ struct Params {
     float *C;
     int *flag;
     int M, rows, pairs, tiles_n, groups_n, tiles_m, block_m, ldc;   // groups_n = ceil(tiles_n / NT)
+    int stages, raw_bytes, a_slots, acc_slots;
 };
 
 struct Ring {
-    uint32_t idx = 0, phase = 0;
-    int n;
-    __device__ explicit Ring(int n_) : n(n_) {}
-    __device__ void advance()
+    uint32_t idx = 0, phase = 0, n;
+    __device__ explicit Ring(uint32_t n_) : n(n_) {}
+    __device__ __forceinline__ void advance()
     {
-        if (++idx == static_cast<uint32_t>(n)) {
+        if (++idx == n) {
             idx = 0;
             phase ^= 1;
         }
     }
 };
 
-// Four nibbles (one per byte of v, already masked) -> four halves q*d + m, as two packed pairs.
-__device__ __forceinline__ void dequant4(uint32_t v, __half2 d2, __half2 m2, uint32_t &out01, uint32_t &out23)
+// Bounded wait; always returns (after an abort the roles finish their loops without waiting).  The probe suspends the thread in
+// hardware: probing in a loop, the roles that wait take issue slots from the dequantising warps (one more such warp: +10 %).
+__device__ __forceinline__ void wait_bounded(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *dev_flag)
 {
-    // byte b -> fp16 bits 0x6400 | b = 1024 + b exactly; subtracting 1024 leaves b exactly
-    const uint32_t h01 = __byte_perm(v, 0x64646464u, 0x4140);
-    const uint32_t h23 = __byte_perm(v, 0x64646464u, 0x4342);
-    const __half2 k1024 = __half2half2(__ushort_as_half(0x6400));
-    const __half2 q01 = __hsub2(*reinterpret_cast<const __half2 *>(&h01), k1024);
-    const __half2 q23 = __hsub2(*reinterpret_cast<const __half2 *>(&h23), k1024);
-    const __half2 w01 = __hfma2(q01, d2, m2);
-    const __half2 w23 = __hfma2(q23, d2, m2);
-    out01 = *reinterpret_cast<const uint32_t *>(&w01);
-    out23 = *reinterpret_cast<const uint32_t *>(&w23);
+    if (mbar_try_wait(bar, parity)) return;
+    const long long t0 = clock64();
+#pragma unroll 1
+    while (!mbar_try_wait_for(bar, parity, 10000u)) {
+        if (*abort_flag != 0) return;
+        if (clock64() - t0 > INKQ_SPIN_LIMIT_CYCLES) {
+            *abort_flag = 1;
+            atomicExch(dev_flag, 1);
+            return;
+        }
+    }
+}
+
+__device__ __forceinline__ uint32_t bits(__half2 h) { return *reinterpret_cast<const uint32_t *>(&h); }
+__device__ __forceinline__ __half2 halves(uint32_t b) { return *reinterpret_cast<const __half2 *>(&b); }
+
+// Four bytes (elements 4i .. 4i + 3 of both blocks of a pair) -> q*d + m of the low and of the high nibbles
+__device__ __forceinline__ void dequant4(uint32_t v, __half2 d_lo, __half2 m_lo, __half2 d_hi, __half2 m_hi, uint32_t *lo, uint32_t *hi)
+{
+    const __half2 k1024 = halves(0x64006400u), k16th = halves(0x2C002C00u), k64 = halves(0xD400D400u);   // 1024, 1/16, -64
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const uint32_t p = __byte_perm(v, 0u, i ? 0x4342 : 0x4140);                     // two bytes, 16 bits apart
+        // fp16 bits 0x6400 | b = 1024 + b exactly: 1024 + q, and 1024 + 16 q whose sixteenth minus 64 is q; all exact
+        const __half2 ql = __hsub2(halves((p & 0x000F000Fu) | 0x64006400u), k1024);
+        const __half2 qh = __hfma2(halves((p & 0x00F000F0u) | 0x64006400u), k16th, k64);
+        lo[i] = bits(__hfma2(ql, d_lo, m_lo));
+        hi[i] = bits(__hfma2(qh, d_hi, m_hi));
+    }
+}
+
+// Worker `who` of `workers` warps of a lane quadrant stores its 16-column chunks of the tile at tensor-memory column `col`.
+__device__ __forceinline__ void store_tile(const Params &prm, uint32_t col, int n, int m0, int quad, int who, int workers)
+{
+    for (int c0 = who * 16; c0 < prm.block_m; c0 += workers * 16) {
+        uint32_t v[16];
+        tmem_ld_x16(col + (static_cast<uint32_t>(quad * 32) << 16) + c0, v);
+        tmem_ld_wait();
+        if (n < prm.rows) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const int m = m0 + c0 + j;
+                if (m < prm.M) prm.C[static_cast<size_t>(m) * prm.ldc + n] = __uint_as_float(v[j]);
+            }
+        }
+    }
 }
 
 template <int NT>
 __global__ void __launch_bounds__(THREADS, 1) k_gemm_w41_tc(const __grid_constant__ CUtensorMap map_a, const Params prm)
 {
-    constexpr int STAGES = Cfg<NT>::STAGES, RAW_STAGE_BYTES = Cfg<NT>::RAW_STAGE_BYTES, RAW_A_BYTES = Cfg<NT>::RAW_A_BYTES;
-    constexpr int U16_STAGE_BYTES = Cfg<NT>::U16_STAGE_BYTES, ACC_STAGES = Cfg<NT>::ACC_STAGES;
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
     unsigned char *smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
-    unsigned char *raw_base = smem;
-    unsigned char *u16_base = raw_base + STAGES * RAW_STAGE_BYTES;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(u16_base + STAGES * U16_STAGE_BYTES);
-    // per stage: raw_full (TMA bytes landed), u16_full (dequantised), consumed (raw operands read by the
-    // dequantisers AND every MMA of the stage complete: the stage's two halves are free together)
-    uint64_t *raw_full = bars, *u16_full = raw_full + STAGES, *consumed = u16_full + STAGES;
-    uint64_t *acc_full = consumed + STAGES, *acc_empty = acc_full + ACC_STAGES;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + ACC_STAGES);
+    uint64_t *raw_full = reinterpret_cast<uint64_t *>(smem + prm.stages * prm.raw_bytes);   // TMA bytes landed
+    uint64_t *done = raw_full + MAX_STAGES, *a_full = done + DONE_RING;                     // a_full: dequantised
+    uint64_t *acc_full = a_full + MAX_A_SLOTS, *acc_empty = acc_full + MAX_ACC_SLOTS, *drain = acc_empty + MAX_ACC_SLOTS;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int total_tiles = prm.groups_n * prm.tiles_m;   // work items: (group of NT weight tiles, activation tile)
+    const int total = prm.groups_n * prm.tiles_m;   // work items: (group of NT weight tiles, activation tile)
+    const int q_bytes = prm.block_m * 128, w_off = q_bytes, s_off = w_off + NT * RAW_W_BYTES;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < STAGES; i++) {
-            mbar_init(&raw_full[i], 1);
-            mbar_init(&u16_full[i], DEQ_WARPS * 32);
-            mbar_init(&consumed[i], DEQ_WARPS + 1);  // the dequantising warps + the MMA commit
-        }
-        for (int i = 0; i < ACC_STAGES; i++) {
+        for (int i = 0; i < prm.stages; i++) mbar_init(&raw_full[i], 2);
+        for (int i = 0; i < DONE_RING; i++) mbar_init(&done[i], 1);
+        for (int i = 0; i < prm.a_slots; i++) mbar_init(&a_full[i], DEQ_WARPS / (NT == 2 ? 2 : 4));
+        for (int i = 0; i < prm.acc_slots; i++) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], EPI_WARPS);
+            mbar_init(&acc_empty[i], prm.acc_slots == 1 ? DEQ_WARPS + EPI_WARPS : EPI_WARPS);
         }
+        mbar_init(drain, 1);
         *abort_flag = 0;
         mbar_fence_init();
+        tma_prefetch_desc(&map_a);
     }
     if (warp == 2) {
         tmem_alloc(tmem_slot, 512);
@@ -141,163 +188,162 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm_w41_tc(const __grid_constan
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = *tmem_slot, tmem_a = tmem_base + prm.acc_slots * NT * prm.block_m;
+    // Launched with programmatic stream serialization: everything above may overlap the tail of the kernel before this one
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-#define INKQ_GIVE_UP()            \
-    {                             \
-        *abort_flag = 1;          \
-        atomicExch(prm.flag, 1);  \
-        dead = true;              \
-        break;                    \
-    }
-
-    if (warp == 0) {
-        // ------------------------------ TMA producer ------------------------------
-        if (lane == 0) {
-            tma_prefetch_desc(&map_a);
-            Ring raw(STAGES);
-            bool dead = false;
-            for (int tile = blockIdx.x; tile < total_tiles && !dead; tile += gridDim.x) {
+    if (warp == 0 || warp == 3) {
+        // ------------------------------ TMA producers: activations, weights ------------------------------
+        if (elect_one()) {
+            Ring raw(prm.stages);
+            uint32_t g = 0;   // stages issued so far, over all tiles of this CTA
+            for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
                 const int tg = tile / prm.tiles_m, tm = tile % prm.tiles_m;
                 const int nvalid = min(NT, prm.tiles_n - tg * NT);   // weight tiles of this group that exist
-                const uint32_t tx = static_cast<uint32_t>(prm.block_m) * 128u + nvalid * (RAW_W_BYTES + RAW_S_BYTES);
-                for (int p = 0; p < prm.pairs; p++) {
-                    if (!mbar_wait_abortable(abort_flag, &consumed[raw.idx], raw.phase ^ 1, 500u)) INKQ_GIVE_UP();
-                    unsigned char *st = raw_base + raw.idx * RAW_STAGE_BYTES;
-                    mbar_arrive_expect_tx(&raw_full[raw.idx], tx);
-                    tma_tensor2d_g2s(st, &map_a, p * 64, tm * prm.block_m, &raw_full[raw.idx]);
-                    for (int wt = 0; wt < nvalid; wt++) {
-                        const size_t slab = static_cast<size_t>(tg * NT + wt) * prm.pairs + p;
-                        tma_bulk_g2s(st + RAW_A_BYTES + wt * RAW_W_BYTES, prm.nibT + slab * RAW_W_BYTES, RAW_W_BYTES, &raw_full[raw.idx]);
-                        tma_bulk_g2s(st + RAW_A_BYTES + NT * RAW_W_BYTES + wt * RAW_S_BYTES,
-                                     reinterpret_cast<const unsigned char *>(prm.sc16) + slab * RAW_S_BYTES, RAW_S_BYTES, &raw_full[raw.idx]);
+                for (int p = 0; p < prm.pairs; p++, g++) {
+                    if (g >= static_cast<uint32_t>(prm.stages)) {   // the slot last held stage g - stages: free once its MMAs have completed
+                        const uint32_t h = g - prm.stages;
+                        wait_bounded(&done[h % DONE_RING], (h / DONE_RING) & 1u, abort_flag, prm.flag);
+                    }
+                    unsigned char *st = smem + raw.idx * prm.raw_bytes;
+                    uint64_t *bar = &raw_full[raw.idx];
+                    if (warp == 0) {
+                        mbar_arrive_expect_tx(bar, q_bytes);
+                        tma_tensor2d_g2s(st, &map_a, p * 64, tm * prm.block_m, bar);
+                    } else {
+                        mbar_arrive_expect_tx(bar, nvalid * (RAW_W_BYTES + RAW_S_BYTES));
+                        for (int wt = 0; wt < nvalid; wt++) {
+                            const size_t slab = static_cast<size_t>(tg * NT + wt) * prm.pairs + p;
+                            tma_bulk_g2s(st + w_off + wt * RAW_W_BYTES, prm.nibT + slab * RAW_W_BYTES, RAW_W_BYTES, bar);
+                            tma_bulk_g2s(st + s_off + wt * RAW_S_BYTES, reinterpret_cast<const unsigned char *>(prm.sc16) + slab * RAW_S_BYTES, RAW_S_BYTES, bar);
+                        }
                     }
                     raw.advance();
                 }
+            }
+            if (*abort_flag != 0) {   // copies nobody consumed may still be in flight: wait (bounded) for each stage's last fill
+                for (uint32_t s = 0; s < static_cast<uint32_t>(prm.stages) && s < g; s++) mbar_wait_drain(&raw_full[s], s < raw.idx ? raw.phase : raw.phase ^ 1);
             }
         }
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc_f16(TILE_N, prm.block_m);
-            Ring raw(STAGES), acc(ACC_STAGES);
-            bool dead = false;
-            for (int tile = blockIdx.x; tile < total_tiles && !dead; tile += gridDim.x) {
+            Ring raw(prm.stages), as(prm.a_slots), acc(prm.acc_slots);
+            uint32_t g = 0;
+            for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
                 const int nvalid = min(NT, prm.tiles_n - (tile / prm.tiles_m) * NT);
-                if (!mbar_wait_abortable(abort_flag, &acc_empty[acc.idx], acc.phase ^ 1, 0u)) INKQ_GIVE_UP();
-                tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + ((NT == 1) ? acc.idx * ACC_COLS : 0);
-                for (int p = 0; p < prm.pairs; p++) {
-                    if (!mbar_wait_abortable(abort_flag, &raw_full[raw.idx], raw.phase, 0u)) INKQ_GIVE_UP();
-                    if (!mbar_wait_abortable(abort_flag, &u16_full[raw.idx], raw.phase, 0u)) INKQ_GIVE_UP();
+                wait_bounded(&acc_empty[acc.idx], acc.phase ^ 1, abort_flag, prm.flag);
+                const uint32_t d = tmem_base + acc.idx * NT * prm.block_m;
+                for (int p = 0; p < prm.pairs; p++, g++) {
+                    wait_bounded(&raw_full[raw.idx], raw.phase, abort_flag, prm.flag);
+                    wait_bounded(&a_full[as.idx], as.phase, abort_flag, prm.flag);
                     tc_fence_after_sync();
-                    // A: dequantised weights, no swizzle: element (row r, k) at (k / 8) * 2048 + r * 16 + (k % 8) * 2:
-                    //    K-adjacent 8x8 core matrices 2048 B apart (leading offset), 8-row groups 128 B apart (stride
-                    //    offset); the j-th K=16 slice starts 4096 B further.
-                    // B: activations, 128-byte swizzled rows of 64 halves; slice j is the j-th 32-byte part of the
-                    //    row; 8-row groups are 1024 B apart.  The start-address field counts 16-byte units.
-                    const uint64_t a_desc0 = umma_smem_desc(smem_u32(u16_base + raw.idx * U16_STAGE_BYTES), 2048, 128, 0);
-                    const uint64_t b_desc0 = umma_smem_desc(smem_u32(raw_base + raw.idx * RAW_STAGE_BYTES), 16, 1024, 2);
+                    // A: lane = weight row, eight columns (16 halves) per MMA.  B: activations, 128-byte swizzled rows of 64
+                    // halves; slice j is the j-th 32-byte part of the row; 8-row groups are 1024 B apart.  The
+                    // start-address field counts 16-byte units.
+                    const uint64_t b0 = umma_smem_desc(smem_u32(smem + raw.idx * prm.raw_bytes), 16, 1024, 2);
+                    const uint32_t a0 = tmem_a + as.idx * NT * A_COLS;
 #pragma unroll
-                    for (int wt = 0; wt < NT; wt++) {
-                        if (wt < nvalid) {
+                    for (int j = 0; j < 4; j++)
 #pragma unroll
-                            for (int j = 0; j < 4; j++)
-                                umma_f16(d_tmem + wt * ACC_COLS, a_desc0 + static_cast<uint64_t>((wt * U16_TILE_BYTES + j * 4096) >> 4),
-                                         b_desc0 + static_cast<uint64_t>(j * (32 >> 4)), idesc, (p > 0 || j > 0) ? 1u : 0u);
-                        }
-                    }
-                    umma_commit(&consumed[raw.idx]);   // the only commit of the stage
+                        for (int wt = 0; wt < NT; wt++)
+                            if (wt < nvalid)
+                                umma_f16_ts(d + wt * prm.block_m, a0 + wt * A_COLS + j * 8, b0 + static_cast<uint64_t>(j * 2), idesc, (p > 0 || j > 0) ? 1u : 0u);
+                    umma_commit(&done[g % DONE_RING]);   // the only commit of the pair
                     raw.advance();
+                    as.advance();
                 }
-                if (dead) break;
                 umma_commit(&acc_full[acc.idx]);
                 acc.advance();
             }
+            umma_commit(drain);   // every MMA has completed before tensor memory is released
+            mbar_wait_drain(drain, 0u);
         }
         __syncwarp();
-    } else if (warp >= 4 && warp < 4 + DEQ_WARPS) {
-        // ------------------------------ dequantise ------------------------------
-        const int t = threadIdx.x - 128;
-        const int r = t & 127;          // weight row inside the tile (32 consecutive rows per warp)
-        const int hi = t >> 7;          // 0: low nibbles = block 2p (k 0..31), 1: high nibbles = block 2p+1 (k 32..63)
-        const int swz = (r >> 2) & 1;   // chunk swizzle of the packed layout
-        Ring raw(STAGES);
-        bool dead = false;
-        for (int tile = blockIdx.x; tile < total_tiles && !dead; tile += gridDim.x) {
-            const int nvalid = min(NT, prm.tiles_n - (tile / prm.tiles_m) * NT);
-            for (int p = 0; p < prm.pairs; p++) {
-                // fresh operands in the stage imply that its previous round is consumed (the producer refills a stage
-                // only then), so the dequantised half of the stage is free as well
-                if (!mbar_wait_abortable(abort_flag, &raw_full[raw.idx], raw.phase, 100u)) INKQ_GIVE_UP();
-#pragma unroll
-                for (int wt = 0; wt < NT; wt++) {
-                if (wt >= nvalid) continue;
-                const unsigned char *wsrc = raw_base + raw.idx * RAW_STAGE_BYTES + RAW_A_BYTES + wt * RAW_W_BYTES;
-                const unsigned char *ssrc = raw_base + raw.idx * RAW_STAGE_BYTES + RAW_A_BYTES + NT * RAW_W_BYTES + wt * RAW_S_BYTES;
-                unsigned char *stage = u16_base + raw.idx * U16_STAGE_BYTES + wt * U16_TILE_BYTES;
-                unsigned char *dst = stage + (4 * hi) * 2048 + r * 16;
-                const uint2 sc = *reinterpret_cast<const uint2 *>(ssrc + r * 8);   // {d_lo, d_hi | m_lo, m_hi}
-                const uint32_t dbits = hi ? (sc.x >> 16) : (sc.x & 0xFFFFu), mbits = hi ? (sc.y >> 16) : (sc.y & 0xFFFFu);
-                const __half2 d2 = __half2half2(__ushort_as_half(static_cast<unsigned short>(dbits)));
-                const __half2 m2 = __half2half2(__ushort_as_half(static_cast<unsigned short>(mbits)));
-#pragma unroll
-                for (int c = 0; c < 2; c++) {   // logical 16-byte chunk c holds elements 16c..16c+15 of both blocks
-                    const uint4 v = *reinterpret_cast<const uint4 *>(wsrc + r * 32 + ((c ^ swz) * 16));
-                    const uint32_t in[4] = {v.x, v.y, v.z, v.w};
-                    uint32_t o[8];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const uint32_t nib = (hi ? (in[i] >> 4) : in[i]) & 0x0F0F0F0Fu;
-                        dequant4(nib, d2, m2, o[2 * i], o[2 * i + 1]);
-                    }
-                    // elements 16c..16c+7 -> core matrix 2c, 16c+8..16c+15 -> core matrix 2c+1 of this block's four
-                    *reinterpret_cast<uint4 *>(dst + (2 * c) * 2048) = make_uint4(o[0], o[1], o[2], o[3]);
-                    *reinterpret_cast<uint4 *>(dst + (2 * c + 1) * 2048) = make_uint4(o[4], o[5], o[6], o[7]);
-                }
-                }   // weight tiles of the group
-                fence_proxy_async_smem();
-                mbar_arrive(&u16_full[raw.idx]);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&consumed[raw.idx]);
-                raw.advance();
-            }
+    } else if (warp >= 4) {
+        const int quad = warp & 3;                            // TMEM lane quadrant this warp may access
+        const int r = quad * 32 + lane;                       // weight row inside the tile
+        const int sub = (warp - 4) >> 2;                      // 0 .. 3: dequantise, 4: epilogue
+        Ring acc(prm.acc_slots);
+        // Two 16-byte chunks per thread and stage: two weight tiles: the same chunk of both, every other stage; one: both
+        // chunks of a row, every fourth stage.  Fewer and longer turns: waiting, storing and handing over cost as many
+        // instructions as one chunk.
+        constexpr uint32_t STEP = (NT == 2) ? 2u : 4u;
+        const int c = (NT == 2) ? sub & 1 : 0, swz = (r >> 2) & 1;
+        const uint32_t t_row = tmem_a + (static_cast<uint32_t>(quad * 32) << 16) + c * 8;
+        const uint32_t nib0 = w_off + r * 32 + ((c ^ swz) << 4), nib1 = (NT == 2) ? nib0 + RAW_W_BYTES : nib0 ^ 16u, sc0 = s_off + r * 8;
+        const uint32_t mask = prm.a_slots - 1, base = smem_u32(smem);
+        uint32_t g = (NT == 2) ? sub >> 1 : sub, end = 0, idx = g, phase = 0;   // this warp's next stage, over all tiles of the CTA
+        if (idx >= static_cast<uint32_t>(prm.stages)) {
+            idx -= prm.stages;
+            phase = 1;
         }
-    } else if (warp >= 4 + DEQ_WARPS) {
-        // ------------------------------ epilogue ------------------------------
-        const int quad = warp & 3;          // TMEM lane quadrant this warp may read (warps 12..15 -> 0..3)
-        const int row = quad * 32 + lane;
-        Ring acc(ACC_STAGES);
-        bool dead = false;
-        for (int tile = blockIdx.x; tile < total_tiles && !dead; tile += gridDim.x) {
-            const int tg = tile / prm.tiles_m, tm = tile % prm.tiles_m;
-            const int nvalid = min(NT, prm.tiles_n - tg * NT);
-            if (!mbar_wait_abortable(abort_flag, &acc_full[acc.idx], acc.phase, 50u)) INKQ_GIVE_UP();
-            tc_fence_after_sync();
-            for (int wt = 0; wt < nvalid; wt++) {
-                const int n = (tg * NT + wt) * TILE_N + row;
-                const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + ((NT == 1) ? acc.idx * ACC_COLS : wt * ACC_COLS);
-                for (int c0 = 0; c0 < prm.block_m; c0 += 16) {
-                    uint32_t v[16];
-                    tmem_ld_x16(taddr + c0, v);
-                    tmem_ld_wait();
-                    if (n < prm.rows) {
-#pragma unroll
-                        for (int j = 0; j < 16; j++) {
-                            const int m = tm * prm.block_m + c0 + j;
-                            if (m < prm.M) prm.C[static_cast<size_t>(m) * prm.ldc + n] = __uint_as_float(v[j]);
-                        }
-                    }
+        for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
+            end += prm.pairs;
+            // ------------------------------ dequantise ------------------------------
+#pragma unroll 1
+            for (; sub < 4 && g < end; g += STEP) {
+                // A barrier's phase may be waited for only when the one before has completed.  With many stages the turns before
+                // this one have seen to that
+                if (static_cast<uint32_t>(prm.stages) < prm.a_slots + STEP && g >= static_cast<uint32_t>(prm.stages)) {
+                    const uint32_t h = g - prm.stages;
+                    wait_bounded(&done[h % DONE_RING], (h / DONE_RING) & 1u, abort_flag, prm.flag);
                 }
+                wait_bounded(&raw_full[idx], phase, abort_flag, prm.flag);
+                const uint32_t st = base + idx * prm.raw_bytes;
+                idx += STEP;
+                if (idx >= static_cast<uint32_t>(prm.stages)) {
+                    idx -= prm.stages;
+                    phase ^= 1;
+                }
+                const uint4 v[2] = {lds_u32x4(st + nib0), lds_u32x4(st + nib1)};   // a missing tile's bytes are old ones: not used
+                const uint2 sc[2] = {lds_u32x2(st + sc0), lds_u32x2(st + sc0 + (NT == 2 ? RAW_S_BYTES : 0))};   // {d_lo, d_hi | m_lo, m_hi}
+                uint32_t lo[2][8], hi[2][8];
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const __half2 d2 = halves(sc[u].x), m2 = halves(sc[u].y);
+                    const __half2 d_lo = __low2half2(d2), d_hi = __high2half2(d2), m_lo = __low2half2(m2), m_hi = __high2half2(m2);
+                    const uint32_t in[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+                    for (int i = 0; i < 4; i++) dequant4(in[i], d_lo, m_lo, d_hi, m_hi, &lo[u][2 * i], &hi[u][2 * i]);
+                }
+                if (g >= static_cast<uint32_t>(prm.a_slots)) {   // the columns last held stage g - a_slots
+                    const uint32_t h = g - prm.a_slots;
+                    wait_bounded(&done[h % DONE_RING], (h / DONE_RING) & 1u, abort_flag, prm.flag);
+                }
+                tc_fence_after_sync();
+                const uint32_t t = t_row + (g & mask) * (NT * A_COLS);
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    tmem_st_x8(t + u * (NT == 2 ? A_COLS : 8), lo[u]);
+                    tmem_st_x8(t + u * (NT == 2 ? A_COLS : 8) + 16, hi[u]);
+                }
+                tmem_st_wait();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (elect_one()) mbar_arrive(&a_full[g & mask]);
             }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[acc.idx]);
+            // ------------------------------ epilogue ------------------------------
+            // The dequantising warps help with the last tile, and with every tile when the next one's products wait for the stores
+            // (a single accumulator).  Tiles of fewer than four stages: the warps may be further ahead than one phase of acc_full
+            const bool help = prm.acc_slots == 1 || (tile + static_cast<int>(gridDim.x) >= total && prm.pairs >= 4);
+            if (sub == 4 || help) {
+                const int tg = tile / prm.tiles_m, tm = tile % prm.tiles_m;
+                const int nvalid = min(NT, prm.tiles_n - tg * NT);
+                wait_bounded(&acc_full[acc.idx], acc.phase, abort_flag, prm.flag);
+                tc_fence_after_sync();
+                for (int wt = 0; wt < nvalid; wt++)
+                    store_tile(prm, tmem_base + (acc.idx * NT + wt) * prm.block_m, (tg * NT + wt) * TILE_N + r, tm * prm.block_m, quad, help ? sub : 0, help ? 5 : 1);
+                tc_fence_before_sync();
+                __syncwarp();
+                if ((sub == 4 || prm.acc_slots == 1) && elect_one()) mbar_arrive(&acc_empty[acc.idx]);
+            }
             acc.advance();
         }
     }
-#undef INKQ_GIVE_UP
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 2) {
@@ -306,28 +352,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm_w41_tc(const __grid_constan
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-}  // namespace w41
+constexpr int MAX_DEVICES = 64;
 
 template <int NT>
-static int launch_w41(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc)
+static int launch(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc, int block_m)
 {
-    using namespace w41;
-    const int tiles_m = (M + Cfg<NT>::MAX_BLOCK_M - 1) / Cfg<NT>::MAX_BLOCK_M;
-    const int block_m = (((M + tiles_m - 1) / tiles_m) + 15) & ~15;   // even split, multiple of 16
-
+    const Shape sh{NT, block_m};
     CUtensorMap map;
-    const cuuint64_t gdim[2] = {static_cast<cuuint64_t>(w->K), static_cast<cuuint64_t>(M)};
-    const cuuint64_t gstride[1] = {static_cast<cuuint64_t>(w->K) * 2};
-    const cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(block_m)};
-    const cuuint32_t estr[2] = {1u, 1u};
-    CUresult cr = reinterpret_cast<EncodeTiledFn>(ctx->encode_tiled)(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t *>(a16), gdim, gstride,
-                                                                     box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                                                     CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) return fail(ctx, INKQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string(static_cast<int>(cr)));
-
+    int rc = encode_map_2d(ctx, &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a16, w->K, M, 64u, block_m, CU_TENSOR_MAP_SWIZZLE_128B, w->K);
+    if (rc) return rc;
     Params prm;
     prm.nibT = w->nibT;
     prm.sc16 = w->sc16;
@@ -338,30 +371,58 @@ static int launch_w41(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w
     prm.pairs = w->pairs;
     prm.tiles_n = w->tiles;
     prm.groups_n = (w->tiles + NT - 1) / NT;
-    prm.tiles_m = tiles_m;
+    prm.tiles_m = (M + block_m - 1) / block_m;
     prm.block_m = block_m;
     prm.ldc = ldc;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_w41_tc<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<NT>::SMEM_BYTES);
-        if (e != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("cudaFuncSetAttribute(k_gemm_w41_tc): ") + cudaGetErrorString(e));
-        configured = true;
+    prm.stages = sh.stages();
+    prm.raw_bytes = sh.raw_bytes();
+    prm.a_slots = sh.a_slots();
+    prm.acc_slots = sh.acc_slots();
+    // The opt-in for large dynamic shared memory is a per-device function attribute
+    static std::mutex mu;
+    static bool configured[MAX_DEVICES] = {};
+    if (ctx->device < 0 || ctx->device >= MAX_DEVICES) return fail(ctx, INKQ_ERR_UNSUPPORTED, "device index beyond the launch table");
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!configured[ctx->device]) {
+            const cudaError_t e = cudaFuncSetAttribute(k_gemm_w41_tc<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+            if (e != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("cudaFuncSetAttribute(k_gemm_w41_tc): ") + cudaGetErrorString(e));
+            configured[ctx->device] = true;
+        }
     }
     const int total = prm.groups_n * prm.tiles_m;
-    const int grid = total < ctx->num_sms ? total : ctx->num_sms;
-    k_gemm_w41_tc<NT><<<grid, THREADS, Cfg<NT>::SMEM_BYTES, ctx->stream>>>(map, prm);
+    const cudaError_t e = launch_pdl(k_gemm_w41_tc<NT>, dim3(total < ctx->num_sms ? total : ctx->num_sms), dim3(THREADS), SMEM_BYTES, ctx->stream, map, prm);
+    if (e != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("k_gemm_w41_tc launch: ") + cudaGetErrorString(e));
     return after_launch(ctx, "k_gemm_w41_tc");
 }
 
+}  // namespace w41
+
 int launch_gemm_w41_tc(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc)
 {
+    using namespace w41;
     if (ctx->encode_tiled == nullptr) return fail(ctx, INKQ_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled entry point not available");
     if ((reinterpret_cast<uintptr_t>(a16) & 15) != 0) return fail(ctx, INKQ_ERR_INVALID, "the fp16 activations must be 16-byte aligned");
-    // two weight tiles per CTA (half the activation bytes fetched per output: 1.10-1.15 vs 0.89-0.92 PFLOP/s at
-    // M >= 2048, 52 vs 63 us at M = 322) unless that leaves more than half of the SMs without a work item
-    const long long items2 = static_cast<long long>((w->tiles + 1) / 2) * ((M + 255) / 256);
-    const bool two = 2 * items2 >= ctx->num_sms;
-    return two ? launch_w41<2>(ctx, a16, M, w, C, ldc) : launch_w41<1>(ctx, a16, M, w, C, ldc);
+    // The split with the least time: waves x time of a wave (us at K = 4096, measured with one tile on every SM; it is
+    // proportional to K).  Dequantising bounds narrow tiles (one weight tile 18.2, two 28.5), the products wide ones.  Two
+    // weight tiles share the activations, one leaves fewer SMs idle where there are few tiles.
+    Shape best{1, 0};
+    float best_time = 0.f;
+    for (int nt = 1; nt <= 2; nt++) {
+        const int max_m = nt == 1 ? 256 : 192;
+        for (int tm = (M + max_m - 1) / max_m; tm <= (M + 15) / 16; tm++) {
+            const int bm = (((M + tm - 1) / tm) + 15) & ~15;
+            const long long total = static_cast<long long>((w->tiles + nt - 1) / nt) * ((M + bm - 1) / bm);
+            const float wave = nt == 1 ? fmaxf(18.2f, 10.6f + 0.0735f * bm) : fmaxf(28.5f, 18.8f + 0.1205f * bm);
+            const float time = static_cast<float>((total + ctx->num_sms - 1) / ctx->num_sms) * wave;
+            if (best_time == 0.f || time < best_time) {
+                best = Shape{nt, bm};
+                best_time = time;
+            }
+            if (total > 64LL * ctx->num_sms) break;   // many waves already: finer splits only dequantise more often
+        }
+    }
+    return best.nt == 2 ? launch<2>(ctx, a16, M, w, C, ldc, best.block_m) : launch<1>(ctx, a16, M, w, C, ldc, best.block_m);
 }
 
 }  // namespace inkq

@@ -261,7 +261,9 @@ def test_mismatched_quantizer_mode_is_rejected(pkg, gpu, oracle):
                                    (16, 128, 64), (322, 384, 512), (200, 136, 1024), (400, 264, 192),
                                    # enough work items for the two-weight-tiles-per-CTA variant: an odd tile count (the last
                                    # group holds one tile), and two activation tiles of 160 rows
-                                   (16, 297 * 128, 64), (300, 74 * 256, 128)])
+                                   (16, 297 * 128, 64), (300, 74 * 256, 128),
+                                   # one and two weight tiles over several waves, tiles of fewer stages than slots, few stages of 256 rows
+                                   (33, 297 * 128, 64), (17, 72, 192), (300, 19000, 320), (250, 18904, 448), (500, 38000, 128)])
 def test_weight_only_w41(pkg, gpu, oracle, M, N, K):
     """Tensor-core kernel (kind::f16, fp32 accumulation inside tensor memory) and its CUDA-core cross-check against
     the oracle.  The dequantised fp16 weights are identical in all three (one rounding of q*d + m); only the fp32
