@@ -241,19 +241,23 @@ int inkq_ctx_set_stream(inkq_ctx *ctx, void *stream)
     return INKQ_OK;
 }
 
-int inkq_ctx_synchronize(inkq_ctx *ctx)
+// Waits for `stream`.  The time-out word travels to a page-locked host word at its end: one wait covers the work and the flag
+static int finish(inkq_ctx *ctx, cudaStream_t stream)
 {
-    int rc = use(ctx);
-    if (rc) return rc;
-    // the time-out word travels to a page-locked host word at the end of the stream: one wait covers the work and the flag
-    INKQ_CUDA(ctx, cudaMemcpyAsync(ctx->host_flag, ctx->dev_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    INKQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    INKQ_CUDA(ctx, cudaMemcpyAsync(ctx->host_flag, ctx->dev_flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    INKQ_CUDA(ctx, cudaStreamSynchronize(stream));
     const int flag = *static_cast<volatile int *>(ctx->host_flag);
     if (flag != 0) {
         cudaMemset(ctx->dev_flag, 0, sizeof(int));
         return fail(ctx, INKQ_ERR_TIMEOUT, "a bounded device-side wait ran out inside a kernel; its output is invalid");
     }
     return INKQ_OK;
+}
+
+int inkq_ctx_synchronize(inkq_ctx *ctx)
+{
+    const int rc = use(ctx);
+    return rc ? rc : finish(ctx, ctx->stream);
 }
 
 const char *inkq_last_error(const inkq_ctx *ctx)
@@ -682,7 +686,7 @@ int inkq_linear_host(inkq_ctx *ctx, const inkq_weight *w, const float *x_host, i
         // early and then never waits: a window's product is ready before its predecessor's rows have left.
         constexpr int MAXC = 8;
         int m0[MAXC + 1], nch = 0, at = 0;
-        const int lead[3] = {48, 80, 96};
+        const int lead[3] = {32, 80, 112};   // (48, 80, 96: 397 us at M = 322; 16, 32, 64: 381; these: 369)
         m0[0] = 0;
         while (nch < 3 && M - at >= lead[nch] + 32) {
             at += lead[nch];
@@ -712,24 +716,28 @@ int inkq_linear_host(inkq_ctx *ctx, const inkq_weight *w, const float *x_host, i
         INKQ_CUDA(ctx, cudaEventRecord(ctx->start_ev, ctx->stream));
         INKQ_CUDA(ctx, cudaStreamWaitEvent(ctx->h2d_stream, ctx->start_ev, 0));
         INKQ_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_stream, ctx->start_ev, 0));
-        for (int c = 0; c < nch; c++) {
+        auto copy_in = [&](int c) -> int {
             const size_t off = static_cast<size_t>(m0[c]) * w->K, cnt = static_cast<size_t>(m0[c + 1] - m0[c]) * w->K;
             INKQ_CUDA(ctx, cudaMemcpyAsync(ctx->lin_x + off, x_host + off, cnt * sizeof(float), cudaMemcpyHostToDevice, ctx->h2d_stream));
             INKQ_CUDA(ctx, cudaEventRecord(ctx->h2d_ev[c], ctx->h2d_stream));
-        }
+            return INKQ_OK;
+        };
+        // Each call into the driver takes 2-4 us of host time: a window's copy is requested right behind the window before it, not
+        // all copies ahead of the first kernel (M = 322: 407 -> 397 us together with the single wait at the end)
+        if ((rc = copy_in(0))) return rc;
         for (int c = 0; c < nch; c++) {
             const int rows = m0[c + 1] - m0[c];
             INKQ_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->h2d_ev[c], 0));
             if ((rc = launch_quantize_rows(ctx, qmode, ctx->lin_x + static_cast<size_t>(m0[c]) * w->K, m0[c], rows, M, w->K, act))) return rc;
             if ((rc = launch_gemm(ctx, act, w, ctx->lin_c, w->rows, nullptr, nullptr, m0[c], rows))) return rc;
             INKQ_CUDA(ctx, cudaEventRecord(ctx->chunk_ev[c], ctx->stream));
+            if (c + 1 < nch && (rc = copy_in(c + 1))) return rc;
             INKQ_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_stream, ctx->chunk_ev[c], 0));
             INKQ_CUDA(ctx, cudaMemcpy2DAsync(C_host + static_cast<size_t>(m0[c]) * ldc, static_cast<size_t>(ldc) * sizeof(float),
                                              ctx->lin_c + static_cast<size_t>(m0[c]) * w->rows, static_cast<size_t>(w->rows) * sizeof(float),
                                              static_cast<size_t>(w->rows) * sizeof(float), rows, cudaMemcpyDeviceToHost, ctx->copy_stream));
         }
-        INKQ_CUDA(ctx, cudaStreamSynchronize(ctx->copy_stream));
-        return inkq_ctx_synchronize(ctx);
+        return finish(ctx, ctx->copy_stream);   // the last copy waits for the last kernel: one wait covers both streams
     }
     INKQ_CUDA(ctx, cudaMemcpyAsync(ctx->lin_x, x_host, xn * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     if ((rc = inkq_linear(ctx, w, ctx->lin_x, M, ctx->lin_c, w->rows))) return rc;
