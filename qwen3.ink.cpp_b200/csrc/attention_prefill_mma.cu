@@ -58,6 +58,8 @@ __global__ void __launch_bounds__(128) k_attention_prefill_mma(const float *__re
     const int kvh = h / (nq / nkv);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tq = lane & 3;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int pos0 = *pos0_dev;
     const int r0 = t0 + warp * 16 + g, r1 = r0 + 8;                      // this thread's two query rows
     const int lim0 = min(pos0 + min(r0, T - 1), max_pos - 1), lim1 = min(pos0 + min(r1, T - 1), max_pos - 1);   // last visible key
@@ -248,9 +250,8 @@ __global__ void __launch_bounds__(128) k_attention_prefill_mma(const float *__re
 int launch_attention_prefill_mma(inkq_ctx *ctx, const float *q, const uint16_t *k_cache, const uint16_t *v_cache, const int *pos0_dev, int T, int nq,
                                  int nkv, int max_pos, float scale, float *out, const QuantOut &qo, int qrow0)
 {
-    k_attention_prefill_mma<<<dim3((T + AM_ROWS - 1) / AM_ROWS, nq), 128, 0, ctx->stream>>>(q, reinterpret_cast<const __half *>(k_cache),
-                                                                                            reinterpret_cast<const __half *>(v_cache), pos0_dev, T, nq,
-                                                                                            nkv, max_pos, scale, out, qo, qrow0);
+    launch_pdl(k_attention_prefill_mma, dim3((T + AM_ROWS - 1) / AM_ROWS, nq), dim3(128), 0, ctx->stream, q, reinterpret_cast<const __half *>(k_cache),
+               reinterpret_cast<const __half *>(v_cache), pos0_dev, T, nq, nkv, max_pos, scale, out, qo, qrow0);
     return after_launch(ctx, "k_attention_prefill_mma");
 }
 

@@ -79,6 +79,8 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_quant_rows(float *__restric
     __shared__ float red[8];
     const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n4 = dim / 4, nb = dim / QK;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (row >= M) {   // padding rows of the scale planes read as zero
         for (int b = threadIdx.x; b < nb; b += 256) {
             const size_t pl = static_cast<size_t>(b) * M_ld + row;
@@ -811,8 +813,8 @@ int inkq_glue_add_rmsnorm_quant_rows(inkq_ctx *ctx, float *x_dev, const float *d
             configured[ctx->device] = true;
         }
     }
-    k_add_rmsnorm_quant_rows<<<M_ld, 256, smem, ctx->stream>>>(x_dev, delta_dev, norm_w_dev, M, K, eps, M_ld, out_qmode, out->q, out->d, out->s,
-                                                                out->isum, xn_out_dev);
+    launch_pdl(k_add_rmsnorm_quant_rows, dim3(M_ld), dim3(256), smem, ctx->stream, x_dev, delta_dev, norm_w_dev, M, K, eps, M_ld, out_qmode, out->q, out->d,
+               out->s, out->isum, xn_out_dev);
     out->M = M;
     out->M_ld = M_ld;
     out->qmode = out_qmode;
