@@ -18,12 +18,14 @@
 // over K (an output's sum may not be split).  Every warp owns 16 weight rows and all columns: each weight byte is fetched once.
 // Stages of four pairs (256 K-elements) are unrolled, so that the fragment loads and products of one pair overlap the scaling of
 // the one before.  More rows: the register file and the FMA pipe.  Alone in registers, a block's 16 x 8 dots take a scheduler 22
-// cycles with four warps (27 with mins, of which 20 are the packed multiplications, three operands of 64 bits each); the kernel
-// runs at 85 to 92 % of that rate.  The weights are read from L2 once per tile of columns (CTAs of one weight tile are neighbours).
+// cycles with four warps (27 with mins, of which 20 are the packed multiplications, three operands of 64 bits each).  A block's
+// chain (fragment loads, product, conversion, scaling) is long and an SM has few warps in a tile of this size, so stages of 4 to 8
+// pairs are unrolled and one CTA of 8 warps gets up to 255 registers a thread.  The weights are read from L2 once per tile of
+// columns (CTAs of one weight tile are neighbours).
 // Measured (prefetched weights of distinct layers; before: the tcgen05 kernel this one replaced), A81W41: 24576 x 4096 with 5 rows
-// 59 -> 15 us (4.2 TB/s), 4096 x 4096 with 5 rows 37 -> 8.5, 12288 x 4096 with 48 rows 39 -> 25, with 128 rows 72 -> 52, with 322
-// rows 128 -> 117, with 2048 rows 728 -> 644; A80W40 with 322 rows 111 -> 98, with 2048 rows 634 -> 562; A80W4Z 4096 x 12288 with
-// 77 rows 83 -> 57.  Slower: scalar multiplications (+12 %), the conversion by a bias in the product's accumulator operand
+// 59 -> 15.7 us (4.2 TB/s), 4096 x 4096 with 5 rows 37 -> 7.1, 12288 x 4096 with 48 rows 39 -> 21, with 128 rows 72 -> 53, with
+// 322 rows 128 -> 107, with 2048 rows 728 -> 643; A80W40 with 322 rows 111 -> 94, with 2048 rows 634 -> 560; A80W4Z 4096 x 12288
+// with 77 rows 83 -> 42.  Slower: scalar multiplications (+12 %), the conversion by a bias in the product's accumulator operand
 // (+20 %: it has to be moved there), fp16 operands with fp32 accumulators (+25 %) and e4m3 parts (x2).
 //
 // Operands: the weights are the MMA's A side, the activation rows its B side.  A packed byte holds element e of both blocks of
@@ -349,7 +351,7 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
     {
         std::lock_guard<std::mutex> lk(mu);
         if (!configured[ctx->device]) {
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM < SMEM_ONE_CTA ? SMEM_ONE_CTA : G::SMEM);
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SM);
             if (e != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("cudaFuncSetAttribute(k_qgemm_rows): ") + cudaGetErrorString(e));
             configured[ctx->device] = true;
         }
@@ -377,32 +379,42 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
     return after_launch(ctx, "k_qgemm_rows");
 }
 
-// Tiles for more than 32 activation rows: shape, then the time (us) of 1 .. CTAS tiles on every SM at K = 4096, without the
-// ~3 us that a launch takes, with the mins of A81W41 and without them.  Measured with prefetched weights of distinct layers;
-// only the ratios matter, and they hardly depend on K.  Per column the wide tiles cost least (fragments and scales of the weight
-// rows are fetched once for more columns) until the accumulators crowd the 128 registers that two CTAs of 256 threads leave
-// (112 columns of 32-row warps spill a little).  Half-height tiles split a layer with few weight rows over more SMs.
-#define QROWS_TILES(X)                                                                    \
-    X(0, (4, 1, 2, 2, 2, 4), (15.7f, 21.4f, 29.9f, 38.6f), (15.4f, 21.2f, 28.3f, 36.7f)) \
-    X(1, (4, 2, 2, 2, 2, 2), (21.7f, 37.1f), (21.0f, 36.3f))                              \
-    X(2, (4, 2, 2, 3, 2, 2), (27.7f, 48.9f), (26.1f, 45.3f))                              \
-    X(3, (4, 2, 2, 4, 2, 2), (34.6f, 62.5f), (31.7f, 55.8f))                              \
-    X(4, (4, 2, 2, 5, 2, 2), (43.3f, 78.1f), (37.6f, 66.7f))                              \
-    X(5, (4, 2, 2, 7, 2, 2), (72.0f, 122.5f), (55.2f, 94.1f))                             \
-    X(6, (4, 2, 1, 3, 2, 2), (17.9f, 29.8f), (16.3f, 26.5f))                              \
-    X(7, (4, 2, 1, 4, 2, 2), (21.9f, 36.4f), (19.3f, 31.5f))                              \
-    X(8, (4, 2, 1, 6, 2, 2), (28.3f, 50.2f), (25.1f, 42.3f))                              \
-    X(9, (4, 2, 1, 7, 2, 2), (31.7f, 56.8f), (28.2f, 48.7f))
+// Tiles for more than 32 activation rows: shape, then the time (us) of one and of two tiles on every SM at K = 4096, without
+// the ~3 us that a launch takes, with the mins of A81W41 and without them.  Measured with prefetched weights of distinct layers;
+// only the ratios matter, and they hardly depend on K.  One CTA of 8 warps per SM with all the registers it wants and 4 to 8
+// unrolled pairs per stage: the fragment loads and products of several pairs overlap the scaling of the ones before (against two CTAs
+// of 128 registers and two-pair stages: 64 x 48 17.9 -> 14.2, 128 x 112 72 -> 51).  Two such CTAs side by side remain for
+// many tiles per SM, where one's set-up and stores hide behind the other's products.
+// Per column the wide tiles cost least: fragments and scales of the weight rows are fetched once for more columns.
+// Half- and quarter-height tiles split a layer with few weight rows over more SMs.
+#define QROWS_TILES(X)                                         \
+    X(0, (2, 4, 1, 2, 8, 1), (10.4f, 22.7f), (9.8f, 21.4f))    \
+    X(1, (4, 2, 1, 2, 8, 1), (11.2f, 24.2f), (10.4f, 23.0f))   \
+    X(2, (4, 1, 2, 2, 4, 2), (12.0f, 18.5f), (11.6f, 17.5f))   \
+    X(3, (4, 2, 1, 3, 8, 1), (14.2f, 30.3f), (12.5f, 26.6f))   \
+    X(4, (4, 2, 1, 4, 6, 1), (18.2f, 38.6f), (16.7f, 35.6f))   \
+    X(5, (4, 2, 1, 5, 6, 1), (22.0f, 46.4f), (18.6f, 39.4f))   \
+    X(6, (4, 2, 1, 7, 4, 1), (29.6f, 61.7f), (25.4f, 52.8f))   \
+    X(7, (4, 2, 2, 2, 8, 1), (17.9f, 37.0f), (17.2f, 35.6f))   \
+    X(8, (4, 2, 2, 3, 6, 1), (24.4f, 50.6f), (22.4f, 46.4f))   \
+    X(9, (4, 2, 2, 4, 4, 1), (31.9f, 65.7f), (28.4f, 58.7f))   \
+    X(10, (4, 2, 2, 5, 4, 1), (38.2f, 78.3f), (34.0f, 69.8f))  \
+    X(11, (4, 2, 2, 6, 4, 1), (45.0f, 91.8f), (39.8f, 81.0f))  \
+    X(12, (4, 2, 2, 7, 4, 1), (51.1f, 104.2f), (44.6f, 91.1f)) \
+    X(13, (4, 2, 1, 4, 2, 2), (21.9f, 36.4f), (19.3f, 31.5f))  \
+    X(14, (4, 2, 1, 7, 2, 2), (31.7f, 56.8f), (28.2f, 48.7f))  \
+    X(15, (4, 2, 2, 4, 2, 2), (34.6f, 62.5f), (31.7f, 55.8f))  \
+    X(16, (4, 2, 2, 5, 2, 2), (43.3f, 78.1f), (37.6f, 66.7f))
 
 #define QROWS_UNWRAP(...) __VA_ARGS__
 struct TileCost {
-    int rows, cols, ctas;
-    float with_min[4], without[4];
+    int rows, cols;
+    float with_min[2], without[2];
 };
 template <class T>
 constexpr TileCost tile_cost(std::initializer_list<float> with_min, std::initializer_list<float> without)
 {
-    TileCost c{16 * T::WR * T::MT, 8 * T::NT * T::WC, T::CTAS, {}, {}};
+    TileCost c{16 * T::WR * T::MT, 8 * T::NT * T::WC, {}, {}};
     int i = 0;
     for (float v : with_min) c.with_min[i++] = v;
     i = 0;
@@ -415,7 +427,7 @@ static constexpr TileCost tile_costs[] = {
 };
 
 // The tile with the least time for M activation rows: a CTA takes one tile, so the busiest SM works through
-// n = ceil(tiles / SMs) of them, CTAS at a time (3 tiles of 128 x 64 on every SM: 94.2 us against 62.5 + 34.6 by the table).
+// n = ceil(tiles / SMs) of them.
 static int pick_tile(const inkq_ctx *ctx, bool has_min, int rows, int M)
 {
     int best = 0;
@@ -425,7 +437,7 @@ static int pick_tile(const inkq_ctx *ctx, bool has_min, int rows, int M)
         const float *t = has_min ? c.with_min : c.without;
         const long long total = static_cast<long long>((rows + c.rows - 1) / c.rows) * ((M + c.cols - 1) / c.cols);
         const long long n = (total + ctx->num_sms - 1) / ctx->num_sms;
-        const float time = static_cast<float>(n / c.ctas) * t[c.ctas - 1] + (n % c.ctas != 0 ? t[n % c.ctas - 1] : 0.f);
+        const float time = static_cast<float>(n / 2) * t[1] + static_cast<float>(n % 2) * t[0];
         if (i == 0 || time < best_time) {
             best = i;
             best_time = time;
@@ -444,15 +456,20 @@ static int launch_sized(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begi
             QROWS_TILES(QROWS_CASE)
         }
     }
-    // Up to 32 rows one tile holds all of them, so every weight byte is fetched once.  64 instead of 128 weight rows per CTA when
-    // the layer has too few 128-row tiles to occupy the SMs (measured: 6144 x 4096 with 24 rows 18.0 -> 13.4 us; 24576 x 4096
-    // with 5 rows 16.3 against 23.1 us the other way round)
-    const bool narrow = w->tiles * 2 <= ctx->num_sms;
+    // Up to 32 rows one tile holds all of them, so every weight byte is fetched once.  No more 128-row tiles than SMs: one CTA
+    // per SM, stages of eight pairs, and 64 instead of 128 weight rows if that still leaves one CTA per SM; otherwise two CTAs per
+    // SM and stages of four (us, against 4 pairs and two CTAs everywhere: 12288 x 4096 with 5 rows 10.6 -> 9.4, with 24 rows 18.8 ->
+    // 16.8; 6144 x 4096 with 5 rows 9.5 -> 7.3, with 24 rows 13.3 -> 12.1; 24576 x 4096 with 5 rows 15.7 against 17.5)
+    const bool narrow = w->tiles * 2 <= ctx->num_sms, single = w->tiles <= ctx->num_sms;
+#define QROWS_SMALL(n)                                                                                              \
+    case n:                                                                                                         \
+        if (narrow) return launch_one<SCH, S16, Tile<4, 1, 1, n, 8, n == 1 ? 2 : 1>>(ctx, a, w, m_begin, prm);      \
+        return single ? launch_one<SCH, S16, Tile<8, 1, 1, n, 8, 1>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, n, 4, 2>>(ctx, a, w, m_begin, prm);
     switch ((prm.M + 7) / 8) {
-        case 1: return narrow ? launch_one<SCH, S16, Tile<4, 1, 1, 1, 4>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, 1, 4>>(ctx, a, w, m_begin, prm);
-        case 2: return narrow ? launch_one<SCH, S16, Tile<4, 1, 1, 2, 4>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, 2, 4>>(ctx, a, w, m_begin, prm);
-        case 3: return narrow ? launch_one<SCH, S16, Tile<4, 1, 1, 3, 4>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, 3, 4>>(ctx, a, w, m_begin, prm);
-        case 4: return narrow ? launch_one<SCH, S16, Tile<4, 1, 1, 4, 4>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, 4, 4>>(ctx, a, w, m_begin, prm);
+        QROWS_SMALL(1)
+        QROWS_SMALL(2)
+        QROWS_SMALL(3)
+        QROWS_SMALL(4)
     }
     return fail(ctx, INKQ_ERR_INVALID, "internal: too many rows for k_qgemm_rows");
 }

@@ -127,10 +127,11 @@ def test_gemm_tile_edges(pkg, gpu, scheme, scale_mode, N, K):
 
 @pytest.mark.parametrize("scheme", [0, 1, 2])
 @pytest.mark.parametrize("scale_mode", [0, 1])
-@pytest.mark.parametrize("M,N,K", [(33, 24576, 192), (281, 8192, 64), (65, 6144, 320), (113, 12232, 192), (481, 12288, 64), (700, 24576, 64),
-                                   (322, 12288, 192), (409, 1000, 320), (57, 24568, 64), (100, 4096, 192), (322, 4096, 64), (322, 6144, 192)])
+@pytest.mark.parametrize("M,N,K", [(33, 504, 576), (257, 1000, 320), (33, 6136, 192), (65, 4096, 576), (49, 6144, 448), (65, 8184, 448), (193, 4096, 320),
+                                   (65, 6144, 1088), (97, 6136, 448), (145, 6144, 320), (289, 4088, 320), (321, 4096, 192), (322, 12288, 320),
+                                   (49, 24576, 64), (97, 24568, 64), (145, 12288, 192), (289, 8192, 192), (8, 19000, 320), (20, 19000, 192)])
 def test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K):
-    """Sizes that between them select every tile of more than 32 columns, ragged in rows, columns and stages."""
+    """Sizes that between them select every tile, ragged in rows, columns and stages."""
     import torch
     w = pkg.synth.weights(N, K, 11)
     wh = gpu.weight(scheme, scale_mode, w["nib"], w["d"], w["m"] if scheme == 0 else None, w["zp"] if scheme == 2 else None)
