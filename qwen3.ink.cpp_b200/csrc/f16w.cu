@@ -110,8 +110,9 @@ __global__ void __launch_bounds__(256) k_f16w_gemv(const uint16_t *__restrict__ 
 // Bound by the weight stream.  The weights come straight from global memory into A fragments: the order of k inside a product
 // is free, so a lane takes 32 contiguous bytes of its two rows per 64 k - the fragments of four products, 128 bytes per row and
 // request - and the activations are read alike.  Each lane keeps F16R_DEPTH such steps in flight across tile borders (128 KB
-// per SM).  Measured: 151936 x 4096, 8 rows 1258 us on the CUDA cores, 230 with 64-byte pieces, 200 now (6.2 TB/s); one row 194
-// on the CUDA cores, 197 now (32000 x 4096: 54 -> 50, 151936 x 2048: 111 -> 100, set-up hidden behind the kernel before).
+// per SM).  Measured (three matrices in turn): 151936 x 4096, 8 rows 1258 us on the CUDA cores, 230 with 64-byte pieces, 200 with
+// slower preparation of the activations, 186 now (6.7 TB/s); one row 194 on the CUDA cores, 179 now (32000 x 4096: 54 -> 46,
+// 151936 x 2048: 111 -> 102).
 constexpr int F16R_WARPS = 16, F16R_DEPTH = 4, F16R_COLS = 8;
 
 // bytes between two rows of the staged activations: 16 modulo 128, so that the 16-byte pieces of an 8-lane phase (two rows, every
@@ -151,38 +152,48 @@ __global__ void __launch_bounds__(F16R_WARPS * 32, 1)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    // two warps per row: scale by the power of two that puts the row's largest value into [2^13, 2^14), split
+    // 16, 8, 4 or 2 warps per row, whatever the number of rows leaves: scale by the power of two that puts the row's largest value
+    // into [2^13, 2^14), split.  Rows past mt stay as they are: each only feeds its own column, which is not stored.  (Two warps per
+    // row whatever their number, each scanning all of it: 3 us before the first product.)
     {
-        const int m = warp >> 1, half = warp & 1, n4 = K / 4;
+        const int wpr = F16R_WARPS / (mt > 4 ? 8 : mt > 2 ? 4 : mt), m = warp / wpr, n4 = K / 4, first = (warp % wpr) * 32 + lane;
         const float4 *row = reinterpret_cast<const float4 *>(x + static_cast<size_t>(m0 + m) * K);
         float amax = 0.f;
-        if (m < mt)
-            for (int i = lane; i < n4; i += 32) {
+        if (m < mt) {
+#pragma unroll 8
+            for (int i = first; i < n4; i += wpr * 32) {
                 const float4 v = row[i];
                 amax = fmaxf(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))), amax);
             }
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        if (lane == 0) part[warp] = amax;   // (free until the first tile is complete)
+        __syncthreads();
+        amax = 0.f;
+        for (int i = 0; i < wpr; i++) amax = fmaxf(amax, part[m * wpr + i]);
         int e = 0;   // rows of zeros, infinities or NaNs are left unscaled
         if (amax > 0.f && amax < 3.0e38f) e = 13 - ilogbf(amax);
         e = max(-100, min(100, e));
         const float sc = ldexpf(1.0f, e);
-        if (lane == 0 && half == 0) inv[m] = ldexpf(1.0f, -e);
-        for (int i = half * 32 + lane; i < n4; i += 64) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (m < mt) v = row[i];
-            const float f[4] = {v.x * sc, v.y * sc, v.z * sc, v.w * sc};
-            __half h[4], l[4];
+        if (m < mt) {
+            if (first == 0) inv[m] = ldexpf(1.0f, -e);
+#pragma unroll 4
+            for (int i = first; i < n4; i += wpr * 32) {
+                const float4 v = row[i];
+                const float f[4] = {v.x * sc, v.y * sc, v.z * sc, v.w * sc};
+                __half h[4], l[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                h[j] = __float2half_rn(f[j]);
-                l[j] = __float2half_rn(f[j] - __half2float(h[j]));   // the difference is exact in fp32
+                for (int j = 0; j < 4; j++) {
+                    h[j] = __float2half_rn(f[j]);
+                    l[j] = __float2half_rn(f[j] - __half2float(h[j]));   // the difference is exact in fp32
+                }
+                __half2 *oh = reinterpret_cast<__half2 *>(xh + m * pitch + i * 8), *ol = reinterpret_cast<__half2 *>(xl + m * pitch + i * 8);
+                oh[0] = __halves2half2(h[0], h[1]);
+                oh[1] = __halves2half2(h[2], h[3]);
+                ol[0] = __halves2half2(l[0], l[1]);
+                ol[1] = __halves2half2(l[2], l[3]);
             }
-            __half2 *oh = reinterpret_cast<__half2 *>(xh + m * pitch + i * 8), *ol = reinterpret_cast<__half2 *>(xl + m * pitch + i * 8);
-            oh[0] = __halves2half2(h[0], h[1]);
-            oh[1] = __halves2half2(h[2], h[3]);
-            ol[0] = __halves2half2(l[0], l[1]);
-            ol[1] = __halves2half2(l[2], l[3]);
         }
     }
     __syncthreads();
