@@ -832,8 +832,8 @@ def run_ours(args, rank, world, local_rank):
         int8_peak = 2.0 * pk["bf16_tflops"]
         full_shape = wl in ("qgemm_pp322", "qgemv_sweep") and world == 1
         roof = {"bound": "tensor", "achieved": ach, "peak": int8_peak, "unit": "TOP/s", "frac": ach / int8_peak,
-                            "traffic": 41.12e6 if full_shape else None,
-                            "traffic_source": "profiles/qgemm_tc_pp322.md: dram__bytes_read.sum + dram__bytes_write.sum of one launch at this shape "
+                            "traffic": 39.56e6 if full_shape else None,
+                            "traffic_source": "profiles/qgemm_pp322.md: dram__bytes_read.sum + dram__bytes_write.sum of one launch at this shape "
                                               "(not measured by this run)" if full_shape else None,
                             "kernel": "k_qgemm_rows", "us_per_launch": ms_g * 1e3,
                             "peak_note": f"2 x the {pk['source']} dense bf16 figure ({pk['bf16_tflops']} TFLOP/s); int8 itself is not in MEASURED_PEAKS.json",
