@@ -43,6 +43,7 @@ struct FusedM1 {
     int accumulate;      // 1: C[n] += result (residual connection), 0: C[n] = result
 };
 enum { PRO_PLAIN = 0, PRO_RMSNORM = 1, PRO_SILU_MUL = 2 };
+enum { FUSED_NONE = 0, FUSED_PLAIN = 1, FUSED_ANY = 2 };
 
 // Builds the quantized activation row in shared memory from fp32 input (two lanes per 32-element block, as
 // k_quantize_q8): optional RMSNorm (x * 1/sqrt(mean(x^2) + eps) * g) or SiLU(gate) * up first.
@@ -128,11 +129,42 @@ __device__ __forceinline__ void fused_prologue(const FusedM1 &f, int K, uint32_t
     }
 }
 
+// The same for a row taken as it is (the linear layer's own forward): four lanes per block, so that a row of 4096 keeps all 512
+// threads of a 16-warp CTA busy, and eight values per lane instead of sixteen.  Beside the weights in flight the general form
+// spills 48 to 220 bytes per thread (4096 x 4096 4.7 -> 3.1 us, 12288 x 4096 8.1 -> 7.1, 4096 x 12288 9.5 -> 8.7).
+template <bool HAS_MIN>
+__device__ __forceinline__ void plain_prologue(const FusedM1 &f, int K, uint32_t *qa, float *da, float *sa)
+{
+    const int nb = K / QK, quarter = threadIdx.x & 3;
+    const unsigned gmask = 0xFu << (threadIdx.x & 28);                     // the four lanes of a block
+    for (int blk = threadIdx.x >> 2; blk < nb; blk += blockDim.x >> 2) {   // the lanes of a block run the same trip count
+        const float4 a = reinterpret_cast<const float4 *>(f.x)[blk * 8 + 2 * quarter], b = reinterpret_cast<const float4 *>(f.x)[blk * 8 + 2 * quarter + 1];
+        float mx = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))), fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))));
+        mx = fmaxf(mx, __shfl_xor_sync(gmask, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(gmask, mx, 2));
+        const float dd = __fdiv_rn(mx, 127.0f);
+        const float id = (mx != 0.0f) ? __fdiv_rn(127.0f, mx) : 0.0f;
+        const int a0 = __float2int_rn(__fmul_rn(a.x, id)), a1 = __float2int_rn(__fmul_rn(a.y, id));
+        const int a2 = __float2int_rn(__fmul_rn(a.z, id)), a3 = __float2int_rn(__fmul_rn(a.w, id));
+        const int b0 = __float2int_rn(__fmul_rn(b.x, id)), b1 = __float2int_rn(__fmul_rn(b.y, id));
+        const int b2 = __float2int_rn(__fmul_rn(b.z, id)), b3 = __float2int_rn(__fmul_rn(b.w, id));
+        int sum = ((a0 + a1) + (a2 + a3)) + ((b0 + b1) + (b2 + b3));
+        *reinterpret_cast<uint2 *>(qa + blk * 8 + 2 * quarter) = make_uint2(pack_sat_s8x4_m1(a0, a1, a2, a3), pack_sat_s8x4_m1(b0, b1, b2, b3));
+        sum += __shfl_xor_sync(gmask, sum, 1);
+        sum += __shfl_xor_sync(gmask, sum, 2);
+        if (quarter == 0) {
+            da[blk] = __half2float(__float2half_rn(dd));
+            if (HAS_MIN) sa[blk] = (f.qmode == INKQ_Q8_1_F16) ? __half2float(__float2half_rn(__fmul_rn(dd, static_cast<float>(sum)))) : 0.0f;
+            else reinterpret_cast<int32_t *>(sa)[blk] = sum;
+        }
+    }
+}
+
 // WARPS = K-slices per CTA: 8 for wide layers, 16 for narrow ones (more bytes in flight per SM when
 // the grid alone cannot fill the machine).  The register budget keeps 3 (resp. 2) CTAs per SM resident so
 // that every Qwen3-8B shape runs as a single wave.  FUSED: the activation row is built from fp32 input in
-// the prologue (FusedM1) instead of being read from a quantizer's output.
-template <bool HAS_MIN, int WARPS, bool FUSED, bool DEEP>
+// the prologue (FusedM1; FUSED_PLAIN: only PRO_PLAIN) instead of being read from a quantizer's output.
+template <bool HAS_MIN, int WARPS, int FUSED, bool DEEP>
 __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_SM) k_qgemv_a8w4(const uint8_t *__restrict__ nibT, const uint2 *__restrict__ sc16,
                                                                const uchar2 *__restrict__ zpT, const int8_t *__restrict__ q,
                                                                const float *__restrict__ d, const float *__restrict__ s,
@@ -164,7 +196,9 @@ __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_S
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    if (FUSED) {
+    if (FUSED == FUSED_PLAIN) {
+        plain_prologue<HAS_MIN>(fused, K, qa, da, sa);
+    } else if (FUSED == FUSED_ANY) {
         fused_prologue<HAS_MIN>(fused, K, qa, da, sa, part);
     } else {
         for (int i = threadIdx.x; i < K / 16; i += blockDim.x)
@@ -195,7 +229,7 @@ __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_S
     }
 }
 
-template <bool HAS_MIN, int WARPS, bool FUSED, bool DEEP = false>
+template <bool HAS_MIN, int WARPS, int FUSED, bool DEEP = false>
 static void launch_gemv_variant(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const ExtraDst &extra, const FusedM1 &fused)
 {
     const size_t smem = static_cast<size_t>(w->K) + 2 * sizeof(float) * (w->K / QK) + sizeof(float) * WARPS * 32;
@@ -219,7 +253,7 @@ static void launch_gemv_variant(inkq_ctx *ctx, const Act *a, const Weight *w, fl
                        static_cast<const int32_t *>(a ? a->isum : nullptr), a ? a->M_ld : 0, C, w->rows, w->K, w->pairs, extra, fused);
 }
 
-template <bool FUSED>
+template <int FUSED>
 static void launch_gemv_any(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const ExtraDst &extra, const FusedM1 &fused)
 {
     // narrow layers (few CTAs) or long rows: 16 K-slices per CTA
@@ -241,7 +275,7 @@ int launch_gemv(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const Ex
 {
     ExtraDst extra = {};
     if (extra_in != nullptr) extra = *extra_in;
-    launch_gemv_any<false>(ctx, a, w, C, extra, FusedM1{});
+    launch_gemv_any<FUSED_NONE>(ctx, a, w, C, extra, FusedM1{});
     return after_launch(ctx, "k_qgemv_a8w4");
 }
 
@@ -254,7 +288,8 @@ int launch_gemv_fused(inkq_ctx *ctx, const Weight *w, const float *x, int pro, c
     f.pro = pro;
     f.qmode = (w->scheme == INKQ_A81W41) ? INKQ_Q8_1_F16 : INKQ_Q8_0_F16;   // as inkq_linear chooses for M == 1
     f.accumulate = accumulate;
-    launch_gemv_any<true>(ctx, nullptr, w, C, ExtraDst{}, f);
+    if (pro == PRO_PLAIN) launch_gemv_any<FUSED_PLAIN>(ctx, nullptr, w, C, ExtraDst{}, f);
+    else launch_gemv_any<FUSED_ANY>(ctx, nullptr, w, C, ExtraDst{}, f);
     return after_launch(ctx, "k_qgemv_a8w4 (fused prologue)");
 }
 
