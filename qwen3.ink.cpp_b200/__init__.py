@@ -9,6 +9,7 @@ calls raise, there is no CPU fallback.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 import numpy as np
@@ -78,6 +79,25 @@ def lib() -> C.CDLL:
     return _lib
 
 
+def _load_call6():
+    """The module that build.build_fast_call compiles, or None (calls then go through ctypes)."""
+    path = os.path.join(HERE, "inkq_fast_call.so")
+    if not os.path.exists(path):
+        return None
+    try:
+        spec = importlib.util.spec_from_file_location("inkq_fast_call", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        return mod.call6
+    except ImportError:      # built for another interpreter
+        return None
+
+
+def _addr(t) -> int:
+    """Device pointer of a torch tensor (or an int address, or None) as an integer."""
+    return 0 if t is None else t if isinstance(t, int) else t.data_ptr()
+
+
 def _dp(t):
     """Device pointer of a torch tensor (or an int address, or None)."""
     if t is None:
@@ -121,6 +141,8 @@ class Context:
             raise InkqError(rc, self.L.inkq_last_error(None).decode())
         self.h = h
         self.device = device
+        self._call6 = _load_call6()
+        self._linear = C.cast(self.L.inkq_linear, C.c_void_p).value
 
     def check(self, rc: int):
         if rc != OK:
@@ -221,8 +243,13 @@ class Context:
         self.check(fn(self.h, act.h, w.h, _dp(dots_dev)))
 
     def linear(self, w, x, M: int, Cdev, ldc: int):
-        """Qwen_Linear_with_bias_Int4::forward on device buffers."""
-        self.check(self.L.inkq_linear(self.h, w.h, _dp(x), M, _dp(Cdev), ldc))
+        """Qwen_Linear_with_bias_Int4::forward on device buffers.  One row takes the device 3 us: the call must not take longer."""
+        if self._call6 is not None and self.h and w.h:
+            rc = self._call6(self._linear, self.h.value, w.h.value, _addr(x), M, _addr(Cdev), ldc)
+        else:
+            rc = self.L.inkq_linear(self.h, w.h, _dp(x), M, _dp(Cdev), ldc)
+        if rc:
+            self.check(rc)
 
     def linear_host(self, w, x_host, M: int, C_host, ldc: int):
         """Same with host buffers (NumPy arrays, or torch CPU tensors, ideally pinned)."""

@@ -12,12 +12,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libinkq.so")
 SHIM = os.path.join(HERE, "libinkq_refshim.so")
+FAST = os.path.join(HERE, "inkq_fast_call.so")
 
 
 def _nvcc() -> str:
@@ -78,12 +80,32 @@ def build_shim(force: bool = False) -> str:
     return SHIM
 
 
+def build_fast_call(force: bool = False) -> str:
+    """CPython entry for the shortest calls.  Optional: without the interpreter's headers the package calls through ctypes."""
+    src = os.path.join(HERE, "pyext", "fast_call.cc")
+    inc = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(inc, "Python.h")):
+        return ""
+    if not force and not _stale(FAST, [src]):
+        return FAST
+    env = dict(os.environ)
+    env.pop("CC", None)
+    env.pop("CXX", None)
+    res = subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-I", inc, "-o", FAST, src], capture_output=True, text=True, env=env)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("g++ failed building the call entry")
+    return FAST
+
+
 def build_all(force: bool = False) -> None:
     build_cuda(force)
     build_shim(force)
+    build_fast_call(force)
 
 
 if __name__ == "__main__":
     build_cuda(force="--force" in sys.argv, verbose=True)
     build_shim(force="--force" in sys.argv)
+    build_fast_call(force="--force" in sys.argv)
     print("built", LIB)
