@@ -135,7 +135,8 @@ __device__ __forceinline__ void cta_rmsnorm_quant(const float *x, const float *g
     }
 }
 
-template <bool HAS_MIN, int WARPS, bool DEEP>
+// PAIR: EPI_PAIR_SILUQ, two 32-row groups per CTA
+template <bool HAS_MIN, int WARPS, bool DEEP, bool PAIR>
 __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_SM) k_qgemv_decode(const uint8_t *__restrict__ nibT, const uint2 *__restrict__ sc16,
                                                                  const uchar2 *__restrict__ zpT, const int8_t *__restrict__ q,
                                                                  const float *__restrict__ d, const float *__restrict__ s,
@@ -149,10 +150,11 @@ __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_S
     float *sa = da + nb;                                            // nb (sums, or integer sums for the A80 schemes)
     float *part = sa + nb;                                          // [WARPS][32]
     __shared__ unsigned ticket_s;
+    __shared__ float early[6][32];   // requested with the row and used after the product, by warp 0: group sums, residual, norm weight
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int groups = (epi.mode == EPI_PAIR_SILUQ) ? 2 : 1;         // 32-row groups per CTA
-    const int per_tile = 4 / groups;
+    constexpr int groups = PAIR ? 2 : 1;                             // 32-row groups per CTA
+    constexpr int per_tile = 4 / groups;
     const int t = blockIdx.x / per_tile;
     const int g0 = (blockIdx.x % per_tile) * groups;
     const int p_begin = (warp * pairs) / WARPS, p_end = ((warp + 1) * pairs) / WARPS;
@@ -165,23 +167,27 @@ __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_S
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // A pending RMS factor f of the input row multiplies the finished sums (W (f v) = f (W v)), so only the warp that
-    // finishes them needs it: warp 0 requests the group sums now (the first 128: a row of 4096 values; four loads in
-    // flight per lane) and adds them up after the product, when they have long arrived.
-    float pv[4] = {0.f, 0.f, 0.f, 0.f};
-    if (pend.parts > 0 && warp == 0) {
+    // finishes them needs it: warp 0 requests the group sums now (the first 128: a row of 4096 values) and adds them up
+    // after the product.  The residual value and the norm weight this lane's result meets in the epilogue are requested now
+    // as well (nobody else touches them while this grid runs).  They wait in shared memory: in registers, and with
+    // the two-group form in the same kernel, the variants of 64 registers spilled 68 to 96 bytes a thread inside the product
+    // (a decode step of 36 layers 1549 -> 1512 us).
+    if (warp == 0) {
+        const int n_early = t * TILE_N + (g0 << 5) + lane;
+        float e[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (pend.parts > 0) {
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int i = u * 32 + lane;
-            pv[u] = (i < pend.parts) ? __ldcg(pend.ssq + i) : 0.0f;
+            for (int u = 0; u < 4; u++) {
+                const int i = u * 32 + lane;
+                e[u] = (i < pend.parts) ? __ldcg(pend.ssq + i) : 0.0f;
+            }
         }
-    }
-    // the residual value and the norm weight this lane's result meets in the epilogue are requested now as well (nobody
-    // else touches them while this grid runs), so their latency passes under the product
-    const int n_early = t * TILE_N + (g0 << 5) + lane;
-    float c_early = 0.0f, g_early = 0.0f;
-    if (warp == 0 && n_early < rows && groups == 1) {
-        if (epi.mode != EPI_STORE) c_early = C[n_early];
-        if (epi.mode == EPI_ACC_QUANT_PENDING) g_early = epi.g[n_early];
+        if (n_early < rows && groups == 1) {
+            if (epi.mode != EPI_STORE) e[4] = C[n_early];
+            if (epi.mode == EPI_ACC_QUANT_PENDING) e[5] = epi.g[n_early];
+        }
+#pragma unroll
+        for (int u = 0; u < 6; u++) early[u][lane] = e[u];
     }
     for (int i = threadIdx.x; i < K / 16; i += blockDim.x) reinterpret_cast<uint4 *>(qa)[i] = reinterpret_cast<const uint4 *>(q)[i];
     for (int b = threadIdx.x; b < nb; b += blockDim.x) {
@@ -213,7 +219,7 @@ __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_S
         // every CTA adds the group sums in the same order (lane-strided ascending, then an xor tree): one factor for all
         float ss = 0.0f;
 #pragma unroll
-        for (int u = 0; u < 4; u++) ss = __fadd_rn(ss, pv[u]);
+        for (int u = 0; u < 4; u++) ss = __fadd_rn(ss, early[u][lane]);
         for (int i = 128 + lane; i < pend.parts; i += 32) ss = __fadd_rn(ss, __ldcg(pend.ssq + i));
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, off));
@@ -222,7 +228,7 @@ __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_S
         tot[1] = __fmul_rn(tot[1], f);
     }
 
-    if (epi.mode == EPI_PAIR_SILUQ) {
+    if (PAIR) {
         if (warp == 0) {
             const int blk = blockIdx.x;                           // output block = CTA index: rows come in (gate32, up32) groups
             const float a = silu_mul(tot[0], tot[1]);
@@ -233,19 +239,19 @@ __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_S
     const int n = t * TILE_N + (g0 << 5) + lane;
     if (epi.mode == EPI_ACC_QUANT_PENDING) {
         if (warp == 0) {   // rows is a multiple of 32 here: the whole warp holds results
-            const float y = __fadd_rn(c_early, tot[0]);
+            const float y = __fadd_rn(early[4][lane], tot[0]);
             C[n] = y;
             float ss = __fmul_rn(y, y);
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, off));
             if (lane == 0) epi.ssq_out[n >> 5] = ss;
-            quantize_block_lanes(__fmul_rn(y, g_early), n >> 5, lane, epi.out);
+            quantize_block_lanes(__fmul_rn(y, early[5][lane]), n >> 5, lane, epi.out);
         }
         return;
     }
     if (warp == 0 && n < rows) {
         float y = tot[0];
-        if (epi.mode != EPI_STORE) y = __fadd_rn(c_early, y);
+        if (epi.mode != EPI_STORE) y = __fadd_rn(early[4][lane], y);
         C[n] = y;
     }
     if (epi.mode != EPI_ACC_NORMQ) return;
@@ -270,13 +276,13 @@ __global__ void __launch_bounds__(512) k_rmsnorm_quant_row(const float *x, const
     cta_rmsnorm_quant(x, g, eps, n, xn, o, red);
 }
 
-template <bool HAS_MIN, int WARPS, bool DEEP = false>
-static void launch_decode_variant(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const DecodeEpi &epi, const PendingNorm &pend)
+template <bool HAS_MIN, int WARPS, bool DEEP, bool PAIR>
+static void launch_decode_epi(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const DecodeEpi &epi, const PendingNorm &pend)
 {
     const size_t smem = static_cast<size_t>(w->K) + 2 * sizeof(float) * (w->K / QK) + sizeof(float) * WARPS * 32;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_qgemv_decode<HAS_MIN, WARPS, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k_qgemv_decode<HAS_MIN, WARPS, DEEP, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(w->tiles) * (epi.mode == EPI_PAIR_SILUQ ? 2 : 4));
+    cfg.gridDim = dim3(static_cast<unsigned>(w->tiles) * (PAIR ? 2 : 4));
     cfg.blockDim = dim3(WARPS * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
@@ -285,9 +291,16 @@ static void launch_decode_variant(inkq_ctx *ctx, const Act *a, const Weight *w, 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_qgemv_decode<HAS_MIN, WARPS, DEEP>, static_cast<const uint8_t *>(w->nibT), static_cast<const uint2 *>(w->sc16),
+    cudaLaunchKernelEx(&cfg, k_qgemv_decode<HAS_MIN, WARPS, DEEP, PAIR>, static_cast<const uint8_t *>(w->nibT), static_cast<const uint2 *>(w->sc16),
                        static_cast<const uchar2 *>(w->zpT), static_cast<const int8_t *>(a->q), static_cast<const float *>(a->d),
                        static_cast<const float *>(a->s), static_cast<const int32_t *>(a->isum), a->M_ld, C, w->rows, w->K, w->pairs, epi, pend);
+}
+
+template <bool HAS_MIN, int WARPS, bool DEEP = false>
+static void launch_decode_variant(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const DecodeEpi &epi, const PendingNorm &pend)
+{
+    if (epi.mode == EPI_PAIR_SILUQ) launch_decode_epi<HAS_MIN, WARPS, DEEP, true>(ctx, a, w, C, epi, pend);
+    else launch_decode_epi<HAS_MIN, WARPS, DEEP, false>(ctx, a, w, C, epi, pend);
 }
 
 }  // namespace inkq
