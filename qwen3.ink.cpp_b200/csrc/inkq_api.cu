@@ -754,8 +754,12 @@ int inkq_gemm_w41_f16act(inkq_ctx *ctx, const uint16_t *a16_dev, int M, const in
     INKQ_REQUIRE(ctx, w != nullptr && a16_dev != nullptr && C_dev != nullptr, "null handle, input or output");
     INKQ_REQUIRE(ctx, w->scheme == INKQ_W41 || w->scheme == INKQ_A81W41, "weight-only matmul needs Q4_1 weights");
     INKQ_REQUIRE(ctx, M >= 1 && ldc >= w->rows, "bad M or ldc");
-    if (M == 1 && (reinterpret_cast<uintptr_t>(a16_dev) & 3) == 0) return launch_gemv_w41(ctx, a16_dev, w, C_dev);   // decode: stream the weights
-    if (M > 1 && gemm_w41_rows_fits(a16_dev, M, w->K)) return launch_gemm_w41_rows(ctx, a16_dev, M, w, C_dev, ldc);
+    // One row streams the weights through the CUDA cores, unless the layer's 32-row CTAs leave half of the SMs idle and K is no
+    // reason to keep them: then the warp-level products split K further (1024 and 2048 x 4096 5.0 -> 3.9 us; 4096 x 4096 5.5 both)
+    const bool few_rows = w->tiles * 8 <= ctx->num_sms && w->pairs < 128;
+    if (M == 1 && (reinterpret_cast<uintptr_t>(a16_dev) & 3) == 0 && !(few_rows && gemm_w41_rows_fits(a16_dev, M, w->K)))
+        return launch_gemv_w41(ctx, a16_dev, w, C_dev);
+    if (gemm_w41_rows_fits(a16_dev, M, w->K)) return launch_gemm_w41_rows(ctx, a16_dev, M, w, C_dev, ldc);
     return launch_gemm_w41_tc(ctx, a16_dev, M, w, C_dev, ldc);
 }
 

@@ -256,7 +256,7 @@ def test_mismatched_quantizer_mode_is_rejected(pkg, gpu, oracle):
 
 
 # ------------------------------------------------------------------ weight-only W41 and fp16 lm_head
-@pytest.mark.parametrize("M,N,K", [(9, 72, 256), (1, 256, 128), (1, 1064, 512), (1, 4096, 4096), (1, 512, 12288),   # M == 1: the streaming kernel
+@pytest.mark.parametrize("M,N,K", [(9, 72, 256), (1, 256, 128), (1, 1064, 512), (1, 4096, 4096), (1, 512, 12288), (1, 6144, 576),   # M == 1: the streaming kernel (many rows, long rows) and the products
                                    # M = 2 .. 16: products in registers, ragged row tiles, fewer and more pairs than warps x depth
                                    (2, 72, 64), (8, 2440, 1088), (10, 136, 8256), (15, 24, 320), (16, 4808, 576), (16, 136, 12288),
                                    (16, 128, 64), (322, 384, 512), (200, 136, 1024), (400, 264, 192),
