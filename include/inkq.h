@@ -214,11 +214,17 @@ int inkq_gemm_w41_f16act_simt(inkq_ctx *ctx, const uint16_t *a16_dev, int M, con
 int inkq_f16w_create(inkq_ctx *ctx, int N, int K, const uint16_t *w16_host, int n_begin, int n_end, inkq_f16w **out);
 int inkq_f16w_create_dev(inkq_ctx *ctx, int N, int K, const uint16_t *w16_dev, int n_begin, int n_end, inkq_f16w **out);
 int inkq_f16w_destroy(inkq_f16w *w);
-/* C[m][n] = sum_k x[m][k] * w[n][k].  M < 16: bandwidth-bound CUDA-core kernel, fp32 activations, exact products.
- * M >= 16 (and K % 64 == 0): tensor cores; the fp32 activations enter as fp16 hi + lo parts (22 significant bits, the
- * K loop runs over both; result within ~1e-5 of the output's rms of an fp32 evaluation) or, with INKQ_F16W_ACT_FP16,
- * as one fp16 value (half the work; each activation rounded with relative error <= 2^-11, about 1e-3 of the
- * output's rms).  inkq_f16w_matmul = INKQ_F16W_ACT_FP32. */
+/* C[m][n] = sum_k x[m][k] * w[n][k].
+ * M < 16 (or an output that is not 16-byte aligned): bandwidth-bound, warp-level products; the fp32 activations enter as
+ * fp16 hi + lo parts of the row scaled by a power of two (22 significant bits), sums in fp32: about 1.3e-7 of the output's
+ * 2-norm from the exact result, and a batch has the bits of its rows one by one.  K % 64 != 0: CUDA cores, fp32
+ * activations, exact products.
+ * M >= 16 (and K % 64 == 0): tensor cores; the same hi + lo parts (result within ~1e-5 of the output's rms of an fp32
+ * evaluation) or, with INKQ_F16W_ACT_FP16, one fp16 value (half the work; each activation rounded with relative error
+ * <= 2^-11, about 1e-3 of the output's rms).
+ * Finite activations of any magnitude are served (with K % 64 == 0 no partial sum overflows, only a result can); infinities
+ * and NaNs among them act as in an fp32 evaluation, infinite weights as well with M < 16 (else a NaN, not the infinity).
+ * inkq_f16w_matmul = INKQ_F16W_ACT_FP32. */
 typedef enum { INKQ_F16W_ACT_FP32 = 0, INKQ_F16W_ACT_FP16 = 1 } inkq_f16w_precision;
 int inkq_f16w_matmul(inkq_ctx *ctx, const inkq_f16w *w, const float *x_dev, int M, float *C_dev, int ldc);
 int inkq_f16w_matmul_prec(inkq_ctx *ctx, const inkq_f16w *w, const float *x_dev, int M, float *C_dev, int ldc, int precision);

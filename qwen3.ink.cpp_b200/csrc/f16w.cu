@@ -17,6 +17,9 @@
 // M*rows*4 output bytes.
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
+#include "f16w_split.cuh"
 #include "inkq_internal.h"
 #include "ptx.cuh"
 
@@ -103,8 +106,8 @@ __global__ void __launch_bounds__(256) k_f16w_gemv(const uint16_t *__restrict__ 
 // The CUDA-core kernel above needs, per weight and row, a conversion, an fp32 fma and its share of a 16-byte shared load: with
 // four rows it is bound by instruction issue (4 rows 631 us for the 1.2 GB lm_head, 194 us with one).  Here 16 weight rows x 8
 // activation rows x 16 k are one warp-level fp16 product with fp32 accumulation; the fp32 activations enter as an fp16 value and
-// an fp16 remainder of the row scaled by a power of two (22 significant bits, as in the tensor-core GEMM), so both products
-// are exact.  A tile's K is split over the CTA's 16 warps, whose partial sums are added in ascending order.  A row's result does
+// an fp16 remainder of the row scaled by a power of two (f16w_split.cuh: 22 significant bits), so both products are exact.
+// Error against 64 bits, 2-norm: 1.2e-7 at K = 2048 and 4096, where the CUDA-core kernel's fp32 sums have 1.6e-7 and 2.1e-7.  A tile's K is split over the CTA's 16 warps, whose partial sums are added in ascending order.  A row's result does
 // not depend on the rows beside it, and one row takes this kernel too: a batch gives the same bits as its rows one by one.
 //
 // Bound by the weight stream.  The weights come straight from global memory into A fragments: the order of k inside a product
@@ -119,6 +122,23 @@ constexpr int F16R_WARPS = 16, F16R_DEPTH = 4, F16R_COLS = 8;
 // other piece of 128 bytes) fall into different banks
 __host__ __device__ constexpr int f16r_pitch(int K) { return (K * 2 + 127) / 128 * 128 + 16; }
 
+// One output in fp32, by one warp: for the outputs that the split operands cannot express
+static __device__ __noinline__ float dot_f16w(const uint16_t *wrow, const float *xrow, int K, int lane)
+{
+    float acc = 0.0f;
+    for (int i = lane; i < K / 4; i += 32) {
+        const float4 v = reinterpret_cast<const float4 *>(xrow)[i];
+        const __half2 *p = reinterpret_cast<const __half2 *>(wrow + i * 4);
+        const float2 a = __half22float2(p[0]), b = __half22float2(p[1]);
+        acc = fmaf(v.x, a.x, acc);
+        acc = fmaf(v.y, a.y, acc);
+        acc = fmaf(v.z, b.x, acc);
+        acc = fmaf(v.w, b.y, acc);
+    }
+    for (int o = 16; o > 0; o >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    return acc;
+}
+
 __global__ void __launch_bounds__(F16R_WARPS * 32, 1)
     k_f16w_rows(const uint16_t *__restrict__ w, const float *__restrict__ x, int m0, int mt, int rows, int K, float *__restrict__ C, int ldc, const ExtraDst extra)
 {
@@ -126,7 +146,8 @@ __global__ void __launch_bounds__(F16R_WARPS * 32, 1)
     const int pitch = f16r_pitch(K);
     unsigned char *xh = smem_raw, *xl = xh + F16R_COLS * pitch;                                  // [8][K] fp16 value and remainder
     float *part = reinterpret_cast<float *>(xl + F16R_COLS * pitch);                              // [2][warps][8 columns][16 rows]
-    float *inv = part + 2 * F16R_WARPS * F16R_COLS * 16;                                           // [8]
+    float *inv = part + 2 * F16R_WARPS * F16R_COLS * 16;                                           // [8] 2^-e of a row
+    int *has_nan = reinterpret_cast<int *>(inv + F16R_COLS);                                       // [8]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int k64 = K / 64, steps = (k64 + F16R_WARPS - 1) / F16R_WARPS;                          // steps of 64 k per warp and tile
     const int tiles = (rows + 15) / 16;
@@ -152,48 +173,44 @@ __global__ void __launch_bounds__(F16R_WARPS * 32, 1)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    // 16, 8, 4 or 2 warps per row, whatever the number of rows leaves: scale by the power of two that puts the row's largest value
-    // into [2^13, 2^14), split.  Rows past mt stay as they are: each only feeds its own column, which is not stored.  (Two warps per
-    // row whatever their number, each scanning all of it: 3 us before the first product.)
+    // 16, 8, 4 or 2 warps per row, whatever the number of rows leaves: scale and split (f16w_split.cuh).  Rows past mt stay
+    // as they are: each only feeds its own column, which is not stored.  (Two warps per row whatever their number, each
+    // scanning all of it: 3 us before the first product.)
     {
         const int wpr = F16R_WARPS / (mt > 4 ? 8 : mt > 2 ? 4 : mt), m = warp / wpr, n4 = K / 4, first = (warp % wpr) * 32 + lane;
         const float4 *row = reinterpret_cast<const float4 *>(x + static_cast<size_t>(m0 + m) * K);
         float amax = 0.f;
         if (m < mt) {
 #pragma unroll 8
-            for (int i = first; i < n4; i += wpr * 32) {
-                const float4 v = row[i];
-                amax = fmaxf(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))), amax);
-            }
+            for (int i = first; i < n4; i += wpr * 32) amax = absmax_nan(amax, row[i]);
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        for (int o = 16; o > 0; o >>= 1) amax = absmax_nan(amax, __shfl_xor_sync(0xffffffffu, amax, o));
         if (lane == 0) part[warp] = amax;   // (free until the first tile is complete)
         __syncthreads();
         amax = 0.f;
-        for (int i = 0; i < wpr; i++) amax = fmaxf(amax, part[m * wpr + i]);
-        int e = 0;   // rows of zeros, infinities or NaNs are left unscaled
-        if (amax > 0.f && amax < 3.0e38f) e = 13 - ilogbf(amax);
-        e = max(-100, min(100, e));
-        const float sc = ldexpf(1.0f, e);
+        for (int i = 0; i < wpr; i++) amax = absmax_nan(amax, part[m * wpr + i]);
         if (m < mt) {
+            const bool special = !(amax <= FLT_MAX);
+            if (first == 0) has_nan[m] = amax != amax;
+            if (special) amax = finite_absmax(row, n4, lane);
+            const int e = split_exponent(amax);
+            const float sc = ldexpf(1.0f, e);
             if (first == 0) inv[m] = ldexpf(1.0f, -e);
+            auto split_row = [&](auto with_special) {
 #pragma unroll 4
-            for (int i = first; i < n4; i += wpr * 32) {
-                const float4 v = row[i];
-                const float f[4] = {v.x * sc, v.y * sc, v.z * sc, v.w * sc};
-                __half h[4], l[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    h[j] = __float2half_rn(f[j]);
-                    l[j] = __float2half_rn(f[j] - __half2float(h[j]));   // the difference is exact in fp32
+                for (int i = first; i < n4; i += wpr * 32) {
+                    __half2 h[2], l[2];
+                    split4<decltype(with_special)::value>(row[i], sc, h, l);
+                    __half2 *oh = reinterpret_cast<__half2 *>(xh + m * pitch + i * 8), *ol = reinterpret_cast<__half2 *>(xl + m * pitch + i * 8);
+                    oh[0] = h[0];
+                    oh[1] = h[1];
+                    ol[0] = l[0];
+                    ol[1] = l[1];
                 }
-                __half2 *oh = reinterpret_cast<__half2 *>(xh + m * pitch + i * 8), *ol = reinterpret_cast<__half2 *>(xl + m * pitch + i * 8);
-                oh[0] = __halves2half2(h[0], h[1]);
-                oh[1] = __halves2half2(h[2], h[3]);
-                ol[0] = __halves2half2(l[0], l[1]);
-                ol[1] = __halves2half2(l[2], l[3]);
-            }
+            };
+            if (special) split_row(std::true_type{});
+            else split_row(std::false_type{});
         }
     }
     __syncthreads();
@@ -234,8 +251,15 @@ __global__ void __launch_bounds__(F16R_WARPS * 32, 1)
                         float v = q[0];
 #pragma unroll
                         for (int i = 1; i < F16R_WARPS; i++) v = __fadd_rn(v, q[i * (F16R_COLS * 16)]);
-                        if (c < mt && n < rows) {
-                            v *= inv[c];   // exact: a power of two
+                        const bool mine = c < mt && n < rows;
+                        if (mine) v *= inv[c];   // exact: a power of two
+                        // An infinite weight meets remainders of zero or of the other sign: a NaN that no fp32 evaluation has
+                        for (unsigned redo = __ballot_sync(0xffffffffu, mine && v != v && has_nan[c] == 0); redo != 0; redo &= redo - 1) {
+                            const int from = __ffs(redo) - 1;
+                            const float y = dot_f16w(w + static_cast<size_t>(tile * 16 + (from & 15)) * K, x + static_cast<size_t>(m0 + warp * 2 + (from >> 4)) * K, K, lane);
+                            if (lane == from) v = y;
+                        }
+                        if (mine) {
                             const size_t off = static_cast<size_t>(m0 + c) * ldc + n;
                             C[off] = v;
 #pragma unroll
@@ -258,7 +282,7 @@ int launch_f16w_matmul(inkq_ctx *ctx, const F16W *w, const float *x, int M, floa
     ExtraDst extra = {};
     if (extra_in != nullptr) extra = *extra_in;
     const int grid = min((w->rows + 7) / 8, ctx->num_sms * 8);
-    const size_t rows_smem = static_cast<size_t>(2 * F16R_COLS) * f16r_pitch(w->K) + sizeof(float) * (2 * F16R_WARPS * F16R_COLS * 16 + F16R_COLS);
+    const size_t rows_smem = static_cast<size_t>(2 * F16R_COLS) * f16r_pitch(w->K) + sizeof(float) * (2 * F16R_WARPS * F16R_COLS * 16 + 2 * F16R_COLS);
     if (w->K % 64 == 0 && rows_smem <= 226 * 1024) {
         INKQ_CUDA(ctx, cudaFuncSetAttribute(k_f16w_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(rows_smem)));
         const int tiles = (w->rows + 15) / 16;

@@ -3,15 +3,15 @@
 //
 // No C++ kernel exists in the reference for this operand format (its lm_head is an int4 linear applied to the
 // last token only, qwen3/src/qwen/QwenForCausalLM.cc:43-46,121); the arithmetic is that of its fp32 row-times-row
-// GEMV gemv_fp32_rcr_mt_impl_1 (qwen3/src/qwen/fp32_gemx_kernels_rcr.cc:494-507).  M == 1 stays on the
-// bandwidth-bound CUDA-core kernel (k_f16w_gemv); this file serves M >= 16.
+// GEMV gemv_fp32_rcr_mt_impl_1 (qwen3/src/qwen/fp32_gemx_kernels_rcr.cc:494-507).  Fewer than 16
+// rows stay on the bandwidth-bound k_f16w_rows (f16w.cu).
 //
 // Numerics.  The tensor cores take 16-bit operands, so the fp32 activations are first written as fp16:
 //   x16[m][k] = fp16(x[m][k] * 2^e_m)      e_m = the power of two that brings the row's largest magnitude to [2^13, 2^14)
-// (k_f16w_split; the scaling is exact and is undone on the finished sum, so the row keeps fp16's full 11 significant
-// bits whatever its magnitude).  With `passes` == 2 a second operand xlo16 = fp16(x * 2^e_m - x16) holds the next 11
-// bits and the K loop runs a second time over it, accumulating sum_k xlo16 * w into the same tensor-memory
-// accumulator: the activations then enter with 22 significant bits and the result agrees with an fp32 evaluation to
+// (k_f16w_split, f16w_split.cuh; the scaling is exact and is undone on the finished sum, so the row keeps fp16's full 11
+// significant bits whatever its magnitude; infinities and NaNs among the activations act as in an fp32 evaluation).
+// With `passes` == 2 a second operand xlo16 = fp16(x * 2^e_m - x16) holds the next 11 bits and the K loop runs a second
+// time over it, accumulating sum_k xlo16 * w into the same tensor-memory accumulator: the activations then enter with 22 significant bits and the result agrees with an fp32 evaluation to
 // ~1e-5 of the output's rms, at twice the tensor-core work.  With `passes` == 1 each activation
 // carries a relative rounding error of at most 2^-11, i.e. |error| <= 2^-11 * sum_k |x_k * w_k| (about 3e-4 of the
 // output's rms for random data).  Products are exact in fp32; the sum is accumulated in fp32 inside tensor memory in
@@ -42,6 +42,7 @@
 
 #include <mutex>
 
+#include "f16w_split.cuh"
 #include "inkq_internal.h"
 #include "ptx.cuh"
 
@@ -269,34 +270,25 @@ __global__ void __launch_bounds__(256) k_f16w_split(const float *__restrict__ x,
     if (m >= M) return;
     const float4 *row = reinterpret_cast<const float4 *>(x + static_cast<size_t>(m) * K);
     float amax = 0.f;
-    for (int i = lane; i < K / 4; i += 32) {
-        const float4 v = row[i];
-        amax = fmaxf(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))), amax);
-    }
+    for (int i = lane; i < K / 4; i += 32) amax = absmax_nan(amax, row[i]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    // 2^e with amax * 2^e in [2^13, 2^14); rows of zeros, infinities or NaNs are left unscaled
-    int e = 0;
-    if (amax > 0.f && amax < 3.0e38f) e = 13 - ilogbf(amax);
-    e = max(-100, min(100, e));
+    for (int o = 16; o > 0; o >>= 1) amax = absmax_nan(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const bool special = !(amax <= FLT_MAX);
+    if (special) amax = finite_absmax(row, K / 4, lane);
+    const int e = split_exponent(amax);
     const float s = ldexpf(1.0f, e);
     if (lane == 0) inv_scale[m] = ldexpf(1.0f, -e);
     __half2 *h2 = reinterpret_cast<__half2 *>(hi + static_cast<size_t>(m) * K);
     __half2 *l2 = (lo != nullptr) ? reinterpret_cast<__half2 *>(lo + static_cast<size_t>(m) * K) : nullptr;
     for (int i = lane; i < K / 4; i += 32) {
-        const float4 v = row[i];
-        const float a[4] = {v.x * s, v.y * s, v.z * s, v.w * s};
-        __half h[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) h[j] = __float2half_rn(a[j]);
-        h2[2 * i] = __halves2half2(h[0], h[1]);
-        h2[2 * i + 1] = __halves2half2(h[2], h[3]);
+        __half2 h[2], l[2];
+        if (special) split4<true>(row[i], s, h, l);
+        else split4<false>(row[i], s, h, l);
+        h2[2 * i] = h[0];
+        h2[2 * i + 1] = h[1];
         if (l2 != nullptr) {
-            __half l[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) l[j] = __float2half_rn(a[j] - __half2float(h[j]));   // the difference is exact in fp32
-            l2[2 * i] = __halves2half2(l[0], l[1]);
-            l2[2 * i + 1] = __halves2half2(l[2], l[3]);
+            l2[2 * i] = l[0];
+            l2[2 * i + 1] = l[1];
         }
     }
 }

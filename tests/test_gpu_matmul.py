@@ -322,3 +322,59 @@ def test_lm_head_f16(pkg, gpu, oracle, M, N, K):
     gpu.f16w_matmul(wh, torch.from_numpy(x).cuda(), M, C, N)
     gpu.synchronize()
     assert rel_err(C.cpu().numpy(), oracle.lmhead_f16w(x, w16)) < 1e-3
+
+
+@pytest.mark.parametrize("M,K", [(1, 512), (5, 512), (8, 1088), (9, 512), (15, 64), (16, 512), (33, 512), (1, 544), (4, 544)])
+@pytest.mark.parametrize("weights", ["finite", "special"])
+def test_lm_head_f16_rows_of_any_magnitude(pkg, gpu, M, K, weights):
+    """Huge, tiny and subnormal rows keep their precision; infinities and NaNs appear in the outputs where a 64-bit
+    evaluation has them.  M < 16 and M >= 16 are different kernels, K % 64 != 0 a third."""
+    import torch
+    if weights == "special" and M >= 16:
+        pytest.skip("infinite weights with 16 and more rows are not part of the contract")
+    N = 200
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M * K)
+    w = (torch.randn((N, K), device="cuda", generator=g) * 0.02).half()
+    w[11] = 0.0
+    if weights == "special":
+        w[5, 8], w[6, K - 1], w[7, 3] = float("inf"), float("-inf"), float("nan")
+        w[150, 1], w[150, 2] = float("inf"), float("-inf")
+    wh = gpu.f16w_dev(w, N, K)
+    base = torch.randn((K,), device="cuda", generator=g)
+    base[7] = 0.0                                             # of a row without remainder there
+
+    def spiked(**at):
+        r = base.clone()
+        for i, v in at.items():
+            r[int(i[1:])] = v
+        return r
+
+    inf = float("inf")
+    rows = [spiked(i7=1e34), spiked(i7=2e35), spiked(i7=3.3e38), spiked(i7=-3.4028234663852886e38), base * 1e-30, base * 1e-36, base * 1e-38, base * 1e-41, base * 0.0,
+            spiked(i7=inf), spiked(i33=-inf), spiked(i3=inf, i9=-inf), spiked(i3=inf, i9=inf, i12=3e38), spiked(i60=float("nan")), base]
+    if K % 64 == 0:                                           # (partial sums of the CUDA-core kernel may overflow here)
+        rows += [base * 1e37, base * 1e38]
+
+    def classes(t):
+        return torch.where(t.isnan(), 3, torch.where(t == inf, 1, torch.where(t == -inf, 2, 0)))
+
+    C = torch.empty((M, N), device="cuda")
+    for i, r in enumerate(rows):
+        x = base.repeat(M, 1)
+        x[i % M] = r
+        gpu.f16w_matmul(wh, x, M, C, N)
+        gpu.synchronize()
+        ref = x.double() @ w.double().t()
+        assert torch.equal(classes(C), classes(ref.float())), (i, int((classes(C) != classes(ref.float())).sum()))
+        ok = classes(ref.float()) == 0
+        err = torch.where(ok, (C.double() - ref).abs(), 0.0)
+        mag = x.double().abs() @ w.double().abs().t()         # sum of |x w|
+        # M < 16: an element's split error 2^-23, fp32 sums of at most 32 + K/512 + 16 (CUDA cores: K/32 + 5) rounded or truncated
+        # partials; one rounding of a subnormal result, for the CUDA cores of each product.  M >= 16: the hardware's accumulation,
+        # as bounded in test_gpu_baseline_shapes.py, 2e-4 of the row's rms (finite rows only)
+        if M < 16:
+            bound = 2.0 ** -23 * 60 * mag + 2.0 ** -149 * (K if K % 64 else 1)
+        else:
+            bound = 2e-4 * ref.pow(2).mean(1, keepdim=True).sqrt() + 2.0 ** -149
+        assert bool((~ok | (err <= bound)).all()), (i, float(torch.where(ok, err / bound, 0.0).max()))
