@@ -284,33 +284,33 @@ int launch_f16w_matmul(inkq_ctx *ctx, const F16W *w, const float *x, int M, floa
     const int grid = min((w->rows + 7) / 8, ctx->num_sms * 8);
     const size_t rows_smem = static_cast<size_t>(2 * F16R_COLS) * f16r_pitch(w->K) + sizeof(float) * (2 * F16R_WARPS * F16R_COLS * 16 + 2 * F16R_COLS);
     if (w->K % 64 == 0 && rows_smem <= 226 * 1024) {
-        INKQ_CUDA(ctx, cudaFuncSetAttribute(k_f16w_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(rows_smem)));
+        int rc = allow_smem<k_f16w_rows>(ctx);
+        if (rc) return rc;
         const int tiles = (w->rows + 15) / 16;
         for (int m0 = 0; m0 < M; m0 += F16R_COLS) {
             const cudaError_t e = launch_pdl(k_f16w_rows, dim3(min(tiles, ctx->num_sms)), dim3(F16R_WARPS * 32), rows_smem, ctx->stream, w->w, x, m0,
                                              min(F16R_COLS, M - m0), w->rows, w->K, C, ldc, extra);
             if (e != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("k_f16w_rows launch: ") + cudaGetErrorString(e));
-            int rc = after_launch(ctx, "k_f16w_rows");
-            if (rc) return rc;
+            if ((rc = after_launch(ctx, "k_f16w_rows"))) return rc;
         }
         return INKQ_OK;
     }
     // other row lengths: one or four rows per pass on the CUDA cores
     if (M == 1) {
         const size_t smem = static_cast<size_t>(w->K) * sizeof(float);
-        if (smem > 48 * 1024) cudaFuncSetAttribute(k_f16w_gemv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        const int rc = allow_smem<k_f16w_gemv<1>>(ctx);
+        if (rc) return rc;
         k_f16w_gemv<1><<<grid, 256, smem, ctx->stream>>>(w->w, x, 0, M, w->rows, w->K, C, ldc, extra);
         return after_launch(ctx, "k_f16w_gemv");
     }
     const size_t smem = 4 * static_cast<size_t>(w->K) * sizeof(float);
     if (smem > 200 * 1024) return fail(ctx, INKQ_ERR_UNSUPPORTED, "K too large for the fp16-weight matmul");
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_f16w_gemv<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    for (int m0 = 0; m0 < M; m0 += 4) {
+    int rc = allow_smem<k_f16w_gemv<4>>(ctx);
+    for (int m0 = 0; m0 < M && !rc; m0 += 4) {
         k_f16w_gemv<4><<<grid, 256, smem, ctx->stream>>>(w->w, x, m0, M, w->rows, w->K, C, ldc, extra);
-        int rc = after_launch(ctx, "k_f16w_gemv");
-        if (rc) return rc;
+        rc = after_launch(ctx, "k_f16w_gemv");
     }
-    return INKQ_OK;
+    return rc;
 }
 
 // Weight-only W41 on the CUDA cores (cross-check of the tensor-core kernel): one output per thread,

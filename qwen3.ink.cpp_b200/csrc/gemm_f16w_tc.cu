@@ -40,8 +40,6 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
-#include <mutex>
-
 #include "f16w_split.cuh"
 #include "inkq_internal.h"
 #include "ptx.cuh"
@@ -350,17 +348,7 @@ int launch_f16w_gemm_tc(inkq_ctx *ctx, const F16W *w, const float *x, int M, flo
     prm.tiles_m = tiles_m;
     prm.block_m = block_m;
     prm.ldc = ldc;
-    {
-        static std::mutex mu;
-        static bool configured[64] = {};
-        if (ctx->device < 0 || ctx->device >= 64) return fail(ctx, INKQ_ERR_UNSUPPORTED, "device index beyond the launch table");
-        std::lock_guard<std::mutex> lk(mu);
-        if (!configured[ctx->device]) {   // the opt-in for large dynamic shared memory is per device
-            cudaError_t e = cudaFuncSetAttribute(k_gemm_f16w_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-            if (e != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("cudaFuncSetAttribute(k_gemm_f16w_tc): ") + cudaGetErrorString(e));
-            configured[ctx->device] = true;
-        }
-    }
+    if ((rc = allow_smem<k_gemm_f16w_tc>(ctx))) return rc;
     const long long total = static_cast<long long>(prm.groups_n) * tiles_m;
     const int grid = static_cast<int>(total < ctx->num_sms ? total : ctx->num_sms);
     k_gemm_f16w_tc<<<grid, THREADS, SMEM_BYTES, ctx->stream>>>(map_w, map_x, map_xlo, prm);

@@ -159,17 +159,23 @@ bool gemm_w41_rows_fits(const uint16_t *a16, int M, int K)
     return nt <= 2 && (reinterpret_cast<uintptr_t>(a16) & 15) == 0 && 8 * nt * (pitch_for(K) + 2 * WARPS * 16 * static_cast<int>(sizeof(float))) <= 226 * 1024;
 }
 
-int launch_gemm_w41_rows(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc)
+template <int NT>
+static int launch_rows(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc)
 {
     using namespace w41rows;
-    const int nt = (M + 7) / 8, smem = 8 * nt * (pitch_for(w->K) + 2 * WARPS * 16 * static_cast<int>(sizeof(float)));
-    auto kernel = nt == 1 ? k_gemm_w41_rows<1> : k_gemm_w41_rows<2>;
-    INKQ_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const int rc = allow_smem<k_gemm_w41_rows<NT>>(ctx);
+    if (rc) return rc;
     const int tiles = (w->rows + 15) / 16;
-    const cudaError_t e = launch_pdl(kernel, dim3(tiles < ctx->num_sms ? tiles : ctx->num_sms), dim3(WARPS * 32), smem, ctx->stream, w->nibT, w->sc16, a16, M,
+    const cudaError_t e = launch_pdl(k_gemm_w41_rows<NT>, dim3(tiles < ctx->num_sms ? tiles : ctx->num_sms), dim3(WARPS * 32),
+                                     8 * NT * (pitch_for(w->K) + 2 * WARPS * 16 * static_cast<int>(sizeof(float))), ctx->stream, w->nibT, w->sc16, a16, M,
                                      w->rows, w->K, C, ldc);
     if (e != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("k_gemm_w41_rows launch: ") + cudaGetErrorString(e));
     return after_launch(ctx, "k_gemm_w41_rows");
+}
+
+int launch_gemm_w41_rows(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc)
+{
+    return M <= 8 ? launch_rows<1>(ctx, a16, M, w, C, ldc) : launch_rows<2>(ctx, a16, M, w, C, ldc);
 }
 
 }  // namespace inkq

@@ -92,20 +92,20 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : 2) k_gemv_w41(con
 }
 
 template <int WARPS>
-static void launch_variant(inkq_ctx *ctx, const uint16_t *a16, const Weight *w, float *C)
+static int launch_variant(inkq_ctx *ctx, const uint16_t *a16, const Weight *w, float *C)
 {
     const size_t smem = sizeof(float) * (static_cast<size_t>(w->K) + WARPS * 32);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_gemv_w41<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const int rc = allow_smem<k_gemv_w41<WARPS>>(ctx);
+    if (rc) return rc;
     launch_pdl(k_gemv_w41<WARPS>, dim3(static_cast<unsigned>(w->tiles) * 4), dim3(WARPS * 32), smem, ctx->stream, static_cast<const uint8_t *>(w->nibT),
                static_cast<const uint2 *>(w->sc16), reinterpret_cast<const __half *>(a16), C, w->rows, w->K, w->pairs);
+    return after_launch(ctx, "k_gemv_w41");
 }
 
 int launch_gemv_w41(inkq_ctx *ctx, const uint16_t *a16, const Weight *w, float *C)
 {
     const bool wide_cta = (w->tiles * 4 <= 2 * ctx->num_sms) || (w->pairs >= 128);
-    if (wide_cta) launch_variant<16>(ctx, a16, w, C);
-    else launch_variant<8>(ctx, a16, w, C);
-    return after_launch(ctx, "k_gemv_w41");
+    return wide_cta ? launch_variant<16>(ctx, a16, w, C) : launch_variant<8>(ctx, a16, w, C);
 }
 
 }  // namespace inkq

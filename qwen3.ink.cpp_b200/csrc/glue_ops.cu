@@ -19,8 +19,6 @@
 #include <cuda_fp16.h>
 #include <math.h>
 
-#include <mutex>
-
 #include "glue_math.cuh"
 #include "inkq_glue.h"
 #include "inkq_internal.h"
@@ -735,7 +733,7 @@ static int attention_impl(inkq_ctx *ctx, const float *q_dev, const uint16_t *k_c
         const int share_max = (max_pos + ATT_S - 1) / ATT_S;
         const size_t smem_s = sizeof(float) * (HEAD_DIM + ATT_SPLIT_NW * HEAD_DIM + 2 * ATT_SPLIT_NW + static_cast<size_t>(share_max));
         INKQ_REQUIRE(ctx, smem_s <= 200 * 1024, "context too long for the decode attention kernel");
-        if (smem_s > 48 * 1024) cudaFuncSetAttribute(k_attention_split, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_s));
+        if ((rc = allow_smem<k_attention_split>(ctx))) return rc;
         launch_pdl(k_attention_split, dim3(nq * ATT_S), dim3(ATT_SPLIT_NT), smem_s, ctx->stream, q_dev, reinterpret_cast<const __half *>(k_cache_dev),
                    reinterpret_cast<const __half *>(v_cache_dev), pos0_dev, nq, nkv, max_pos, scale, out_dev, qo, fz);
         return after_launch(ctx, "k_attention_split");
@@ -748,10 +746,10 @@ static int attention_impl(inkq_ctx *ctx, const float *q_dev, const uint16_t *k_c
     INKQ_REQUIRE(ctx, smem <= 200 * 1024, "context too long for the simple attention kernel");
     const __half *kc = reinterpret_cast<const __half *>(k_cache_dev), *vc = reinterpret_cast<const __half *>(v_cache_dev);
     if (wide) {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(k_attention<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if ((rc = allow_smem<k_attention<512>>(ctx))) return rc;
         launch_pdl(k_attention<512>, dim3(T * nq), dim3(512), smem, ctx->stream, q_dev, kc, vc, pos0_dev, T, nq, nkv, max_pos, scale, out_dev, qo);
     } else {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(k_attention<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if ((rc = allow_smem<k_attention<128>>(ctx))) return rc;
         k_attention<128><<<T * nq, 128, smem, ctx->stream>>>(q_dev, kc, vc, pos0_dev, T, nq, nkv, max_pos, scale, out_dev, qo);
     }
     return after_launch(ctx, "k_attention");
@@ -803,16 +801,7 @@ int inkq_glue_add_rmsnorm_quant_rows(inkq_ctx *ctx, float *x_dev, const float *d
     INKQ_REQUIRE(ctx, out_qmode == INKQ_Q8_1_F16 || out_qmode == INKQ_Q8_0_F16 || out_qmode == INKQ_Q8_1_F32, "bad output quantization mode");
     const int M_ld = (M + 3) & ~3;
     const size_t smem = static_cast<size_t>(K) * sizeof(float);
-    if (smem + 64 > 48 * 1024) {   // the kernel also holds 32 bytes of static shared memory
-        static std::mutex mu;
-        static bool configured[64] = {};
-        std::lock_guard<std::mutex> g(mu);
-        if (ctx->device < 0 || ctx->device >= 64) return fail(ctx, INKQ_ERR_INVALID, "device index out of range");
-        if (!configured[ctx->device]) {
-            INKQ_CUDA(ctx, cudaFuncSetAttribute(k_add_rmsnorm_quant_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
-            configured[ctx->device] = true;
-        }
-    }
+    if ((rc = allow_smem<k_add_rmsnorm_quant_rows>(ctx))) return rc;
     launch_pdl(k_add_rmsnorm_quant_rows, dim3(M_ld), dim3(256), smem, ctx->stream, x_dev, delta_dev, norm_w_dev, M, K, eps, M_ld, out_qmode, out->q, out->d,
                out->s, out->isum, xn_out_dev);
     out->M = M;

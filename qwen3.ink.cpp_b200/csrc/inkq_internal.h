@@ -6,6 +6,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
 #include <string>
 
 #include "inkq.h"
@@ -162,6 +163,26 @@ static inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 b
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+constexpr int MAX_DEVICES = 64;
+
+// Lets `kernel` be launched with all the dynamic shared memory that an SM has beside the kernel's static part.  The limit is an
+// attribute of the function on a device, which every context and thread shares: set once to the most a launch may ask for.  Set to
+// what a call needs, it was lowered by a call with shorter rows between another thread's setting and launch.
+template <auto kernel>
+inline int allow_smem(inkq_ctx *ctx)
+{
+    static std::atomic<bool> done[MAX_DEVICES];
+    if (ctx->device < 0 || ctx->device >= MAX_DEVICES) return fail(ctx, INKQ_ERR_UNSUPPORTED, "device index beyond the launch table");
+    if (done[ctx->device].load(std::memory_order_acquire)) return INKQ_OK;
+    cudaFuncAttributes fa;
+    int optin = 0;
+    INKQ_CUDA(ctx, cudaFuncGetAttributes(&fa, kernel));
+    INKQ_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    INKQ_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - static_cast<int>(fa.sharedSizeBytes)));
+    done[ctx->device].store(true, std::memory_order_release);
+    return INKQ_OK;
 }
 
 // Tiled 2-D tensor map (rows of dim0 elements, pitch_elems apart), 128-byte L2 promotion, zero fill outside

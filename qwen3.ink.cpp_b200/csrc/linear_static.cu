@@ -41,7 +41,6 @@ static_assert(STATIC_BYTES == 40 * 1024, "the documented size of the static scra
 // In host code this name is only a handle for cudaGetSymbolAddress, never a pointer to pass on.
 static __device__ __align__(256) unsigned char g_static_scratch[STATIC_BYTES];
 
-constexpr int MAX_DEVICES = 64;
 static std::mutex g_static_mu;
 static unsigned char *g_static_ptr[MAX_DEVICES];  // device address of the array, per device
 

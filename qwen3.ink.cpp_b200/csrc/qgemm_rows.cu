@@ -42,7 +42,6 @@
 #include <cuda_fp16.h>
 
 #include <initializer_list>
-#include <mutex>
 
 #include "inkq_internal.h"
 #include "ptx.cuh"
@@ -337,30 +336,18 @@ __global__ void __launch_bounds__(32 * T::WR * T::WC, T::CTAS)
         }
 }
 
-constexpr int MAX_DEVICES = 64;
-
 template <int SCH, bool S16, class T, bool DUMP = false>
 static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin, Params prm)
 {
     using G = Cfg<SCH, S16, T>;
     auto kernel = k_qgemm_rows<SCH, S16, T, DUMP>;
-    // The opt-in for large dynamic shared memory is a per-device function attribute: remembered per device and instantiation
-    static std::mutex mu;
-    static bool configured[MAX_DEVICES] = {};
-    if (ctx->device < 0 || ctx->device >= MAX_DEVICES) return fail(ctx, INKQ_ERR_UNSUPPORTED, "device index beyond the launch table");
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!configured[ctx->device]) {
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SM);
-            if (e != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("cudaFuncSetAttribute(k_qgemm_rows): ") + cudaGetErrorString(e));
-            configured[ctx->device] = true;
-        }
-    }
+    int rc = allow_smem<k_qgemm_rows<SCH, S16, T, DUMP>>(ctx);
+    if (rc) return rc;
     const int nb = a->K / QK;
     CUtensorMap mq, md, ms;
     // a row window starts m_begin rows into q and m_begin entries into every block's line of the planes
-    int rc = encode_map_2d(ctx, &mq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->q + static_cast<size_t>(m_begin) * a->K, a->K, prm.M, 128u, G::BM,
-                           CU_TENSOR_MAP_SWIZZLE_128B, a->K);
+    rc = encode_map_2d(ctx, &mq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->q + static_cast<size_t>(m_begin) * a->K, a->K, prm.M, 128u, G::BM,
+                       CU_TENSOR_MAP_SWIZZLE_128B, a->K);
     if (!rc) rc = encode_map_2d(ctx, &md, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->d + m_begin, a->M_ld - m_begin, nb, G::BM, 2 * G::SP, CU_TENSOR_MAP_SWIZZLE_NONE,
                                 a->M_ld);
     ms = md;

@@ -44,8 +44,6 @@
 
 #include <math.h>
 
-#include <mutex>
-
 #include "inkq_internal.h"
 #include "ptx.cuh"
 
@@ -352,8 +350,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm_w41_tc(const __grid_constan
     }
 }
 
-constexpr int MAX_DEVICES = 64;
-
 template <int NT>
 static int launch(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc, int block_m)
 {
@@ -378,18 +374,7 @@ static int launch(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, fl
     prm.raw_bytes = sh.raw_bytes();
     prm.a_slots = sh.a_slots();
     prm.acc_slots = sh.acc_slots();
-    // The opt-in for large dynamic shared memory is a per-device function attribute
-    static std::mutex mu;
-    static bool configured[MAX_DEVICES] = {};
-    if (ctx->device < 0 || ctx->device >= MAX_DEVICES) return fail(ctx, INKQ_ERR_UNSUPPORTED, "device index beyond the launch table");
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!configured[ctx->device]) {
-            const cudaError_t e = cudaFuncSetAttribute(k_gemm_w41_tc<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-            if (e != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("cudaFuncSetAttribute(k_gemm_w41_tc): ") + cudaGetErrorString(e));
-            configured[ctx->device] = true;
-        }
-    }
+    if ((rc = allow_smem<k_gemm_w41_tc<NT>>(ctx))) return rc;
     const int total = prm.groups_n * prm.tiles_m;
     const cudaError_t e = launch_pdl(k_gemm_w41_tc<NT>, dim3(total < ctx->num_sms ? total : ctx->num_sms), dim3(THREADS), SMEM_BYTES, ctx->stream, map, prm);
     if (e != cudaSuccess) return fail(ctx, INKQ_ERR_CUDA, std::string("k_gemm_w41_tc launch: ") + cudaGetErrorString(e));

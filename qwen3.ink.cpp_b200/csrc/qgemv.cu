@@ -230,11 +230,11 @@ __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_S
 }
 
 template <bool HAS_MIN, int WARPS, int FUSED, bool DEEP = false>
-static void launch_gemv_variant(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const ExtraDst &extra, const FusedM1 &fused)
+static int launch_gemv_variant(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const ExtraDst &extra, const FusedM1 &fused)
 {
     const size_t smem = static_cast<size_t>(w->K) + 2 * sizeof(float) * (w->K / QK) + sizeof(float) * WARPS * 32;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_qgemv_a8w4<HAS_MIN, WARPS, FUSED, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const int rc = allow_smem<k_qgemv_a8w4<HAS_MIN, WARPS, FUSED, DEEP>>(ctx);
+    if (rc) return rc;
     // launched with programmatic stream serialization: the grid may begin (and prefetch weights) before the
     // previous kernel in the stream has finished; it waits for that kernel inside (griddepcontrol.wait)
     cudaLaunchConfig_t cfg = {};
@@ -251,23 +251,22 @@ static void launch_gemv_variant(inkq_ctx *ctx, const Act *a, const Weight *w, fl
                        static_cast<const uchar2 *>(w->zpT), static_cast<const int8_t *>(a ? a->q : nullptr),
                        static_cast<const float *>(a ? a->d : nullptr), static_cast<const float *>(a ? a->s : nullptr),
                        static_cast<const int32_t *>(a ? a->isum : nullptr), a ? a->M_ld : 0, C, w->rows, w->K, w->pairs, extra, fused);
+    return after_launch(ctx, FUSED == FUSED_NONE ? "k_qgemv_a8w4" : "k_qgemv_a8w4 (fused prologue)");
 }
 
 template <int FUSED>
-static void launch_gemv_any(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const ExtraDst &extra, const FusedM1 &fused)
+static int launch_gemv_any(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const ExtraDst &extra, const FusedM1 &fused)
 {
     // narrow layers (few CTAs) or long rows: 16 K-slices per CTA
     const bool wide_cta = (w->tiles * 4 <= 2 * ctx->num_sms) || (w->pairs >= 128);
     // no more CTAs than SMs and long rows: one CTA per SM with four batches in flight per lane (same accumulation order)
     const bool deep = wide_cta && gemv_deep(w->tiles * 4, w->pairs, 16, ctx->num_sms);
     if (w->scheme == INKQ_A81W41) {
-        if (deep) launch_gemv_variant<true, 16, FUSED, true>(ctx, a, w, C, extra, fused);
-        else if (wide_cta) launch_gemv_variant<true, 16, FUSED>(ctx, a, w, C, extra, fused);
-        else launch_gemv_variant<true, 8, FUSED>(ctx, a, w, C, extra, fused);
+        if (deep) return launch_gemv_variant<true, 16, FUSED, true>(ctx, a, w, C, extra, fused);
+        return wide_cta ? launch_gemv_variant<true, 16, FUSED>(ctx, a, w, C, extra, fused) : launch_gemv_variant<true, 8, FUSED>(ctx, a, w, C, extra, fused);
     } else {
-        if (deep) launch_gemv_variant<false, 16, FUSED, true>(ctx, a, w, C, extra, fused);
-        else if (wide_cta) launch_gemv_variant<false, 16, FUSED>(ctx, a, w, C, extra, fused);
-        else launch_gemv_variant<false, 8, FUSED>(ctx, a, w, C, extra, fused);
+        if (deep) return launch_gemv_variant<false, 16, FUSED, true>(ctx, a, w, C, extra, fused);
+        return wide_cta ? launch_gemv_variant<false, 16, FUSED>(ctx, a, w, C, extra, fused) : launch_gemv_variant<false, 8, FUSED>(ctx, a, w, C, extra, fused);
     }
 }
 
@@ -275,8 +274,7 @@ int launch_gemv(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const Ex
 {
     ExtraDst extra = {};
     if (extra_in != nullptr) extra = *extra_in;
-    launch_gemv_any<FUSED_NONE>(ctx, a, w, C, extra, FusedM1{});
-    return after_launch(ctx, "k_qgemv_a8w4");
+    return launch_gemv_any<FUSED_NONE>(ctx, a, w, C, extra, FusedM1{});
 }
 
 int launch_gemv_fused(inkq_ctx *ctx, const Weight *w, const float *x, int pro, const float *g, float eps, float *C, int accumulate)
@@ -288,9 +286,7 @@ int launch_gemv_fused(inkq_ctx *ctx, const Weight *w, const float *x, int pro, c
     f.pro = pro;
     f.qmode = (w->scheme == INKQ_A81W41) ? INKQ_Q8_1_F16 : INKQ_Q8_0_F16;   // as inkq_linear chooses for M == 1
     f.accumulate = accumulate;
-    if (pro == PRO_PLAIN) launch_gemv_any<FUSED_PLAIN>(ctx, nullptr, w, C, ExtraDst{}, f);
-    else launch_gemv_any<FUSED_ANY>(ctx, nullptr, w, C, ExtraDst{}, f);
-    return after_launch(ctx, "k_qgemv_a8w4 (fused prologue)");
+    return pro == PRO_PLAIN ? launch_gemv_any<FUSED_PLAIN>(ctx, nullptr, w, C, ExtraDst{}, f) : launch_gemv_any<FUSED_ANY>(ctx, nullptr, w, C, ExtraDst{}, f);
 }
 
 }  // namespace inkq

@@ -277,10 +277,11 @@ __global__ void __launch_bounds__(512) k_rmsnorm_quant_row(const float *x, const
 }
 
 template <bool HAS_MIN, int WARPS, bool DEEP, bool PAIR>
-static void launch_decode_epi(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const DecodeEpi &epi, const PendingNorm &pend)
+static int launch_decode_epi(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const DecodeEpi &epi, const PendingNorm &pend)
 {
     const size_t smem = static_cast<size_t>(w->K) + 2 * sizeof(float) * (w->K / QK) + sizeof(float) * WARPS * 32;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_qgemv_decode<HAS_MIN, WARPS, DEEP, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const int rc = allow_smem<k_qgemv_decode<HAS_MIN, WARPS, DEEP, PAIR>>(ctx);
+    if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(w->tiles) * (PAIR ? 2 : 4));
     cfg.blockDim = dim3(WARPS * 32);
@@ -294,13 +295,14 @@ static void launch_decode_epi(inkq_ctx *ctx, const Act *a, const Weight *w, floa
     cudaLaunchKernelEx(&cfg, k_qgemv_decode<HAS_MIN, WARPS, DEEP, PAIR>, static_cast<const uint8_t *>(w->nibT), static_cast<const uint2 *>(w->sc16),
                        static_cast<const uchar2 *>(w->zpT), static_cast<const int8_t *>(a->q), static_cast<const float *>(a->d),
                        static_cast<const float *>(a->s), static_cast<const int32_t *>(a->isum), a->M_ld, C, w->rows, w->K, w->pairs, epi, pend);
+    return after_launch(ctx, "k_qgemv_decode");
 }
 
 template <bool HAS_MIN, int WARPS, bool DEEP = false>
-static void launch_decode_variant(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const DecodeEpi &epi, const PendingNorm &pend)
+static int launch_decode_variant(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, const DecodeEpi &epi, const PendingNorm &pend)
 {
-    if (epi.mode == EPI_PAIR_SILUQ) launch_decode_epi<HAS_MIN, WARPS, DEEP, true>(ctx, a, w, C, epi, pend);
-    else launch_decode_epi<HAS_MIN, WARPS, DEEP, false>(ctx, a, w, C, epi, pend);
+    if (epi.mode == EPI_PAIR_SILUQ) return launch_decode_epi<HAS_MIN, WARPS, DEEP, true>(ctx, a, w, C, epi, pend);
+    return launch_decode_epi<HAS_MIN, WARPS, DEEP, false>(ctx, a, w, C, epi, pend);
 }
 
 }  // namespace inkq
@@ -371,15 +373,12 @@ int inkq_glue_decode_gemv(inkq_ctx *ctx, const inkq_weight *w, const inkq_act *i
     const int ctas = w->tiles * (epilogue == EPI_PAIR_SILUQ ? 2 : 4);
     const bool deep = wide_cta && gemv_deep(ctas, w->pairs, 16, ctx->num_sms);
     if (w->scheme == INKQ_A81W41) {
-        if (deep) launch_decode_variant<true, 16, true>(ctx, in, w, C_dev, epi, pend);
-        else if (wide_cta) launch_decode_variant<true, 16>(ctx, in, w, C_dev, epi, pend);
-        else launch_decode_variant<true, 8>(ctx, in, w, C_dev, epi, pend);
+        if (deep) return launch_decode_variant<true, 16, true>(ctx, in, w, C_dev, epi, pend);
+        return wide_cta ? launch_decode_variant<true, 16>(ctx, in, w, C_dev, epi, pend) : launch_decode_variant<true, 8>(ctx, in, w, C_dev, epi, pend);
     } else {
-        if (deep) launch_decode_variant<false, 16, true>(ctx, in, w, C_dev, epi, pend);
-        else if (wide_cta) launch_decode_variant<false, 16>(ctx, in, w, C_dev, epi, pend);
-        else launch_decode_variant<false, 8>(ctx, in, w, C_dev, epi, pend);
+        if (deep) return launch_decode_variant<false, 16, true>(ctx, in, w, C_dev, epi, pend);
+        return wide_cta ? launch_decode_variant<false, 16>(ctx, in, w, C_dev, epi, pend) : launch_decode_variant<false, 8>(ctx, in, w, C_dev, epi, pend);
     }
-    return after_launch(ctx, "k_qgemv_decode");
 }
 
 int inkq_glue_rmsnorm_quant(inkq_ctx *ctx, const float *x_dev, const float *norm_w_dev, float eps, int K, inkq_act *out, int out_qmode,
