@@ -214,7 +214,7 @@ int inkq_gemm_w41_f16act_simt(inkq_ctx *ctx, const uint16_t *a16_dev, int M, con
 int inkq_f16w_create(inkq_ctx *ctx, int N, int K, const uint16_t *w16_host, int n_begin, int n_end, inkq_f16w **out);
 int inkq_f16w_create_dev(inkq_ctx *ctx, int N, int K, const uint16_t *w16_dev, int n_begin, int n_end, inkq_f16w **out);
 int inkq_f16w_destroy(inkq_f16w *w);
-/* C[m][n] = sum_k x[m][k] * w[n][k].
+/* C[m][n] = sum_k x[m][k] * w[n][k].  x_dev must be 16-byte aligned (INKQ_ERR_INVALID otherwise).
  * M < 16 (or an output that is not 16-byte aligned): bandwidth-bound, warp-level products; the fp32 activations enter as
  * fp16 hi + lo parts of the row scaled by a power of two (22 significant bits), sums in fp32: about 1.3e-7 of the output's
  * 2-norm from the exact result, and a batch has the bits of its rows one by one.  K % 64 != 0: CUDA cores, fp32

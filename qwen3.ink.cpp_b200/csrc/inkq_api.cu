@@ -852,10 +852,10 @@ int inkq::f16w_matmul_impl(inkq_ctx *ctx, const inkq_f16w *w, const float *x_dev
     INKQ_REQUIRE(ctx, w != nullptr && x_dev != nullptr && C_dev != nullptr, "null handle, input or output");
     INKQ_REQUIRE(ctx, M >= 1 && ldc >= w->rows, "bad M or ldc");
     INKQ_REQUIRE(ctx, precision == INKQ_F16W_ACT_FP32 || precision == INKQ_F16W_ACT_FP16, "unknown precision");
+    INKQ_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(x_dev) & 15) == 0, "x must be 16-byte aligned");   // every kernel below reads 16-byte pieces
     // few rows: the weights are streamed once per 8 rows
     const bool aligned = w->rows % 4 == 0 && ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C_dev) & 15) == 0;
     if (M < 16 || w->K % 64 != 0 || !aligned) return launch_f16w_matmul(ctx, w, x_dev, M, C_dev, ldc, extra);
-    INKQ_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(x_dev) & 15) == 0, "x must be 16-byte aligned");
     const int passes = precision == INKQ_F16W_ACT_FP32 ? 2 : 1;
     const size_t need = static_cast<size_t>(M) * w->K * passes;
     if (ctx->f16_x_cap < need) {

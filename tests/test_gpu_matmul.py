@@ -378,3 +378,20 @@ def test_lm_head_f16_rows_of_any_magnitude(pkg, gpu, M, K, weights):
         else:
             bound = 2e-4 * ref.pow(2).mean(1, keepdim=True).sqrt() + 2.0 ** -149
         assert bool((~ok | (err <= bound)).all()), (i, float(torch.where(ok, err / bound, 0.0).max()))
+
+
+@pytest.mark.parametrize("M,K", [(1, 64), (8, 64), (9, 64), (16, 64), (2, 40)])
+def test_lm_head_f16_refuses_unaligned_activations(pkg, gpu, M, K):
+    """Every kernel of the head reads the activations in 16-byte pieces: the host refuses a pointer that does not allow it."""
+    import torch
+    wh = gpu.f16w(pkg.synth.lm_head(16, K, 6))
+    x = torch.zeros((M * K + 4,), device="cuda")
+    C = torch.full((M, 16), -5.0, device="cuda")
+    before = gpu.launches
+    with pytest.raises(pkg.InkqError) as e:
+        gpu.f16w_matmul(wh, x[1:], M, C, 16)
+    gpu.synchronize()
+    assert e.value.code == pkg.ERR_INVALID and gpu.launches == before and bool((C == -5.0).all())
+    gpu.f16w_matmul(wh, x[4:], M, C, 16)
+    gpu.synchronize()
+    assert bool((C == 0.0).all())
