@@ -17,7 +17,8 @@ shape: M=322 activations x K=4096, N=12288 A81W41 weights (fp32 block scales).
           and a barrier kernel completes the step (strong scaling; the same step with an
           NCCL all-gather is timed beside it, and is the fallback when peer mapping fails)
   --impl reference   the reference project's own AVX kernels (oracle/_ref, compiled
-          unmodified) on this box's host cores, same shape, all host threads
+          unmodified) on this box's host cores, same shape, all host threads; a line that
+          says "unavailable" where they were never compiled
 The line also carries the roofline of the dominant kernel, the reference's CPU kernels timed on
 this box, the decode QGEMV sweep, the scheme matrix and pp322 / tg128 of a synthetic Qwen3-8B
 (--no-gemv / --no-model skip the last three).  Other workloads (--workload): qgemv_sweep,
@@ -150,34 +151,24 @@ def cuda_time_ms(torch, fn, iters):
 def run_reference(args, rank, world):
     if rank != 0:
         return
-    from oracle.inkq_oracle import Oracle, Reference
+    from oracle.inkq_oracle import Reference
+    if Reference.available_path()[0] is None:
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's kernels are not compiled here for this host (oracle/_ref: make -C oracle ref, where its checkout is present)"}),
+              flush=True)
+        return
     pkg = load_package()
     M, K, N = M_PP, K_PP, N_PP
     x = pkg.synth.activations(M, K)
     w = pkg.synth.weights(N, K)
     cores = host_threads()
-    kind = "reference" if Reference.available_path()[0] else "port"
-    isa = "scalar"
-    if kind == "reference":
-        ref = Reference()
-        isa = ref.isa
-        B = ref.repack(w["nib"], w["d"], w["m"], 2)
+    ref = Reference()
+    B = ref.repack(w["nib"], w["d"], w["m"], 2)
 
-        def step():
-            A = ref.quantize_struct(x, 2, pad_rows=6 * K // 64, prefill=0)     # quantize_row_q8_1_repack_fp32
-            return ref.matmul("gemm_repack_A81W41_fp32", A, B, M, N, K)       # gemm_repack_A81W41_fp32
-        sample = (f"full workload: quantize_row_q8_1_repack_fp32 (1 thread, as the reference) + gemm_repack_A81W41_fp32 at {M}x{N}x{K} "
-                  f"with an OpenMP team of {cores} threads (omp_get_max_threads after omp_set_num_threads)")
-        ops = 2.0 * M * N * K
-    else:
-        orc = Oracle()
-        ncols = 1536
-
-        def step():
-            q, d, s = orc.quantize(x, 2)
-            return orc.gemm(0, q, d, s, w["nib"][:ncols], w["d"][:ncols], w["m"][:ncols])
-        sample = f"first {ncols} of {N} output columns (oracle port, OpenMP over columns)"
-        ops = 2.0 * M * ncols * K
+    def step():
+        A = ref.quantize_struct(x, 2, pad_rows=6 * K // 64, prefill=0)     # quantize_row_q8_1_repack_fp32
+        return ref.matmul("gemm_repack_A81W41_fp32", A, B, M, N, K)       # gemm_repack_A81W41_fp32
+    sample = (f"full workload: quantize_row_q8_1_repack_fp32 (1 thread, as the reference) + gemm_repack_A81W41_fp32 at {M}x{N}x{K} "
+              f"with an OpenMP team of {cores} threads (omp_get_max_threads after omp_set_num_threads)")
     for _ in range(args.warmup):
         step()
     t0 = time.perf_counter()
@@ -189,13 +180,13 @@ def run_reference(args, rank, world):
         step()
     total = time.perf_counter() - t0
     dt = total / (args.steps * repeats)
-    tops = ops / dt / 1e12
+    tops = 2.0 * M * N * K / dt / 1e12
     line = {"impl": "reference", "metric": "qgemm_int8_tops_pp322", "value": tops, "unit": "TOPS", "n_gpus": args.gpus,
             "steps": args.steps, "warmup": args.warmup, "repeats": repeats, "timed_region_s": total,
-            "ms_per_step": dt * 1e3 * (2.0 * M * N * K / ops), "higher_is_better": True,
+            "ms_per_step": dt * 1e3, "higher_is_better": True,
             "scaling": "strong", "vs_baseline": None, "dtype": "s8 x u4 -> s32, fp32 scale/accumulate", "data": "synthetic",
-            "config": base_config("qgemm_pp322", M, N, K), "host": {"isa": isa, "omp_threads": cores},
-            "cpu_baseline": {"value": tops, "unit": "TOPS", "cores": cores, "kind": kind, "sample": sample},
+            "config": base_config("qgemm_pp322", M, N, K), "host": {"isa": ref.isa, "omp_threads": cores},
+            "cpu_baseline": {"value": tops, "unit": "TOPS", "cores": cores, "kind": "reference", "sample": sample},
             "e2e": {"value": tops, "unit": "TOPS", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}, "gpu_launches": 0}
     print(json.dumps(line), flush=True)
 
