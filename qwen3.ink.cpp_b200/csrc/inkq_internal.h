@@ -170,8 +170,9 @@ constexpr int MAX_DEVICES = 64;
 // Lets `kernel` be launched with all the dynamic shared memory that an SM has beside the kernel's static part.  The limit is an
 // attribute of the function on a device, which every context and thread shares: set once to the most a launch may ask for.  Set to
 // what a call needs, it was lowered by a call with shorter rows between another thread's setting and launch.
+// (static: `done` of an inline function is one object for every copy of this library in a process, the attribute is not)
 template <auto kernel>
-inline int allow_smem(inkq_ctx *ctx)
+static int allow_smem(inkq_ctx *ctx)
 {
     static std::atomic<bool> done[MAX_DEVICES];
     if (ctx->device < 0 || ctx->device >= MAX_DEVICES) return fail(ctx, INKQ_ERR_UNSUPPORTED, "device index beyond the launch table");

@@ -2,6 +2,10 @@
 attribute of the function that all contexts and threads of a device share.  Without the opt-in a launch is refused on the
 host (an error status), nothing runs."""
 import ctypes as C
+import importlib.util
+import os
+import shutil
+import sys
 import threading
 
 import pytest
@@ -96,3 +100,34 @@ def test_threads_with_long_and_short_rows(pkg, gpu, kind):
     for t in threads:
         t.join()
     assert not errors and not wrong, (errors, wrong)
+
+
+def test_two_copies_of_the_library_in_one_process(pkg, gpu, tmp_path):
+    """Each copy has functions of its own and opts them in itself."""
+    import torch
+    src = os.path.dirname(os.path.abspath(pkg.__file__))
+    for f in os.listdir(src):
+        if f.endswith((".py", ".so")):
+            shutil.copy(os.path.join(src, f), tmp_path)
+    spec = importlib.util.spec_from_file_location("inkq_b200_copy", tmp_path / "__init__.py", submodule_search_locations=[str(tmp_path)])
+    copy = importlib.util.module_from_spec(spec)
+    sys.modules["inkq_b200_copy"] = copy
+    try:
+        spec.loader.exec_module(copy)
+        N, K, M = 136, 5120, 40
+        w, x = pkg.synth.weights(N, K, 7), torch.from_numpy(pkg.synth.activations(M, K, 5)).cuda()
+        out = []
+        for p, ctx in ((pkg, gpu), (copy, copy.Context(0, torch.cuda.current_stream().cuda_stream))):
+            wh, w41, lm = ctx.weight(p.A81W41, p.SCALES_F16, w["nib"], w["d"], w["m"]), ctx.weight(p.W41, p.SCALES_F16, w["nib"], w["d"], w["m"]), ctx.f16w(pkg.synth.lm_head(N, K, 6))
+            c = torch.zeros((6, M, N), device="cuda")
+            ctx.linear(wh, x, M, c[0], N)
+            for i, m in ((1, 8), (2, M)):
+                ctx.gemm_w41_f16act(x.half(), m, w41, c[i], N)
+            for i, m in ((3, 1), (4, M)):
+                ctx.f16w_matmul(lm, x, m, c[i], N)
+            ctx.linear(wh, x, 1, c[5], N)
+            ctx.synchronize()
+            out.append(c)
+        assert torch.equal(*out)
+    finally:
+        del sys.modules["inkq_b200_copy"]
