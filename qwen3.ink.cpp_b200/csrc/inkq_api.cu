@@ -682,11 +682,14 @@ int inkq_linear_host(inkq_ctx *ctx, const inkq_weight *w, const float *x_host, i
         // Both copies (M*K*4 bytes in, M*N*4 bytes out over PCIe) take longer than the arithmetic, so the call works on
         // windows of rows: window i's activations travel to the device on one stream while window i-1 is quantized and
         // multiplied on the context's stream and window i-2's finished rows (contiguous in the result) travel back on
-        // a third.  The first windows are small, so that the device-to-host link, which carries the most bytes, starts
-        // early and then never waits: a window's product is ready before its predecessor's rows have left.
+        // a third.  The first windows are small, so that the way back to the host, which carries the most bytes where N > K,
+        // starts early; the sizes depend on M alone.  Median us over 40 layers with M = 96 to 512, N from 512 to 24576, K from 1088
+        // to 12288: 48, 80, 96 is 1.6 % below 32, 80, 112 (12288 x 4096 with 322 rows 382 -> 368, 4096 x 12288 437 both, single layers
+        // from -12 to +5 %); 64, 96, 96 and 32, 64, 96 are 0.5 and 0.2 % above that.  The bare copies of 12288 x 4096 with 322
+        // rows take 357 us with both directions at once (123 in and 298 out on their own).
         constexpr int MAXC = 8;
         int m0[MAXC + 1], nch = 0, at = 0;
-        const int lead[3] = {32, 80, 112};   // (48, 80, 96: 397 us at M = 322; 16, 32, 64: 381; these: 369)
+        const int lead[3] = {48, 80, 96};
         m0[0] = 0;
         while (nch < 3 && M - at >= lead[nch] + 32) {
             at += lead[nch];
