@@ -170,8 +170,6 @@ int inkq_ctx_create(int device, void *stream, inkq_ctx **out)
     ctx->f16_x_cap = ctx->f16_scale_cap = 0;
     ctx->lin_x = ctx->lin_c = nullptr;
     ctx->lin_x_cap = ctx->lin_c_cap = 0;
-    ctx->pin_x = ctx->pin_c = nullptr;
-    ctx->pin_x_cap = ctx->pin_c_cap = 0;
     ctx->dev_flag = nullptr;
     ctx->host_flag = nullptr;
     ctx->encode_tiled = nullptr;

@@ -1,7 +1,7 @@
 // Thin inline-PTX wrappers for sm_100a: mbarrier, bulk/tensor TMA copies, tcgen05
-// (tensor memory allocation, UMMA issue/commit, TMEM loads), proxy fences.
-// Every wait is bounded: after INKQ_SPIN_LIMIT_CYCLES the wait gives up and
-// returns false so that the kernel can record the failure and leave cleanly.
+// (tensor memory allocation, UMMA issue/commit, TMEM loads), fences.
+// Every wait built on these probes is bounded by INKQ_SPIN_LIMIT_CYCLES, after which
+// the kernel records the failure and leaves cleanly.
 #pragma once
 #include <cuda.h>
 #include <stdint.h>
@@ -72,24 +72,6 @@ __device__ __forceinline__ bool mbar_try_wait_for(uint64_t *bar, uint32_t parity
         : "memory");
     return ok != 0;
 }
-// Bounded wait.  Returns false when the limit ran out, or as soon as *abort (a
-// shared-memory word another role sets when its own wait ran out) is non-zero.
-// After `eager` failed probes the thread sleeps `sleep_ns` between probes (0 = never:
-// for waits on the critical path, a sleep costs far more than the probes it saves), so
-// a role that is far ahead of its consumer does not take issue slots from the warps
-// doing the arithmetic; the clock is read only every 64 probes.
-__device__ __forceinline__ bool mbar_wait_abortable(volatile int *abort, uint64_t *bar, uint32_t parity, uint32_t sleep_ns = 256u,
-                                                    uint32_t eager = 2u)
-{
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-#pragma unroll 1
-    for (uint32_t spin = 1;; spin++) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (sleep_ns != 0u && spin > eager) __nanosleep(sleep_ns);
-        if ((spin & 63u) == 0u && (*abort != 0 || clock64() - t0 > INKQ_SPIN_LIMIT_CYCLES)) return false;
-    }
-}
 // Wait used when a kernel leaves after a failed wait: its own asynchronous copies may still be in flight and must
 // land before the CTA's shared memory is given up.  Ignores any abort word; bounded by `limit_cycles` (copies complete
 // within microseconds; the default is about a millisecond).
@@ -104,11 +86,6 @@ __device__ __forceinline__ bool mbar_wait_drain(uint64_t *bar, uint32_t parity, 
     }
 }
 // ---- fences -------------------------------------------------------------------
-// Make generic-proxy shared-memory writes visible to the async proxy (UMMA / TMA reads).
-__device__ __forceinline__ void fence_proxy_async_smem()
-{
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
