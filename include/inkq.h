@@ -126,7 +126,7 @@ int inkq_quantize_host(inkq_ctx *ctx, int qmode, const float *x_host, int M, int
 int inkq_act_import(inkq_ctx *ctx, inkq_act *act, int qmode, int M, const int8_t *q, const float *d, const float *s);
 
 /* ---- matmuls ---------------------------------------------------------------
- * inkq_gemm  : tcgen05 int8 tensor-core path, any M >= 1. Replaces
+ * inkq_gemm  : int8 tensor-core path (warp-level products), any M >= 1. Replaces
  *              gemm_repack_A81W41_fp32 / gemm_repack_A80W40 (QwenOperator.h:280-298).
  * inkq_gemv  : bandwidth path, M == 1. Replaces gemv_repack_A81W41_fp16 /
  *              gemv_repack_A80W40 (QwenOperator.h:286-304).

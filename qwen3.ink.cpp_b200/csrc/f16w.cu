@@ -1,4 +1,4 @@
-// fp16-weight matmul (lm_head: fp32 activations x fp16 weights, fp32 accumulate) and
+// fp16-weight matmul for few rows (lm_head: fp32 activations x fp16 weights, fp32 accumulate) and
 // the CUDA-core weight-only W41 matmul (fp16 activations x dequantised Q4_1 weights).
 //
 // Neither has a C++ kernel in the reference.  lm_head follows the arithmetic of
@@ -106,16 +106,18 @@ __global__ void __launch_bounds__(256) k_f16w_gemv(const uint16_t *__restrict__ 
 // The CUDA-core kernel above needs, per weight and row, a conversion, an fp32 fma and its share of a 16-byte shared load: with
 // four rows it is bound by instruction issue (4 rows 631 us for the 1.2 GB lm_head, 194 us with one).  Here 16 weight rows x 8
 // activation rows x 16 k are one warp-level fp16 product with fp32 accumulation; the fp32 activations enter as an fp16 value and
-// an fp16 remainder of the row scaled by a power of two (f16w_split.cuh: 22 significant bits), so both products are exact.
-// Error against 64 bits, 2-norm: 1.2e-7 at K = 2048 and 4096, where the CUDA-core kernel's fp32 sums have 1.6e-7 and 2.1e-7.  A tile's K is split over the CTA's 16 warps, whose partial sums are added in ascending order.  A row's result does
-// not depend on the rows beside it, and one row takes this kernel too: a batch gives the same bits as its rows one by one.
+// an fp16 remainder of the row scaled by a power of two (f16w_split.cuh: 22 significant bits), so both products are exact. Error
+// against 64 bits, 2-norm: 1.2e-7 at K = 2048 and 4096, where the CUDA-core kernel's fp32 sums have 1.6e-7 and 2.1e-7.  A tile's
+// K is split over the CTA's 16 warps, whose partial sums are added in ascending order.  A row's result does not depend on the
+// rows beside it, and one row takes this kernel too: a batch gives the same bits as its rows one by one. Nine to 15 rows are two
+// passes and read the weights twice (151936 x 4096: 9 rows 372 us, 15 rows 397, where 16 on the tensor cores take 280).
 //
 // Bound by the weight stream.  The weights come straight from global memory into A fragments: the order of k inside a product
 // is free, so a lane takes 32 contiguous bytes of its two rows per 64 k - the fragments of four products, 128 bytes per row and
 // request - and the activations are read alike.  Each lane keeps F16R_DEPTH such steps in flight across tile borders (128 KB
 // per SM).  Measured (three matrices in turn): 151936 x 4096, 8 rows 1258 us on the CUDA cores, 230 with 64-byte pieces, 200 with
-// slower preparation of the activations, 186 now (6.7 TB/s); one row 194 on the CUDA cores, 179 now (32000 x 4096: 54 -> 46,
-// 151936 x 2048: 111 -> 102).
+// slower preparation of the activations, 186 to 193 now (6.5 to 6.7 TB/s); one row 194 on the CUDA cores, 177 now (32000 x 4096:
+// 54 -> 46, 151936 x 2048: 111 -> 102).
 constexpr int F16R_WARPS = 16, F16R_DEPTH = 4, F16R_COLS = 8;
 
 // bytes between two rows of the staged activations: 16 modulo 128, so that the 16-byte pieces of an 8-lane phase (two rows, every

@@ -1,18 +1,20 @@
-// Weight-only W41 for a few activation rows (2 to 16): fp16 activations x Q4_1 weights dequantised in registers, warp-level
-// fp16 products with fp32 accumulation.
+// Weight-only W41 for a few activation rows (up to 16; one row of a wide layer takes gemv_w41.cu): fp16 activations x Q4_1
+// weights dequantised in registers, warp-level fp16 products with fp32 accumulation.
 //
 // No C++ kernel exists in the reference for this scheme; it follows notebooks/evaluate-qwen3_8b_W4.ipynb cell 13, like the
 // tensor-core kernel (qgemm_w41_tc.cu), and dequantises alike:  w16[n][k] = fp16(q[n][k] * d[n][k/32] + m[n][k/32])  with one
 // rounding, C[m][n] = sum_k a16[m][k] * w16[n][k].
 //
-// Bound by the weight stream (0.625 bytes per weight).  The tensor-core kernel expands every stage of packed weights into
-// shared memory and pays for it whatever the number of rows: 29 us for 12288 x 4096 from 2 to 64 rows.  Here the packed weights
-// go from global memory straight into A fragments: the order of k inside a product is free, so a lane takes 8
-// contiguous bytes of its two rows per pair of blocks - 8 weights of the low and 8 of the high block, the fragments of four
-// products - and the activations, staged once per CTA in shared memory, are read alike.  A tile of 16 weight rows is split
-// along K over the CTA's 16 warps, so the work is even to one tile per SM; each lane keeps DEPTH pairs in flight across tile borders.
-// The products of one pair accumulate from zero and are added to the running sums in fp32 (the hardware's own accumulation
-// truncates), the warps' partials are added in ascending order.
+// The least it has to move is the weight stream (0.625 bytes per weight), which it reaches a third of: 12288 x 4096 with 8 rows
+// 13.6 us = 2.35 TB/s, with 16 rows 16.4; 24576 x 4096 24.6 = 2.6 TB/s; 4096 x 4096 5.3.  Dequantising and multiplying is 12.4k
+// instructions per scheduler (6.3 us of the 13.6); for the rest the 16 warps of an SM wait for loads of 32 bytes per row and
+// request.  The tensor-core kernel dequantises every stage for its tile whatever the number of rows: 29 us for 12288 x 4096 from
+// 2 to 64 rows when this kernel took its place, 21 today.  Here the packed weights go from global memory straight into A
+// fragments: the order of k inside a product is free, so a lane takes 8 contiguous bytes of its two rows per pair of blocks - 8
+// weights of the low and 8 of the high block, the fragments of four products - and the activations, staged once per CTA in shared
+// memory, are read alike.  A tile of 16 weight rows is split along K over the CTA's 16 warps, so the work is even to one tile per
+// SM; each lane keeps DEPTH pairs in flight across tile borders. The products of one pair accumulate from zero and are added to
+// the running sums in fp32 (the hardware's own accumulation truncates), the warps' partials are added in ascending order.
 #include <cuda_fp16.h>
 
 #include "inkq_internal.h"

@@ -114,7 +114,7 @@ def full_lm_head(pkg, gpu):
 
 @pytest.mark.parametrize("M", [1, 16, 322, 8192])
 def test_lm_head_real_vocabulary(pkg, gpu, oracle, full_lm_head, M):
-    """M == 1: the CUDA-core kernel (fp32 products and sums): 1e-3 per element.  M >= 16: tensor cores.  Products are
+    """M == 1: the warp-level kernel (activations as fp16 hi + lo, fp32 sums): 1e-3 per element.  M >= 16: tensor cores.  Products are
     exact there too, but the K-long sum is accumulated in fp32 inside tensor memory in the hardware's own order and
     rounding, which moves a result by up to ~1e-4 of the OUTPUT'S rms whatever its own size; the bound is therefore
     norm-wise: 2e-4 of the rms with the activations as fp16 hi + lo (the default), 3e-3 with one fp16 value."""
