@@ -41,8 +41,6 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
-#include <initializer_list>
-
 #include "inkq_internal.h"
 #include "ptx.cuh"
 
@@ -68,13 +66,13 @@ struct Params {
 // CTAS resident CTAs per SM.
 template <int WR_, int WC_, int MT_, int NT_, int SP_, int CTAS_ = 2>
 struct Tile {
-    static constexpr int WR = WR_, WC = WC_, MT = MT_, NT = NT_, SP = SP_, CTAS = CTAS_;
+    static constexpr int WR = WR_, WC = WC_, MT = MT_, NT = NT_, SP = SP_, CTAS = CTAS_, ROWS = 16 * WR * MT, COLS = 8 * NT * WC;
 };
 
 // SCH: weight scheme; S16: fp16 scale records
 template <int SCH, bool S16, class T>
 struct Cfg {
-    static constexpr int SP = T::SP, ROWS = 16 * T::WR * T::MT, BM = 8 * T::NT * T::WC, WARPS = T::WR * T::WC, THREADS = 32 * WARPS;
+    static constexpr int SP = T::SP, ROWS = T::ROWS, BM = T::COLS, WARPS = T::WR * T::WC, THREADS = 32 * WARPS;
     static constexpr int PLANES = (SCH == INKQ_A81W41) ? 2 : 1;
     static constexpr int Q_BYTES = BM * 64 * SP, PLANE_BYTES = 2 * SP * BM * 4;
     static constexpr int W_PAIR = ROWS * 32, SC_REC = S16 ? 8 : 16, SC_PAIR = ROWS * SC_REC, Z_PAIR = (SCH == INKQ_A80W4Z) ? ROWS * 2 : 0;
@@ -369,64 +367,60 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
 }
 
 // Tiles for more than 32 activation rows: shape, then the time (us) of one and of two tiles on every SM at K = 4096, without
-// the ~3 us that a launch takes, with the mins of A81W41 and without them.  Measured with prefetched weights of distinct layers;
+// the ~3 us that a launch takes, for A81W41, A80W40 and A80W4Z with fp16 scale records, and what a tile takes more with fp32
+// records.  Measured with weights of distinct layers;
 // only the ratios matter, and they hardly depend on K.  One CTA of 8 warps per SM with all the registers it wants and 4 to 8
 // unrolled pairs per stage: the fragment loads and products of several pairs overlap the scaling of the ones before (against two CTAs
 // of 128 registers and two-pair stages: 64 x 48 17.9 -> 14.2, 128 x 112 72 -> 51).  Two such CTAs side by side remain for
 // many tiles per SM, where one's set-up and stores hide behind the other's products.
 // Per column the wide tiles cost least: fragments and scales of the weight rows are fetched once for more columns.
-// Half- and quarter-height tiles split a layer with few weight rows over more SMs.
-#define QROWS_TILES(X)                                         \
-    X(0, (2, 4, 1, 2, 8, 1), (10.4f, 22.7f), (9.8f, 21.4f))    \
-    X(1, (4, 2, 1, 2, 8, 1), (11.2f, 24.2f), (10.4f, 23.0f))   \
-    X(2, (4, 1, 2, 2, 4, 2), (12.0f, 18.5f), (11.6f, 17.5f))   \
-    X(3, (4, 2, 1, 3, 8, 1), (14.2f, 30.3f), (12.5f, 26.6f))   \
-    X(4, (4, 2, 1, 4, 6, 1), (18.2f, 38.6f), (16.7f, 35.6f))   \
-    X(5, (4, 2, 1, 5, 6, 1), (22.0f, 46.4f), (18.6f, 39.4f))   \
-    X(6, (4, 2, 1, 7, 4, 1), (29.6f, 61.7f), (25.4f, 52.8f))   \
-    X(7, (4, 2, 2, 2, 8, 1), (17.9f, 37.0f), (17.2f, 35.6f))   \
-    X(8, (4, 2, 2, 3, 6, 1), (24.4f, 50.6f), (22.4f, 46.4f))   \
-    X(9, (4, 2, 2, 4, 4, 1), (31.9f, 65.7f), (28.4f, 58.7f))   \
-    X(10, (4, 2, 2, 5, 4, 1), (38.2f, 78.3f), (34.0f, 69.8f))  \
-    X(11, (4, 2, 2, 6, 4, 1), (45.0f, 91.8f), (39.8f, 81.0f))  \
-    X(12, (4, 2, 2, 7, 4, 1), (51.1f, 104.2f), (44.6f, 91.1f)) \
-    X(13, (4, 2, 1, 4, 2, 2), (21.9f, 36.4f), (19.3f, 31.5f))  \
-    X(14, (4, 2, 1, 7, 2, 2), (31.7f, 56.8f), (28.2f, 48.7f))  \
-    X(15, (4, 2, 2, 4, 2, 2), (34.6f, 62.5f), (31.7f, 55.8f))  \
-    X(16, (4, 2, 2, 5, 2, 2), (43.3f, 78.1f), (37.6f, 66.7f))
+// Half- and quarter-height tiles split a layer with few weight rows over more SMs.  64 x 40 with one warp per scheduler costs less per
+// column than 64 x 48 with two, which fetch and unpack every weight fragment twice (77 rows of 4096 x 12288, A80W4Z: 41 -> 36 us).
+#define QROWS_TILES(X)                                                               \
+    X(0, (2, 4, 1, 2, 8, 1), (9.9f, 21.9f), (9.1f, 20.5f), (11.2f, 24.3f), 0.0f)     \
+    X(1, (4, 2, 1, 2, 8, 1), (10.6f, 23.1f), (9.9f, 22.0f), (12.0f, 26.1f), 0.0f)    \
+    X(2, (4, 1, 2, 2, 4, 2), (10.8f, 17.5f), (10.2f, 16.3f), (11.9f, 19.2f), 2.6f)   \
+    X(3, (4, 2, 1, 3, 8, 1), (13.2f, 28.1f), (11.6f, 24.5f), (13.6f, 28.9f), 0.0f)   \
+    X(4, (4, 2, 1, 4, 6, 1), (17.0f, 35.8f), (15.5f, 32.7f), (17.8f, 37.1f), 0.0f)   \
+    X(5, (4, 2, 1, 5, 6, 1), (20.5f, 43.0f), (16.9f, 36.7f), (19.5f, 39.6f), 1.1f)   \
+    X(6, (4, 2, 1, 7, 4, 1), (27.0f, 56.2f), (23.0f, 47.7f), (25.3f, 52.2f), 0.0f)   \
+    X(7, (4, 2, 2, 2, 8, 1), (16.8f, 34.1f), (16.0f, 32.6f), (18.5f, 37.6f), 0.0f)   \
+    X(8, (4, 2, 2, 3, 6, 1), (22.2f, 45.7f), (20.4f, 41.8f), (23.3f, 47.7f), 0.0f)   \
+    X(9, (4, 2, 2, 4, 4, 1), (29.0f, 59.3f), (25.6f, 52.7f), (27.8f, 57.3f), 0.0f)   \
+    X(10, (4, 2, 2, 5, 4, 1), (34.1f, 69.6f), (30.4f, 62.1f), (32.8f, 67.2f), 0.0f)  \
+    X(11, (4, 2, 2, 6, 4, 1), (40.6f, 82.7f), (35.1f, 72.0f), (37.5f, 76.9f), 0.0f)  \
+    X(12, (4, 2, 2, 7, 4, 1), (45.8f, 92.9f), (39.7f, 80.9f), (41.8f, 85.2f), 1.4f)  \
+    X(13, (4, 2, 1, 4, 2, 2), (20.9f, 34.8f), (17.9f, 29.6f), (21.7f, 34.0f), 0.0f)  \
+    X(14, (4, 2, 1, 7, 2, 2), (29.2f, 54.0f), (25.8f, 45.7f), (28.2f, 47.9f), 0.0f)  \
+    X(15, (4, 2, 2, 4, 2, 2), (31.8f, 58.8f), (28.9f, 52.4f), (31.8f, 57.9f), 0.0f)  \
+    X(16, (4, 2, 2, 5, 2, 2), (39.7f, 73.4f), (33.9f, 61.8f), (36.4f, 67.2f), 0.0f)  \
+    X(17, (4, 1, 1, 5, 8, 1), (12.4f, 26.4f), (10.9f, 23.8f), (12.9f, 27.3f), -0.4f)
 
 #define QROWS_UNWRAP(...) __VA_ARGS__
 struct TileCost {
     int rows, cols;
-    float with_min[2], without[2];
+    float time[3][2];   // by weight scheme (A81W41, A80W40, A80W4Z), one and two tiles
+    float f32;          // more with fp32 scale records
 };
-template <class T>
-constexpr TileCost tile_cost(std::initializer_list<float> with_min, std::initializer_list<float> without)
-{
-    TileCost c{16 * T::WR * T::MT, 8 * T::NT * T::WC, {}, {}};
-    int i = 0;
-    for (float v : with_min) c.with_min[i++] = v;
-    i = 0;
-    for (float v : without) c.without[i++] = v;
-    return c;
-}
+static_assert(INKQ_A81W41 == 0 && INKQ_A80W40 == 1 && INKQ_A80W4Z == 2, "the schemes index the table");
 static constexpr TileCost tile_costs[] = {
-#define QROWS_COST(i, shape, with_min, without) tile_cost<Tile<QROWS_UNWRAP shape>>({QROWS_UNWRAP with_min}, {QROWS_UNWRAP without}),
+#define QROWS_COST(i, shape, w41, w40, w4z, f32) \
+    {Tile<QROWS_UNWRAP shape>::ROWS, Tile<QROWS_UNWRAP shape>::COLS, {{QROWS_UNWRAP w41}, {QROWS_UNWRAP w40}, {QROWS_UNWRAP w4z}}, f32},
     QROWS_TILES(QROWS_COST)
 };
 
 // The tile with the least time for M activation rows: a CTA takes one tile, so the busiest SM works through
 // n = ceil(tiles / SMs) of them.
-static int pick_tile(const inkq_ctx *ctx, bool has_min, int rows, int M)
+static int pick_tile(const inkq_ctx *ctx, int scheme, bool s16, int rows, int M)
 {
     int best = 0;
     float best_time = 0.f;
     for (int i = 0; i < static_cast<int>(sizeof(tile_costs) / sizeof(tile_costs[0])); i++) {
         const TileCost &c = tile_costs[i];
-        const float *t = has_min ? c.with_min : c.without;
+        const float *t = c.time[scheme];
         const long long total = static_cast<long long>((rows + c.rows - 1) / c.rows) * ((M + c.cols - 1) / c.cols);
         const long long n = (total + ctx->num_sms - 1) / ctx->num_sms;
-        const float time = static_cast<float>(n / 2) * t[1] + static_cast<float>(n % 2) * t[0];
+        const float time = static_cast<float>(n / 2) * t[1] + static_cast<float>(n % 2) * t[0] + (s16 ? 0.f : static_cast<float>(n) * c.f32);
         if (i == 0 || time < best_time) {
             best = i;
             best_time = time;
@@ -439,21 +433,22 @@ template <int SCH, bool S16>
 static int launch_sized(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin, const Params &prm)
 {
     if (prm.M > 32) {
-        const int tile = pick_tile(ctx, SCH == INKQ_A81W41, prm.rows, prm.M);
+        const int tile = pick_tile(ctx, SCH, S16, prm.rows, prm.M);
         switch (tile) {
-#define QROWS_CASE(i, shape, with_min, without) case i: return launch_one<SCH, S16, Tile<QROWS_UNWRAP shape>>(ctx, a, w, m_begin, prm);
+#define QROWS_CASE(i, shape, w41, w40, w4z, f32) case i: return launch_one<SCH, S16, Tile<QROWS_UNWRAP shape>>(ctx, a, w, m_begin, prm);
             QROWS_TILES(QROWS_CASE)
         }
     }
     // Up to 32 rows one tile holds all of them, so every weight byte is fetched once.  No more 128-row tiles than SMs: one CTA
-    // per SM, stages of eight pairs, and 64 instead of 128 weight rows if that still leaves one CTA per SM; otherwise two CTAs per
-    // SM and stages of four (us, against 4 pairs and two CTAs everywhere: 12288 x 4096 with 5 rows 10.6 -> 9.4, with 24 rows 18.8 ->
-    // 16.8; 6144 x 4096 with 5 rows 9.5 -> 7.3, with 24 rows 13.3 -> 12.1; 24576 x 4096 with 5 rows 15.7 against 17.5)
+    // per SM, stages of eight pairs, and 64 instead of 128 weight rows if that still leaves one CTA per SM (us, against 4 pairs and
+    // two CTAs everywhere: 12288 x 4096 with 5 rows 10.6 -> 9.4, with 24 rows 18.8 -> 16.8; 6144 x 4096 with 5 rows 9.5 -> 7.3, with
+    // 24 rows 13.3 -> 12.1).  More: 64-row CTAs, up to three to an SM, and stages of four.  The busiest SM then has 192 rows of
+    // 24576 instead of the 256 of two 128-row CTAs (5 rows 15.6 -> 14.1 = 5.0 TB/s, 12 rows 22.1 -> 19.0)
     const bool narrow = w->tiles * 2 <= ctx->num_sms, single = w->tiles <= ctx->num_sms;
 #define QROWS_SMALL(n)                                                                                              \
     case n:                                                                                                         \
         if (narrow) return launch_one<SCH, S16, Tile<4, 1, 1, n, 8, n == 1 ? 2 : 1>>(ctx, a, w, m_begin, prm);      \
-        return single ? launch_one<SCH, S16, Tile<8, 1, 1, n, 8, 1>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, n, 4, 2>>(ctx, a, w, m_begin, prm);
+        return single ? launch_one<SCH, S16, Tile<8, 1, 1, n, 8, 1>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<4, 1, 1, n, 4, 3>>(ctx, a, w, m_begin, prm);
     switch ((prm.M + 7) / 8) {
         QROWS_SMALL(1)
         QROWS_SMALL(2)
