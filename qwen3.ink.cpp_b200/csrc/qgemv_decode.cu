@@ -189,7 +189,11 @@ __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_S
 #pragma unroll
         for (int u = 0; u < 6; u++) early[u][lane] = e[u];
     }
+    // Not unrolled: with four copies of each loop's body in flight beside the weights most variants spilled 12 to 40 bytes a thread, and a
+    // CTA runs these loops once or twice (a decode step of 36 layers 1514 -> 1473 us)
+#pragma unroll 1
     for (int i = threadIdx.x; i < K / 16; i += blockDim.x) reinterpret_cast<uint4 *>(qa)[i] = reinterpret_cast<const uint4 *>(q)[i];
+#pragma unroll 1
     for (int b = threadIdx.x; b < nb; b += blockDim.x) {
         da[b] = d[static_cast<size_t>(b) * M_ld];
         if (HAS_MIN) sa[b] = s[static_cast<size_t>(b) * M_ld];
@@ -220,6 +224,7 @@ __global__ void __launch_bounds__(WARPS * 32, GemvShape<WARPS, DEEP>::CTAS_PER_S
         float ss = 0.0f;
 #pragma unroll
         for (int u = 0; u < 4; u++) ss = __fadd_rn(ss, early[u][lane]);
+#pragma unroll 1
         for (int i = 128 + lane; i < pend.parts; i += 32) ss = __fadd_rn(ss, __ldcg(pend.ssq + i));
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, off));
