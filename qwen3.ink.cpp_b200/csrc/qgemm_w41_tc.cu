@@ -14,11 +14,13 @@
 // the UMMA N side.  One stage = one pair of quantization blocks = 64 K-elements = four K=16 MMAs per weight tile.
 // The dequantised weights go from registers straight into tensor memory and are the MMA's A operand there: with A in
 // shared memory (16 KB written and read again per stage and tile) the shared-memory port was as busy as the tensor pipe.
-// What bounds it: up to ~100 columns the dequantising warps (~740 cycles per stage of two weight tiles: fp16 and ALU pipes at half
-// rate, plus waiting, storing and handing over), above the tensor pipe.  Measured at K = 4096 (before: A in shared memory, 8
-// dequantising warps): 12288 rows x 17 columns 29 -> 22 us, x 64 31 -> 22, x 322 53 -> 33, x 2048 178 -> 157 (1.31 PFLOP/s); 4096 x
-// 322 33 -> 22; 24576 x 512 123 -> 78.  Slower: one chunk per thread and turn (+15 %), the stores of a stage completing under the
-// next one's arithmetic (+5 %: one slot less), two stages per copy (+10 %).
+// What bounds it: up to ~100 columns the turns of the dequantising warps and of the thread that issues the products (~260 cycles a
+// stage of one weight tile: waits of ~60 cycles each, instruction fetch of six warps with different code on a scheduler, hand-over),
+// above the tensor pipe.  Measured at K = 4096: 12288 rows x 17 columns 17 us, x 64 17.8 (22.3 before the waits' slow path left the
+// loops and the issuing thread stopped waiting for the copies itself), x 322 33.5, x 2048 160 (1.29 PFLOP/s); 4096 x 322 17.7 (22.6),
+// 4096 x 12288 with 322 rows 44 (58).  Slower: A in shared memory with 8 dequantising warps (12288 x 322 53 us), one chunk per thread and
+// turn (+15 %), the stores of a stage completing under the next one's arithmetic (+5 %: one slot less), two stages per copy (+10 %), the two
+// chunks of a turn in a rolled loop (192 columns +8 %).
 //
 // Persistent, warp-specialised, one CTA per SM, 768 threads:
 //   warps 0, 3   TMA producers (activations; weights): per stage one tiled 2-D copy of the fp16 activations
@@ -99,11 +101,12 @@ struct Ring {
     }
 };
 
-// Bounded wait; always returns (after an abort the roles finish their loops without waiting).  The probe suspends the thread in
+// Bounded wait; always returns (after an abort the roles finish their loops without waiting).  The probes suspend the thread in
 // hardware: probing in a loop, the roles that wait take issue slots from the dequantising warps (one more such warp: +10 %).
-__device__ __forceinline__ void wait_bounded(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *dev_flag)
+// Not inlined: the loops of all roles share the schedulers' small instruction caches, and a loop that spans fewer lines turns faster
+// (one weight tile, a stage ~330 -> 260 cycles together with the shorter loop of the products).
+__device__ __noinline__ void wait_slow(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *dev_flag)
 {
-    if (mbar_try_wait(bar, parity)) return;
     const long long t0 = clock64();
 #pragma unroll 1
     while (!mbar_try_wait_for(bar, parity, 10000u)) {
@@ -114,6 +117,10 @@ __device__ __forceinline__ void wait_bounded(uint64_t *bar, uint32_t parity, vol
             return;
         }
     }
+}
+__device__ __forceinline__ void wait_bounded(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *dev_flag)
+{
+    if (__builtin_expect(!mbar_try_wait(bar, parity), 0)) wait_slow(bar, parity, abort_flag, dev_flag);
 }
 
 __device__ __forceinline__ uint32_t bits(__half2 h) { return *reinterpret_cast<const uint32_t *>(&h); }
@@ -229,29 +236,31 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm_w41_tc(const __grid_constan
         // ------------------------------ MMA issuer ------------------------------
         if (elect_one()) {
             const uint32_t idesc = umma_idesc_f16(TILE_N, prm.block_m);
-            Ring raw(prm.stages), as(prm.a_slots), acc(prm.acc_slots);
-            uint32_t g = 0;
+            // A: lane = weight row, eight columns (16 halves) per MMA.  B: activations, 128-byte swizzled rows of 64 halves; slice j is the
+            // j-th 32-byte part of the row; 8-row groups are 1024 B apart.  The start-address field counts 16-byte units.
+            const uint64_t b_first = umma_smem_desc(smem_u32(smem), 16, 1024, 2);
+            const uint32_t b_step = prm.raw_bytes >> 4;
+            Ring as(prm.a_slots), acc(prm.acc_slots);
+            uint32_t stage = 0, ring = 0;
             for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
-                const int nvalid = min(NT, prm.tiles_n - (tile / prm.tiles_m) * NT);
+                const bool both = NT == 2 && prm.tiles_n - (tile / prm.tiles_m) * NT > 1;
                 wait_bounded(&acc_empty[acc.idx], acc.phase ^ 1, abort_flag, prm.flag);
                 const uint32_t d = tmem_base + acc.idx * NT * prm.block_m;
-                for (int p = 0; p < prm.pairs; p++, g++) {
-                    wait_bounded(&raw_full[raw.idx], raw.phase, abort_flag, prm.flag);
+#pragma unroll 1
+                for (int p = 0; p < prm.pairs; p++) {
+                    // The dequantising warps have waited for the whole stage, the activations among it, before they arrive here
                     wait_bounded(&a_full[as.idx], as.phase, abort_flag, prm.flag);
                     tc_fence_after_sync();
-                    // A: lane = weight row, eight columns (16 halves) per MMA.  B: activations, 128-byte swizzled rows of 64
-                    // halves; slice j is the j-th 32-byte part of the row; 8-row groups are 1024 B apart.  The
-                    // start-address field counts 16-byte units.
-                    const uint64_t b0 = umma_smem_desc(smem_u32(smem + raw.idx * prm.raw_bytes), 16, 1024, 2);
+                    const uint64_t b0 = b_first + stage * b_step;
                     const uint32_t a0 = tmem_a + as.idx * NT * A_COLS;
 #pragma unroll
-                    for (int j = 0; j < 4; j++)
-#pragma unroll
-                        for (int wt = 0; wt < NT; wt++)
-                            if (wt < nvalid)
-                                umma_f16_ts(d + wt * prm.block_m, a0 + wt * A_COLS + j * 8, b0 + static_cast<uint64_t>(j * 2), idesc, (p > 0 || j > 0) ? 1u : 0u);
-                    umma_commit(&done[g % DONE_RING]);   // the only commit of the pair
-                    raw.advance();
+                    for (int j = 0; j < 4; j++) {
+                        umma_f16_ts(d, a0 + j * 8, b0 + static_cast<uint64_t>(j * 2), idesc, (p > 0 || j > 0) ? 1u : 0u);
+                        if (both) umma_f16_ts(d + prm.block_m, a0 + A_COLS + j * 8, b0 + static_cast<uint64_t>(j * 2), idesc, (p > 0 || j > 0) ? 1u : 0u);
+                    }
+                    umma_commit(&done[ring]);   // the only commit of the pair
+                    ring = (ring + 1) % DONE_RING;
+                    if (++stage == static_cast<uint32_t>(prm.stages)) stage = 0;
                     as.advance();
                 }
                 umma_commit(&acc_full[acc.idx]);
@@ -388,9 +397,10 @@ int launch_gemm_w41_tc(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *
     using namespace w41;
     if (ctx->encode_tiled == nullptr) return fail(ctx, INKQ_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled entry point not available");
     if ((reinterpret_cast<uintptr_t>(a16) & 15) != 0) return fail(ctx, INKQ_ERR_INVALID, "the fp16 activations must be 16-byte aligned");
-    // The split with the least time: waves x time of a wave (us at K = 4096, measured with one tile on every SM; it is
-    // proportional to K).  Dequantising bounds narrow tiles (one weight tile 18.2, two 28.5), the products wide ones.  Two
-    // weight tiles share the activations, one leaves fewer SMs idle where there are few tiles.
+    // The split with the least time: waves x time of a wave (us at K = 4096, measured as what a second tile on every SM adds; it
+    // is proportional to K).  Dequantising bounds narrow tiles (one weight tile
+    // 13.4, two 26.4), the products wide ones.  One weight tile leaves fewer SMs idle where there are few tiles; two share the
+    // activations, which pays beyond ~190 rows (192 rows: 22.6 twice against 42.6).
     Shape best{1, 0};
     float best_time = 0.f;
     for (int nt = 1; nt <= 2; nt++) {
@@ -398,7 +408,7 @@ int launch_gemm_w41_tc(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *
         for (int tm = (M + max_m - 1) / max_m; tm <= (M + 15) / 16; tm++) {
             const int bm = (((M + tm - 1) / tm) + 15) & ~15;
             const long long total = static_cast<long long>((w->tiles + nt - 1) / nt) * ((M + bm - 1) / bm);
-            const float wave = nt == 1 ? fmaxf(18.2f, 10.6f + 0.0735f * bm) : fmaxf(28.5f, 18.8f + 0.1205f * bm);
+            const float wave = nt == 1 ? fmaxf(13.4f, 5.0f + 0.098f * bm) : fmaxf(26.4f, 17.2f + 0.131f * bm);
             const float time = static_cast<float>((total + ctx->num_sms - 1) / ctx->num_sms) * wave;
             if (best_time == 0.f || time < best_time) {
                 best = Shape{nt, bm};
