@@ -10,59 +10,32 @@
 //   both: byte[32 g + e] = q[64 g + e] | q[64 g + 32 + e] << 4                  (:61-64, :120-123)
 //
 // Bound by memory: 4 bytes read and 0.78 written per weight.  Eight lanes share a pair of blocks (64 weights): a lane holds
-// four consecutive elements of each, so both loads and the packed store of a warp are whole 128-byte lines, the reductions
-// take three exchanges, and four pairs per lane keep eight 16-byte loads in flight.  (One element per lane and block, five
-// exchanges and byte stores ran at 1.26 TB/s, 190 us for 12288 x 4096.)
+// four consecutive elements of each, so both loads and the packed store of a warp are whole 128-byte lines, and four pairs per
+// lane keep eight 16-byte loads in flight.  (One element per lane and block, five exchanges and byte stores ran at 1.26 TB/s, 190 us
+// for 12288 x 4096.)  The eight blocks of eight lanes are reduced together: each exchange hands half of the remaining blocks to the
+// partner, seven exchanges in place of 24, after which lane t owns block t, divides once for all and hands the factors back.  With
+// every lane reducing and dividing for every block, 12288 x 4096 took 45.6 us in Q4_1 and 60.8 in Q4_0 (whose 64-bit keys are now built
+// only where a block's extremes tie); now 39.8 and 39.3 = 6.0 TB/s.
 #include "inkq_internal.h"
 
 namespace inkq {
 
 constexpr int WQ_PAIRS = 4;   // pairs of blocks per group of eight lanes
 
-// Scale, minimum and the four codes (one per byte) of this lane's elements 4t .. 4t+3 of a block shared by eight lanes.
-template <int FORMAT>   // 0: Q4_0, 1: Q4_1
-__device__ __forceinline__ uint32_t quantize_block(const float4 x4, int t, float &dd, float &mm)
+// Reduces v[k] of eight lanes (t = 0 .. 7) for each of eight blocks k; lane t returns with block t's result
+template <typename T, typename Op>
+__device__ __forceinline__ T reduce_scatter8(T (&v)[8], int t, Op op)
 {
-    const float x[4] = {x4.x, x4.y, x4.z, x4.w};
-    float v[4];
-    if (FORMAT == 1) {
-        float mx = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])), mn = fminf(fminf(x[0], x[1]), fminf(x[2], x[3]));
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    for (int o = 4; o > 0; o >>= 1) {
+        const bool up = (t & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; i++) {
+            const T keep = up ? v[i + o] : v[i], give = up ? v[i] : v[i + o];
+            v[i] = op(keep, __shfl_xor_sync(0xffffffffu, give, o));
         }
-        mm = mn;
-        dd = __fdiv_rn(__fsub_rn(mx, mn), 15.0f);
-        const float id = (dd != 0.0f) ? __fdiv_rn(1.0f, dd) : 0.0f;
-#pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = rintf(__fmul_rn(__fsub_rn(x[i], mn), id));
-    } else {
-        // the value of the largest magnitude, lowest index on ties (np.argmax): the key orders by magnitude, then by
-        // descending index, and carries the sign along
-        unsigned long long key = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t bits = __float_as_uint(x[i]);
-            const unsigned long long k = (static_cast<unsigned long long>(bits & 0x7fffffffu) << 6) | static_cast<unsigned>((31 - 4 * t - i) << 1) | (bits >> 31);
-            key = k > key ? k : key;
-        }
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            const unsigned long long k = __shfl_xor_sync(0xffffffffu, key, o);
-            key = k > key ? k : key;
-        }
-        const float val = __uint_as_float(static_cast<uint32_t>(key >> 6) | (static_cast<uint32_t>(key & 1u) << 31));
-        dd = __fdiv_rn(val, -8.0f);
-        mm = 0.0f;
-        const float id = (dd != 0.0f) ? __fdiv_rn(1.0f, dd) : 0.0f;
-#pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = __fadd_rn(__fmul_rn(x[i], id), 8.5f);
     }
-    uint32_t q = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) q |= static_cast<uint32_t>(fminf(fmaxf(v[i], 0.0f), 15.0f)) << (8 * i);   // truncation, as astype(np.uint8) of a value in [0, 15]
-    return q;
+    return v[0];
 }
 
 // ALIGNED: every pointer suits the vector accesses (the callers' usual case); otherwise element by element.
@@ -90,31 +63,85 @@ __global__ void __launch_bounds__(256) k_quantize_weight_q4(const float *__restr
             }
         }
     }
+    // block 2u: the low one of pair u, 2u + 1: its high one
+    static_assert(WQ_PAIRS == 4, "eight blocks for eight lanes");
+    float dd, mm = 0.0f;
+    if (FORMAT == 1) {
+        float mx[8], mn[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float4 x = (k & 1) ? hi[k >> 1] : lo[k >> 1];
+            mx[k] = fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w));
+            mn[k] = fminf(fminf(x.x, x.y), fminf(x.z, x.w));
+        }
+        mm = reduce_scatter8(mn, t, [](float a, float b) { return fminf(a, b); });
+        dd = __fdiv_rn(__fsub_rn(reduce_scatter8(mx, t, [](float a, float b) { return fmaxf(a, b); }), mm), 15.0f);
+    } else {
+        // The value of the largest magnitude (as bits: a NaN is larger than any number): the larger of the positive and the negative
+        // side's maximum
+        int pos[8], neg[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float4 x = (k & 1) ? hi[k >> 1] : lo[k >> 1];
+            const int b[4] = {__float_as_int(x.x), __float_as_int(x.y), __float_as_int(x.z), __float_as_int(x.w)};
+            pos[k] = max(max(max(b[0], b[1]), max(b[2], b[3])), 0);
+            constexpr int sign = static_cast<int>(0x80000000u);
+            neg[k] = max(max(max(b[0] ^ sign, b[1] ^ sign), max(b[2] ^ sign, b[3] ^ sign)), 0);
+        }
+        const auto larger = [](int a, int b) { return max(a, b); };
+        const int above = reduce_scatter8(pos, t, larger), below = reduce_scatter8(neg, t, larger);
+        uint32_t val = above > below ? static_cast<uint32_t>(above) : static_cast<uint32_t>(below) | 0x80000000u;
+        if (__any_sync(0xffffffffu, above == below)) {
+            // Both sides reach it (or the block is zero): the lowest index decides (np.argmax).  The key orders by magnitude, then by
+            // descending index, and carries the sign along
+            unsigned long long key[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const float4 x4 = (k & 1) ? hi[k >> 1] : lo[k >> 1];
+                const float x[4] = {x4.x, x4.y, x4.z, x4.w};
+                key[k] = 0;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const uint32_t bits = __float_as_uint(x[i]);
+                    const unsigned long long c = (static_cast<unsigned long long>(bits & 0x7fffffffu) << 6) | static_cast<unsigned>((31 - 4 * t - i) << 1) | (bits >> 31);
+                    key[k] = c > key[k] ? c : key[k];
+                }
+            }
+            const unsigned long long best = reduce_scatter8(key, t, [](unsigned long long a, unsigned long long b) { return a > b ? a : b; });
+            val = static_cast<uint32_t>(best >> 6) | (static_cast<uint32_t>(best & 1u) << 31);
+        }
+        dd = __fdiv_rn(__uint_as_float(val), -8.0f);
+    }
+    const float id = (dd != 0.0f) ? __fdiv_rn(1.0f, dd) : 0.0f;
+    const long long mine = p0 + 4 * (t >> 1);   // the pair of this lane's block
+    if (mine < pairs) {
+        const long long e = 2 * mine + (t & 1);
+        d[e] = dd;
+        m[e] = mm;
+        if (zp != nullptr) zp[e] = (FORMAT == 0) ? 8 : 0;
+    }
 #pragma unroll
     for (int u = 0; u < WQ_PAIRS; u++) {
+        uint32_t q[2] = {0u, 0u};
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int from = (lane & 24) + 2 * u + h;
+            const float f = __shfl_sync(0xffffffffu, id, from), mn = (FORMAT == 1) ? __shfl_sync(0xffffffffu, mm, from) : 0.0f;
+            const float4 x4 = h ? hi[u] : lo[u];
+            const float x[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float v = (FORMAT == 1) ? rintf(__fmul_rn(__fsub_rn(x[i], mn), f)) : __fadd_rn(__fmul_rn(x[i], f), 8.5f);
+                q[h] |= static_cast<uint32_t>(fminf(fmaxf(v, 0.0f), 15.0f)) << (8 * i);   // truncation, as astype(np.uint8) of a value in [0, 15]
+            }
+        }
         const long long p = p0 + 4 * u;
-        float2 dd, mm;
-        const uint32_t q_lo = quantize_block<FORMAT>(lo[u], t, dd.x, mm.x);
-        const uint32_t q_hi = quantize_block<FORMAT>(hi[u], t, dd.y, mm.y);
         if (p < pairs) {
-            const uint32_t q = q_lo | (q_hi << 4);
-            constexpr int z = (FORMAT == 0) ? 8 : 0;
+            const uint32_t both = q[0] | (q[1] << 4);
             if (ALIGNED) {
-                reinterpret_cast<uint32_t *>(nib)[p * 8 + t] = q;
-                if (t == 0) {
-                    reinterpret_cast<float2 *>(d)[p] = dd;
-                    reinterpret_cast<float2 *>(m)[p] = mm;
-                    if (zp != nullptr) reinterpret_cast<char2 *>(zp)[p] = make_char2(z, z);
-                }
+                reinterpret_cast<uint32_t *>(nib)[p * 8 + t] = both;
             } else {
-                for (int i = 0; i < 4; i++) nib[p * 32 + 4 * t + i] = static_cast<uint8_t>(q >> (8 * i));
-                if (t == 0) {
-                    d[2 * p] = dd.x;
-                    d[2 * p + 1] = dd.y;
-                    m[2 * p] = mm.x;
-                    m[2 * p + 1] = mm.y;
-                    if (zp != nullptr) zp[2 * p] = zp[2 * p + 1] = z;
-                }
+                for (int i = 0; i < 4; i++) nib[p * 32 + 4 * t + i] = static_cast<uint8_t>(both >> (8 * i));
             }
         }
     }

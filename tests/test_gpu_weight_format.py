@@ -65,3 +65,19 @@ def test_gpu_weight_quantizer_list_ends_and_alignment(pkg, gpu, oracle, fmt, N, 
     for got, want in zip((nib, d, m), oracle.quantize_weight(fmt, w[shift:shift + N * K].reshape(N, K))):
         assert np.array_equal(got, want)
     assert (zp == (8 if fmt == 0 else 0)).all()
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+def test_gpu_weight_quantizer_ties_and_zeros(pkg, gpu, oracle, fmt):
+    """Blocks whose largest magnitude occurs with both signs (the first one counts), blocks of zeros of either sign, extreme values."""
+    import torch
+    rng = np.random.default_rng(12)
+    w = rng.choice(np.array([-1.5, -1.0, -0.0, 0.0, 1.0, 1.5], dtype=np.float32), size=(70, 320))
+    w[:8, :64] = 0.0
+    w[4:12, :32] = -0.0
+    w[12, :] *= np.float32(2e38)
+    w[13, :] *= np.float32(1e-42)
+    w[20:40] *= rng.choice(np.array([0, 0, 0, 1], dtype=np.float32), size=(20, 320))     # mostly zeros, one or few extremes
+    nib, d, m, _ = (t.cpu().numpy() for t in gpu.quantize_weights(fmt, torch.from_numpy(w).cuda()))
+    for got, want in zip((nib, d, m), oracle.quantize_weight(fmt, w)):
+        assert np.array_equal(got, want)
