@@ -88,7 +88,9 @@ int inkq_glue_attention_quant_rows(inkq_ctx *ctx, const float *q_dev, const uint
 /* One token: inkq_glue_qknorm_rope_cache and inkq_glue_attention_quant in one kernel.  Starts from the fused qkv
  * projection's output row [(nq + 2 nkv) * 128]: per-head RMSNorm + RoPE of the query heads and of the new key, the new
  * key and value appended to the caches at position *pos0, attention over positions 0 .. *pos0, output quantized into
- * `out`.  Same arithmetic as the two calls; nq * 4 must not exceed twice the SM count. */
+ * `out`.  Same arithmetic as the two calls; nq * 4 must not exceed twice the SM count.  The position and the cached rows before
+ * it are read while the kernel in front of this call (which produces qkv_dev) still runs: a kernel of the caller's own that
+ * writes them directly in front of it must not let its successor start early (programmatic launch). */
 int inkq_glue_qkv_attention_quant(inkq_ctx *ctx, const float *qkv_dev, const float *q_norm_w, const float *k_norm_w, const float *cos_dev,
                                   const float *sin_dev, const int *pos0_dev, int nq, int nkv, int max_pos, float eps, float scale,
                                   uint16_t *k_cache_dev, uint16_t *v_cache_dev, inkq_act *out, int out_qmode);

@@ -319,8 +319,11 @@ __global__ void __cluster_dims__(ATT_S, 1, 1) __launch_bounds__(ATT_SPLIT_NT)
                       const int *__restrict__ pos0_dev, int nq, int nkv, int max_pos, float scale, float *__restrict__ out, const QuantOut qo,
                       const FusedQkv fz)
 {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // In the fused form the position and the cached keys and values come from kernels before the predecessor (the qkv projection), and
+    // those have completed: every kernel of this library lets its successor start only behind its own wait.  So they are
+    // requested while the projection still runs, and only its output row waits for it.
+    const bool fused = fz.qkv != nullptr;
+    if (!fused) asm volatile("griddepcontrol.wait;" ::: "memory");
     extern __shared__ float sm[];
     float *qs = sm;                               // 128
     float *part = sm + HEAD_DIM;                  // NW * 128
@@ -341,7 +344,6 @@ __global__ void __cluster_dims__(ATT_S, 1, 1) __launch_bounds__(ATT_SPLIT_NT)
     // more than 128 keys (contexts beyond 512 positions) takes the remaining ones in further, unprefetched passes.
     constexpr int KPASS = ATT_SPLIT_NT / 4, VPRE = 8;
     __shared__ __align__(16) __half knew[HEAD_DIM], vnew[HEAD_DIM];
-    const bool fused = fz.qkv != nullptr;
     // the newest key is the last one of the last share that holds any; in the fused form it comes from shared memory
     const int j_new = (fused && pos_raw < max_pos && n > 0 && k0 + n == nkeys) ? n - 1 : -1;   // (a position past the caches is not stored)
     uint4 pk0[4];
@@ -357,6 +359,8 @@ __global__ void __cluster_dims__(ATT_S, 1, 1) __launch_bounds__(ATT_SPLIT_NT)
         const int j = warp + u * ATT_SPLIT_NW;
         pv0[u] = (j < n && j != j_new) ? reinterpret_cast<const uint2 *>(vb + static_cast<size_t>(j) * HEAD_DIM)[lane] : make_uint2(0, 0);
     }
+    if (fused) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (!fused) {
         if (tid < HEAD_DIM) qs[tid] = q[static_cast<size_t>(h) * HEAD_DIM + tid];
     } else if (warp < 3) {

@@ -42,12 +42,13 @@ __global__ void __launch_bounds__(256) k_quantize_q8(const float4 *__restrict__ 
     // x, q and the planes point at the first of the M rows this launch quantizes; M_ld = M rounded up to 4 (the padding
     // rows of the planes are zeroed), ld = distance between two blocks' entries in the planes (>= M_ld: a launch may fill
     // a window of rows of a larger matrix)
-    // lets a dependent kernel launched with programmatic stream serialization (QGEMV, QGEMM) start its weight prefetch while
-    // this grid runs; it still waits for this grid's completion before reading.  Launched that way itself: its own launch
-    // overlaps the tail of the kernel before it, whose results (x) and readers (q and the planes) it waits for here (linear of
-    // 4096 x 4096 with 5 rows 13.4 -> 10.6 us)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // Launched with programmatic stream serialization: the launch overlaps the tail of the kernel before it, whose results (x) and
+    // readers (q and the planes) it waits for here (linear of 4096 x 4096 with 5 rows 13.4 -> 10.6 us).  Then a dependent kernel
+    // launched the same way (QGEMV, QGEMM) may start its weight prefetch while this grid runs; it still waits for this grid's
+    // completion before reading.  In this order, as in every kernel of the library: a kernel that starts early knows that all
+    // before its predecessor has completed (k_attention_split relies on it).
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int nb = K / QK;
     const long long gthread = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const long long blk = gthread >> 1;  // global block index over [M_ld][nb]; two lanes per block
