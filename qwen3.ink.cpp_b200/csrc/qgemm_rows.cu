@@ -11,8 +11,7 @@
 // Why mma.sync: it leaves the 16 x 8 dots of one block (K = 32) in the registers of the threads that scale them.  Every block
 // of every output needs its own fp32 conversion, scale product and one or two fused multiply-adds in the reference's order, so
 // the CUDA cores bound this path and not the tensor cores: a tcgen05 form (block dots in tensor memory, or as e4m3 parts with
-// the weights in tensor memory) keeps the tensor pipe 94 % idle and pays for the way back to registers, ~350 cycles of
-// hand-shakes per pair of blocks in narrow tiles and shared-memory bandwidth in wide ones.
+// the weights in tensor memory) keeps the tensor pipe ~90 % idle and pays for the way back to registers and for hand-shakes.
 //
 // What bounds it.  Up to 32 rows: the weight stream, and for layers with few rows the chain of a warp's dependent instructions
 // over K (an output's sum may not be split).  Every warp owns 16 weight rows and all columns: each weight byte is fetched once.
@@ -22,11 +21,15 @@
 // chain (fragment loads, product, conversion, scaling) is long and an SM has few warps in a tile of this size, so stages of 4 to 8
 // pairs are unrolled and one CTA of 8 warps gets up to 255 registers a thread.  The weights are read from L2 once per tile of
 // columns (CTAs of one weight tile are neighbours).
-// Measured (prefetched weights of distinct layers; before: the tcgen05 kernel this one replaced), A81W41: 24576 x 4096 with 5 rows
-// 59 -> 15.7 us (4.2 TB/s), 4096 x 4096 with 5 rows 37 -> 7.1, 12288 x 4096 with 48 rows 39 -> 21, with 128 rows 72 -> 53, with
-// 322 rows 128 -> 107, with 2048 rows 728 -> 643; A80W40 with 322 rows 111 -> 94, with 2048 rows 634 -> 560; A80W4Z 4096 x 12288
-// with 77 rows 83 -> 42.  Slower: scalar multiplications (+12 %), the conversion by a bias in the product's accumulator operand
-// (+20 %: it has to be moved there), fp16 operands with fp32 accumulators (+25 %) and e4m3 parts (x2).
+// Measured (weights of distinct layers), A81W41: 24576 x 4096 with 5 rows 14.1 us (5.0 TB/s), 4096 x 4096 with 5 rows 7.0, 12288 x 4096
+// with 24 rows 16, with 322 rows 99 (fp32 records), 24576 x 4096 with 322 rows 190; A80W40 12288 x 4096 with 2048 rows 525; A80W4Z 4096 x
+// 12288 with 77 rows 36.  Slower: scalar multiplications (+12 %), the conversion by a bias in the product's accumulator operand (+20 %: it
+// has to be moved there), fp16 operands with fp32 accumulators (+25 %), e4m3 parts (x2), the results staged in shared memory for whole-line
+// stores (+1 to 2 %), a stage's pairs unrolled by two (+1 to 8 %), a resident CTA that requests its next tile's stages during the stores
+// (K = 1024: -10 %, 322 and 77 rows at K = 4096 and 12288: +4 %, from the registers it takes).
+// A tcgen05 form (kind::i8 with the weights in tensor memory, dots read back 16 x 256 bits at a time, a relay warp and named barriers in
+// front of the scaling warps) takes 694 (A81W41) and 575 ns (A80W40) per pair of a 128 x 112 tile, exact fp16 operands 684 and 559, this
+// kernel 706 and 612: the scaling bounds them all alike, two packed operations and a conversion per dot at ~0.55 instructions a cycle.
 //
 // Operands: the weights are the MMA's A side, the activation rows its B side.  A packed byte holds element e of both blocks of
 // a pair, so one ldmatrix.x4 fetches the A fragments of two blocks.  Stages pass through a ring in shared memory: tiled TMA
@@ -393,7 +396,7 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
     X(13, (4, 2, 1, 4, 2, 2), (20.9f, 34.8f), (17.9f, 29.6f), (21.7f, 34.0f), 0.0f)  \
     X(14, (4, 2, 1, 7, 2, 2), (29.2f, 54.0f), (25.8f, 45.7f), (28.2f, 47.9f), 0.0f)  \
     X(15, (4, 2, 2, 4, 2, 2), (31.8f, 58.8f), (28.9f, 52.4f), (31.8f, 57.9f), 0.0f)  \
-    X(16, (4, 2, 2, 5, 2, 2), (39.7f, 73.4f), (33.9f, 61.8f), (36.4f, 67.2f), 0.0f)  \
+    X(16, (4, 2, 2, 5, 2, 2), (39.7f, 73.4f), (33.9f, 61.3f), (36.4f, 67.2f), 0.0f)  \
     X(17, (4, 1, 1, 5, 8, 1), (12.4f, 26.4f), (10.9f, 23.8f), (12.9f, 27.3f), -0.4f)
 
 #define QROWS_UNWRAP(...) __VA_ARGS__
