@@ -88,12 +88,16 @@ int inkq_glue_attention_quant_rows(inkq_ctx *ctx, const float *q_dev, const uint
 /* One token: inkq_glue_qknorm_rope_cache and inkq_glue_attention_quant in one kernel.  Starts from the fused qkv
  * projection's output row [(nq + 2 nkv) * 128]: per-head RMSNorm + RoPE of the query heads and of the new key, the new
  * key and value appended to the caches at position *pos0, attention over positions 0 .. *pos0, output quantized into
- * `out`.  Same arithmetic as the two calls; nq * 4 must not exceed twice the SM count.  The position and the cached rows before
- * it are read while the kernel in front of this call (which produces qkv_dev) still runs: a kernel of the caller's own that
- * writes them directly in front of it must not let its successor start early (programmatic launch). */
+ * `out`.  Same arithmetic as the two calls; nq * 4 must not exceed twice the SM count. */
 int inkq_glue_qkv_attention_quant(inkq_ctx *ctx, const float *qkv_dev, const float *q_norm_w, const float *k_norm_w, const float *cos_dev,
                                   const float *sin_dev, const int *pos0_dev, int nq, int nkv, int max_pos, float eps, float scale,
                                   uint16_t *k_cache_dev, uint16_t *v_cache_dev, inkq_act *out, int out_qmode);
+/* inkq_glue_decode_gemv (epilogue 0) of a layer of (nq + 2 nkv) * 128 rows into qkv_dev, and inkq_glue_qkv_attention_quant
+ * directly behind it: the same results as the two calls, with the position and the cached rows before it read while the product
+ * still runs.  So the product must not write them: qkv_dev must not overlap the caches or *pos0_dev. */
+int inkq_glue_decode_qkv_attention(inkq_ctx *ctx, const inkq_weight *w_qkv, const inkq_act *in, float *qkv_dev, const float *q_norm_w,
+                                   const float *k_norm_w, const float *cos_dev, const float *sin_dev, const int *pos0_dev, int nq, int nkv, int max_pos,
+                                   float eps, float scale, uint16_t *k_cache_dev, uint16_t *v_cache_dev, inkq_act *out, int out_qmode);
 /* a += b (residual).  qwen3/src/qwen/QwenDecoderLayer.cc:73,105 */
 int inkq_glue_add_inplace(inkq_ctx *ctx, float *a_dev, const float *b_dev, long long n);
 /* Greedy sampling: *token_out = argmax(logits) (first index on ties), appended to generated

@@ -313,17 +313,20 @@ struct FusedQkv {
     const float *qkv, *q_norm_w, *k_norm_w, *cos_t, *sin_t;
     float eps;
     __half *k_cache_w, *v_cache_w;
+    bool early;   // the launch in front is the qkv projection and nothing else: see the kernel
 };
 __global__ void __cluster_dims__(ATT_S, 1, 1) __launch_bounds__(ATT_SPLIT_NT)
     k_attention_split(const float *__restrict__ q, const __half *__restrict__ k_cache, const __half *__restrict__ v_cache,
                       const int *__restrict__ pos0_dev, int nq, int nkv, int max_pos, float scale, float *__restrict__ out, const QuantOut qo,
                       const FusedQkv fz)
 {
-    // In the fused form the position and the cached keys and values come from kernels before the predecessor (the qkv projection), and
-    // those have completed: every kernel of this library lets its successor start only behind its own wait.  So they are
-    // requested while the projection still runs, and only its output row waits for it.
+    // Behind a qkv projection that inkq_glue_decode_qkv_attention has launched itself, the position and the cached keys and values
+    // are requested while the projection still runs (-1 us a layer, a decode step 1473 -> 1437 us), and only its output row waits for
+    // it.  The projection writes neither, and what stands before it has completed: it lets this kernel start only behind its own wait.
+    // Behind anything else that does not hold: k_qknorm_rope_cache and this kernel append to the caches after they have let
+    // their successor start, so every other call waits first.
     const bool fused = fz.qkv != nullptr;
-    if (!fused) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!fz.early) asm volatile("griddepcontrol.wait;" ::: "memory");
     extern __shared__ float sm[];
     float *qs = sm;                               // 128
     float *part = sm + HEAD_DIM;                  // NW * 128
@@ -359,7 +362,7 @@ __global__ void __cluster_dims__(ATT_S, 1, 1) __launch_bounds__(ATT_SPLIT_NT)
         const int j = warp + u * ATT_SPLIT_NW;
         pv0[u] = (j < n && j != j_new) ? reinterpret_cast<const uint2 *>(vb + static_cast<size_t>(j) * HEAD_DIM)[lane] : make_uint2(0, 0);
     }
-    if (fused) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (fz.early) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (!fused) {
         if (tid < HEAD_DIM) qs[tid] = q[static_cast<size_t>(h) * HEAD_DIM + tid];
@@ -675,24 +678,55 @@ int inkq_glue_attention_quant(inkq_ctx *ctx, const float *q_dev, const uint16_t 
     return attention_impl(ctx, q_dev, k_cache_dev, v_cache_dev, pos0_dev, 1, nq, nkv, max_pos, scale, nullptr, quant_out_of(out, nq * HEAD_DIM, out_qmode));
 }
 
+// checks the arguments that the two calls below share, and gathers them
+static int fused_qkv_of(inkq_ctx *ctx, const float *qkv_dev, const float *q_norm_w, const float *k_norm_w, const float *cos_dev, const float *sin_dev,
+                        const int *pos0_dev, int nq, int nkv, int max_pos, float eps, uint16_t *k_cache_dev, uint16_t *v_cache_dev,
+                        const inkq_act *out, int out_qmode, FusedQkv *fz)
+{
+    INKQ_REQUIRE(ctx, qkv_dev && q_norm_w && k_norm_w && cos_dev && sin_dev && pos0_dev && k_cache_dev && v_cache_dev, "null argument");
+    INKQ_REQUIRE(ctx, nq >= 1 && nkv >= 1 && nq % nkv == 0 && max_pos >= 1, "bad head configuration");
+    INKQ_REQUIRE(ctx, out != nullptr && out->K == nq * HEAD_DIM, "the output activation handle must have been created for K = nq * 128");
+    INKQ_REQUIRE(ctx, out_qmode == INKQ_Q8_1_F16 || out_qmode == INKQ_Q8_0_F16 || out_qmode == INKQ_Q8_1_F32, "bad output quantization mode");
+    INKQ_REQUIRE(ctx, nq * ATT_S <= 2 * ctx->num_sms, "the form that starts from the qkv row serves at most SMs / 2 query heads");
+    fz->qkv = qkv_dev;
+    fz->q_norm_w = q_norm_w;
+    fz->k_norm_w = k_norm_w;
+    fz->cos_t = cos_dev;
+    fz->sin_t = sin_dev;
+    fz->eps = eps;
+    fz->k_cache_w = reinterpret_cast<__half *>(k_cache_dev);
+    fz->v_cache_w = reinterpret_cast<__half *>(v_cache_dev);
+    fz->early = false;
+    return INKQ_OK;
+}
+
 int inkq_glue_qkv_attention_quant(inkq_ctx *ctx, const float *qkv_dev, const float *q_norm_w, const float *k_norm_w, const float *cos_dev,
                                   const float *sin_dev, const int *pos0_dev, int nq, int nkv, int max_pos, float eps, float scale,
                                   uint16_t *k_cache_dev, uint16_t *v_cache_dev, inkq_act *out, int out_qmode)
 {
     int rc = glue_use(ctx);
     if (rc) return rc;
-    INKQ_REQUIRE(ctx, qkv_dev && q_norm_w && k_norm_w && cos_dev && sin_dev, "null argument");
-    INKQ_REQUIRE(ctx, out != nullptr && out->K == nq * HEAD_DIM, "the output activation handle must have been created for K = nq * 128");
-    INKQ_REQUIRE(ctx, out_qmode == INKQ_Q8_1_F16 || out_qmode == INKQ_Q8_0_F16 || out_qmode == INKQ_Q8_1_F32, "bad output quantization mode");
-    FusedQkv fz;
-    fz.qkv = qkv_dev;
-    fz.q_norm_w = q_norm_w;
-    fz.k_norm_w = k_norm_w;
-    fz.cos_t = cos_dev;
-    fz.sin_t = sin_dev;
-    fz.eps = eps;
-    fz.k_cache_w = reinterpret_cast<__half *>(k_cache_dev);
-    fz.v_cache_w = reinterpret_cast<__half *>(v_cache_dev);
+    FusedQkv fz{};
+    rc = fused_qkv_of(ctx, qkv_dev, q_norm_w, k_norm_w, cos_dev, sin_dev, pos0_dev, nq, nkv, max_pos, eps, k_cache_dev, v_cache_dev, out, out_qmode, &fz);
+    if (rc) return rc;
+    return attention_impl(ctx, nullptr, k_cache_dev, v_cache_dev, pos0_dev, 1, nq, nkv, max_pos, scale, nullptr, quant_out_of(out, nq * HEAD_DIM, out_qmode), 0,
+                          fz);
+}
+
+int inkq_glue_decode_qkv_attention(inkq_ctx *ctx, const inkq_weight *w_qkv, const inkq_act *in, float *qkv_dev, const float *q_norm_w,
+                                   const float *k_norm_w, const float *cos_dev, const float *sin_dev, const int *pos0_dev, int nq, int nkv, int max_pos,
+                                   float eps, float scale, uint16_t *k_cache_dev, uint16_t *v_cache_dev, inkq_act *out, int out_qmode)
+{
+    int rc = glue_use(ctx);
+    if (rc) return rc;
+    INKQ_REQUIRE(ctx, w_qkv != nullptr && w_qkv->rows == (nq + 2 * nkv) * HEAD_DIM, "the layer must have (nq + 2 nkv) * 128 rows");
+    INKQ_REQUIRE(ctx, out != in, "the output handle must not be the input");   // (quant_out_of marks it before the product has been launched)
+    FusedQkv fz{};
+    rc = fused_qkv_of(ctx, qkv_dev, q_norm_w, k_norm_w, cos_dev, sin_dev, pos0_dev, nq, nkv, max_pos, eps, k_cache_dev, v_cache_dev, out, out_qmode, &fz);
+    if (rc) return rc;
+    rc = inkq_glue_decode_gemv(ctx, w_qkv, in, qkv_dev, 0, nullptr, 0.0f, nullptr, out_qmode, nullptr);
+    if (rc) return rc;
+    fz.early = true;
     return attention_impl(ctx, nullptr, k_cache_dev, v_cache_dev, pos0_dev, 1, nq, nkv, max_pos, scale, nullptr, quant_out_of(out, nq * HEAD_DIM, out_qmode), 0,
                           fz);
 }
@@ -727,8 +761,6 @@ static int attention_impl(inkq_ctx *ctx, const float *q_dev, const uint16_t *k_c
     int rc = INKQ_OK;
     INKQ_REQUIRE(ctx, (q_dev || fz.qkv) && k_cache_dev && v_cache_dev && pos0_dev, "null argument");
     INKQ_REQUIRE(ctx, T >= 1 && nq % nkv == 0 && max_pos >= 1, "bad head configuration");
-    INKQ_REQUIRE(ctx, fz.qkv == nullptr || (T == 1 && nq * ATT_S <= 2 * ctx->num_sms),
-                 "the form that starts from the qkv row serves one token and at most SMs / 2 query heads");
     const bool quant_rows = qo.q != nullptr && (T > 1 || qrow0 > 0 || qo.M_ld > 4);
     if (T >= 16 || quant_rows)   // a prompt: tensor-core kernel (attention_prefill_mma.cu), 64 tokens of one query head per CTA
         return launch_attention_prefill_mma(ctx, q_dev, k_cache_dev, v_cache_dev, pos0_dev, T, nq, nkv, max_pos, scale, out_dev, qo, qrow0);

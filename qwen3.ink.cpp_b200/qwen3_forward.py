@@ -11,7 +11,7 @@ linear goes through Context.linear (Qwen_Linear_with_bias_Int4::forward: quantiz
 a prompt, + QGEMV for a single token); everything between them is the thin glue of
 csrc/glue_ops.cu.  In a decode step (one token) the norms, SiLU*up, the activation quantizer and the residual
 additions run in the epilogues of the kernels that produce each row (inkq_glue_decode_gemv,
-inkq_glue_qkv_attention_quant): 5 launches per layer instead of 11.  One decode step is captured once as a CUDA
+inkq_glue_decode_qkv_attention): 5 launches per layer instead of 11.  One decode step is captured once as a CUDA
 graph and replayed.
 
 Column-sharded form (world > 1, one process per GPU): every linear holds the weight rows [rank*N/P, (rank+1)*N/P) of the
@@ -196,12 +196,12 @@ class Qwen3Synthetic:
             nl = len(self.layers)
             self._chk(L.inkq_glue_rmsnorm_quant(h, _p(b["x"]), _p(self.layers[0]["ln1"]), eps, H, self.act_h.h, Q, None))
             for i, ly in enumerate(self.layers):
-                self._chk(L.inkq_glue_decode_gemv(h, ly["qkv"].h, self.act_h.h, _p(b["qkv"]), 0, None, eps, None, Q, None))
                 if cfg.decode_qkv_attention:
-                    self._chk(L.inkq_glue_qkv_attention_quant(h, _p(b["qkv"]), _p(ly["qn"]), _p(ly["kn"]), _p(self.cos), _p(self.sin), _p(self.pos),
-                                                              cfg.nq, cfg.nkv, cfg.max_pos, eps, C.c_float(scale), _p(ly["k_cache"][0]),
-                                                              _p(ly["v_cache"][0]), self.act_attn.h, Q))
+                    self._chk(L.inkq_glue_decode_qkv_attention(h, ly["qkv"].h, self.act_h.h, _p(b["qkv"]), _p(ly["qn"]), _p(ly["kn"]), _p(self.cos),
+                                                               _p(self.sin), _p(self.pos), cfg.nq, cfg.nkv, cfg.max_pos, eps, C.c_float(scale),
+                                                               _p(ly["k_cache"][0]), _p(ly["v_cache"][0]), self.act_attn.h, Q))
                 else:
+                    self._chk(L.inkq_glue_decode_gemv(h, ly["qkv"].h, self.act_h.h, _p(b["qkv"]), 0, None, eps, None, Q, None))
                     self._chk(L.inkq_glue_qknorm_rope_cache(h, _p(b["qkv"]), _p(ly["qn"]), _p(ly["kn"]), _p(self.cos), _p(self.sin), _p(self.pos), T,
                                                             cfg.nq, cfg.nkv, cfg.max_pos, eps, _p(b["q"]), _p(ly["k_cache"][0]), _p(ly["v_cache"][0])))
                     self._chk(L.inkq_glue_attention_quant(h, _p(b["q"]), _p(ly["k_cache"][0]), _p(ly["v_cache"][0]), _p(self.pos), cfg.nq, cfg.nkv,
