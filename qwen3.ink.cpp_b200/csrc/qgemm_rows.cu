@@ -445,13 +445,27 @@ static int launch_sized(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begi
     // Up to 32 rows one tile holds all of them, so every weight byte is fetched once.  No more 128-row tiles than SMs: one CTA
     // per SM, stages of eight pairs, and 64 instead of 128 weight rows if that still leaves one CTA per SM (us, against 4 pairs and
     // two CTAs everywhere: 12288 x 4096 with 5 rows 10.6 -> 9.4, with 24 rows 18.8 -> 16.8; 6144 x 4096 with 5 rows 9.5 -> 7.3, with
-    // 24 rows 13.3 -> 12.1).  More: 64-row CTAs, up to three to an SM, and stages of four.  The busiest SM then has 192 rows of
-    // 24576 instead of the 256 of two 128-row CTAs (5 rows 15.6 -> 14.1 = 5.0 TB/s, 12 rows 22.1 -> 19.0)
+    // 24 rows 13.3 -> 12.1).
+    // More tiles, stages of four pairs: 64-row CTAs, three to an SM, as long as all of them are resident at once.  The busiest SM then
+    // has 192 rows at most instead of the 256 of two 128-row CTAs.  Past that the fourth CTA of an SM is a second pass over K, and
+    // 128-row CTAs are faster up to the widest layers.  us with 64- and 128-row CTAs, A81W41, K = 4096, fp16 records:
+    //     weight rows (64-row CTAs)   8 activation rows   20 rows        32 rows
+    //     24576 (384)                 13.9    15.2        22.8    28.8   30.2    35.1
+    //     28416 (444)                 14.1    15.4        23.0    28.8   30.4    35.1
+    //     28672 (448)                 20.1    15.4        32.3    29.0   52.5    35.1
+    //     34816 (544)                 21.3    16.1        35.3    29.2   59.2    35.4
+    //     51200 (800)                 26.6    29.4        44.5    44.1   59.9    53.1
+    //     151936 (2374)               72.9    66.9       132     128    178     151
+    // (640 CTAs, 8 to 20 rows of an A8xW4x layer without zero points, 3 to 13 % faster with 64: not worth a rule).  Up to four rows the
+    // planes are narrower than the boxes of eight that fetch them, and with the two planes of A81W41 the larger number of
+    // 64-row CTAs pays for that: 24576 x 4096 with 2 rows 16.4 against 15.5, with fp32 records 17.9 against 16.1; A80W40 15.5 and 15.5.
     const bool narrow = w->tiles * 2 <= ctx->num_sms, single = w->tiles <= ctx->num_sms;
+    const bool half = (w->rows + 63) / 64 <= 3 * ctx->num_sms && (SCH != INKQ_A81W41 || prm.M > 4);
 #define QROWS_SMALL(n)                                                                                              \
     case n:                                                                                                         \
         if (narrow) return launch_one<SCH, S16, Tile<4, 1, 1, n, 8, n == 1 ? 2 : 1>>(ctx, a, w, m_begin, prm);      \
-        return single ? launch_one<SCH, S16, Tile<8, 1, 1, n, 8, 1>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<4, 1, 1, n, 4, 3>>(ctx, a, w, m_begin, prm);
+        if (single) return launch_one<SCH, S16, Tile<8, 1, 1, n, 8, 1>>(ctx, a, w, m_begin, prm);                   \
+        return half ? launch_one<SCH, S16, Tile<4, 1, 1, n, 4, 3>>(ctx, a, w, m_begin, prm) : launch_one<SCH, S16, Tile<8, 1, 1, n, 4, 2>>(ctx, a, w, m_begin, prm);
     switch ((prm.M + 7) / 8) {
         QROWS_SMALL(1)
         QROWS_SMALL(2)
