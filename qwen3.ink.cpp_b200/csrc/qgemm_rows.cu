@@ -369,40 +369,41 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
     return after_launch(ctx, "k_qgemm_rows");
 }
 
-// Tiles for more than 32 activation rows: shape, then the time (us) of one and of two tiles on every SM at K = 4096, without
-// the ~3 us that a launch takes, for A81W41, A80W40 and A80W4Z with fp16 scale records, and what a tile takes more with fp32
-// records.  Measured with weights of distinct layers;
-// only the ratios matter, and they hardly depend on K.  One CTA of 8 warps per SM with all the registers it wants and 4 to 8
-// unrolled pairs per stage: the fragment loads and products of several pairs overlap the scaling of the ones before (against two CTAs
-// of 128 registers and two-pair stages: 64 x 48 17.9 -> 14.2, 128 x 112 72 -> 51).  Two such CTAs side by side remain for
-// many tiles per SM, where one's set-up and stores hide behind the other's products.
+// Tiles for more than 32 activation rows: shape, then for A81W41, A80W40 and A80W4Z with fp16 scale records the time (us) of a launch
+// with one and with two tiles on every SM at K = 4096 and of every two tiles more (a third of the way from two to eight), and what a
+// tile takes more with fp32 records.  All times measured in one way: 148 tiles of weight rows, as many tiles of columns as the count
+// says, three layers in turn, the least of sixteen loops; two such measurements differ by 1 to 2 %.  Only the ratios matter, and they
+// hardly depend on K.  One CTA of 8 warps per SM with all the registers it wants and 4 to 8 unrolled pairs per stage: the fragment loads
+// and products of several pairs overlap the scaling of the ones before (against two CTAs of 128 registers and two-pair stages: 64 x 48
+// 17.9 -> 14.2, 128 x 112 72 -> 51).  Two such CTAs side by side remain for many tiles per SM, where one's set-up and stores hide behind
+// the other's products.
 // Per column the wide tiles cost least: fragments and scales of the weight rows are fetched once for more columns.
 // Half- and quarter-height tiles split a layer with few weight rows over more SMs.  64 x 40 with one warp per scheduler costs less per
 // column than 64 x 48 with two, which fetch and unpack every weight fragment twice (77 rows of 4096 x 12288, A80W4Z: 41 -> 36 us).
-#define QROWS_TILES(X)                                                               \
-    X(0, (2, 4, 1, 2, 8, 1), (9.9f, 21.9f), (9.1f, 20.5f), (11.2f, 24.3f), 0.0f)     \
-    X(1, (4, 2, 1, 2, 8, 1), (10.6f, 23.1f), (9.9f, 22.0f), (12.0f, 26.1f), 0.0f)    \
-    X(2, (4, 1, 2, 2, 4, 2), (10.8f, 17.5f), (10.2f, 16.3f), (11.9f, 19.2f), 2.6f)   \
-    X(3, (4, 2, 1, 3, 8, 1), (13.2f, 28.1f), (11.6f, 24.5f), (13.6f, 28.9f), 0.0f)   \
-    X(4, (4, 2, 1, 4, 6, 1), (17.0f, 35.8f), (15.5f, 32.7f), (17.8f, 37.1f), 0.0f)   \
-    X(5, (4, 2, 1, 5, 6, 1), (20.5f, 43.0f), (16.9f, 36.7f), (19.5f, 39.6f), 1.1f)   \
-    X(6, (4, 2, 1, 7, 4, 1), (27.0f, 56.2f), (23.0f, 47.7f), (25.3f, 52.2f), 0.0f)   \
-    X(7, (4, 2, 2, 2, 8, 1), (16.8f, 34.1f), (16.0f, 32.6f), (18.5f, 37.6f), 0.0f)   \
-    X(8, (4, 2, 2, 3, 6, 1), (22.2f, 45.7f), (20.4f, 41.8f), (23.3f, 47.7f), 0.0f)   \
-    X(9, (4, 2, 2, 4, 4, 1), (29.0f, 59.3f), (25.6f, 52.7f), (27.8f, 57.3f), 0.0f)   \
-    X(10, (4, 2, 2, 5, 4, 1), (34.1f, 69.6f), (30.4f, 62.1f), (32.8f, 67.2f), 0.0f)  \
-    X(11, (4, 2, 2, 6, 4, 1), (40.6f, 82.7f), (35.1f, 72.0f), (37.5f, 76.9f), 0.0f)  \
-    X(12, (4, 2, 2, 7, 4, 1), (45.8f, 92.9f), (39.7f, 80.9f), (41.8f, 85.2f), 1.4f)  \
-    X(13, (4, 2, 1, 4, 2, 2), (20.9f, 34.8f), (17.9f, 29.6f), (21.7f, 34.0f), 0.0f)  \
-    X(14, (4, 2, 1, 7, 2, 2), (29.2f, 54.0f), (25.8f, 45.7f), (28.2f, 47.9f), 0.0f)  \
-    X(15, (4, 2, 2, 4, 2, 2), (31.8f, 58.8f), (28.9f, 52.4f), (31.8f, 57.9f), 0.0f)  \
-    X(16, (4, 2, 2, 5, 2, 2), (39.7f, 73.4f), (33.9f, 61.3f), (36.4f, 67.2f), 0.0f)  \
-    X(17, (4, 1, 1, 5, 8, 1), (12.4f, 26.4f), (10.9f, 23.8f), (12.9f, 27.3f), -0.4f)
+#define QROWS_TILES(X)                                                                                    \
+    X(0, (2, 4, 1, 2, 8, 1), (12.2f, 24.1f, 23.7f), (11.6f, 22.7f, 22.3f), (13.5f, 26.6f, 26.3f), 0.0f)   \
+    X(1, (4, 2, 1, 2, 8, 1), (13.1f, 25.7f, 25.2f), (12.4f, 24.4f, 23.8f), (14.5f, 28.6f, 28.1f), 0.0f)   \
+    X(2, (4, 1, 2, 2, 4, 2), (13.3f, 19.8f, 18.4f), (12.7f, 18.7f, 17.4f), (14.4f, 21.5f, 20.3f), 2.6f)   \
+    X(3, (4, 2, 1, 3, 8, 1), (15.8f, 30.9f, 30.3f), (13.9f, 27.2f, 26.8f), (16.1f, 31.6f, 31.2f), 0.0f)   \
+    X(4, (4, 2, 1, 4, 6, 1), (19.4f, 38.5f, 38.0f), (17.9f, 35.5f, 35.0f), (20.1f, 39.9f, 39.3f), 0.0f)   \
+    X(5, (4, 2, 1, 5, 6, 1), (23.0f, 45.8f, 45.2f), (19.5f, 38.6f, 38.0f), (21.4f, 42.4f, 41.9f), 1.1f)   \
+    X(6, (4, 2, 1, 7, 4, 1), (29.6f, 59.0f, 58.3f), (25.5f, 50.4f, 49.9f), (27.8f, 54.9f, 54.4f), 0.0f)   \
+    X(7, (4, 2, 2, 2, 8, 1), (19.2f, 36.8f, 35.5f), (18.3f, 35.2f, 33.9f), (20.9f, 40.3f, 38.9f), 0.0f)   \
+    X(8, (4, 2, 2, 3, 6, 1), (24.8f, 48.4f, 47.4f), (22.9f, 44.4f, 43.3f), (25.8f, 50.3f, 49.4f), 0.0f)   \
+    X(9, (4, 2, 2, 4, 4, 1), (31.6f, 61.9f, 61.0f), (28.1f, 55.2f, 54.3f), (30.5f, 59.7f, 58.8f), 0.0f)   \
+    X(10, (4, 2, 2, 5, 4, 1), (36.6f, 72.3f, 71.3f), (32.8f, 64.7f, 63.9f), (35.4f, 69.8f, 69.1f), 0.0f)  \
+    X(11, (4, 2, 2, 6, 4, 1), (43.2f, 85.5f, 84.7f), (37.6f, 74.5f, 73.6f), (40.1f, 79.4f, 78.6f), 0.0f)  \
+    X(12, (4, 2, 2, 7, 4, 1), (48.4f, 95.7f, 94.9f), (42.2f, 83.4f, 82.5f), (44.3f, 87.7f, 86.9f), 1.4f)  \
+    X(13, (4, 2, 1, 4, 2, 2), (23.2f, 37.5f, 35.8f), (20.5f, 32.3f, 31.2f), (24.3f, 36.6f, 35.5f), 0.0f)  \
+    X(14, (4, 2, 1, 7, 2, 2), (31.8f, 56.7f, 54.6f), (28.2f, 48.4f, 46.2f), (30.8f, 50.7f, 48.8f), 0.0f)  \
+    X(15, (4, 2, 2, 4, 2, 2), (34.4f, 61.4f, 58.1f), (31.3f, 54.9f, 52.0f), (34.2f, 60.3f, 57.6f), 0.0f)  \
+    X(16, (4, 2, 2, 5, 2, 2), (42.4f, 76.0f, 72.2f), (36.3f, 64.5f, 61.4f), (39.0f, 69.7f, 66.2f), 0.0f)  \
+    X(17, (4, 1, 1, 5, 8, 1), (14.9f, 29.1f, 28.7f), (13.3f, 26.2f, 25.8f), (15.3f, 30.0f, 29.6f), -0.4f)
 
 #define QROWS_UNWRAP(...) __VA_ARGS__
 struct TileCost {
     int rows, cols;
-    float time[3][2];   // by weight scheme (A81W41, A80W40, A80W4Z), one and two tiles
+    float time[3][3];   // by weight scheme (A81W41, A80W40, A80W4Z): one tile, two, every two more
     float f32;          // more with fp32 scale records
 };
 static_assert(INKQ_A81W41 == 0 && INKQ_A80W40 == 1 && INKQ_A80W4Z == 2, "the schemes index the table");
@@ -423,7 +424,7 @@ static int pick_tile(const inkq_ctx *ctx, int scheme, bool s16, int rows, int M)
         const float *t = c.time[scheme];
         const long long total = static_cast<long long>((rows + c.rows - 1) / c.rows) * ((M + c.cols - 1) / c.cols);
         const long long n = (total + ctx->num_sms - 1) / ctx->num_sms;
-        const float time = static_cast<float>(n / 2) * t[1] + static_cast<float>(n % 2) * t[0] + (s16 ? 0.f : static_cast<float>(n) * c.f32);
+        const float time = t[(n - 1) % 2] + static_cast<float>((n - 1) / 2) * t[2] + (s16 ? 0.f : static_cast<float>(n) * c.f32);
         if (i == 0 || time < best_time) {
             best = i;
             best_time = time;
