@@ -369,47 +369,68 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
     return after_launch(ctx, "k_qgemm_rows");
 }
 
-// Tiles for more than 32 activation rows: shape, then for A81W41, A80W40 and A80W4Z with fp16 scale records the time (us) of a launch
-// with one and with two tiles on every SM at K = 4096 and of every two tiles more (a third of the way from two to eight), and what a
-// tile takes more with fp32 records.  All times measured in one way: 148 tiles of weight rows, as many tiles of columns as the count
-// says, three layers in turn, the least of sixteen loops; two such measurements differ by 1 to 2 %.  Only the ratios matter, and they
-// hardly depend on K.  One CTA of 8 warps per SM with all the registers it wants and 4 to 8 unrolled pairs per stage: the fragment loads
-// and products of several pairs overlap the scaling of the ones before (against two CTAs of 128 registers and two-pair stages: 64 x 48
+// Tiles for more than 32 activation rows: shape, then for A81W41, A80W40 and A80W4Z, first with fp16 and then with fp32 scale records,
+// the time (us) of a launch with one and with two tiles on every SM at K = 4096 and of every two tiles more (a third of the way from
+// two to eight).  All measured in one way: 148 tiles of weight rows, as many tiles of columns as the count says, three layers in turn,
+// the least of sixteen loops; two such measurements differ by 1 to 2 %.  The records' size makes up to 24 % of difference in either
+// direction, by tile and scheme: it changes the ring's stages and the registers.  Only the ratios matter, and they hardly depend on K:
+// over 240 random layers (33 to 2048 rows, K from 1024 to 12288) the chosen tile takes 0.6 % more than the best of the eighteen, at
+// most 20 % (2248 x 1088 with 73 rows); with the times of fp16 records for both it was 0.7 %, at most 26 %.
+// Mostly one CTA of 8 warps per SM with all the registers it wants and 4 to 8 unrolled pairs per stage: the fragment loads and products
+// of several pairs overlap the scaling of the ones before (against two CTAs of 128 registers and two-pair stages: 64 x 48
 // 17.9 -> 14.2, 128 x 112 72 -> 51).  Two such CTAs side by side remain for many tiles per SM, where one's set-up and stores hide behind
 // the other's products.
 // Per column the wide tiles cost least: fragments and scales of the weight rows are fetched once for more columns.
 // Half- and quarter-height tiles split a layer with few weight rows over more SMs.  64 x 40 with one warp per scheduler costs less per
 // column than 64 x 48 with two, which fetch and unpack every weight fragment twice (77 rows of 4096 x 12288, A80W4Z: 41 -> 36 us).
-#define QROWS_TILES(X)                                                                                    \
-    X(0, (2, 4, 1, 2, 8, 1), (12.2f, 24.1f, 23.7f), (11.6f, 22.7f, 22.3f), (13.5f, 26.6f, 26.3f), 0.0f)   \
-    X(1, (4, 2, 1, 2, 8, 1), (13.1f, 25.7f, 25.2f), (12.4f, 24.4f, 23.8f), (14.5f, 28.6f, 28.1f), 0.0f)   \
-    X(2, (4, 1, 2, 2, 4, 2), (13.3f, 19.8f, 18.4f), (12.7f, 18.7f, 17.4f), (14.4f, 21.5f, 20.3f), 2.6f)   \
-    X(3, (4, 2, 1, 3, 8, 1), (15.8f, 30.9f, 30.3f), (13.9f, 27.2f, 26.8f), (16.1f, 31.6f, 31.2f), 0.0f)   \
-    X(4, (4, 2, 1, 4, 6, 1), (19.4f, 38.5f, 38.0f), (17.9f, 35.5f, 35.0f), (20.1f, 39.9f, 39.3f), 0.0f)   \
-    X(5, (4, 2, 1, 5, 6, 1), (23.0f, 45.8f, 45.2f), (19.5f, 38.6f, 38.0f), (21.4f, 42.4f, 41.9f), 1.1f)   \
-    X(6, (4, 2, 1, 7, 4, 1), (29.6f, 59.0f, 58.3f), (25.5f, 50.4f, 49.9f), (27.8f, 54.9f, 54.4f), 0.0f)   \
-    X(7, (4, 2, 2, 2, 8, 1), (19.2f, 36.8f, 35.5f), (18.3f, 35.2f, 33.9f), (20.9f, 40.3f, 38.9f), 0.0f)   \
-    X(8, (4, 2, 2, 3, 6, 1), (24.8f, 48.4f, 47.4f), (22.9f, 44.4f, 43.3f), (25.8f, 50.3f, 49.4f), 0.0f)   \
-    X(9, (4, 2, 2, 4, 4, 1), (31.6f, 61.9f, 61.0f), (28.1f, 55.2f, 54.3f), (30.5f, 59.7f, 58.8f), 0.0f)   \
-    X(10, (4, 2, 2, 5, 4, 1), (36.6f, 72.3f, 71.3f), (32.8f, 64.7f, 63.9f), (35.4f, 69.8f, 69.1f), 0.0f)  \
-    X(11, (4, 2, 2, 6, 4, 1), (43.2f, 85.5f, 84.7f), (37.6f, 74.5f, 73.6f), (40.1f, 79.4f, 78.6f), 0.0f)  \
-    X(12, (4, 2, 2, 7, 4, 1), (48.4f, 95.7f, 94.9f), (42.2f, 83.4f, 82.5f), (44.3f, 87.7f, 86.9f), 1.4f)  \
-    X(13, (4, 2, 1, 4, 2, 2), (23.2f, 37.5f, 35.8f), (20.5f, 32.3f, 31.2f), (24.3f, 36.6f, 35.5f), 0.0f)  \
-    X(14, (4, 2, 1, 7, 2, 2), (31.8f, 56.7f, 54.6f), (28.2f, 48.4f, 46.2f), (30.8f, 50.7f, 48.8f), 0.0f)  \
-    X(15, (4, 2, 2, 4, 2, 2), (34.4f, 61.4f, 58.1f), (31.3f, 54.9f, 52.0f), (34.2f, 60.3f, 57.6f), 0.0f)  \
-    X(16, (4, 2, 2, 5, 2, 2), (42.4f, 76.0f, 72.2f), (36.3f, 64.5f, 61.4f), (39.0f, 69.7f, 66.2f), 0.0f)  \
-    X(17, (4, 1, 1, 5, 8, 1), (14.9f, 29.1f, 28.7f), (13.3f, 26.2f, 25.8f), (15.3f, 30.0f, 29.6f), -0.4f)
+#define QROWS_TILES(X)                                                                             \
+    X(0, (2, 4, 1, 2, 8, 1), (12.2f, 24.1f, 23.7f), (11.6f, 22.7f, 22.3f), (13.5f, 26.6f, 26.3f),  \
+      (12.6f, 24.4f, 24.0f), (11.6f, 22.4f, 22.0f), (13.6f, 26.8f, 26.4f))                         \
+    X(1, (4, 2, 1, 2, 8, 1), (13.1f, 25.7f, 25.2f), (12.4f, 24.4f, 23.8f), (14.5f, 28.6f, 28.1f),  \
+      (13.2f, 26.1f, 25.5f), (12.2f, 24.0f, 23.5f), (14.6f, 28.8f, 28.2f))                         \
+    X(2, (4, 1, 2, 2, 4, 2), (13.3f, 19.8f, 18.4f), (12.7f, 18.7f, 17.4f), (14.4f, 21.5f, 20.3f),  \
+      (15.6f, 21.0f, 19.8f), (15.8f, 20.9f, 20.0f), (17.2f, 23.9f, 22.4f))                         \
+    X(3, (4, 2, 1, 3, 8, 1), (15.8f, 30.9f, 30.3f), (13.9f, 27.2f, 26.8f), (16.1f, 31.6f, 31.2f),  \
+      (15.9f, 31.4f, 30.9f), (13.8f, 27.0f, 26.4f), (15.8f, 31.1f, 30.6f))                         \
+    X(4, (4, 2, 1, 4, 6, 1), (19.4f, 38.5f, 38.0f), (17.9f, 35.5f, 35.0f), (20.1f, 39.9f, 39.3f),  \
+      (19.9f, 39.5f, 39.1f), (16.8f, 33.5f, 32.8f), (19.1f, 37.8f, 37.2f))                         \
+    X(5, (4, 2, 1, 5, 6, 1), (23.0f, 45.8f, 45.2f), (19.5f, 38.6f, 38.0f), (21.4f, 42.4f, 41.9f),  \
+      (26.1f, 51.5f, 51.6f), (19.5f, 38.7f, 38.1f), (21.1f, 41.9f, 41.4f))                         \
+    X(6, (4, 2, 1, 7, 4, 1), (29.6f, 59.0f, 58.3f), (25.5f, 50.4f, 49.9f), (27.8f, 54.9f, 54.4f),  \
+      (30.1f, 59.9f, 59.4f), (25.4f, 50.2f, 49.3f), (27.7f, 54.9f, 54.2f))                         \
+    X(7, (4, 2, 2, 2, 8, 1), (19.2f, 36.8f, 35.5f), (18.3f, 35.2f, 33.9f), (20.9f, 40.3f, 38.9f),  \
+      (18.3f, 34.8f, 33.4f), (18.4f, 35.2f, 33.7f), (21.0f, 40.2f, 38.6f))                         \
+    X(8, (4, 2, 2, 3, 6, 1), (24.8f, 48.4f, 47.4f), (22.9f, 44.4f, 43.3f), (25.8f, 50.3f, 49.4f),  \
+      (24.5f, 47.6f, 46.2f), (23.5f, 45.7f, 44.3f), (26.1f, 50.9f, 49.8f))                         \
+    X(9, (4, 2, 2, 4, 4, 1), (31.6f, 61.9f, 61.0f), (28.1f, 55.2f, 54.3f), (30.5f, 59.7f, 58.8f),  \
+      (30.7f, 59.8f, 58.8f), (27.9f, 54.5f, 53.5f), (30.8f, 60.2f, 59.2f))                         \
+    X(10, (4, 2, 2, 5, 4, 1), (36.6f, 72.3f, 71.3f), (32.8f, 64.7f, 63.9f), (35.4f, 69.8f, 69.1f), \
+      (36.1f, 71.0f, 70.0f), (32.2f, 63.6f, 62.7f), (34.8f, 68.7f, 67.5f))                         \
+    X(11, (4, 2, 2, 6, 4, 1), (43.2f, 85.5f, 84.7f), (37.6f, 74.5f, 73.6f), (40.1f, 79.4f, 78.6f), \
+      (41.6f, 82.0f, 81.0f), (36.8f, 72.9f, 72.0f), (38.7f, 76.6f, 75.7f))                         \
+    X(12, (4, 2, 2, 7, 4, 1), (48.4f, 95.7f, 94.9f), (42.2f, 83.4f, 82.5f), (44.3f, 87.7f, 86.9f), \
+      (49.6f, 99.0f, 97.9f), (43.2f, 86.0f, 85.2f), (45.9f, 91.3f, 90.4f))                         \
+    X(13, (4, 2, 1, 4, 2, 2), (23.2f, 37.5f, 35.8f), (20.5f, 32.3f, 31.2f), (24.3f, 36.6f, 35.5f), \
+      (22.5f, 37.2f, 36.0f), (20.7f, 32.5f, 31.4f), (23.6f, 35.7f, 34.7f))                         \
+    X(14, (4, 2, 1, 7, 2, 2), (31.8f, 56.7f, 54.6f), (28.2f, 48.4f, 46.2f), (30.8f, 50.7f, 48.8f), \
+      (32.1f, 57.7f, 55.3f), (27.6f, 47.2f, 45.2f), (30.0f, 49.9f, 47.9f))                         \
+    X(15, (4, 2, 2, 4, 2, 2), (34.4f, 61.4f, 58.1f), (31.3f, 54.9f, 52.0f), (34.2f, 60.3f, 57.6f), \
+      (34.4f, 60.3f, 56.8f), (31.2f, 54.7f, 51.7f), (33.6f, 59.6f, 56.4f))                         \
+    X(16, (4, 2, 2, 5, 2, 2), (42.4f, 76.0f, 72.2f), (36.3f, 64.5f, 61.4f), (39.0f, 69.7f, 66.2f), \
+      (42.7f, 75.8f, 71.8f), (36.0f, 63.9f, 60.5f), (38.1f, 68.9f, 65.3f))                         \
+    X(17, (4, 1, 1, 5, 8, 1), (14.9f, 29.1f, 28.7f), (13.3f, 26.2f, 25.8f), (15.3f, 30.0f, 29.6f), \
+      (14.8f, 28.9f, 28.3f), (12.6f, 24.7f, 24.2f), (14.4f, 28.2f, 27.8f))
 
 #define QROWS_UNWRAP(...) __VA_ARGS__
 struct TileCost {
     int rows, cols;
-    float time[3][3];   // by weight scheme (A81W41, A80W40, A80W4Z): one tile, two, every two more
-    float f32;          // more with fp32 scale records
+    float time[2][3][3];   // by scale records (fp16, fp32) and weight scheme (A81W41, A80W40, A80W4Z): one tile, two, every two more
 };
 static_assert(INKQ_A81W41 == 0 && INKQ_A80W40 == 1 && INKQ_A80W4Z == 2, "the schemes index the table");
 static constexpr TileCost tile_costs[] = {
-#define QROWS_COST(i, shape, w41, w40, w4z, f32) \
-    {Tile<QROWS_UNWRAP shape>::ROWS, Tile<QROWS_UNWRAP shape>::COLS, {{QROWS_UNWRAP w41}, {QROWS_UNWRAP w40}, {QROWS_UNWRAP w4z}}, f32},
+#define QROWS_COST(i, shape, h41, h40, h4z, f41, f40, f4z)           \
+    {Tile<QROWS_UNWRAP shape>::ROWS, Tile<QROWS_UNWRAP shape>::COLS, \
+     {{{QROWS_UNWRAP h41}, {QROWS_UNWRAP h40}, {QROWS_UNWRAP h4z}}, {{QROWS_UNWRAP f41}, {QROWS_UNWRAP f40}, {QROWS_UNWRAP f4z}}}},
     QROWS_TILES(QROWS_COST)
 };
 
@@ -421,10 +442,10 @@ static int pick_tile(const inkq_ctx *ctx, int scheme, bool s16, int rows, int M)
     float best_time = 0.f;
     for (int i = 0; i < static_cast<int>(sizeof(tile_costs) / sizeof(tile_costs[0])); i++) {
         const TileCost &c = tile_costs[i];
-        const float *t = c.time[scheme];
+        const float *t = c.time[s16 ? 0 : 1][scheme];
         const long long total = static_cast<long long>((rows + c.rows - 1) / c.rows) * ((M + c.cols - 1) / c.cols);
         const long long n = (total + ctx->num_sms - 1) / ctx->num_sms;
-        const float time = t[(n - 1) % 2] + static_cast<float>((n - 1) / 2) * t[2] + (s16 ? 0.f : static_cast<float>(n) * c.f32);
+        const float time = t[(n - 1) % 2] + static_cast<float>((n - 1) / 2) * t[2];
         if (i == 0 || time < best_time) {
             best = i;
             best_time = time;
@@ -439,7 +460,7 @@ static int launch_sized(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begi
     if (prm.M > 32) {
         const int tile = pick_tile(ctx, SCH, S16, prm.rows, prm.M);
         switch (tile) {
-#define QROWS_CASE(i, shape, w41, w40, w4z, f32) case i: return launch_one<SCH, S16, Tile<QROWS_UNWRAP shape>>(ctx, a, w, m_begin, prm);
+#define QROWS_CASE(i, shape, h41, h40, h4z, f41, f40, f4z) case i: return launch_one<SCH, S16, Tile<QROWS_UNWRAP shape>>(ctx, a, w, m_begin, prm);
             QROWS_TILES(QROWS_CASE)
         }
     }

@@ -155,6 +155,15 @@ def test_gemm_tiles_of_64_rows(pkg, gpu, scheme, scale_mode, M, N, K):
 
 @pytest.mark.parametrize("scheme", [0, 1, 2])
 @pytest.mark.parametrize("scale_mode", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(41, 6280, 576), (161, 12552, 192), (241, 15808, 64), (1572, 264, 448), (225, 18952, 64), (81, 3096, 576), (33, 9528, 320),
+                                   (241, 7072, 192)])
+def test_gemm_tiles_that_one_scheme_or_record_size_takes(pkg, gpu, scheme, scale_mode, M, N, K):
+    """With the sizes above: every tile in every combination of weight scheme and scale records that the times of the tiles choose."""
+    test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K)
+
+
+@pytest.mark.parametrize("scheme", [0, 1, 2])
+@pytest.mark.parametrize("scale_mode", [0, 1])
 @pytest.mark.parametrize("M,N,K", [(4, 20480, 320), (5, 28416, 64), (32, 28416, 576), (5, 28424, 64), (20, 34816, 320), (9, 37888, 64), (2, 37896, 64),
                                    (32, 37896, 576)])
 def test_gemm_up_to_32_rows_of_wide_layers(pkg, gpu, scheme, scale_mode, M, N, K):
