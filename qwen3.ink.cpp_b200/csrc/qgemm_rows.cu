@@ -16,8 +16,9 @@
 // What bounds it.  Up to 32 rows: the weight stream, and for layers with few rows the chain of a warp's dependent instructions
 // over K (an output's sum may not be split).  Every warp owns 16 weight rows and all columns: each weight byte is fetched once.
 // Stages of four pairs (256 K-elements) are unrolled, so that the fragment loads and products of one pair overlap the scaling of
-// the one before.  More rows: the register file and the FMA pipe.  Alone in registers, a block's 16 x 8 dots take a scheduler 22
-// cycles with four warps (27 with mins, of which 20 are the packed multiplications, three operands of 64 bits each).  A block's
+// the one before.  More rows: conversions, register file and FMA pipe.  Alone in registers, with two warps of 32 x 56 dots a scheduler,
+// a block's 16 x 8 dots (a product, four conversions, two packed multiplications and two packed multiply-adds, four with mins) take it
+// 19 cycles, 23 with mins; 10.7 and 15.6 of them the packed operations, three operands of 64 bits each.  A block's
 // chain (fragment loads, product, conversion, scaling) is long and an SM has few warps in a tile of this size, so stages of 4 to 8
 // pairs are unrolled and one CTA of 8 warps gets up to 255 registers a thread.  The weights are read from L2 once per tile of
 // columns (CTAs of one weight tile are neighbours).

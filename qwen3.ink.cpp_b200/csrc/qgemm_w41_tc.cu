@@ -16,9 +16,9 @@
 // shared memory (16 KB written and read again per stage and tile) the shared-memory port was as busy as the tensor pipe.
 // What bounds it: up to ~100 columns the turns of the dequantising warps and of the thread that issues the products (~260 cycles a
 // stage of one weight tile: waits of ~60 cycles each, instruction fetch of six warps with different code on a scheduler, hand-over),
-// above the tensor pipe.  Measured at K = 4096: 12288 rows x 17 columns 17 us, x 64 17.8 (22.3 before the waits' slow path left the
-// loops and the issuing thread stopped waiting for the copies itself), x 322 33.5, x 2048 160 (1.29 PFLOP/s); 4096 x 322 17.7 (22.6),
-// 4096 x 12288 with 322 rows 44 (58).  Slower: A in shared memory with 8 dequantising warps (12288 x 322 53 us), one chunk per thread and
+// above the tensor pipe.  Measured at K = 4096: 12288 rows x 17 columns 16.8 us, x 64 17.7 (21.4 and 22.1 before the waits' slow path left the
+// loops and the issuing thread stopped waiting for the copies itself), x 322 32.4 (32.8: two weight tiles per CTA), x 2048 158 (157;
+// 1.31 PFLOP/s); 4096 x 322 17.4 (22.4), 4096 x 12288 with 322 rows 44 (58).  Slower: A in shared memory with 8 dequantising warps (12288 x 322 53 us), one chunk per thread and
 // turn (+15 %), the stores of a stage completing under the next one's arithmetic (+5 %: one slot less), two stages per copy (+10 %), the two
 // chunks of a turn in a rolled loop (192 columns +8 %).
 //
