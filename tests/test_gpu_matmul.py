@@ -149,7 +149,7 @@ def test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K):
 @pytest.mark.parametrize("scale_mode", [0, 1])
 @pytest.mark.parametrize("M,N,K", [(41, 3848, 192), (77, 4088, 1088), (80, 3912, 576), (42, 21976, 64), (2, 18952, 64), (9, 18960, 320), (32, 18952, 576)])
 def test_gemm_tiles_of_64_rows(pkg, gpu, scheme, scale_mode, M, N, K):
-    """64 x 40 and 64 x 48 tiles, and 64-row CTAs with up to 32 rows at both sides of 148 weight tiles."""
+    """64 x 40 and 64 x 48 tiles, and 64-row CTAs with up to 32 rows (A81W41 with two: 128-row ones) above 148 weight tiles."""
     test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K)
 
 
