@@ -11,6 +11,17 @@ namespace inkq {
 
 constexpr int GEMV_UNROLL = 2;   // pairs per batch; two batches are in flight per lane
 
+// Four products of an unsigned and a signed byte, added to c
+__device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c)
+{
+    int d;
+    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+
+// The dots of a pair's two blocks.  Until the first batch is used the weights wait for the activations and not the other way round, so
+// instructions between the two are what a layer's product takes on top of its launch: without a shift per word of high nibbles a decode
+// step of 36 layers takes 1408 us instead of 1433.
 __device__ __forceinline__ void dots_of_pair(const uint4 c0, const uint4 c1, const uint32_t *__restrict__ a_lo,
                                              const uint32_t *__restrict__ a_hi, int &ilo, int &ihi)
 {
@@ -20,8 +31,9 @@ __device__ __forceinline__ void dots_of_pair(const uint4 c0, const uint4 c1, con
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         ilo = __dp4a(static_cast<int>(w[i] & 0x0F0F0F0Fu), static_cast<int>(a_lo[i]), ilo);
-        ihi = __dp4a(static_cast<int>((w[i] >> 4) & 0x0F0F0F0Fu), static_cast<int>(a_hi[i]), ihi);
+        ihi = dp4a_us(w[i] & 0xF0F0F0F0u, a_hi[i], ihi);   // bytes of 16 q: no shift per word
     }
+    ihi >>= 4;   // exact: a multiple of 16, below 2^20 in magnitude
 }
 
 // One batch of GEMV_UNROLL pairs of this lane's row, as loaded.
