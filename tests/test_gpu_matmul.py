@@ -162,6 +162,15 @@ def test_gemm_tiles_that_one_scheme_or_record_size_takes(pkg, gpu, scheme, scale
     test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K)
 
 
+@pytest.mark.parametrize("scheme", [1, 2])
+@pytest.mark.parametrize("scale_mode", [0, 1])
+@pytest.mark.parametrize("cols", range(40, 121, 8))
+def test_gemm_tiles_of_schemes_without_mins(pkg, gpu, scheme, scale_mode, cols):
+    """128 x 40 to 128 x 120 tiles, 8 warps of 16 rows by all columns: one on every SM, ragged in rows and stages, a column short and full."""
+    test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, cols - 1, 18936, 448)
+    test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, cols, 18936, 64)
+
+
 @pytest.mark.parametrize("scheme", [0, 1, 2])
 @pytest.mark.parametrize("scale_mode", [0, 1])
 @pytest.mark.parametrize("M,N,K", [(4, 20480, 320), (5, 28416, 64), (32, 28416, 576), (5, 28424, 64), (20, 34816, 320), (9, 37888, 64), (2, 37896, 64),
