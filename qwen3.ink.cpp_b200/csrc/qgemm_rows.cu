@@ -67,10 +67,12 @@ struct Params {
 };
 
 // Shape of a tile: WR x WC warps, each with MT groups of 16 weight rows and NT groups of 8 activation rows; SP pairs per stage;
-// CTAS resident CTAs per SM.
-template <int WR_, int WC_, int MT_, int NT_, int SP_, int CTAS_ = 2>
+// CTAS resident CTAs per SM; SHORT: the second column of warps has one group of activation rows less (each scheduler has a warp of both).
+template <int WR_, int WC_, int MT_, int NT_, int SP_, int CTAS_ = 2, bool SHORT_ = false>
 struct Tile {
-    static constexpr int WR = WR_, WC = WC_, MT = MT_, NT = NT_, SP = SP_, CTAS = CTAS_, ROWS = 16 * WR * MT, COLS = 8 * NT * WC;
+    static constexpr int WR = WR_, WC = WC_, MT = MT_, NT = NT_, SP = SP_, CTAS = CTAS_, ROWS = 16 * WR * MT, COLS = 8 * (NT * WC - (SHORT_ ? 1 : 0));
+    static constexpr bool SHORT = SHORT_;
+    static_assert(!SHORT || (WC == 2 && WR == 4), "warps w and w + 4 share a scheduler");
 };
 
 // SCH: weight scheme; S16: fp16 scale records
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(32 * T::WR * T::WC, T::CTAS)
     __syncthreads();
 
     const int row0 = (warp % T::WR) * (16 * MT), col0 = (warp / T::WR) * (8 * NT);   // the warp's first row and column inside the tile
+    const bool is_short = T::SHORT && warp >= T::WR;         // this warp leaves its last group of activation rows out
     const int g = lane >> 2, t2 = (lane & 3) * 2;            // fragment coordinates: rows g, g + 8; columns t2, t2 + 1
     // ldmatrix row addresses.  A: matrices (rows 0-7, chunk 0), (rows 8-15, chunk 0), (rows 0-7, chunk 1), (rows 8-15, chunk 1)
     const int a_row = row0 + ((lane >> 3) & 1) * 8 + (lane & 7);
@@ -234,6 +237,7 @@ __global__ void __launch_bounds__(32 * T::WR * T::WC, T::CTAS)
         }
 #pragma unroll
         for (int j = 0; j < NT; j++) {
+            if (T::SHORT && j == NT - 1 && is_short) break;
             uint32_t b[4];
             ldmatrix_x4(b, st + (pj >> 1) * (G::BM * 128) + (b_off ^ ((pj & 1) << 6)) + j * (8 * 128));
             const uint32_t pl = st + (2 * pj) * (G::BM * 4) + (col0 + j * 8 + t2) * 4;
@@ -323,7 +327,7 @@ __global__ void __launch_bounds__(32 * T::WR * T::WC, T::CTAS)
 #pragma unroll
             for (int c = 0; c < 2; c++) {
                 const int m = m_base + col0 + j * 8 + t2 + c;
-                if (m < prm.M) {
+                if (m < prm.M && !(T::SHORT && j == NT - 1 && is_short)) {
 #pragma unroll
                     for (int i = 0; i < MT; i++)
 #pragma unroll
@@ -389,6 +393,9 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
 // us with 4 x 2 and with 8 x 1 warps: 48 columns A80W40 22.9, 21.6, A80W4Z 25.8, 22.7; 64: 28.1, 27.4 and 30.5, 28.2; 96: 37.6, 37.1 and
 // 40.1, 37.7; 112: 42.2, 41.7 and 44.3, 43.6; and sizes between the multiples of 16 that two columns of warps have.  With mins it is the other
 // way round: 48 columns 24.8, 26.5, 64: 31.6, 33.8; 322 rows of 4096 x 4096 47.1 with 96 columns by 4 x 2 warps, 48.2 with 88 by 8.
+// With mins 88 columns are 48 for one column of warps and 40 for the other (41.5 us a tile, 96 columns 43.2; 322 rows of 4096 x 4096 47.1 -> 45.8,
+// of 4096 x 12288 129.5 -> 126.1): the last group of the longer ones stands in a block of its own, which costs half of what is left out, and
+// 72 and 104 columns gain nothing over 80 and 112.  With two bodies of code instead 88 columns take 58 us (instruction fetch).
 // 12288 x 4096 with 2048 rows, A80W40 541 -> 518 us (128 x 104); 4096 x 12288 with 322 rows 113 -> 101, A80W4Z 120 -> 106 (128 x 88).
 enum Who { ANY, MINS, PLAIN };   // schemes that a tile serves: all, A81W41, the ones without mins
 constexpr bool serves(Who who, int scheme) { return who == ANY || (who == MINS) == (scheme == INKQ_A81W41); }
@@ -451,7 +458,9 @@ constexpr bool serves(Who who, int scheme) { return who == ANY || (who == MINS) 
     X(27, PLAIN, (8, 1, 1, 14, 4, 1), NEVER, (41.7f, 82.5f, 81.0f), (43.6f, 85.9f, 84.5f),                 \
       NEVER, (43.5f, 85.8f, 84.2f), (44.1f, 87.3f, 86.0f))                                                 \
     X(28, PLAIN, (8, 1, 1, 15, 4, 1), NEVER, (44.7f, 88.4f, 86.9f), (45.6f, 90.4f, 88.9f),                 \
-      NEVER, (45.5f, 89.6f, 87.9f), (46.6f, 92.7f, 91.3f))
+      NEVER, (45.5f, 89.6f, 87.9f), (46.6f, 92.7f, 91.3f))                                                 \
+    X(29, MINS, (4, 2, 2, 6, 4, 1, true), (41.5f, 81.7f, 80.2f), NEVER, NEVER,                             \
+      (40.7f, 79.9f, 78.5f), NEVER, NEVER)
 
 #define QROWS_UNWRAP(...) __VA_ARGS__
 struct TileCost {

@@ -171,6 +171,13 @@ def test_gemm_tiles_of_schemes_without_mins(pkg, gpu, scheme, scale_mode, cols):
     test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, cols, 18936, 64)
 
 
+@pytest.mark.parametrize("scale_mode", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(88, 18936, 448), (81, 18944, 64), (261, 4088, 320), (352, 4096, 576)])
+def test_gemm_tile_with_a_short_column_of_warps(pkg, gpu, scale_mode, M, N, K):
+    """128 x 88 tiles of A81W41: their last columns belong to the next tile."""
+    test_gemm_tile_shapes(pkg, gpu, 0, scale_mode, M, N, K)
+
+
 @pytest.mark.parametrize("scheme", [0, 1, 2])
 @pytest.mark.parametrize("scale_mode", [0, 1])
 @pytest.mark.parametrize("M,N,K", [(4, 20480, 320), (5, 28416, 64), (32, 28416, 576), (5, 28424, 64), (20, 34816, 320), (9, 37888, 64), (2, 37896, 64),
