@@ -374,13 +374,16 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
     return after_launch(ctx, "k_qgemm_rows");
 }
 
-// Tiles for more than 32 activation rows: shape, then for A81W41, A80W40 and A80W4Z, first with fp16 and then with fp32 scale records,
-// the time (us) of a launch with one and with two tiles on every SM at K = 4096 and of every two tiles more (a third of the way from
-// two to eight).  All measured in one way: 148 tiles of weight rows, as many tiles of columns as the count says, three layers in turn,
-// the least of sixteen loops; two such measurements differ by 1 to 2 %.  The records' size makes up to 24 % of difference in either
-// direction, by tile and scheme: it changes the ring's stages and the registers.  Only the ratios matter, and they hardly depend on K:
-// over 240 random layers (33 to 2048 rows, K from 1024 to 12288) the chosen of eighteen tiles took 0.6 % more than the best, at
-// most 20 % (2248 x 1088 with 73 rows); with the times of fp16 records for both it was 0.7 %, at most 26 %.
+// Tiles for more than 32 activation rows: shape, the part of a launch's time (us) that does not depend on K, and for A81W41, A80W40 and
+// A80W4Z, first with fp16 and then with fp32 scale records, the whole time at K = 4096; each with one and with two tiles on every SM and of
+// every two tiles more (a third of the way from two to eight).  All measured in one way: 148 tiles of weight rows, as many tiles of columns
+// as the count says, three layers in turn, the least of sixteen loops; two such measurements differ by 1 to 2 %.  The records' size makes up
+// to 24 % of difference in either direction, by tile and scheme: it changes the ring's stages and the registers.  The fixed part is a CTA's
+// set-up and its stores, from times at K = 512 and 4096; it hardly depends on scheme and records (their mean, mostly 0.3 us from each).
+// Only the ratios matter.  Over 240 random layers each (33 to 2048 rows) the chosen tile takes 0.3 % more than the best one, at most 18 %
+// (1248 x 1920 with 224 rows), for K from 1024 to 12288, and 1.5 %, at most 25 % (5360 x 576 with 42 rows: 4.2 us), for K from 64 to 1023.
+// By the times at K = 4096 alone the latter took 5.7 % more, at most 80 %: two CTAs per SM hide set-up and stores behind each other's
+// products, and short rows are little else (818 rows of 16832 x 384, A80W4Z with fp32 records: 49.8 -> 40.3 us).
 // Mostly one CTA of 8 warps per SM with all the registers it wants and 4 to 8 unrolled pairs per stage: the fragment loads and products
 // of several pairs overlap the scaling of the ones before (against two CTAs of 128 registers and two-pair stages: 64 x 48
 // 17.9 -> 14.2, 128 x 112 72 -> 51).  Two such CTAs side by side remain for many tiles per SM, where one's set-up and stores hide behind
@@ -400,93 +403,97 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
 enum Who { ANY, MINS, PLAIN };   // schemes that a tile serves: all, A81W41, the ones without mins
 constexpr bool serves(Who who, int scheme) { return who == ANY || (who == MINS) == (scheme == INKQ_A81W41); }
 #define NEVER (1e30f, 1e30f, 1e30f)
-#define QROWS_TILES(X)                                                                                     \
-    X(0, ANY, (2, 4, 1, 2, 8, 1), (12.2f, 24.1f, 23.7f), (11.6f, 22.7f, 22.3f), (13.5f, 26.6f, 26.3f),     \
-      (12.6f, 24.4f, 24.0f), (11.6f, 22.4f, 22.0f), (13.6f, 26.8f, 26.4f))                                 \
-    X(1, ANY, (4, 2, 1, 2, 8, 1), (13.1f, 25.7f, 25.2f), (12.4f, 24.4f, 23.8f), (14.5f, 28.6f, 28.1f),     \
-      (13.2f, 26.1f, 25.5f), (12.2f, 24.0f, 23.5f), (14.6f, 28.8f, 28.2f))                                 \
-    X(2, ANY, (4, 1, 2, 2, 4, 2), (13.3f, 19.8f, 18.4f), (12.7f, 18.7f, 17.4f), (14.4f, 21.5f, 20.3f),     \
-      (15.6f, 21.0f, 19.8f), (15.8f, 20.9f, 20.0f), (17.2f, 23.9f, 22.4f))                                 \
-    X(3, ANY, (4, 2, 1, 3, 8, 1), (15.8f, 30.9f, 30.3f), (13.9f, 27.2f, 26.8f), (16.1f, 31.6f, 31.2f),     \
-      (15.9f, 31.4f, 30.9f), (13.8f, 27.0f, 26.4f), (15.8f, 31.1f, 30.6f))                                 \
-    X(4, ANY, (4, 2, 1, 4, 6, 1), (19.4f, 38.5f, 38.0f), (17.9f, 35.5f, 35.0f), (20.1f, 39.9f, 39.3f),     \
-      (19.9f, 39.5f, 39.1f), (16.8f, 33.5f, 32.8f), (19.1f, 37.8f, 37.2f))                                 \
-    X(5, ANY, (4, 2, 1, 5, 6, 1), (23.0f, 45.8f, 45.2f), (19.5f, 38.6f, 38.0f), (21.4f, 42.4f, 41.9f),     \
-      (26.1f, 51.5f, 51.6f), (19.5f, 38.7f, 38.1f), (21.1f, 41.9f, 41.4f))                                 \
-    X(6, ANY, (4, 2, 1, 7, 4, 1), (29.6f, 59.0f, 58.3f), (25.5f, 50.4f, 49.9f), (27.8f, 54.9f, 54.4f),     \
-      (30.1f, 59.9f, 59.4f), (25.4f, 50.2f, 49.3f), (27.7f, 54.9f, 54.2f))                                 \
-    X(7, ANY, (4, 2, 2, 2, 8, 1), (19.2f, 36.8f, 35.5f), (18.3f, 35.2f, 33.9f), (20.9f, 40.3f, 38.9f),     \
-      (18.3f, 34.8f, 33.4f), (18.4f, 35.2f, 33.7f), (21.0f, 40.2f, 38.6f))                                 \
-    X(8, MINS, (4, 2, 2, 3, 6, 1), (24.8f, 48.4f, 47.4f), NEVER, NEVER,                                    \
-      (24.5f, 47.6f, 46.2f), NEVER, NEVER)                                                                 \
-    X(9, MINS, (4, 2, 2, 4, 4, 1), (31.6f, 61.9f, 61.0f), NEVER, NEVER,                                    \
-      (30.7f, 59.8f, 58.8f), NEVER, NEVER)                                                                 \
-    X(10, MINS, (4, 2, 2, 5, 4, 1), (36.6f, 72.3f, 71.3f), NEVER, NEVER,                                   \
-      (36.1f, 71.0f, 70.0f), NEVER, NEVER)                                                                 \
-    X(11, MINS, (4, 2, 2, 6, 4, 1), (43.2f, 85.5f, 84.7f), NEVER, NEVER,                                   \
-      (41.6f, 82.0f, 81.0f), NEVER, NEVER)                                                                 \
-    X(12, MINS, (4, 2, 2, 7, 4, 1), (48.4f, 95.7f, 94.9f), NEVER, NEVER,                                   \
-      (49.6f, 99.0f, 97.9f), NEVER, NEVER)                                                                 \
-    X(13, ANY, (4, 2, 1, 4, 2, 2), (23.2f, 37.5f, 35.8f), (20.5f, 32.3f, 31.2f), (24.3f, 36.6f, 35.5f),    \
-      (22.5f, 37.2f, 36.0f), (20.7f, 32.5f, 31.4f), (23.6f, 35.7f, 34.7f))                                 \
-    X(14, ANY, (4, 2, 1, 7, 2, 2), (31.8f, 56.7f, 54.6f), (28.2f, 48.4f, 46.2f), (30.8f, 50.7f, 48.8f),    \
-      (32.1f, 57.7f, 55.3f), (27.6f, 47.2f, 45.2f), (30.0f, 49.9f, 47.9f))                                 \
-    X(15, ANY, (4, 2, 2, 4, 2, 2), (34.4f, 61.4f, 58.1f), (31.3f, 54.9f, 52.0f), (34.2f, 60.3f, 57.6f),    \
-      (34.4f, 60.3f, 56.8f), (31.2f, 54.7f, 51.7f), (33.6f, 59.6f, 56.4f))                                 \
-    X(16, ANY, (4, 2, 2, 5, 2, 2), (42.4f, 76.0f, 72.2f), (36.3f, 64.5f, 61.4f), (39.0f, 69.7f, 66.2f),    \
-      (42.7f, 75.8f, 71.8f), (36.0f, 63.9f, 60.5f), (38.1f, 68.9f, 65.3f))                                 \
-    X(17, ANY, (4, 1, 1, 5, 8, 1), (14.9f, 29.1f, 28.7f), (13.3f, 26.2f, 25.8f), (15.3f, 30.0f, 29.6f),    \
-      (14.8f, 28.9f, 28.3f), (12.6f, 24.7f, 24.2f), (14.4f, 28.2f, 27.8f))                                 \
-    X(18, PLAIN, (8, 1, 1, 5, 6, 1), NEVER, (19.3f, 36.8f, 35.4f), (20.3f, 38.9f, 37.3f),                  \
-      NEVER, (19.4f, 36.8f, 35.4f), (20.4f, 38.7f, 37.4f))                                                 \
-    X(19, PLAIN, (8, 1, 1, 6, 6, 1), NEVER, (21.6f, 41.7f, 40.1f), (22.7f, 43.6f, 42.2f),                  \
-      NEVER, (22.0f, 42.1f, 40.4f), (23.5f, 45.1f, 43.5f))                                                 \
-    X(20, PLAIN, (8, 1, 1, 7, 6, 1), NEVER, (24.0f, 46.2f, 44.8f), (25.9f, 50.0f, 48.3f),                  \
-      NEVER, (24.3f, 46.7f, 45.2f), (25.4f, 49.1f, 47.4f))                                                 \
-    X(21, PLAIN, (8, 1, 1, 8, 4, 1), NEVER, (27.4f, 53.0f, 51.7f), (28.2f, 54.6f, 53.4f),                  \
-      NEVER, (27.7f, 53.2f, 52.1f), (28.6f, 55.1f, 53.9f))                                                 \
-    X(22, PLAIN, (8, 1, 1, 9, 4, 1), NEVER, (29.9f, 58.2f, 56.8f), (31.0f, 60.4f, 59.3f),                  \
-      NEVER, (29.7f, 57.6f, 56.4f), (30.9f, 60.5f, 59.1f))                                                 \
-    X(23, PLAIN, (8, 1, 1, 10, 4, 1), NEVER, (32.6f, 63.8f, 62.4f), (33.3f, 65.3f, 64.1f),                 \
-      NEVER, (31.7f, 61.9f, 60.6f), (32.8f, 64.6f, 63.2f))                                                 \
-    X(24, PLAIN, (8, 1, 1, 11, 4, 1), NEVER, (34.3f, 67.2f, 66.1f), (35.7f, 70.5f, 69.1f),                 \
-      NEVER, (34.5f, 67.8f, 66.4f), (35.7f, 70.2f, 68.8f))                                                 \
-    X(25, PLAIN, (8, 1, 1, 12, 4, 1), NEVER, (37.1f, 72.8f, 72.0f), (37.7f, 74.4f, 73.0f),                 \
-      NEVER, (37.1f, 73.1f, 71.7f), (38.0f, 74.9f, 73.6f))                                                 \
-    X(26, PLAIN, (8, 1, 1, 13, 4, 1), NEVER, (39.4f, 77.7f, 76.2f), (40.6f, 79.7f, 78.3f),                 \
-      NEVER, (39.9f, 78.5f, 77.0f), (40.5f, 80.0f, 78.7f))                                                 \
-    X(27, PLAIN, (8, 1, 1, 14, 4, 1), NEVER, (41.7f, 82.5f, 81.0f), (43.6f, 85.9f, 84.5f),                 \
-      NEVER, (43.5f, 85.8f, 84.2f), (44.1f, 87.3f, 86.0f))                                                 \
-    X(28, PLAIN, (8, 1, 1, 15, 4, 1), NEVER, (44.7f, 88.4f, 86.9f), (45.6f, 90.4f, 88.9f),                 \
-      NEVER, (45.5f, 89.6f, 87.9f), (46.6f, 92.7f, 91.3f))                                                 \
-    X(29, MINS, (4, 2, 2, 6, 4, 1, true), (41.5f, 81.7f, 80.2f), NEVER, NEVER,                             \
+#define QROWS_TILES(X)                                                                                                          \
+    X(0, ANY, (2, 4, 1, 2, 8, 1), (2.2f, 3.6f, 3.2f), (12.2f, 24.1f, 23.7f), (11.6f, 22.7f, 22.3f), (13.5f, 26.6f, 26.3f),      \
+      (12.6f, 24.4f, 24.0f), (11.6f, 22.4f, 22.0f), (13.6f, 26.8f, 26.4f))                                                      \
+    X(1, ANY, (4, 2, 1, 2, 8, 1), (2.0f, 3.3f, 2.9f), (13.1f, 25.7f, 25.2f), (12.4f, 24.4f, 23.8f), (14.5f, 28.6f, 28.1f),      \
+      (13.2f, 26.1f, 25.5f), (12.2f, 24.0f, 23.5f), (14.6f, 28.8f, 28.2f))                                                      \
+    X(2, ANY, (4, 1, 2, 2, 4, 2), (2.1f, 2.1f, 1.0f), (13.3f, 19.8f, 18.4f), (12.7f, 18.7f, 17.4f), (14.4f, 21.5f, 20.3f),      \
+      (15.6f, 21.0f, 19.8f), (15.8f, 20.9f, 20.0f), (17.2f, 23.9f, 22.4f))                                                      \
+    X(3, ANY, (4, 2, 1, 3, 8, 1), (2.0f, 3.8f, 3.4f), (15.8f, 30.9f, 30.3f), (13.9f, 27.2f, 26.8f), (16.1f, 31.6f, 31.2f),      \
+      (15.9f, 31.4f, 30.9f), (13.8f, 27.0f, 26.4f), (15.8f, 31.1f, 30.6f))                                                      \
+    X(4, ANY, (4, 2, 1, 4, 6, 1), (2.6f, 4.9f, 4.5f), (19.4f, 38.5f, 38.0f), (17.9f, 35.5f, 35.0f), (20.1f, 39.9f, 39.3f),      \
+      (19.9f, 39.5f, 39.1f), (16.8f, 33.5f, 32.8f), (19.1f, 37.8f, 37.2f))                                                      \
+    X(5, ANY, (4, 2, 1, 5, 6, 1), (2.7f, 5.2f, 4.6f), (23.0f, 45.8f, 45.2f), (19.5f, 38.6f, 38.0f), (21.4f, 42.4f, 41.9f),      \
+      (26.1f, 51.5f, 51.6f), (19.5f, 38.7f, 38.1f), (21.1f, 41.9f, 41.4f))                                                      \
+    X(6, ANY, (4, 2, 1, 7, 4, 1), (2.7f, 5.1f, 4.9f), (29.6f, 59.0f, 58.3f), (25.5f, 50.4f, 49.9f), (27.8f, 54.9f, 54.4f),      \
+      (30.1f, 59.9f, 59.4f), (25.4f, 50.2f, 49.3f), (27.7f, 54.9f, 54.2f))                                                      \
+    X(7, ANY, (4, 2, 2, 2, 8, 1), (2.1f, 3.4f, 2.5f), (19.2f, 36.8f, 35.5f), (18.3f, 35.2f, 33.9f), (20.9f, 40.3f, 38.9f),      \
+      (18.3f, 34.8f, 33.4f), (18.4f, 35.2f, 33.7f), (21.0f, 40.2f, 38.6f))                                                      \
+    X(8, MINS, (4, 2, 2, 3, 6, 1), (2.7f, 4.4f, 3.6f), (24.8f, 48.4f, 47.4f), NEVER, NEVER,                                     \
+      (24.5f, 47.6f, 46.2f), NEVER, NEVER)                                                                                      \
+    X(9, MINS, (4, 2, 2, 4, 4, 1), (2.7f, 4.5f, 3.7f), (31.6f, 61.9f, 61.0f), NEVER, NEVER,                                     \
+      (30.7f, 59.8f, 58.8f), NEVER, NEVER)                                                                                      \
+    X(10, MINS, (4, 2, 2, 5, 4, 1), (3.0f, 5.0f, 4.2f), (36.6f, 72.3f, 71.3f), NEVER, NEVER,                                    \
+      (36.1f, 71.0f, 70.0f), NEVER, NEVER)                                                                                      \
+    X(11, MINS, (4, 2, 2, 6, 4, 1), (3.2f, 5.4f, 4.9f), (43.2f, 85.5f, 84.7f), NEVER, NEVER,                                    \
+      (41.6f, 82.0f, 81.0f), NEVER, NEVER)                                                                                      \
+    X(12, MINS, (4, 2, 2, 7, 4, 1), (3.3f, 5.5f, 5.3f), (48.4f, 95.7f, 94.9f), NEVER, NEVER,                                    \
+      (49.6f, 99.0f, 97.9f), NEVER, NEVER)                                                                                      \
+    X(13, ANY, (4, 2, 1, 4, 2, 2), (2.7f, 2.7f, 2.5f), (23.2f, 37.5f, 35.8f), (20.5f, 32.3f, 31.2f), (24.3f, 36.6f, 35.5f),     \
+      (22.5f, 37.2f, 36.0f), (20.7f, 32.5f, 31.4f), (23.6f, 35.7f, 34.7f))                                                      \
+    X(14, ANY, (4, 2, 1, 7, 2, 2), (2.4f, 2.9f, 2.3f), (31.8f, 56.7f, 54.6f), (28.2f, 48.4f, 46.2f), (30.8f, 50.7f, 48.8f),     \
+      (32.1f, 57.7f, 55.3f), (27.6f, 47.2f, 45.2f), (30.0f, 49.9f, 47.9f))                                                      \
+    X(15, ANY, (4, 2, 2, 4, 2, 2), (2.2f, 2.7f, 1.9f), (34.4f, 61.4f, 58.1f), (31.3f, 54.9f, 52.0f), (34.2f, 60.3f, 57.6f),     \
+      (34.4f, 60.3f, 56.8f), (31.2f, 54.7f, 51.7f), (33.6f, 59.6f, 56.4f))                                                      \
+    X(16, ANY, (4, 2, 2, 5, 2, 2), (2.3f, 3.1f, 1.9f), (42.4f, 76.0f, 72.2f), (36.3f, 64.5f, 61.4f), (39.0f, 69.7f, 66.2f),     \
+      (42.7f, 75.8f, 71.8f), (36.0f, 63.9f, 60.5f), (38.1f, 68.9f, 65.3f))                                                      \
+    X(17, ANY, (4, 1, 1, 5, 8, 1), (2.3f, 4.1f, 3.6f), (14.9f, 29.1f, 28.7f), (13.3f, 26.2f, 25.8f), (15.3f, 30.0f, 29.6f),     \
+      (14.8f, 28.9f, 28.3f), (12.6f, 24.7f, 24.2f), (14.4f, 28.2f, 27.8f))                                                      \
+    X(18, PLAIN, (8, 1, 1, 5, 6, 1), (2.7f, 4.2f, 3.5f), NEVER, (19.3f, 36.8f, 35.4f), (20.3f, 38.9f, 37.3f),                   \
+      NEVER, (19.4f, 36.8f, 35.4f), (20.4f, 38.7f, 37.4f))                                                                      \
+    X(19, PLAIN, (8, 1, 1, 6, 6, 1), (2.7f, 4.3f, 3.6f), NEVER, (21.6f, 41.7f, 40.1f), (22.7f, 43.6f, 42.2f),                   \
+      NEVER, (22.0f, 42.1f, 40.4f), (23.5f, 45.1f, 43.5f))                                                                      \
+    X(20, PLAIN, (8, 1, 1, 7, 6, 1), (2.8f, 4.6f, 3.9f), NEVER, (24.0f, 46.2f, 44.8f), (25.9f, 50.0f, 48.3f),                   \
+      NEVER, (24.3f, 46.7f, 45.2f), (25.4f, 49.1f, 47.4f))                                                                      \
+    X(21, PLAIN, (8, 1, 1, 8, 4, 1), (2.6f, 4.3f, 3.6f), NEVER, (27.4f, 53.0f, 51.7f), (28.2f, 54.6f, 53.4f),                   \
+      NEVER, (27.7f, 53.2f, 52.1f), (28.6f, 55.1f, 53.9f))                                                                      \
+    X(22, PLAIN, (8, 1, 1, 9, 4, 1), (2.8f, 4.6f, 4.0f), NEVER, (29.9f, 58.2f, 56.8f), (31.0f, 60.4f, 59.3f),                   \
+      NEVER, (29.7f, 57.6f, 56.4f), (30.9f, 60.5f, 59.1f))                                                                      \
+    X(23, PLAIN, (8, 1, 1, 10, 4, 1), (2.9f, 4.8f, 4.2f), NEVER, (32.6f, 63.8f, 62.4f), (33.3f, 65.3f, 64.1f),                  \
+      NEVER, (31.7f, 61.9f, 60.6f), (32.8f, 64.6f, 63.2f))                                                                      \
+    X(24, PLAIN, (8, 1, 1, 11, 4, 1), (3.1f, 5.1f, 4.5f), NEVER, (34.3f, 67.2f, 66.1f), (35.7f, 70.5f, 69.1f),                  \
+      NEVER, (34.5f, 67.8f, 66.4f), (35.7f, 70.2f, 68.8f))                                                                      \
+    X(25, PLAIN, (8, 1, 1, 12, 4, 1), (3.2f, 5.4f, 4.9f), NEVER, (37.1f, 72.8f, 72.0f), (37.7f, 74.4f, 73.0f),                  \
+      NEVER, (37.1f, 73.1f, 71.7f), (38.0f, 74.9f, 73.6f))                                                                      \
+    X(26, PLAIN, (8, 1, 1, 13, 4, 1), (3.3f, 5.6f, 5.2f), NEVER, (39.4f, 77.7f, 76.2f), (40.6f, 79.7f, 78.3f),                  \
+      NEVER, (39.9f, 78.5f, 77.0f), (40.5f, 80.0f, 78.7f))                                                                      \
+    X(27, PLAIN, (8, 1, 1, 14, 4, 1), (3.3f, 5.7f, 5.5f), NEVER, (41.7f, 82.5f, 81.0f), (43.6f, 85.9f, 84.5f),                  \
+      NEVER, (43.5f, 85.8f, 84.2f), (44.1f, 87.3f, 86.0f))                                                                      \
+    X(28, PLAIN, (8, 1, 1, 15, 4, 1), (3.4f, 5.8f, 5.8f), NEVER, (44.7f, 88.4f, 86.9f), (45.6f, 90.4f, 88.9f),                  \
+      NEVER, (45.5f, 89.6f, 87.9f), (46.6f, 92.7f, 91.3f))                                                                      \
+    X(29, MINS, (4, 2, 2, 6, 4, 1, true), (2.7f, 4.3f, 3.7f), (41.5f, 81.7f, 80.2f), NEVER, NEVER,                              \
       (40.7f, 79.9f, 78.5f), NEVER, NEVER)
 
 #define QROWS_UNWRAP(...) __VA_ARGS__
 struct TileCost {
     int rows, cols;
+    float fixed[3];        // part of the times below that does not depend on K
     float time[2][3][3];   // by scale records (fp16, fp32) and weight scheme (A81W41, A80W40, A80W4Z): one tile, two, every two more
 };
 static_assert(INKQ_A81W41 == 0 && INKQ_A80W40 == 1 && INKQ_A80W4Z == 2, "the schemes index the table");
 static constexpr TileCost tile_costs[] = {
-#define QROWS_COST(i, who, shape, h41, h40, h4z, f41, f40, f4z)           \
-    {Tile<QROWS_UNWRAP shape>::ROWS, Tile<QROWS_UNWRAP shape>::COLS, \
+#define QROWS_COST(i, who, shape, fixed, h41, h40, h4z, f41, f40, f4z)                      \
+    {Tile<QROWS_UNWRAP shape>::ROWS, Tile<QROWS_UNWRAP shape>::COLS, {QROWS_UNWRAP fixed}, \
      {{{QROWS_UNWRAP h41}, {QROWS_UNWRAP h40}, {QROWS_UNWRAP h4z}}, {{QROWS_UNWRAP f41}, {QROWS_UNWRAP f40}, {QROWS_UNWRAP f4z}}}},
     QROWS_TILES(QROWS_COST)
 };
 
 // The tile with the least time for M activation rows: a CTA takes one tile, so the busiest SM works through
 // n = ceil(tiles / SMs) of them.
-static int pick_tile(const inkq_ctx *ctx, int scheme, bool s16, int rows, int M)
+static int pick_tile(int num_sms, int scheme, bool s16, int rows, int pairs, int M)
 {
+    const float length = static_cast<float>(pairs) / 64.0f;   // of a row, in units of the K = 4096 of the table
     int best = 0;
     float best_time = 0.f;
     for (int i = 0; i < static_cast<int>(sizeof(tile_costs) / sizeof(tile_costs[0])); i++) {
         const TileCost &c = tile_costs[i];
         const float *t = c.time[s16 ? 0 : 1][scheme];
         const long long total = static_cast<long long>((rows + c.rows - 1) / c.rows) * ((M + c.cols - 1) / c.cols);
-        const long long n = (total + ctx->num_sms - 1) / ctx->num_sms;
-        const float time = t[(n - 1) % 2] + static_cast<float>((n - 1) / 2) * t[2];
+        const long long n = (total + num_sms - 1) / num_sms;
+        const float whole = t[(n - 1) % 2] + static_cast<float>((n - 1) / 2) * t[2];
+        const float fixed = c.fixed[(n - 1) % 2] + static_cast<float>((n - 1) / 2) * c.fixed[2];
+        const float time = fixed + (whole - fixed) * length;
         if (i == 0 || time < best_time) {
             best = i;
             best_time = time;
@@ -499,9 +506,9 @@ template <int SCH, bool S16>
 static int launch_sized(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin, const Params &prm)
 {
     if (prm.M > 32) {
-        const int tile = pick_tile(ctx, SCH, S16, prm.rows, prm.M);
+        const int tile = pick_tile(ctx->num_sms, SCH, S16, prm.rows, prm.pairs, prm.M);
         switch (tile) {
-#define QROWS_CASE(i, who, shape, h41, h40, h4z, f41, f40, f4z) \
+#define QROWS_CASE(i, who, shape, fixed, h41, h40, h4z, f41, f40, f4z) \
     case i:                                                     \
         if constexpr (serves(who, SCH)) return launch_one<SCH, S16, Tile<QROWS_UNWRAP shape>>(ctx, a, w, m_begin, prm); \
         break;
