@@ -145,6 +145,9 @@ int inkq_gemv_host(inkq_ctx *ctx, const inkq_act *act, const inkq_weight *w, flo
 int inkq_debug_block_dots(inkq_ctx *ctx, const inkq_act *act, const inkq_weight *w, int32_t *dots_dev);
 /* As inkq_debug_block_dots but produced by the tensor-core kernel's own MMA path. */
 int inkq_debug_block_dots_tc(inkq_ctx *ctx, const inkq_act *act, const inkq_weight *w, int32_t *dots_dev);
+/* Which of its tiles inkq_gemm takes for M > 32 activation rows and a layer of `rows` x K on a device of num_sms SMs: tile[0] its index,
+ * tile[1] and tile[2] its weight and activation rows.  Needs no context and no device: lets tests check that their sizes cover every tile. */
+int inkq_debug_gemm_tile(int num_sms, int scheme, int scale_mode, int rows, int K, int M, int *tile);
 
 /* ---- the linear layer's forward ---------------------------------------------
  * Replaces Qwen_Linear_with_bias_Int4::forward (QwenOperator.h:224,

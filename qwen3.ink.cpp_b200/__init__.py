@@ -34,7 +34,7 @@ SYMBOLS = [
     "inkq_ctx_create", "inkq_ctx_destroy", "inkq_ctx_set_stream", "inkq_ctx_synchronize", "inkq_last_error",
     "inkq_launch_count", "inkq_weight_create", "inkq_weight_create_dev", "inkq_weight_destroy", "inkq_weight_info",
     "inkq_weight_export", "inkq_act_create", "inkq_act_destroy", "inkq_quantize", "inkq_act_export", "inkq_act_import", "inkq_quantize_host", "inkq_gemm_host", "inkq_gemv_host", "inkq_gemm",
-    "inkq_gemv", "inkq_gemm_simt", "inkq_debug_block_dots", "inkq_debug_block_dots_tc", "inkq_linear",
+    "inkq_gemv", "inkq_gemm_simt", "inkq_debug_block_dots", "inkq_debug_block_dots_tc", "inkq_debug_gemm_tile", "inkq_linear",
     "inkq_linear_host", "inkq_linear_m1_static", "inkq_gemm_w41_f16act", "inkq_gemm_w41_f16act_simt", "inkq_f16w_create", "inkq_f16w_create_dev", "inkq_f16w_destroy", "inkq_f16w_matmul_prec",
     "inkq_f16w_matmul", "inkq_peer_export", "inkq_peerset_open", "inkq_peerset_from_pointers", "inkq_peerset_destroy",
     "inkq_linear_scatter", "inkq_gemm_scatter", "inkq_peer_barrier", "inkq_f16w_matmul_scatter", "inkq_weight_quantize_dev",

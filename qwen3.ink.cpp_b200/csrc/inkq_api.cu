@@ -587,6 +587,17 @@ int inkq_debug_block_dots_tc(inkq_ctx *ctx, const inkq_act *act, const inkq_weig
     return launch_gemm(ctx, act, w, nullptr, 0, dots_dev);
 }
 
+int inkq_debug_gemm_tile(int num_sms, int scheme, int scale_mode, int rows, int K, int M, int *tile)
+{
+    INKQ_REQUIRE(nullptr, tile != nullptr, "null output");
+    INKQ_REQUIRE(nullptr, scheme >= INKQ_A81W41 && scheme <= INKQ_A80W4Z, "unknown weight scheme");
+    INKQ_REQUIRE(nullptr, scale_mode == INKQ_SCALES_F32 || scale_mode == INKQ_SCALES_F16, "unknown scale mode");
+    INKQ_REQUIRE(nullptr, num_sms > 0 && rows > 0 && M > 32, "needs SMs, weight rows and more than 32 activation rows");
+    INKQ_REQUIRE(nullptr, K > 0 && K % (2 * QK) == 0, "K must be a multiple of 64");
+    gemm_tile(num_sms, scheme, scale_mode == INKQ_SCALES_F16, rows, K, M, tile);
+    return INKQ_OK;
+}
+
 // ---- linear forward ---------------------------------------------------------------------
 // The context's activation scratch (the reference's ModelContext::activation_buffer, sized once for the
 // largest layer, QwenForCausalLM.cc:101-113): one allocation that serves every (M, K) whose M*K fits.  It

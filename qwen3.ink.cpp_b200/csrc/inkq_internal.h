@@ -211,6 +211,7 @@ int launch_block_dots(inkq_ctx *ctx, const Act *a, const Weight *w, int32_t *dot
 // QGEMM (qgemm_rows.cu); m_begin / m_count: a window of the activation rows (m_begin a multiple of 4; C and the extra
 // destinations still point at row 0).  dots: raw int32 block dots instead of C
 int launch_gemm(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc, int32_t *dots, const ExtraDst *extra = nullptr, int m_begin = 0, int m_count = -1);
+void gemm_tile(int num_sms, int scheme, bool s16, int rows, int K, int M, int *tile);   // M > 32: index, weight rows and columns of launch_gemm's tile
 int launch_gemm_w41_f16(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc);   // CUDA cores
 int launch_gemm_w41_tc(inkq_ctx *ctx, const uint16_t *a16, int M, const Weight *w, float *C, int ldc);    // tcgen05 kind::f16
 bool gemm_w41_rows_fits(const uint16_t *a16, int M, int K);                                                   // whether the next one serves this call

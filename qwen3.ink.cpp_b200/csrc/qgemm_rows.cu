@@ -550,6 +550,13 @@ static int launch_sized(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begi
 
 }  // namespace qrows
 
+void gemm_tile(int num_sms, int scheme, bool s16, int rows, int K, int M, int *tile)
+{
+    tile[0] = qrows::pick_tile(num_sms, scheme, s16, rows, K / (2 * QK), M);
+    tile[1] = qrows::tile_costs[tile[0]].rows;
+    tile[2] = qrows::tile_costs[tile[0]].cols;
+}
+
 int launch_gemm(inkq_ctx *ctx, const Act *a, const Weight *w, float *C, int ldc, int32_t *dots, const ExtraDst *extra, int m_begin, int m_count)
 {
     using namespace qrows;

@@ -108,7 +108,7 @@ def test_gemm_bit_identical_to_oracle(pkg, gpu, oracle, impl, scheme, scale_mode
 @pytest.mark.parametrize("scale_mode", [0, 1])
 @pytest.mark.parametrize("N,K", [(200, 64), (264, 448), (9736, 320)])     # few and many weight tiles, ragged last tile, partial last stages
 def test_gemm_tile_edges(pkg, gpu, scheme, scale_mode, N, K):
-    """Both sides of every tile width (8-row steps up to 32 rows, 16-row steps above) against the CUDA-core kernel."""
+    """Both sides of tile widths (8-row steps up to 32 rows, 8- and 16-row steps above) against the CUDA-core kernel."""
     import torch
     w = pkg.synth.weights(N, K, 7)
     if scale_mode == 0:
@@ -131,7 +131,7 @@ def test_gemm_tile_edges(pkg, gpu, scheme, scale_mode, N, K):
                                    (65, 6144, 1088), (97, 6136, 448), (145, 6144, 320), (289, 4088, 320), (321, 4096, 192), (322, 12288, 320),
                                    (49, 24576, 64), (97, 24568, 64), (145, 12288, 192), (289, 8192, 192), (8, 19000, 320), (20, 19000, 192)])
 def test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K):
-    """Sizes that between them select every tile, ragged in rows, columns and stages."""
+    """Narrow, ordinary and wide layers, ragged in rows, columns and stages."""
     import torch
     w = pkg.synth.weights(N, K, 11)
     wh = gpu.weight(scheme, scale_mode, w["nib"], w["d"], w["m"] if scheme == 0 else None, w["zp"] if scheme == 2 else None)
@@ -149,7 +149,7 @@ def test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K):
 @pytest.mark.parametrize("scale_mode", [0, 1])
 @pytest.mark.parametrize("M,N,K", [(41, 3848, 192), (77, 4088, 1088), (80, 3912, 576), (42, 21976, 64), (2, 18952, 64), (9, 18960, 320), (32, 18952, 576)])
 def test_gemm_tiles_of_64_rows(pkg, gpu, scheme, scale_mode, M, N, K):
-    """64 x 40 and 64 x 48 tiles, and 64-row CTAs with up to 32 rows (A81W41 with two: 128-row ones) above 148 weight tiles."""
+    """Tiles of 64 weight rows, and 64-row CTAs with up to 32 rows (A81W41 with two: 128-row ones) above 148 weight tiles."""
     test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K)
 
 
@@ -158,8 +158,55 @@ def test_gemm_tiles_of_64_rows(pkg, gpu, scheme, scale_mode, M, N, K):
 @pytest.mark.parametrize("M,N,K", [(41, 6280, 576), (161, 12552, 192), (241, 15808, 64), (1572, 264, 448), (225, 18952, 64), (81, 3096, 576), (33, 9528, 320),
                                    (241, 7072, 192)])
 def test_gemm_tiles_that_one_scheme_or_record_size_takes(pkg, gpu, scheme, scale_mode, M, N, K):
-    """With the sizes above: every tile in every combination of weight scheme and scale records that the times of the tiles choose."""
+    """Sizes around the borders between tiles."""
     test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K)
+
+
+# (M, N) that with rows of each length K select every tile that layers of up to 24576 weight rows select with up to 2048 activation rows, in
+# every combination of weight scheme and scale records (checked on the CPU by test_gemm_tiles.py).  Ragged in weight and activation rows.
+TILE_SIZES = [(1569, 136), (1857, 136), (81, 3096), (125, 3096), (177, 3096), (197, 3096), (201, 3096), (321, 3096), (365, 3096), (389, 3096),
+              (401, 3096), (441, 3096), (617, 3096), (821, 3096), (65, 5480), (125, 5480), (149, 5480), (197, 5480), (293, 5480), (341, 5480),
+              (365, 5480), (41, 9736), (57, 9736), (321, 11640), (185, 12568), (365, 23960)]
+TILE_KS = [64, 320, 1088]
+
+
+def device_weight(gpu, scheme, scale_mode, N, K):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(N + K)
+    nib = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device="cuda", generator=g)
+    d = torch.rand((N, K // 32), device="cuda", generator=g) * 0.018 + 0.002
+    m = torch.rand((N, K // 32), device="cuda", generator=g) * -0.1
+    zp = torch.randint(0, 16, (N, K // 32), dtype=torch.uint8, device="cuda", generator=g)
+    w = gpu.weight_dev(scheme, scale_mode, N, K, nib, d, m if scheme == 0 else None, zp if scheme == 2 else None)
+    gpu.synchronize()
+    return w
+
+
+def assert_gemm_equals_simt(gpu, scheme, w, act, x, M, N):
+    import torch
+    C, ref = torch.full((M + 1, N), -5.0, device="cuda"), torch.empty((M, N), device="cuda")
+    gpu.quantize(act, x, M, 2 if scheme == 0 else 0)
+    gpu.gemm(act, w, C, N)
+    gpu.gemm_simt(act, w, ref, N)
+    gpu.synchronize()
+    assert torch.equal(C[:M], ref) and bool((C[M] == -5.0).all()), (M, N)
+
+
+@pytest.mark.parametrize("scheme", [0, 1, 2])
+@pytest.mark.parametrize("scale_mode", [0, 1])
+@pytest.mark.parametrize("K", TILE_KS)
+def test_gemm_every_tile(pkg, gpu, scheme, scale_mode, K):
+    """Every tile against the CUDA-core kernel."""
+    import torch
+    M_max = max(m for m, _ in TILE_SIZES)
+    x = torch.randn((M_max, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    act = gpu.act(M_max, K)
+    for N in sorted({n for _, n in TILE_SIZES}):
+        w = device_weight(gpu, scheme, scale_mode, N, K)
+        for M in [m for m, n in TILE_SIZES if n == N]:
+            assert_gemm_equals_simt(gpu, scheme, w, act, x, M, N)
+        w.close()
 
 
 @pytest.mark.parametrize("scheme", [1, 2])
