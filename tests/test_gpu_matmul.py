@@ -167,7 +167,19 @@ def test_gemm_tiles_that_one_scheme_or_record_size_takes(pkg, gpu, scheme, scale
 TILE_SIZES = [(1569, 136), (1857, 136), (81, 3096), (125, 3096), (177, 3096), (197, 3096), (201, 3096), (321, 3096), (365, 3096), (389, 3096),
               (401, 3096), (441, 3096), (617, 3096), (821, 3096), (65, 5480), (125, 5480), (149, 5480), (197, 5480), (293, 5480), (341, 5480),
               (365, 5480), (41, 9736), (57, 9736), (321, 11640), (185, 12568), (365, 23960)]
-TILE_KS = [64, 320, 1088]
+# The longest rows: 129 pairs are more than two rounds of any tile's ring (at most 8 stages of 8 pairs) and leave a ragged last stage, so that
+# every slot is refilled and every barrier passes both phases.
+TILE_KS = [64, 320, 1088, 64 * 129]
+
+
+def gemm_tile(gpu, scheme, scale_mode, N, K, M):
+    """(index, weight rows, activation rows) of the tile that this device takes"""
+    import ctypes
+    import torch
+    t = (ctypes.c_int * 3)()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    gpu.check(gpu.L.inkq_debug_gemm_tile(sms, scheme, scale_mode, N, K, M, t))
+    return tuple(t)
 
 
 def device_weight(gpu, scheme, scale_mode, N, K):
@@ -213,7 +225,16 @@ def test_gemm_every_tile(pkg, gpu, scheme, scale_mode, K):
 @pytest.mark.parametrize("scale_mode", [0, 1])
 @pytest.mark.parametrize("cols", range(40, 121, 8))
 def test_gemm_tiles_of_schemes_without_mins(pkg, gpu, scheme, scale_mode, cols):
-    """128 x 40 to 128 x 120 tiles, 8 warps of 16 rows by all columns: one on every SM, ragged in rows and stages, a column short and full."""
+    """128 x 40 to 128 x 120 tiles, 8 warps of 16 rows by all columns: one on every SM, ragged in rows and stages, a column short and full,
+    each slot of the ring filled more than twice."""
+    import torch
+    N, K = 18936, TILE_KS[-1]
+    x = torch.randn((cols, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(cols))
+    w, act = device_weight(gpu, scheme, scale_mode, N, K), gpu.act(cols, K)
+    for M in (cols - 1, cols):
+        assert gemm_tile(gpu, scheme, scale_mode, N, K, M)[1:] == (128, cols)
+        assert_gemm_equals_simt(gpu, scheme, w, act, x, M, N)
+    w.close()
     test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, cols - 1, 18936, 448)
     test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, cols, 18936, 64)
 
