@@ -156,7 +156,7 @@ def test_gemm_tiles_of_64_rows(pkg, gpu, scheme, scale_mode, M, N, K):
 @pytest.mark.parametrize("scheme", [0, 1, 2])
 @pytest.mark.parametrize("scale_mode", [0, 1])
 @pytest.mark.parametrize("M,N,K", [(41, 6280, 576), (161, 12552, 192), (241, 15808, 64), (1572, 264, 448), (225, 18952, 64), (81, 3096, 576), (33, 9528, 320),
-                                   (241, 7072, 192)])
+                                   (241, 7072, 192), (261, 4088, 320)])
 def test_gemm_tiles_that_one_scheme_or_record_size_takes(pkg, gpu, scheme, scale_mode, M, N, K):
     """Sizes around the borders between tiles."""
     test_gemm_tile_shapes(pkg, gpu, scheme, scale_mode, M, N, K)
@@ -240,9 +240,10 @@ def test_gemm_tiles_of_schemes_without_mins(pkg, gpu, scheme, scale_mode, cols):
 
 
 @pytest.mark.parametrize("scale_mode", [0, 1])
-@pytest.mark.parametrize("M,N,K", [(88, 18936, 448), (81, 18944, 64), (261, 4088, 320), (352, 4096, 576)])
+@pytest.mark.parametrize("M,N,K", [(88, 18936, 448), (81, 18944, 64), (345, 4088, 1088), (322, 4088, 4160), (352, 4096, 576)])
 def test_gemm_tile_with_a_short_column_of_warps(pkg, gpu, scale_mode, M, N, K):
-    """128 x 88 tiles of A81W41: their last columns belong to the next tile."""
+    """128 x 88 tiles of A81W41: their last columns belong to the next tile, which may be ragged."""
+    assert gemm_tile(gpu, 0, scale_mode, N, K, M)[1:] == (128, 88)
     test_gemm_tile_shapes(pkg, gpu, 0, scale_mode, M, N, K)
 
 
