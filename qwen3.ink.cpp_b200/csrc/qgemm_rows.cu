@@ -400,69 +400,67 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
 // of 4096 x 12288 129.5 -> 126.1): the last group of the longer ones stands in a block of its own, which costs half of what is left out, and
 // 72 and 104 columns gain nothing over 80 and 112.  With two bodies of code instead 88 columns take 58 us (instruction fetch).
 // 12288 x 4096 with 2048 rows, A80W40 541 -> 518 us (128 x 104); 4096 x 12288 with 322 rows 113 -> 101, A80W4Z 120 -> 106 (128 x 88).
-enum Who { ANY, MINS, PLAIN };   // schemes that a tile serves: all, A81W41, the ones without mins
-constexpr bool serves(Who who, int scheme) { return who == ANY || (who == MINS) == (scheme == INKQ_A81W41); }
-#define NEVER (1e30f, 1e30f, 1e30f)
-#define QROWS_TILES(X)                                                                                                          \
-    X(0, ANY, (2, 4, 1, 2, 8, 1), (2.2f, 3.6f, 3.2f), (12.2f, 24.1f, 23.7f), (11.6f, 22.7f, 22.3f), (13.5f, 26.6f, 26.3f),      \
-      (12.6f, 24.4f, 24.0f), (11.6f, 22.4f, 22.0f), (13.6f, 26.8f, 26.4f))                                                      \
-    X(1, ANY, (4, 2, 1, 2, 8, 1), (2.0f, 3.3f, 2.9f), (13.1f, 25.7f, 25.2f), (12.4f, 24.4f, 23.8f), (14.5f, 28.6f, 28.1f),      \
-      (13.2f, 26.1f, 25.5f), (12.2f, 24.0f, 23.5f), (14.6f, 28.8f, 28.2f))                                                      \
-    X(2, ANY, (4, 1, 2, 2, 4, 2), (2.1f, 2.1f, 1.0f), (13.3f, 19.8f, 18.4f), (12.7f, 18.7f, 17.4f), (14.4f, 21.5f, 20.3f),      \
-      (15.6f, 21.0f, 19.8f), (15.8f, 20.9f, 20.0f), (17.2f, 23.9f, 22.4f))                                                      \
-    X(3, ANY, (4, 2, 1, 3, 8, 1), (2.0f, 3.8f, 3.4f), (15.8f, 30.9f, 30.3f), (13.9f, 27.2f, 26.8f), (16.1f, 31.6f, 31.2f),      \
-      (15.9f, 31.4f, 30.9f), (13.8f, 27.0f, 26.4f), (15.8f, 31.1f, 30.6f))                                                      \
-    X(4, ANY, (4, 2, 1, 4, 6, 1), (2.6f, 4.9f, 4.5f), (19.4f, 38.5f, 38.0f), (17.9f, 35.5f, 35.0f), (20.1f, 39.9f, 39.3f),      \
-      (19.9f, 39.5f, 39.1f), (16.8f, 33.5f, 32.8f), (19.1f, 37.8f, 37.2f))                                                      \
-    X(5, ANY, (4, 2, 1, 5, 6, 1), (2.7f, 5.2f, 4.6f), (23.0f, 45.8f, 45.2f), (19.5f, 38.6f, 38.0f), (21.4f, 42.4f, 41.9f),      \
-      (26.1f, 51.5f, 51.6f), (19.5f, 38.7f, 38.1f), (21.1f, 41.9f, 41.4f))                                                      \
-    X(6, ANY, (4, 2, 1, 7, 4, 1), (2.7f, 5.1f, 4.9f), (29.6f, 59.0f, 58.3f), (25.5f, 50.4f, 49.9f), (27.8f, 54.9f, 54.4f),      \
-      (30.1f, 59.9f, 59.4f), (25.4f, 50.2f, 49.3f), (27.7f, 54.9f, 54.2f))                                                      \
-    X(7, ANY, (4, 2, 2, 2, 8, 1), (2.1f, 3.4f, 2.5f), (19.2f, 36.8f, 35.5f), (18.3f, 35.2f, 33.9f), (20.9f, 40.3f, 38.9f),      \
-      (18.3f, 34.8f, 33.4f), (18.4f, 35.2f, 33.7f), (21.0f, 40.2f, 38.6f))                                                      \
-    X(8, MINS, (4, 2, 2, 3, 6, 1), (2.7f, 4.4f, 3.6f), (24.8f, 48.4f, 47.4f), NEVER, NEVER,                                     \
-      (24.5f, 47.6f, 46.2f), NEVER, NEVER)                                                                                      \
-    X(9, MINS, (4, 2, 2, 4, 4, 1), (2.7f, 4.5f, 3.7f), (31.6f, 61.9f, 61.0f), NEVER, NEVER,                                     \
-      (30.7f, 59.8f, 58.8f), NEVER, NEVER)                                                                                      \
-    X(10, MINS, (4, 2, 2, 5, 4, 1), (3.0f, 5.0f, 4.2f), (36.6f, 72.3f, 71.3f), NEVER, NEVER,                                    \
-      (36.1f, 71.0f, 70.0f), NEVER, NEVER)                                                                                      \
-    X(11, MINS, (4, 2, 2, 6, 4, 1), (3.2f, 5.4f, 4.9f), (43.2f, 85.5f, 84.7f), NEVER, NEVER,                                    \
-      (41.6f, 82.0f, 81.0f), NEVER, NEVER)                                                                                      \
-    X(12, MINS, (4, 2, 2, 7, 4, 1), (3.3f, 5.5f, 5.3f), (48.4f, 95.7f, 94.9f), NEVER, NEVER,                                    \
-      (49.6f, 99.0f, 97.9f), NEVER, NEVER)                                                                                      \
-    X(13, ANY, (4, 2, 1, 4, 2, 2), (2.7f, 2.7f, 2.5f), (23.2f, 37.5f, 35.8f), (20.5f, 32.3f, 31.2f), (24.3f, 36.6f, 35.5f),     \
-      (22.5f, 37.2f, 36.0f), (20.7f, 32.5f, 31.4f), (23.6f, 35.7f, 34.7f))                                                      \
-    X(14, ANY, (4, 2, 1, 7, 2, 2), (2.4f, 2.9f, 2.3f), (31.8f, 56.7f, 54.6f), (28.2f, 48.4f, 46.2f), (30.8f, 50.7f, 48.8f),     \
-      (32.1f, 57.7f, 55.3f), (27.6f, 47.2f, 45.2f), (30.0f, 49.9f, 47.9f))                                                      \
-    X(15, ANY, (4, 2, 2, 4, 2, 2), (2.2f, 2.7f, 1.9f), (34.4f, 61.4f, 58.1f), (31.3f, 54.9f, 52.0f), (34.2f, 60.3f, 57.6f),     \
-      (34.4f, 60.3f, 56.8f), (31.2f, 54.7f, 51.7f), (33.6f, 59.6f, 56.4f))                                                      \
-    X(16, ANY, (4, 2, 2, 5, 2, 2), (2.3f, 3.1f, 1.9f), (42.4f, 76.0f, 72.2f), (36.3f, 64.5f, 61.4f), (39.0f, 69.7f, 66.2f),     \
-      (42.7f, 75.8f, 71.8f), (36.0f, 63.9f, 60.5f), (38.1f, 68.9f, 65.3f))                                                      \
-    X(17, ANY, (4, 1, 1, 5, 8, 1), (2.3f, 4.1f, 3.6f), (14.9f, 29.1f, 28.7f), (13.3f, 26.2f, 25.8f), (15.3f, 30.0f, 29.6f),     \
-      (14.8f, 28.9f, 28.3f), (12.6f, 24.7f, 24.2f), (14.4f, 28.2f, 27.8f))                                                      \
-    X(18, PLAIN, (8, 1, 1, 5, 6, 1), (2.7f, 4.2f, 3.5f), NEVER, (19.3f, 36.8f, 35.4f), (20.3f, 38.9f, 37.3f),                   \
-      NEVER, (19.4f, 36.8f, 35.4f), (20.4f, 38.7f, 37.4f))                                                                      \
-    X(19, PLAIN, (8, 1, 1, 6, 6, 1), (2.7f, 4.3f, 3.6f), NEVER, (21.6f, 41.7f, 40.1f), (22.7f, 43.6f, 42.2f),                   \
-      NEVER, (22.0f, 42.1f, 40.4f), (23.5f, 45.1f, 43.5f))                                                                      \
-    X(20, PLAIN, (8, 1, 1, 7, 6, 1), (2.8f, 4.6f, 3.9f), NEVER, (24.0f, 46.2f, 44.8f), (25.9f, 50.0f, 48.3f),                   \
-      NEVER, (24.3f, 46.7f, 45.2f), (25.4f, 49.1f, 47.4f))                                                                      \
-    X(21, PLAIN, (8, 1, 1, 8, 4, 1), (2.6f, 4.3f, 3.6f), NEVER, (27.4f, 53.0f, 51.7f), (28.2f, 54.6f, 53.4f),                   \
-      NEVER, (27.7f, 53.2f, 52.1f), (28.6f, 55.1f, 53.9f))                                                                      \
-    X(22, PLAIN, (8, 1, 1, 9, 4, 1), (2.8f, 4.6f, 4.0f), NEVER, (29.9f, 58.2f, 56.8f), (31.0f, 60.4f, 59.3f),                   \
-      NEVER, (29.7f, 57.6f, 56.4f), (30.9f, 60.5f, 59.1f))                                                                      \
-    X(23, PLAIN, (8, 1, 1, 10, 4, 1), (2.9f, 4.8f, 4.2f), NEVER, (32.6f, 63.8f, 62.4f), (33.3f, 65.3f, 64.1f),                  \
-      NEVER, (31.7f, 61.9f, 60.6f), (32.8f, 64.6f, 63.2f))                                                                      \
-    X(24, PLAIN, (8, 1, 1, 11, 4, 1), (3.1f, 5.1f, 4.5f), NEVER, (34.3f, 67.2f, 66.1f), (35.7f, 70.5f, 69.1f),                  \
-      NEVER, (34.5f, 67.8f, 66.4f), (35.7f, 70.2f, 68.8f))                                                                      \
-    X(25, PLAIN, (8, 1, 1, 12, 4, 1), (3.2f, 5.4f, 4.9f), NEVER, (37.1f, 72.8f, 72.0f), (37.7f, 74.4f, 73.0f),                  \
-      NEVER, (37.1f, 73.1f, 71.7f), (38.0f, 74.9f, 73.6f))                                                                      \
-    X(26, PLAIN, (8, 1, 1, 13, 4, 1), (3.3f, 5.6f, 5.2f), NEVER, (39.4f, 77.7f, 76.2f), (40.6f, 79.7f, 78.3f),                  \
-      NEVER, (39.9f, 78.5f, 77.0f), (40.5f, 80.0f, 78.7f))                                                                      \
-    X(27, PLAIN, (8, 1, 1, 14, 4, 1), (3.3f, 5.7f, 5.5f), NEVER, (41.7f, 82.5f, 81.0f), (43.6f, 85.9f, 84.5f),                  \
-      NEVER, (43.5f, 85.8f, 84.2f), (44.1f, 87.3f, 86.0f))                                                                      \
-    X(28, PLAIN, (8, 1, 1, 15, 4, 1), (3.4f, 5.8f, 5.8f), NEVER, (44.7f, 88.4f, 86.9f), (45.6f, 90.4f, 88.9f),                  \
-      NEVER, (45.5f, 89.6f, 87.9f), (46.6f, 92.7f, 91.3f))                                                                      \
-    X(29, MINS, (4, 2, 2, 6, 4, 1, true), (2.7f, 4.3f, 3.7f), (41.5f, 81.7f, 80.2f), NEVER, NEVER,                              \
+#define NEVER (0.f, 0.f, 0.f)   // a tile that a scheme does not have
+#define QROWS_TILES(X)                                                                                                    \
+    X(0, (2, 4, 1, 2, 8, 1), (2.2f, 3.6f, 3.2f), (12.2f, 24.1f, 23.7f), (11.6f, 22.7f, 22.3f), (13.5f, 26.6f, 26.3f),     \
+      (12.6f, 24.4f, 24.0f), (11.6f, 22.4f, 22.0f), (13.6f, 26.8f, 26.4f))                                                \
+    X(1, (4, 2, 1, 2, 8, 1), (2.0f, 3.3f, 2.9f), (13.1f, 25.7f, 25.2f), (12.4f, 24.4f, 23.8f), (14.5f, 28.6f, 28.1f),     \
+      (13.2f, 26.1f, 25.5f), (12.2f, 24.0f, 23.5f), (14.6f, 28.8f, 28.2f))                                                \
+    X(2, (4, 1, 2, 2, 4, 2), (2.1f, 2.1f, 1.0f), (13.3f, 19.8f, 18.4f), (12.7f, 18.7f, 17.4f), (14.4f, 21.5f, 20.3f),     \
+      (15.6f, 21.0f, 19.8f), (15.8f, 20.9f, 20.0f), (17.2f, 23.9f, 22.4f))                                                \
+    X(3, (4, 2, 1, 3, 8, 1), (2.0f, 3.8f, 3.4f), (15.8f, 30.9f, 30.3f), (13.9f, 27.2f, 26.8f), (16.1f, 31.6f, 31.2f),     \
+      (15.9f, 31.4f, 30.9f), (13.8f, 27.0f, 26.4f), (15.8f, 31.1f, 30.6f))                                                \
+    X(4, (4, 2, 1, 4, 6, 1), (2.6f, 4.9f, 4.5f), (19.4f, 38.5f, 38.0f), (17.9f, 35.5f, 35.0f), (20.1f, 39.9f, 39.3f),     \
+      (19.9f, 39.5f, 39.1f), (16.8f, 33.5f, 32.8f), (19.1f, 37.8f, 37.2f))                                                \
+    X(5, (4, 2, 1, 5, 6, 1), (2.7f, 5.2f, 4.6f), (23.0f, 45.8f, 45.2f), (19.5f, 38.6f, 38.0f), (21.4f, 42.4f, 41.9f),     \
+      (26.1f, 51.5f, 51.6f), (19.5f, 38.7f, 38.1f), (21.1f, 41.9f, 41.4f))                                                \
+    X(6, (4, 2, 1, 7, 4, 1), (2.7f, 5.1f, 4.9f), (29.6f, 59.0f, 58.3f), (25.5f, 50.4f, 49.9f), (27.8f, 54.9f, 54.4f),     \
+      (30.1f, 59.9f, 59.4f), (25.4f, 50.2f, 49.3f), (27.7f, 54.9f, 54.2f))                                                \
+    X(7, (4, 2, 2, 2, 8, 1), (2.1f, 3.4f, 2.5f), (19.2f, 36.8f, 35.5f), (18.3f, 35.2f, 33.9f), (20.9f, 40.3f, 38.9f),     \
+      (18.3f, 34.8f, 33.4f), (18.4f, 35.2f, 33.7f), (21.0f, 40.2f, 38.6f))                                                \
+    X(8, (4, 2, 2, 3, 6, 1), (2.7f, 4.4f, 3.6f), (24.8f, 48.4f, 47.4f), NEVER, NEVER,                                     \
+      (24.5f, 47.6f, 46.2f), NEVER, NEVER)                                                                                \
+    X(9, (4, 2, 2, 4, 4, 1), (2.7f, 4.5f, 3.7f), (31.6f, 61.9f, 61.0f), NEVER, NEVER,                                     \
+      (30.7f, 59.8f, 58.8f), NEVER, NEVER)                                                                                \
+    X(10, (4, 2, 2, 5, 4, 1), (3.0f, 5.0f, 4.2f), (36.6f, 72.3f, 71.3f), NEVER, NEVER,                                    \
+      (36.1f, 71.0f, 70.0f), NEVER, NEVER)                                                                                \
+    X(11, (4, 2, 2, 6, 4, 1), (3.2f, 5.4f, 4.9f), (43.2f, 85.5f, 84.7f), NEVER, NEVER,                                    \
+      (41.6f, 82.0f, 81.0f), NEVER, NEVER)                                                                                \
+    X(12, (4, 2, 2, 7, 4, 1), (3.3f, 5.5f, 5.3f), (48.4f, 95.7f, 94.9f), NEVER, NEVER,                                    \
+      (49.6f, 99.0f, 97.9f), NEVER, NEVER)                                                                                \
+    X(13, (4, 2, 1, 4, 2, 2), (2.7f, 2.7f, 2.5f), (23.2f, 37.5f, 35.8f), (20.5f, 32.3f, 31.2f), (24.3f, 36.6f, 35.5f),    \
+      (22.5f, 37.2f, 36.0f), (20.7f, 32.5f, 31.4f), (23.6f, 35.7f, 34.7f))                                                \
+    X(14, (4, 2, 1, 7, 2, 2), (2.4f, 2.9f, 2.3f), (31.8f, 56.7f, 54.6f), (28.2f, 48.4f, 46.2f), (30.8f, 50.7f, 48.8f),    \
+      (32.1f, 57.7f, 55.3f), (27.6f, 47.2f, 45.2f), (30.0f, 49.9f, 47.9f))                                                \
+    X(15, (4, 2, 2, 4, 2, 2), (2.2f, 2.7f, 1.9f), (34.4f, 61.4f, 58.1f), (31.3f, 54.9f, 52.0f), (34.2f, 60.3f, 57.6f),    \
+      (34.4f, 60.3f, 56.8f), (31.2f, 54.7f, 51.7f), (33.6f, 59.6f, 56.4f))                                                \
+    X(16, (4, 2, 2, 5, 2, 2), (2.3f, 3.1f, 1.9f), (42.4f, 76.0f, 72.2f), (36.3f, 64.5f, 61.4f), (39.0f, 69.7f, 66.2f),    \
+      (42.7f, 75.8f, 71.8f), (36.0f, 63.9f, 60.5f), (38.1f, 68.9f, 65.3f))                                                \
+    X(17, (4, 1, 1, 5, 8, 1), (2.3f, 4.1f, 3.6f), (14.9f, 29.1f, 28.7f), (13.3f, 26.2f, 25.8f), (15.3f, 30.0f, 29.6f),    \
+      (14.8f, 28.9f, 28.3f), (12.6f, 24.7f, 24.2f), (14.4f, 28.2f, 27.8f))                                                \
+    X(18, (8, 1, 1, 5, 6, 1), (2.7f, 4.2f, 3.5f), NEVER, (19.3f, 36.8f, 35.4f), (20.3f, 38.9f, 37.3f),                    \
+      NEVER, (19.4f, 36.8f, 35.4f), (20.4f, 38.7f, 37.4f))                                                                \
+    X(19, (8, 1, 1, 6, 6, 1), (2.7f, 4.3f, 3.6f), NEVER, (21.6f, 41.7f, 40.1f), (22.7f, 43.6f, 42.2f),                    \
+      NEVER, (22.0f, 42.1f, 40.4f), (23.5f, 45.1f, 43.5f))                                                                \
+    X(20, (8, 1, 1, 7, 6, 1), (2.8f, 4.6f, 3.9f), NEVER, (24.0f, 46.2f, 44.8f), (25.9f, 50.0f, 48.3f),                    \
+      NEVER, (24.3f, 46.7f, 45.2f), (25.4f, 49.1f, 47.4f))                                                                \
+    X(21, (8, 1, 1, 8, 4, 1), (2.6f, 4.3f, 3.6f), NEVER, (27.4f, 53.0f, 51.7f), (28.2f, 54.6f, 53.4f),                    \
+      NEVER, (27.7f, 53.2f, 52.1f), (28.6f, 55.1f, 53.9f))                                                                \
+    X(22, (8, 1, 1, 9, 4, 1), (2.8f, 4.6f, 4.0f), NEVER, (29.9f, 58.2f, 56.8f), (31.0f, 60.4f, 59.3f),                    \
+      NEVER, (29.7f, 57.6f, 56.4f), (30.9f, 60.5f, 59.1f))                                                                \
+    X(23, (8, 1, 1, 10, 4, 1), (2.9f, 4.8f, 4.2f), NEVER, (32.6f, 63.8f, 62.4f), (33.3f, 65.3f, 64.1f),                   \
+      NEVER, (31.7f, 61.9f, 60.6f), (32.8f, 64.6f, 63.2f))                                                                \
+    X(24, (8, 1, 1, 11, 4, 1), (3.1f, 5.1f, 4.5f), NEVER, (34.3f, 67.2f, 66.1f), (35.7f, 70.5f, 69.1f),                   \
+      NEVER, (34.5f, 67.8f, 66.4f), (35.7f, 70.2f, 68.8f))                                                                \
+    X(25, (8, 1, 1, 12, 4, 1), (3.2f, 5.4f, 4.9f), NEVER, (37.1f, 72.8f, 72.0f), (37.7f, 74.4f, 73.0f),                   \
+      NEVER, (37.1f, 73.1f, 71.7f), (38.0f, 74.9f, 73.6f))                                                                \
+    X(26, (8, 1, 1, 13, 4, 1), (3.3f, 5.6f, 5.2f), NEVER, (39.4f, 77.7f, 76.2f), (40.6f, 79.7f, 78.3f),                   \
+      NEVER, (39.9f, 78.5f, 77.0f), (40.5f, 80.0f, 78.7f))                                                                \
+    X(27, (8, 1, 1, 14, 4, 1), (3.3f, 5.7f, 5.5f), NEVER, (41.7f, 82.5f, 81.0f), (43.6f, 85.9f, 84.5f),                   \
+      NEVER, (43.5f, 85.8f, 84.2f), (44.1f, 87.3f, 86.0f))                                                                \
+    X(28, (8, 1, 1, 15, 4, 1), (3.4f, 5.8f, 5.8f), NEVER, (44.7f, 88.4f, 86.9f), (45.6f, 90.4f, 88.9f),                   \
+      NEVER, (45.5f, 89.6f, 87.9f), (46.6f, 92.7f, 91.3f))                                                                \
+    X(29, (4, 2, 2, 6, 4, 1, true), (2.7f, 4.3f, 3.7f), (41.5f, 81.7f, 80.2f), NEVER, NEVER,                              \
       (40.7f, 79.9f, 78.5f), NEVER, NEVER)
 
 #define QROWS_UNWRAP(...) __VA_ARGS__
@@ -473,20 +471,24 @@ struct TileCost {
 };
 static_assert(INKQ_A81W41 == 0 && INKQ_A80W40 == 1 && INKQ_A80W4Z == 2, "the schemes index the table");
 static constexpr TileCost tile_costs[] = {
-#define QROWS_COST(i, who, shape, fixed, h41, h40, h4z, f41, f40, f4z)                      \
+#define QROWS_COST(i, shape, fixed, h41, h40, h4z, f41, f40, f4z)                           \
     {Tile<QROWS_UNWRAP shape>::ROWS, Tile<QROWS_UNWRAP shape>::COLS, {QROWS_UNWRAP fixed}, \
      {{{QROWS_UNWRAP h41}, {QROWS_UNWRAP h40}, {QROWS_UNWRAP h4z}}, {{QROWS_UNWRAP f41}, {QROWS_UNWRAP f40}, {QROWS_UNWRAP f4z}}}},
     QROWS_TILES(QROWS_COST)
 };
+constexpr int TILES = static_cast<int>(sizeof(tile_costs) / sizeof(tile_costs[0]));
+// What is compiled and what is chosen from: the tiles with times
+static constexpr bool has_tile(int i, bool s16, int scheme) { return tile_costs[i].time[s16 ? 0 : 1][scheme][0] > 0.f; }
 
 // The tile with the least time for M activation rows: a CTA takes one tile, so the busiest SM works through
 // n = ceil(tiles / SMs) of them.
 static int pick_tile(int num_sms, int scheme, bool s16, int rows, int pairs, int M)
 {
     const float length = static_cast<float>(pairs) / 64.0f;   // of a row, in units of the K = 4096 of the table
-    int best = 0;
+    int best = -1;
     float best_time = 0.f;
-    for (int i = 0; i < static_cast<int>(sizeof(tile_costs) / sizeof(tile_costs[0])); i++) {
+    for (int i = 0; i < TILES; i++) {
+        if (!has_tile(i, s16, scheme)) continue;
         const TileCost &c = tile_costs[i];
         const float *t = c.time[s16 ? 0 : 1][scheme];
         const long long total = static_cast<long long>((rows + c.rows - 1) / c.rows) * ((M + c.cols - 1) / c.cols);
@@ -494,7 +496,7 @@ static int pick_tile(int num_sms, int scheme, bool s16, int rows, int pairs, int
         const float whole = t[(n - 1) % 2] + static_cast<float>((n - 1) / 2) * t[2];
         const float fixed = c.fixed[(n - 1) % 2] + static_cast<float>((n - 1) / 2) * c.fixed[2];
         const float time = fixed + (whole - fixed) * length;
-        if (i == 0 || time < best_time) {
+        if (best < 0 || time < best_time) {
             best = i;
             best_time = time;
         }
@@ -508,9 +510,9 @@ static int launch_sized(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begi
     if (prm.M > 32) {
         const int tile = pick_tile(ctx->num_sms, SCH, S16, prm.rows, prm.pairs, prm.M);
         switch (tile) {
-#define QROWS_CASE(i, who, shape, fixed, h41, h40, h4z, f41, f40, f4z) \
-    case i:                                                     \
-        if constexpr (serves(who, SCH)) return launch_one<SCH, S16, Tile<QROWS_UNWRAP shape>>(ctx, a, w, m_begin, prm); \
+#define QROWS_CASE(i, shape, fixed, h41, h40, h4z, f41, f40, f4z)                                                             \
+    case i:                                                                                                                   \
+        if constexpr (has_tile(i, S16, SCH)) return launch_one<SCH, S16, Tile<QROWS_UNWRAP shape>>(ctx, a, w, m_begin, prm);  \
         break;
             QROWS_TILES(QROWS_CASE)
         }
