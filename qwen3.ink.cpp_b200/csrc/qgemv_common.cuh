@@ -158,9 +158,10 @@ struct QuantOut {     // one quantized activation row (M == 1) in the device lay
 __device__ __forceinline__ void quantize_block_lanes(float v, int blk, int lane, const QuantOut &o)
 {
     // One instruction for the largest magnitude and one for the sum, in place of five shuffles and operations each: every CTA of a decode
-    // step ends in this (a step of 36 layers 1414 -> 1400 us).  NaNs are left out of the maximum as by fmaxf.
+    // step ends in this (a step of 36 layers 1414 -> 1400 us).  NaNs are left out of the maximum as by fmaxf.  volatile: every lane takes
+    // part, so the instruction may not be moved under a condition on a lane.
     float mx;
-    asm("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(mx) : "f"(v));
+    asm volatile("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(mx) : "f"(v));
     const float dd = __fdiv_rn(mx, 127.0f);
     const float id = (mx != 0.0f) ? __fdiv_rn(127.0f, mx) : 0.0f;
     const int qi = __float2int_rn(__fmul_rn(v, id));
