@@ -25,7 +25,7 @@ constexpr int TILE_N = 128;  // weight rows per device tile (one UMMA M=128 oper
 //                                  of block 2p+1); its two 16-byte chunks are stored at chunk
 //                                  position c ^ ((r >> 2) & 1) so that 8 consecutive rows read
 //                                  the same logical chunk from 8 distinct bank groups.
-//   sc32  float4 [T][P][128]       {d_lo, d_hi, m_lo, m_hi}, only when scales are kept in fp32
+//   sc32  float4 [T][P][128]       {d_lo, d_hi, m_lo, m_hi}: as given or, with fp16 scales, rounded and widened again; none for W41
 //   sc16  half x4[T][P][128]       the same rounded to fp16 (always present)
 //   zpT   u8 x2  [T][P][128]       {z_lo, z_hi}: 0 (Q4_1), 8 (Q4_0) or the block zero point
 // Rows beyond R inside the last tile hold zero nibbles, zero scales, zero z.

@@ -63,8 +63,8 @@ __global__ void __launch_bounds__(256) k_retile_scales(const float *__restrict__
     const __half2 h0 = __floats2half2_rn(sc.x, sc.y);
     const __half2 h1 = __floats2half2_rn(sc.z, sc.w);
     if (sc32 != nullptr) {
-        // the prefill kernel reads fp32 records either way (widening fp16 in its inner loop costs more than the
-        // extra bytes): the values as given, or the fp16-rounded ones widened again
+        // the values as given, or the fp16-rounded ones widened again for the cross-check and the block-dot dump (the QGEMM of a
+        // layer with fp16 scales reads the fp16 records)
         if (round16) {
             const float2 a = __half22float2(h0), b = __half22float2(h1);
             sc = make_float4(a.x, a.y, b.x, b.y);

@@ -22,8 +22,8 @@
 // chain (fragment loads, product, conversion, scaling) is long and an SM has few warps in a tile of this size, so stages of 4 to 8
 // pairs are unrolled and one CTA of 8 warps gets up to 255 registers a thread.  The weights are read from L2 once per tile of
 // columns (CTAs of one weight tile are neighbours).
-// Measured (weights of distinct layers), A81W41: 24576 x 4096 with 5 rows 14.1 us (5.0 TB/s), 4096 x 4096 with 5 rows 7.0, 12288 x 4096
-// with 24 rows 16, with 322 rows 99 (fp32 records), 24576 x 4096 with 322 rows 190; A80W40 12288 x 4096 with 2048 rows 525; A80W4Z 4096 x
+// Measured (weights of distinct layers), A81W41: 24576 x 4096 with 5 rows 14 us (4.6 TB/s), 4096 x 4096 with 5 rows 6.6, 12288 x 4096
+// with 24 rows 15.5, with 322 rows 99 (fp32 records), 24576 x 4096 with 322 rows 191; A80W40 12288 x 4096 with 2048 rows 502; A80W4Z 4096 x
 // 12288 with 77 rows 36.  Slower: scalar multiplications (+12 %), the conversion by a bias in the product's accumulator operand (+20 %: it
 // has to be moved there), fp16 operands with fp32 accumulators (+25 %), e4m3 parts (x2), the results staged in shared memory for whole-line
 // stores (+1 to 2 %), a stage's pairs unrolled by two (+1 to 8 %), a resident CTA that requests its next tile's stages during the stores
@@ -397,9 +397,9 @@ static int launch_one(inkq_ctx *ctx, const Act *a, const Weight *w, int m_begin,
 // 40.1, 37.7; 112: 42.2, 41.7 and 44.3, 43.6; and sizes between the multiples of 16 that two columns of warps have.  With mins it is the other
 // way round: 48 columns 24.8, 26.5, 64: 31.6, 33.8; 322 rows of 4096 x 4096 47.1 with 96 columns by 4 x 2 warps, 48.2 with 88 by 8.
 // With mins 88 columns are 48 for one column of warps and 40 for the other (41.5 us a tile, 96 columns 43.2; 322 rows of 4096 x 4096 47.1 -> 45.8,
-// of 4096 x 12288 129.5 -> 126.1): the last group of the longer ones stands in a block of its own, which costs half of what is left out, and
-// 72 and 104 columns gain nothing over 80 and 112.  With two bodies of code instead 88 columns take 58 us (instruction fetch).
-// 12288 x 4096 with 2048 rows, A80W40 541 -> 518 us (128 x 104); 4096 x 12288 with 322 rows 113 -> 101, A80W4Z 120 -> 106 (128 x 88).
+// of 4096 x 12288 129.5 -> 126.1): the last group of the longer ones stands in a block of its own, which costs half of what is left out.  72
+// columns take 36.3 us a tile (fp16 records; fp32 35.3) where 80 take 36.8 (36.3), 104 take 49.0 (49.6) and 112 48.7 (49.9).  With two bodies of code instead 88 columns take 58 us (instruction fetch).
+// Layers with their quantizer: 12288 x 4096 with 2048 rows, A80W40 541 -> 518 us (128 x 104); 4096 x 12288 with 322 rows 113 -> 101, A80W4Z 120 -> 106 (128 x 88).
 #define NEVER (0.f, 0.f, 0.f)   // a tile that a scheme does not have
 #define QROWS_TILES(X)                                                                                                    \
     X(0, (2, 4, 1, 2, 8, 1), (2.2f, 3.6f, 3.2f), (12.2f, 24.1f, 23.7f), (11.6f, 22.7f, 22.3f), (13.5f, 26.6f, 26.3f),     \

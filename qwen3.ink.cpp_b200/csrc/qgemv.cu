@@ -19,9 +19,12 @@
 // narrow or long-row layers: the choice depends only on the layer's shape).  Every int32
 // block dot is exact.
 //
-// Algorithmic bytes per launch: rows*K/2 nibbles + rows*(K/32)*4 scale bytes
+// Bytes streamed per launch: rows*K/2 nibbles + rows*(K/32)*4 scale bytes
 // (+ rows*(K/32) zero-point bytes for the A80 schemes) + K + (K/32)*8 activation
-// bytes + rows*4 output bytes, i.e. 0.625 B per weight for A81W41.
+// bytes + rows*4 output bytes, i.e. 0.625 B per weight for A81W41, which needs all of
+// them.  The schemes without mins do not: half of their 8-byte records is zero, and
+// A80W40's zero points are all 8.  Of 42 bytes per row and pair A80W40 needs 36 and
+// A80W4Z 38 (4096 x 12288: 33.0 MB where 28.3 and 29.9 would do).
 #include <cuda_fp16.h>
 
 #include "glue_math.cuh"
